@@ -385,6 +385,9 @@ static size_t workspace_bytes(uint32_t M, uint32_t n_out) {
     return (size_t)kTicketBytes * 4 + (split > streamk ? split : streamk);
 }
 
+// Behind those, where the caller's workspace has room: up to 16 rows of activations reordered (linear_mma4.cu).
+static size_t x_scratch_bytes(uint32_t K) { return K ? (size_t)K * 16 * sizeof(uint16_t) + 256 : 0; }
+
 template <int MT>
 static int launch_linear(LinArgs a, cudaStream_t s) {
     size_t smem = kProbScale * 4 + (size_t)kLinWarps * kLinStage;
@@ -450,7 +453,7 @@ using namespace ci;
 extern "C" {
 
 size_t ci_linear_workspace_bytes(uint32_t M, uint32_t n_out, uint32_t K, uint32_t tile_h) {
-    size_t small = workspace_bytes(M, n_out);
+    size_t small = workspace_bytes(M, n_out) + x_scratch_bytes(K);
     size_t big = (size_t)kTicketBytes * 4 + gemm_workspace_bytes(M, n_out, K, tile_h);    // prefill path, split-K partials
     return small > big ? small : big;
 }
@@ -475,6 +478,9 @@ static int linear_impl(const ci_tiled_weight *w, const uint16_t *d_x, int64_t ld
     a.tickets = reinterpret_cast<uint32_t *>(d_ws);
     a.partial = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(d_ws) + kTicketBytes * 4);
     a.bias = d_bias; a.ldx = ldx; a.ldy = ldy;
+    if (have_ws && ws_bytes >= workspace_bytes(M, w->N) + x_scratch_bytes(w->K))
+        a.x_scratch = reinterpret_cast<uint16_t *>(reinterpret_cast<uint8_t *>(d_ws) +
+                                                   ((workspace_bytes(M, w->N) + 255) & ~(size_t)255));
     cudaStream_t s = (cudaStream_t)stream;
     if (ar != nullptr) {
         // output all-reduced inside the kernel: only the staged GEMV kernels do that, for one or two rows
@@ -504,8 +510,9 @@ static int linear_impl(const ci_tiled_weight *w, const uint16_t *d_x, int64_t ld
         a.y = d_y + (size_t)m0 * ldy;
         a.M = mc;
         // staged tensor-core kernel when the weight qualifies (tile width <= 32, known maximum tile
-        // depth, aligned buffers, a workspace); split_k != 0 asks for the generic split-K kernel
-        if (split_k == 0 && have_ws) {
+        // depth, aligned buffers, a workspace): it splits K by itself, so split_k -- a hint about how to run,
+        // not about the result -- only shapes the generic kernel that takes the rest
+        if (have_ws) {
             rc = launch_linear_mma4(a, w->max_tile_len, s);     // 32-wide tiles, whole tile rows
             if (rc == CI_OK) continue;
             if (rc < 0) return rc;

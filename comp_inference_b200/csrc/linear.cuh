@@ -18,6 +18,7 @@ struct LinArgs {
     uint32_t stream_aligned;
     const uint16_t *x;
     int64_t ldx;
+    uint16_t *x_scratch; // room for 16 rows of activations in another order, or null
     const uint16_t *bias;
     uint16_t *y;
     int64_t ldy;

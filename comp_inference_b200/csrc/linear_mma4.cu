@@ -22,32 +22,40 @@
 //    window of 128-byte rows (upper tile in bytes 0..63, lower tile in 64..127).  The four streams of a
 //    lane are the four bytes of one word column, so every lane reads its own bank whatever row each of
 //    its cursors is on;
-//  * sign+mantissa bytes never enter shared memory: one 32-bit global load per row covers the lane's
-//    four columns (a warp reads four full 32-byte sectors), issued one 4-row group ahead of its use;
-//    the unit's two 4 KB blocks are pulled into L2 when the unit's copies are queued;
+//  * sign+mantissa bytes: chunks of 16 rows of the four segments, double buffered per warp by cp.async, the segments
+//    8 banks apart so that a row of the warp's 128 columns is one conflict-free wavefront (read straight from
+//    global memory a row took four, one per 32-byte sector: a quarter of the pipe's load);
 //  * initial states arrive by bulk copy with the rest of the unit (no global load at a unit's start).
-// Units are double buffered per warp; byte ranges of the next units are loaded one unit ahead by all
-// lanes in parallel.
+// The byte windows are double buffered per warp where they fit (tall tiles: one window); byte ranges of the next units
+// are loaded one unit ahead by all lanes in parallel.
 //
 // Scheduling: warp-level stream-K as in linear_mma.cu (units ordered by column group then tile-row
 // pair, equal contiguous runs per warp, fp32 partials + ticket, fixed summation order).
+//
+// Measured (graph replays over more than L2 of weights), before -> after the chunks, the in-place renormalisation, the
+// wider choice of warp counts and the reordered activations: 4096 x 22016 at tile height 128, 1 row 90.4 -> 82.3 us,
+// 16 rows 126.7 -> 89.6; 4096 x 4096 at 1024 (was the generic kernel) 551 -> 68.
 #include "linear.cuh"
 #include "ptx.cuh"
 
 namespace ci {
 
-constexpr uint32_t kBar4Bytes = 256;         // up to 16 warps x 2 stages x 8 B
-constexpr uint32_t kMma4Warps = 14;          // 448 threads x 128 registers; an instantiation for 12 warps with 158
-                                             // registers executes 7 % fewer instructions but was slower (fewer warps)
+constexpr uint32_t kBar4Bytes = 512;         // up to 16 warps x (2 window stages + 2 mantissa chunks) x 8 B
+constexpr uint32_t kChunkRows = 16;          // rows of sign+mantissa bytes per chunk and segment
+constexpr uint32_t kSegPitch = kChunkRows * 32 + 32;   // the four segments of a chunk start 8 banks apart
+constexpr uint32_t kManBytes = 2 * 4 * kSegPitch;      // two chunks per warp
+constexpr uint32_t kMma4Warps = 16;          // x 32 threads x 128 registers = the register file
 
 struct Mma4Args {
     LinArgs a;
     uint32_t cap_rows;     // rows of a byte window (>= every tile_max_len)
     uint32_t stage_bytes;  // window + 128 initial states
-    uint32_t per_warp;     // units per warp
+    uint32_t slots;        // warps of the grid: warp i takes units [i * total / slots, (i + 1) * total / slots)
     uint32_t total;        // units in the matrix
     uint32_t pairs_k;      // tile-row pairs = ceil(tiles_k / 2)
+    uint32_t stages;       // byte windows per warp: 2, or 1 where tall tiles leave no room for two
     uint32_t y_vec;        // outputs can be written as 16-byte rows of eight
+    uint32_t x_step;       // elements from one row's activations k .. k+3 to k+4 .. k+7
     uint32_t *status;      // set non-zero if a wait ran out
 };
 
@@ -67,34 +75,9 @@ __device__ __forceinline__ uint32_t weight_pair4(uint32_t e_lo, uint32_t e_hi, u
     // place in a bf16 pair; whatever else the shift drags along is masked out by the bit-select.
     const uint32_t ee = __byte_perm(e_lo, e_hi, 0x6521) << 3;
     const uint32_t vv = __byte_perm(m_lo, m_hi, 0x4400 + 0x1111 * C);
-    return (ee & 0x7F807F80u) | (vv & 0x807F807Fu);
-}
-
-__device__ __forceinline__ void prefetch_l2(const void *src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ uint32_t ldg_stream_u32(const void *src) {
-    uint32_t v;
-    asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(src));
-    return v;
-}
-
-// Renormalisation of a lane's four streams.  The first byte (about one symbol in three needs it) is merged
-// under a predicate; a second byte is needed only after a symbol of frequency below 16, so the whole
-// warp tests for it with one vote and skips those instructions otherwise.
-__device__ __forceinline__ void renorm4(uint32_t &s0, uint32_t &s1, uint32_t &s2, uint32_t &s3, uint32_t &p0, uint32_t &p1,
-                                        uint32_t &p2, uint32_t &p3, uint32_t y0, uint32_t y1, uint32_t y2, uint32_t y3) {
-    const uint32_t lowest = min(min(s0, s1), min(s2, s3));
-    renorm_first<128>(s0, p0, y0);
-    renorm_first<128>(s1, p1, y1);
-    renorm_first<128>(s2, p2, y2);
-    renorm_first<128>(s3, p3, y3);
-    if (__any_sync(kFull, lowest < 256u)) {
-        renorm_fast<128>(s0, p0);
-        renorm_fast<128>(s1, p1);
-        renorm_fast<128>(s2, p2);
-        renorm_fast<128>(s3, p3);
-    }
+    uint32_t w;                                                 // bit-select in one instruction
+    asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(w) : "r"(ee), "r"(vv), "n"(0x7F807F80));
+    return w;
 }
 
 // Four symbols of each of the lane's streams -> four packed weight pairs per column -> tensor core.
@@ -105,32 +88,7 @@ __device__ __forceinline__ void renorm4(uint32_t &s0, uint32_t &s1, uint32_t &s2
 // operand (one mma per column) this halves the mma count and the accumulators for up to 8 rows and needs
 // no interleaving of the activation registers.
 template <bool HI>
-__device__ __forceinline__ void group4(float (&acc)[4][4], uint32_t &s0, uint32_t &s1, uint32_t &s2, uint32_t &s3,
-                                       uint32_t &p0, uint32_t &p1, uint32_t &p2, uint32_t &p3, uint32_t lut_s,
-                                       const uint32_t (&m)[4], const uint32_t (&xf)[4]) {
-    uint32_t b[4][2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {                               // two rows -> one packed pair per column
-        uint32_t y0 = lds_u8(p0), y1 = lds_u8(p1), y2 = lds_u8(p2), y3 = lds_u8(p3);
-        const uint32_t e0 = decode_aligned(s0, lut_s);
-        const uint32_t e1 = decode_aligned(s1, lut_s);
-        const uint32_t e2 = decode_aligned(s2, lut_s);
-        const uint32_t e3 = decode_aligned(s3, lut_s);
-        renorm4(s0, s1, s2, s3, p0, p1, p2, p3, y0, y1, y2, y3);
-        y0 = lds_u8(p0);
-        y1 = lds_u8(p1);
-        y2 = lds_u8(p2);
-        y3 = lds_u8(p3);
-        const uint32_t f0 = decode_aligned(s0, lut_s);
-        const uint32_t f1 = decode_aligned(s1, lut_s);
-        const uint32_t f2 = decode_aligned(s2, lut_s);
-        const uint32_t f3 = decode_aligned(s3, lut_s);
-        renorm4(s0, s1, s2, s3, p0, p1, p2, p3, y0, y1, y2, y3);
-        b[0][h] = weight_pair4<0>(e0, f0, m[2 * h], m[2 * h + 1]);
-        b[1][h] = weight_pair4<1>(e1, f1, m[2 * h], m[2 * h + 1]);
-        b[2][h] = weight_pair4<2>(e2, f2, m[2 * h], m[2 * h + 1]);
-        b[3][h] = weight_pair4<3>(e3, f3, m[2 * h], m[2 * h + 1]);
-    }
+__device__ __forceinline__ void mma4(float (&acc)[4][4], const uint32_t (&b)[4][2], const uint32_t (&xf)[4]) {
     const uint32_t w01[4] = {b[0][0], b[1][0], b[0][1], b[1][1]};
     const uint32_t w23[4] = {b[2][0], b[3][0], b[2][1], b[3][1]};
     mma_bf16(acc[0], w01, xf[0], xf[1]);
@@ -138,6 +96,18 @@ __device__ __forceinline__ void group4(float (&acc)[4][4], uint32_t &s0, uint32_
     if constexpr (HI) {
         mma_bf16(acc[2], w01, xf[2], xf[3]);
         mma_bf16(acc[3], w23, xf[2], xf[3]);
+    }
+}
+__device__ __forceinline__ void group4(uint32_t (&b)[4][2], Quad &z, uint32_t lut_s, const uint32_t (&m)[4]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {                               // two rows -> one packed pair per column
+        uint32_t e[4], f[4];
+        z.step(lut_s, e);
+        z.step(lut_s, f);
+        b[0][h] = weight_pair4<0>(e[0], f[0], m[2 * h], m[2 * h + 1]);
+        b[1][h] = weight_pair4<1>(e[1], f[1], m[2 * h], m[2 * h + 1]);
+        b[2][h] = weight_pair4<2>(e[2], f[2], m[2 * h], m[2 * h + 1]);
+        b[3][h] = weight_pair4<3>(e[3], f[3], m[2 * h], m[2 * h + 1]);
     }
 }
 
@@ -159,8 +129,9 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     // (state << 2 & 0x3FFC) | base: one shift and one three-input logic operation, no addition.
     const uint32_t lut_s = (smem_s + kLutBytes - 1) & ~(kLutBytes - 1);
     uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + (lut_s - smem_s));
-    const uint32_t wbase_s = lut_s + kLutBytes + kBar4Bytes + warp * 2 * p.stage_bytes;
-    const uint32_t bar_base = lut_s + kLutBytes + warp * 16;
+    const uint32_t wbase_s = lut_s + kLutBytes + kBar4Bytes + W * kManBytes + warp * p.stages * p.stage_bytes;
+    const uint32_t man_s = lut_s + kLutBytes + kBar4Bytes + warp * kManBytes;
+    const uint32_t bar_base = lut_s + kLutBytes + warp * 32, man_bar = bar_base + 16;
     const uint32_t seg_bytes = g.th * 16;                       // half a tile of sign+mantissa bytes
     const uint32_t st_off = p.cap_rows * 128;
 
@@ -168,8 +139,8 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     const uint32_t tsel = q >> 1, hsel = q & 1;                 // upper / lower tile, top / bottom half
 
     const uint32_t gw = blockIdx.x * W + warp;                  // this warp's rank in the grid
-    const uint32_t lo = gw * p.per_warp;
-    const uint32_t hi = min(lo + p.per_warp, p.total);
+    const uint32_t lo = gw < p.slots ? (uint32_t)((uint64_t)gw * p.total / p.slots) : p.total;
+    const uint32_t hi = gw < p.slots ? (uint32_t)((uint64_t)(gw + 1) * p.total / p.slots) : p.total;
 
     // Byte ranges of this warp's units, 32 at a time: lane j holds unit dbase + j.
     uint32_t d_off0 = 0, d_ml0 = 0, d_off1 = 0, d_ml1 = 0, dbase = lo;
@@ -204,8 +175,6 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
             mbar_expect_tx(bar, two ? 512u : 256u);
             bulk_load(dst + st_off, a.states + (size_t)t0 * 64, 256, bar);
             if (two) bulk_load(dst + st_off + 256, a.states + ((size_t)t0 + g.tiles_n) * 64, 256, bar);
-            prefetch_l2(a.mantissa + (size_t)t0 * (2 * seg_bytes), 2 * seg_bytes);
-            if (two) prefetch_l2(a.mantissa + ((size_t)t0 + g.tiles_n) * (2 * seg_bytes), 2 * seg_bytes);
         }
         // byte blocks: 16-byte pieces, piece i of a tile = (row i / 4, quarter i % 4)
         const uint8_t *s0 = a.stream + off0, *s1 = a.stream + off1;
@@ -214,16 +183,38 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
         cp_async_arrive(bar);
     };
 
+    // Sign+mantissa rows [kChunkRows * c, + kChunkRows) of the four segments of unit u into chunk buffer `buf`.
+    auto issue_man = [&](uint32_t u, uint32_t c, uint32_t buf) {
+        const uint32_t grp = u / p.pairs_k, pk = u - grp * p.pairs_k;
+        const uint8_t *src = a.mantissa + ((size_t)2 * pk * g.tiles_n + grp) * (2 * seg_bytes) + c * (kChunkRows * 32) + lane * 16;
+        const uint32_t dst = man_s + buf * (4 * kSegPitch) + lane * 16;
+        if (c * kChunkRows + (lane >> 1) < g.half) {
+            cp_async16(dst, src);
+            cp_async16(dst + kSegPitch, src + seg_bytes);
+            if (2 * pk + 1 < g.tiles_k) {
+                src += (size_t)g.tiles_n * (2 * seg_bytes);
+                cp_async16(dst + 2 * kSegPitch, src);
+                cp_async16(dst + 3 * kSegPitch, src + seg_bytes);
+            }
+        }
+        cp_async_arrive(man_bar + buf * 8);
+    };
+
     if (lane == 0) {
         mbar_init(bar_base, 33);                                // 32 cp.async arrivals + the bulk copies' expect_tx
         mbar_init(bar_base + 8, 33);
+        mbar_init(man_bar, 32);
+        mbar_init(man_bar + 8, 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
     load_desc();
     uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
     uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
-    if (lo < hi) issue(lo, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
+    if (lo < hi) {
+        issue(lo, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
+        issue_man(lo, 0, 0);
+    }
     load_lut(s_lut, a.lut, a.tables, a.slot_map);
     __syncthreads();
     // Everything above touches only the weight, which no kernel writes.  When this launch was allowed to
@@ -247,8 +238,8 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     // Writes the finished (or partial) sums of column group grp.  After a lane exchange (below) a lane
     // works on rows gq and gq + 8 of the activation batch, columns 8q .. 8q+7 of the group.
     auto flush = [&](uint32_t grp) {
-        const uint32_t first_w = (grp * p.pairs_k) / p.per_warp;
-        const uint32_t last_w = ((grp + 1) * p.pairs_k - 1) / p.per_warp;
+        auto warp_of = [&](uint32_t u) { return (uint32_t)(((uint64_t)(u + 1) * p.slots - 1) / p.total); };
+        const uint32_t first_w = warp_of(grp * p.pairs_k), last_w = warp_of((grp + 1) * p.pairs_k - 1);
         const uint32_t count = last_w - first_w + 1;
         const uint32_t n0 = grp * 32 + 8 * q;
         auto store_row = [&](uint32_t m, const float (&v)[8]) {
@@ -409,38 +400,21 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
         if (lane == 0) a.tickets[grp] = 0;                      // ready for the next call
     };
 
-    // Activations of rows gq and gq + 8 as the A fragment: columns k .. k+3 are (a0, a2) resp. (a1, a3).
+    // Activations of rows gq and gq + 8, eight consecutive k at a time (two groups of four rows).
     // Rows beyond the batch read the last real row instead: their products land in output rows that are
     // never stored, so no guard (and no branch) is needed in the loop.
     const uint32_t m_last = a.M - 1;
     const uint16_t *x0 = a.x + (size_t)min(gq, m_last) * a.ldx;
     const uint16_t *x1 = a.x + (size_t)min(gq + 8, m_last) * a.ldx;
-
     uint32_t parity0 = 0, parity1 = 0, stage = 0;
     uint32_t cur_grp = lo / p.pairs_k;
     zero_acc();
-    const uint32_t n_groups = g.half / 4;                       // 4-symbol groups per stream (even)
+    const uint32_t n_blocks = g.half / 4;                       // blocks of four symbols per stream
+    const uint32_t n_chunks = (g.half + kChunkRows - 1) / kChunkRows;
     const uint32_t ragged_pk = (g.K % (2 * g.th)) ? p.pairs_k - 1 : 0xFFFFFFFFu;   // the unit index with rows beyond K
+    uint32_t chunk = 0;                                         // sign+mantissa chunks consumed: buffer and phase parity
 
-    uint32_t s0, s1, s2, s3, pos0, pos1, pos2, pos3;
-    // Four symbols of each of the lane's streams -> four B fragments -> four mma.  m = sign+mantissa words
-    // of the four rows, xf = the activations of those rows.
-    // Operands of one group straight from global memory: four 32-byte-strided words of the sign+mantissa
-    // plane and two 8-byte quads of activations.
-    auto fetch = [&](const uint8_t *mp, const uint16_t *xp0, const uint16_t *xp1, uint32_t (&m)[4], uint32_t (&xf)[4]) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) m[i] = ldg_stream_u32(mp + i * 32);
-        const uint2 v0 = __ldg(reinterpret_cast<const uint2 *>(xp0));
-        xf[0] = v0.x;
-        xf[1] = v0.y;
-        xf[2] = xf[3] = 0;
-        if constexpr (HI) {
-            const uint2 v1 = __ldg(reinterpret_cast<const uint2 *>(xp1));
-            xf[2] = v1.x;
-            xf[3] = v1.y;
-        }
-    };
-
+    Quad z;
     for (uint32_t t = lo; t < hi; ++t) {
         const uint32_t grp = t / p.pairs_k, pk = t - grp * p.pairs_k;
         if (grp != cur_grp) {
@@ -448,9 +422,9 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
             zero_acc();
             cur_grp = grp;
         }
-        // Groups of this lane's segment that exist (n_my) and of the stream it decodes (len); see the kernel's header.
-        uint32_t n_my = n_groups, len = n_groups;
-        uint32_t tsel_d = tsel, hsel_d = hsel;                  // the segment whose stream and bytes this lane decodes
+        // Blocks of this lane's segment that exist (n_my) and of the stream it decodes (len); see the kernel's header.
+        uint32_t n_my = n_blocks, len = n_blocks;
+        uint32_t tsel_d = tsel, hsel_d = hsel;                  // the segment whose stream this lane decodes
         if (RAGGED && pk == ragged_pk) {
             const uint32_t r0 = (2 * pk + tsel) * g.th;
             const uint32_t rows_t = r0 < g.K ? min(g.th, g.K - r0) : 0u;
@@ -461,18 +435,16 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
                 len = min(g.half, g.K - 2 * pk * g.th) >> 2;
             }
         }
-        // (row 0 of this lane's segment, its four columns) of the sign+mantissa plane, and its activations
         const uint32_t krow = (2 * pk + tsel) * g.th + hsel * g.half;
-        const uint8_t *mp = a.mantissa + ((size_t)(2 * pk + tsel_d) * g.tiles_n + grp) * (2 * seg_bytes) +
-                            hsel_d * seg_bytes + gq * 4;
-        const uint16_t *xp0 = x0 + krow + 0, *xp1 = x1 + krow;
-        if (RAGGED && n_my == 0) xp0 = xp1 = g_zero_activations;
-        uint32_t mA[4], xA[4], mB[4], xB[4];
-        fetch(mp, xp0, xp1, mA, xA);                            // in flight while the copies are awaited
-
+        uint32_t xs = p.x_step;
+        const uint16_t *xp0 = x0 + (size_t)(krow >> 2) * xs, *xp1 = x1 + (size_t)(krow >> 2) * xs;
+        if (RAGGED && n_my == 0) {
+            xp0 = xp1 = g_zero_activations;
+            xs = 0;
+        }
         const uint32_t ml = (RAGGED ? tsel_d : tsel) ? nx_ml1 : nx_ml0;
-        __syncwarp();                                           // every lane is done with the other stage
-        if (t + 1 < hi) {
+        auto next_unit = [&]() {                                // every lane is done with the window it goes to
+            if (t + 1 >= hi) return;
             if (t + 1 - dbase == 32) {
                 dbase = t + 1;
                 load_desc();
@@ -482,71 +454,94 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
             nx_ml0 = __shfl_sync(kFull, d_ml0, j);
             nx_off1 = __shfl_sync(kFull, d_off1, j);
             nx_ml1 = __shfl_sync(kFull, d_ml1, j);
-            issue(t + 1, stage ^ 1, nx_off0, nx_ml0, nx_off1, nx_ml1);
-        }
+            issue(t + 1, p.stages == 1 ? 0u : stage ^ 1, nx_off0, nx_ml0, nx_off1, nx_ml1);
+        };
+        __syncwarp();
 
         // ---- this lane's four streams --------------------------------------
         const uint32_t win_s = wbase_s + stage * p.stage_bytes;
         const uint32_t st_s = win_s + st_off + (RAGGED ? tsel_d : tsel) * 256 + ((RAGGED ? hsel_d : hsel) * 32 + gq * 4) * 4;
-        pos0 = win_s + (RAGGED ? tsel_d : tsel) * 64 + (RAGGED ? hsel_d : hsel) * 32 + gq * 4;
-        if (ml <= p.cap_rows) pos0 += (ml - 1) * 128;           // last byte row; an empty tile starts one row below
-        const uint32_t pos_first = pos0;
-        pos1 = pos0 + 1;
-        pos2 = pos0 + 2;
-        pos3 = pos0 + 3;
+        uint32_t first = win_s + (RAGGED ? tsel_d : tsel) * 64 + (RAGGED ? hsel_d : hsel) * 32 + gq * 4;
+        if (ml <= p.cap_rows) first += (ml - 1) * 128;          // last byte row; an empty tile starts one row below
 
         // ---- wait for the bytes (bounded) -------------------------------------
         {
             const uint32_t bar = bar_base + stage * 8, par = stage ? parity1 : parity0;
             uint32_t ok = 0;
-            if (lane == 0)
-                for (uint32_t it = 0; it < kWaitPolls && !ok; ++it) ok = mbar_try_wait(bar, par);
-            ok = __shfl_sync(kFull, ok, 0);
+            for (uint32_t it = 0; it < kWaitPolls && !ok; ++it) ok = mbar_try_wait(bar, par);
             if (stage) parity1 ^= 1; else parity0 ^= 1;
-            if (!ok) {
-                if (lane == 0) atomicExch(p.status, 1u);
-                stage ^= 1;
-                continue;
-            }
-            (void)mbar_try_wait(bar, par);                      // each lane observes the completed phase itself
+            if (!ok) atomicExch(p.status, 1u);                  // the result is invalid; the loop still ends
         }
-        s0 = lds_u32(st_s);
-        s1 = lds_u32(st_s + 4);
-        s2 = lds_u32(st_s + 8);
-        s3 = lds_u32(st_s + 12);
+        z.start(st_s, first);
 
-        uint32_t left = len;                                    // groups until this lane's stream is used up (RAGGED)
+        uint32_t wb[4][2] = {};
+        uint32_t xf[4] = {};                                     // the group before: its weights, its activations
+        uint32_t blk = 0, left = len;                           // left: blocks until this lane's stream is used up (RAGGED)
 #pragma unroll 1
-        for (uint32_t gi = 0; gi < n_groups; gi += 2) {         // operands are fetched one group ahead
-            fetch(mp + 128, xp0 + 4, xp1 + 4, mB, xB);
-            group4<HI>(acc, s0, s1, s2, s3, pos0, pos1, pos2, pos3, lut_s, mA, xA);
-            mp += 256;
-            xp0 += 8;
-            xp1 += 8;
-            if constexpr (RAGGED) {
-                if (gi + 2 == n_my) xp0 = xp1 = g_zero_activations;   // rows beyond K from the next group on
+        for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
+            const uint32_t buf = chunk & 1;
+            __syncwarp();                                       // every lane is done with the other chunk buffer
+            if (c + 1 < n_chunks) issue_man(t, c + 1, buf ^ 1);
+            else if (t + 1 < hi) issue_man(t + 1, 0, buf ^ 1);
+            if (c == 0 && p.stages == 2) next_unit();   // behind it: a chunk's arrival waits for older copies
+            {
+                uint32_t ok = 0;
+                for (uint32_t it = 0; it < kWaitPolls && !ok; ++it) ok = mbar_try_wait(man_bar + buf * 8, (chunk >> 1) & 1);
+                if (!ok) atomicExch(p.status, 1u);
             }
-            if (gi + 2 < n_groups) fetch(mp, xp0, xp1, mA, xA);
-            group4<HI>(acc, s0, s1, s2, s3, pos0, pos1, pos2, pos3, lut_s, mB, xB);
-            if constexpr (RAGGED) {
-                left -= 2;
-                if (left == 0) {                                // stream used up: start it over (its products meet zeros)
-                    left = len;
-                    s0 = lds_u32(st_s);
-                    s1 = lds_u32(st_s + 4);
-                    s2 = lds_u32(st_s + 8);
-                    s3 = lds_u32(st_s + 12);
-                    pos0 = pos_first;
-                    pos1 = pos0 + 1;
-                    pos2 = pos0 + 2;
-                    pos3 = pos0 + 3;
-                    mp -= len * 128;                            // and its sign+mantissa rows with it
+            z.clamp(win_s);
+            uint32_t ms = man_s + (buf * 4 + q) * kSegPitch + gq * 4;
+            const uint32_t end = min(blk + kChunkRows / 4, n_blocks);
+#pragma unroll 1
+            for (; blk < end; ++blk) {
+                const uint2 v0 = __ldg(reinterpret_cast<const uint2 *>(xp0));   // used by the mma at the end
+                uint2 v1 = make_uint2(0u, 0u);
+                if constexpr (HI) v1 = __ldg(reinterpret_cast<const uint2 *>(xp1));
+                const uint32_t m[4] = {lds_u32(ms), lds_u32(ms + 32), lds_u32(ms + 64), lds_u32(ms + 96)};
+                // The tensor instruction of the group before comes first: behind it the compiler knows that the warp is
+                // converged and drops the divergence checks (and the register copies they need) of the votes.
+                mma4<HI>(acc, wb, xf);
+                group4(wb, z, lut_s, m);
+                xf[0] = v0.x; xf[1] = v0.y; xf[2] = v1.x; xf[3] = v1.y;
+                ms += 128;
+                xp0 += xs;
+                if constexpr (HI) xp1 += xs;
+                if constexpr (RAGGED) {
+                    if (blk + 1 == n_my) {                      // rows beyond K from the next block on
+                        xp0 = xp1 = g_zero_activations;
+                        xs = 0;
+                    }
+                }
+                if constexpr (RAGGED) {
+                    if (--left == 0) {                          // stream used up: start it over (its products meet zeros)
+                        left = len;
+                        z.start(st_s, first);
+                    }
                 }
             }
         }
-        stage ^= 1;
+        mma4<HI>(acc, wb, xf);
+        if (p.stages == 1) {
+            __syncwarp();                                       // every lane is done with the only window
+            next_unit();
+        } else {
+            stage ^= 1;
+        }
     }
     flush(cur_grp);
+}
+
+// x[M][K] -> scratch[K / 4][M][4].  A warp's activation load reads four consecutive k of every row: from rows K elements
+// apart that is a cache line, and a wavefront of the load pipe, per row and segment (32 a load for 8 rows, 60 % of the
+// kernel's pipe time at 16 rows); in this order a segment's rows are neighbours.
+__global__ void __launch_bounds__(256) k_interleave_x(const uint16_t *__restrict__ x, int64_t ldx, uint32_t M, uint32_t quads,
+                                                      uint2 *__restrict__ out) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");          // the activations may be the previous kernel's product
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t k4 = blockIdx.x * 256 + threadIdx.x;
+    if (k4 >= quads) return;
+    for (uint32_t m = blockIdx.y; m < M; m += gridDim.y)
+        out[(size_t)k4 * M + m] = __ldg(reinterpret_cast<const uint2 *>(x + (size_t)m * ldx) + k4);
 }
 
 // ------------------------------------------------------------------------ host
@@ -560,10 +555,6 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
         (reinterpret_cast<uintptr_t>(a.states) & 15u))
         return 1;
     if ((reinterpret_cast<uintptr_t>(a.x) & 7u) || (a.ldx & 3)) return 1;      // activations are read as 8-byte quads
-    // The kernel does not bounds-test stream cursors; a malformed stream can walk at most tile_h rows of
-    // 128 bytes below its window, which must still be inside the CTA's shared memory.
-    if (g.th * 128u > kLutBytes) return 1;
-
     int dev = 0, max_smem = 0;
     CI_CUDA(cudaGetDevice(&dev));
     CI_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -572,56 +563,74 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     p.cap_rows = max_tile_len;
     p.stage_bytes = (p.cap_rows * 128u + 512u + 127u) & ~127u;
     const uint32_t fixed = 2 * kLutBytes + kBar4Bytes;         // up to one table size is lost to the table's alignment
-    const uint32_t warp_bytes = 2 * p.stage_bytes;
-    if ((uint32_t)max_smem < fixed + 4 * warp_bytes) return 1;
-    uint32_t w_max = ((uint32_t)max_smem - fixed) / warp_bytes;
-    if (w_max > kMma4Warps) w_max = kMma4Warps;
-
-    // Units per warp must be a whole number: pick the warp count whose grid wastes the least.
+    const uint32_t room = (uint32_t)max_smem - fixed;
     const uint32_t P = (uint32_t)sm_count();
     p.pairs_k = (g.tiles_k + 1) / 2;
     p.total = g.groups * p.pairs_k;
-    // A unit here is a serial chain twice as long as in the two-streams kernel (two tiles instead of one).
-    // That pays once the multiprocessors are saturated (about eight warps each); a small matrix -- a
-    // tensor-parallel shard, say -- is latency bound and finishes sooner with the shorter units
-    // (measured cross-over: 4096 x 2048 at tile height 128).
 #ifndef CI_MMA4_MIN_UNITS
 #define CI_MMA4_MIN_UNITS 6
 #endif
-    if (p.total < P * CI_MMA4_MIN_UNITS) return 1;
-    uint32_t best_w = w_max;
-    double best = -1.0;
-    for (uint32_t w = 4; w <= w_max; ++w) {
-        uint64_t slots = (uint64_t)P * w, per = (p.total + slots - 1) / slots;
-        double eff = (double)p.total / (double)(slots * per);
-        if (w < 8) eff *= w / 8.0;                              // too few warps cannot hide the decode chain
-        if (eff >= best) { best = eff; best_w = w; }
+    // A unit here is a serial chain twice as long as in the two-streams kernel (two tiles instead of one).
+    // That pays once the multiprocessors are saturated (about eight warps each); a small matrix -- a
+    // tensor-parallel shard, say -- is latency bound and finishes sooner with the shorter units
+    // (measured cross-over: 4096 x 2048 at tile height 128).  The two-streams kernel takes tiles of up to 256 rows.
+    if (g.th <= 256 && p.total < P * CI_MMA4_MIN_UNITS) return 1;
+    // One CTA per multiprocessor, the units dealt out in equal runs (they differ by one at most).  The time of a round of
+    // units grows as 3.4 + 0.75 x warps us at 64 symbols per stream (measured for 11 to 16 warps; one warp alone on its
+    // scheduler takes about twice the constant), so the warp count decides how well the last round is filled: 4096 x 22016
+    // runs in five rounds of 15 warps, 79 us, against 90 for 14 warps or 11.  A second window per warp, which hides the
+    // copies of the next unit, is worth 2 %: less than a warp that would not fit beside it.
+    uint32_t warps = 0;
+    double best = 0.0;
+    for (uint32_t stages = 2; stages >= 1; --stages) {
+        uint32_t w_max = room / (stages * p.stage_bytes + kManBytes);
+        if (w_max > kMma4Warps) w_max = kMma4Warps;
+        for (uint32_t w = 1; w <= w_max; ++w) {
+            const uint64_t rounds = (p.total + (uint64_t)P * w - 1) / ((uint64_t)P * w);
+            const double round = w < 5 ? 7.15 : 3.4 + 0.75 * w, cost = (double)rounds * round * (stages == 1 ? 1.02 : 1.0);
+            if (warps == 0 || cost < best) { best = cost; warps = w; p.stages = stages; }
+        }
     }
-    const uint64_t slots = (uint64_t)P * best_w;
-    p.per_warp = (uint32_t)((p.total + slots - 1) / slots);
-    const uint32_t warps_needed = (p.total + p.per_warp - 1) / p.per_warp;
-    const uint32_t blocks = (warps_needed + best_w - 1) / best_w;
+    if (warps == 0 || (g.th <= 256 && warps < 4)) return 1;
+    const uint32_t warp_bytes = p.stages * p.stage_bytes + kManBytes;
+    uint32_t blocks = (p.total + warps - 1) / warps;
+    if (blocks > P) blocks = P;
+    p.slots = blocks * warps < p.total ? blocks * warps : p.total;
     p.y_vec = ((reinterpret_cast<uintptr_t>(a.y) & 15u) == 0 && (a.ldy & 7) == 0) ? 1u : 0u;
+    p.x_step = 4;
     p.status = a.tickets + (kTicketBytes - 1);
     if (a.dry_run) return CI_OK;                                // qualification only
 
     const bool ragged = g.K % (2 * g.th) != 0;
-    void (*kernel)(Mma4Args) = a.M <= 8 ? (ragged ? k_linear_mma4<false, true> : k_linear_mma4<false, false>)
-                                        : (ragged ? k_linear_mma4<true, true> : k_linear_mma4<true, false>);
+    static void (*const kernels[4])(Mma4Args) = {k_linear_mma4<false, false>, k_linear_mma4<true, false>,
+                                                  k_linear_mma4<false, true>, k_linear_mma4<true, true>};
     static SmemLimit lim[4] = {};
-    if (int rc = ensure_smem_limit(lim[(a.M > 8) * 2 + ragged], (const void *)kernel, (size_t)max_smem)) return rc;
+    const int which = (a.M > 8) + 2 * ragged;
+    void (*kernel)(Mma4Args) = kernels[which];
+    if (int rc = ensure_smem_limit(lim[which], (const void *)kernel, (size_t)max_smem)) return rc;
     // Programmatic dependent launch: the grid may be scheduled while the previous kernel of the stream
     // drains; the kernel itself waits for that kernel before it reads activations or touches the workspace.
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(best_w * 32);
-    cfg.dynamicSmemBytes = fixed + (size_t)best_w * warp_bytes;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    // The extra launch takes 2.7 us and saves about 1.7e-8 us per activation row and weight, where the multiprocessors are
+    // busy at all: it pays from 1.6e8 of them (4096 x 22016: 119 -> 90 us at 16 rows, 94 -> 85 at 8, 87 -> 85 at 4).
+    if (a.x_scratch != nullptr && a.M >= 3 && p.total >= 6 * P && (uint64_t)a.M * g.K * g.N >= 160000000ull) {
+        const uint32_t quads = g.K / 4;
+        cfg.gridDim = dim3((quads + 255) / 256, a.M);
+        cfg.blockDim = dim3(256);
+        CI_CUDA(cudaLaunchKernelEx(&cfg, k_interleave_x, a.x, a.ldx, a.M, quads, reinterpret_cast<uint2 *>(a.x_scratch)));
+        p.a.x = a.x_scratch;
+        p.a.ldx = 4;
+        p.x_step = 4 * a.M;
+    }
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(warps * 32);
+    cfg.dynamicSmemBytes = fixed + (size_t)warps * warp_bytes;
     CI_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
     return CI_OK;
 }

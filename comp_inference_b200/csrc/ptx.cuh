@@ -131,6 +131,76 @@ __device__ __forceinline__ void renorm_fast(uint32_t &state, uint32_t &pos) {
         : "n"(STRIDE));
 }
 
+// Four streams of one lane whose bytes are the four byte columns of one word column (rows 128 bytes apart).
+//
+// step() decodes one symbol of each stream and returns the table entries.  The next byte of every stream is loaded
+// before it is known to be needed (its address does not depend on the new state, and some lane needs it on nearly
+// every step), which takes one shared-memory latency off the decode chain; about one symbol in three merges it, under
+// a predicate.  A second byte is needed only after a symbol of frequency below 16: the warp tests for it with one vote.
+// The whole renormalisation is one asm block so that the rare branch updates the registers in place; with the branch in
+// C++ the compiler copies all eight of them on the common path (2 of 22 instructions per symbol).
+struct Quad {
+    uint32_t s[4], p[4];                                        // states, shared addresses of the next bytes
+
+    __device__ __forceinline__ void start(uint32_t states_s, uint32_t first) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            s[j] = lds_u32(states_s + 4 * j);
+            p[j] = first + j;
+        }
+    }
+    __device__ __forceinline__ void step(uint32_t lut_s, uint32_t (&e)[4]) {
+        uint32_t y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = lds_u8(p[j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e[j] = decode_aligned(s[j], lut_s);
+        asm volatile(
+            "{\n\t.reg .pred p0, p1, p2, p3, r;\n\t.reg .u32 m0, m1;\n\t"
+            "setp.lt.u32 p0, %0, 65536;\n\t"
+            "setp.lt.u32 p1, %1, 65536;\n\t"
+            "setp.lt.u32 p2, %2, 65536;\n\t"
+            "setp.lt.u32 p3, %3, 65536;\n\t"
+            "@p0 mad.lo.u32 %0, %0, 256, %8;\n\t"
+            "@p1 mad.lo.u32 %1, %1, 256, %9;\n\t"
+            "@p2 mad.lo.u32 %2, %2, 256, %10;\n\t"
+            "@p3 mad.lo.u32 %3, %3, 256, %11;\n\t"
+            "@p0 sub.u32 %4, %4, 128;\n\t"
+            "@p1 sub.u32 %5, %5, 128;\n\t"
+            "@p2 sub.u32 %6, %6, 128;\n\t"
+            "@p3 sub.u32 %7, %7, 128;\n\t"
+            "min.u32 m0, %0, %1;\n\t"
+            "min.u32 m1, %2, %3;\n\t"
+            "min.u32 m0, m0, m1;\n\t"
+            "setp.lt.u32 r, m0, 65536;\n\t"
+            "vote.sync.any.pred r, r, 0xffffffff;\n\t"
+            "@!r bra.uni DONE;\n\t"
+            "setp.lt.u32 p0, %0, 65536;\n\t"
+            "setp.lt.u32 p1, %1, 65536;\n\t"
+            "setp.lt.u32 p2, %2, 65536;\n\t"
+            "setp.lt.u32 p3, %3, 65536;\n\t"
+            "@p0 ld.shared.u8 m0, [%4];\n\t"
+            "@p0 mad.lo.u32 %0, %0, 256, m0;\n\t"
+            "@p0 sub.u32 %4, %4, 128;\n\t"
+            "@p1 ld.shared.u8 m0, [%5];\n\t"
+            "@p1 mad.lo.u32 %1, %1, 256, m0;\n\t"
+            "@p1 sub.u32 %5, %5, 128;\n\t"
+            "@p2 ld.shared.u8 m0, [%6];\n\t"
+            "@p2 mad.lo.u32 %2, %2, 256, m0;\n\t"
+            "@p2 sub.u32 %6, %6, 128;\n\t"
+            "@p3 ld.shared.u8 m0, [%7];\n\t"
+            "@p3 mad.lo.u32 %3, %3, 256, m0;\n\t"
+            "@p3 sub.u32 %7, %7, 128;\n\t"
+            "DONE:\n\t}"
+            : "+r"(s[0]), "+r"(s[1]), "+r"(s[2]), "+r"(s[3]), "+r"(p[0]), "+r"(p[1]), "+r"(p[2]), "+r"(p[3])
+            : "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]));
+    }
+    // Keeps a malformed stream's cursors within reach of the window at `low`: call it at least every 32 symbols.
+    __device__ __forceinline__ void clamp(uint32_t low) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = max(p[j], low);
+    }
+};
 
 __device__ __forceinline__ void sts_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
