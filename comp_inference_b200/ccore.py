@@ -69,6 +69,31 @@ def _tables_host(freqs, cdf):
     return torch.from_numpy(tables), torch.from_numpy(slot_map)
 
 
+class tiled_arrays:
+    """Device arrays of one run of the one-pass encoder (ci_compress_bf16 / ci_compress_plane, 32-wide tiles)."""
+
+    def __init__(self, K, N, th, tw, dev):
+        tiles = -(-K // th) * -(-N // tw)
+        self.dims = (K, N, th, tw)
+        self.states = torch.empty(tiles * 2 * tw, dtype=torch.uint32, device=dev)
+        self.sizes = torch.empty(tiles * 2 * tw, dtype=torch.uint32, device=dev)
+        self.offsets = torch.empty(tiles, dtype=torch.uint32, device=dev)
+        self.max_lens = torch.empty(tiles, dtype=torch.uint32, device=dev)
+        self.tables = torch.empty(256, dtype=torch.uint32, device=dev)
+        self.slot_map = torch.empty(4096, dtype=torch.uint8, device=dev)
+        self.scratch = torch.empty(_lib.load().ci_compress_scratch_bytes(K, N, th, tw), dtype=torch.uint8, device=dev)
+        self.pointers = [_lib.ptr(t) for t in (self.states, self.sizes, self.offsets, self.max_lens, self.tables,
+                                               self.slot_map, self.scratch)] + [self.scratch.numel()]
+
+    def pack(self, n):
+        """The stream, n bytes, from the scratch; gives the scratch back."""
+        self.stream = torch.empty(n, dtype=torch.uint8, device=self.states.device)
+        _lib.check(_lib.load().ci_compress_pack(*self.dims, _lib.ptr(self.sizes), _lib.ptr(self.offsets),
+                                                _lib.ptr(self.max_lens), _lib.ptr(self.scratch), self.scratch.numel(),
+                                                _lib.ptr(self.stream), n, _lib.stream()))
+        self.scratch = None
+
+
 class RansManager:
     """ccore.RansManager (src/python_bindings.cpp:222-471, src/cpp/rans.hpp:9-96)."""
 
@@ -94,12 +119,24 @@ class RansManager:
         plane = data.to(dev, non_blocking=True).contiguous()
         tk, tn = -(-K // th), -(-N // tw)
         T, S = tk * tn, tk * tn * 2 * tw
+        lib = _lib.load()
+        need = lib.ci_compress_scratch_bytes(K, N, th, tw)
+        if need and f.min() >= 1 and int(c[0]) == 0 and np.array_equal(c[1:], np.cumsum(f, dtype=np.uint32)[:-1]):
+            a = tiled_arrays(K, N, th, tw, dev)
+            n = C.c_uint64(0)
+            _lib.check(lib.ci_compress_plane(_lib.ptr(plane), K, N, f.ctypes.data, c.ctypes.data, th, tw, *a.pointers,
+                                             C.byref(n), _lib.stream()))
+            a.pack(n.value)
+            mv = (lambda t: t) if _keep_on_device else (lambda t: t.cpu())
+            return TiledTensorCompressResult(
+                success=True, stream=mv(a.stream), states=mv(a.states), tables=mv(a.tables), slot_map=mv(a.slot_map),
+                output_sizes=mv(a.sizes), num_streams=S, stream_len=int(n.value), tile_offsets=mv(a.offsets),
+                tile_max_lens=mv(a.max_lens), num_tiles_n=tn, num_tiles_k=tk, tile_height=th, tile_width=tw)
         states = torch.empty(S, dtype=torch.uint32, device=dev)
         sizes = torch.empty(S, dtype=torch.uint32, device=dev)
         offs = torch.empty(T, dtype=torch.uint32, device=dev)
         lens = torch.empty(T, dtype=torch.uint32, device=dev)
         n = C.c_uint64(0)
-        lib = _lib.load()
         _lib.check(lib.ci_encode_tiled_sizes(_lib.ptr(plane), K, N, f.ctypes.data, c.ctypes.data, th, tw,
                                              _lib.ptr(states), _lib.ptr(sizes), _lib.ptr(offs), _lib.ptr(lens),
                                              C.byref(n), _lib.stream()))

@@ -4,6 +4,7 @@ GPU through libci_b200.so.  Inputs may live on the CPU (the reference's scripts
 pass CPU tensors); they are moved to the current CUDA device, results come back
 on the device the reference would have left them on.
 """
+import ctypes as C
 from typing import Tuple
 
 import numpy as np
@@ -71,8 +72,8 @@ def uninterleave_mantissas(interleaved_mantissas, K, N, TILE_K=1024, TILE_N=32):
     return tiled.permute(0, 2, 1, 3).contiguous().view(tk * TILE_K, tn * TILE_N)[:K, :N]
 
 
-def _normalize(hist_dev):
-    hist = hist_dev.cpu().numpy().astype(np.uint64)
+def _normalize(hist):
+    hist = np.ascontiguousarray(hist).astype(np.uint64)
     freqs = np.empty(256, np.uint16)
     cdf = np.empty(256, np.uint16)
     _lib.check(_lib.load().ci_normalize_freqs(hist.ctypes.data, freqs.ctypes.data, cdf.ctypes.data))
@@ -87,7 +88,45 @@ def get_rans_lut(data: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     d = _cuda(data).contiguous().view(-1)
     hist = torch.empty(256, dtype=torch.int64, device=d.device)
     _lib.check(_lib.load().ci_histogram_u8(_lib.ptr(d), d.numel(), _lib.ptr(hist), _lib.stream()))
-    return _normalize(hist)
+    return _normalize(hist.cpu().numpy())
+
+
+def _compress(w, tile_height, tile_width, uncoalesced, keep_on_device, want_man_freqs=False):
+    """Encoder result, tiled sign+mantissa bytes (on the device), and the frequency tables of both byte planes (the second
+    pair None unless asked for) of a contiguous bf16 CUDA matrix [K,N]."""
+    K, N = w.shape
+    th, tw = ccore.effective_tile(K, N, int(tile_height), int(tile_width))
+    tk, tn = -(-K // th), -(-N // tw)
+    dev, lib = w.device, _lib.load()
+    man = torch.empty(tk * tn * th * tw, dtype=torch.uint8, device=dev)
+    mfreqs = mcdf = None
+    if not uncoalesced and lib.ci_compress_scratch_bytes(K, N, th, tw):
+        # 32-wide tiles: histogram, tables, split and encoder in one queue with one wait
+        a = ccore.tiled_arrays(K, N, th, tw, dev)
+        freqs, cdf = np.empty(256, np.uint16), np.empty(256, np.uint16)
+        mhist = np.empty(256, np.uint64) if want_man_freqs else None
+        n = C.c_uint64(0)
+        _lib.check(lib.ci_compress_bf16(_lib.ptr(w), K, N, th, tw, _lib.ptr(man), *a.pointers, freqs.ctypes.data,
+                                        cdf.ctypes.data, mhist.ctypes.data if want_man_freqs else None, C.byref(n),
+                                        _lib.stream()))
+        a.pack(n.value)
+        if want_man_freqs:
+            mfreqs, mcdf = _normalize(mhist)
+        mv = (lambda t: t) if keep_on_device else (lambda t: t.cpu())
+        r = ccore.TiledTensorCompressResult(
+            success=True, stream=mv(a.stream), states=mv(a.states), tables=mv(a.tables), slot_map=mv(a.slot_map),
+            output_sizes=mv(a.sizes), num_streams=tk * tn * 2 * tw, stream_len=int(n.value), tile_offsets=mv(a.offsets),
+            tile_max_lens=mv(a.max_lens), num_tiles_n=tn, num_tiles_k=tk, tile_height=th, tile_width=tw)
+        return r, man, torch.from_numpy(freqs), torch.from_numpy(cdf), mfreqs, mcdf
+    exp = torch.empty((K, N), dtype=torch.uint8, device=dev)
+    hist = torch.empty((2, 256), dtype=torch.int64, device=dev)
+    _lib.check(lib.ci_split_bf16(_lib.ptr(w), K, N, th, tw, _lib.ptr(exp), _lib.ptr(man), _lib.ptr(hist[0]),
+                                 _lib.ptr(hist[1]) if want_man_freqs else None, _lib.stream()))
+    freqs, cdf = _normalize(hist[0].cpu().numpy())
+    if want_man_freqs:
+        mfreqs, mcdf = _normalize(hist[1].cpu().numpy())
+    encode = ccore.RansManager(K * N).compress_tiled_uncoalesced if uncoalesced else ccore.RansManager(K * N).compress_tiled
+    return encode(exp, freqs, cdf, th, tw, _keep_on_device=keep_on_device), man, freqs, cdf, mfreqs, mcdf
 
 
 def compress_weight_cuda(weight_kn: torch.Tensor, tile_height=1024, tile_width=32, uncoalesced_interleaving=False):
@@ -100,24 +139,10 @@ def compress_weight_cuda(weight_kn: torch.Tensor, tile_height=1024, tile_width=3
     w = _cuda(weight_kn).contiguous()
     if w.dtype != torch.bfloat16 or w.dim() != 2:
         raise ValueError("expected a 2-D bfloat16 tensor")
-    K, N = w.shape
-    th, tw = ccore.effective_tile(K, N, int(tile_height), int(tile_width))
-    tk, tn = -(-K // th), -(-N // tw)
-    dev = w.device
-    exp = torch.empty((K, N), dtype=torch.uint8, device=dev)
-    man = torch.empty(tk * tn * th * tw, dtype=torch.uint8, device=dev)
-    hist = torch.empty(256, dtype=torch.int64, device=dev)
-    _lib.check(_lib.load().ci_split_bf16(_lib.ptr(w), K, N, th, tw, _lib.ptr(exp), _lib.ptr(man), _lib.ptr(hist), None,
-                                         _lib.stream()))
-    freqs, cdf = _normalize(hist)
-    mgr = ccore.RansManager(K * N)
-    if uncoalesced_interleaving:
-        r = mgr.compress_tiled_uncoalesced(exp, freqs, cdf, th, tw, _keep_on_device=True)
-    else:
-        r = mgr.compress_tiled(exp, freqs, cdf, th, tw, _keep_on_device=True)
+    r, man, freqs, cdf, _, _ = _compress(w, tile_height, tile_width, uncoalesced_interleaving, True)
     out = dict(rans_exp_stream=r.stream, rans_exp_states=r.states, rans_exp_tables=r.tables,
                rans_exp_slot_map=r.slot_map, rans_man_raw=man, exponent_freqs=freqs, exponent_cdf=cdf,
-               output_sizes=r.output_sizes, shape=(K, N), tile_height=r.tile_height, tile_width=r.tile_width,
+               output_sizes=r.output_sizes, shape=tuple(w.shape), tile_height=r.tile_height, tile_width=r.tile_width,
                num_tiles_k=r.num_tiles_k, num_tiles_n=r.num_tiles_n, num_streams=r.num_streams)
     if uncoalesced_interleaving:
         out["rans_exp_stream_offsets"] = r.stream_offsets
@@ -147,25 +172,8 @@ def rans_compress_module_weight_bf16(module: nn.Module, skip_mantissa=True, tile
     wk = _cuda(weight).contiguous()
     module.input_shape = list(wk.shape)
     module.expanded_size = wk.numel()
-    K, N = wk.shape
-    th, tw = ccore.effective_tile(K, N, int(tile_height), int(tile_width))
-    tk, tn = -(-K // th), -(-N // tw)
-    dev = wk.device
-    exp = torch.empty((K, N), dtype=torch.uint8, device=dev)
-    man = torch.empty(tk * tn * th * tw, dtype=torch.uint8, device=dev)
-    hist = torch.empty(256, dtype=torch.int64, device=dev)
-    mhist = torch.empty(256, dtype=torch.int64, device=dev)
-    _lib.check(_lib.load().ci_split_bf16(_lib.ptr(wk), K, N, th, tw, _lib.ptr(exp), _lib.ptr(man), _lib.ptr(hist),
-                                         _lib.ptr(mhist), _lib.stream()))
-    module.exponent_freqs, module.exponent_cdf = _normalize(hist)
-    module.mantissa_freqs, module.mantissa_cdf = _normalize(mhist)
-    mgr = ccore.RansManager(module.expanded_size)
-    if uncoalesced_interleaving:
-        r = mgr.compress_tiled_uncoalesced(exp, module.exponent_freqs, module.exponent_cdf, th, tw,
-                                           _keep_on_device=keep_on_device)
-    else:
-        r = mgr.compress_tiled(exp, module.exponent_freqs, module.exponent_cdf, th, tw,
-                               _keep_on_device=keep_on_device)
+    r, man, module.exponent_freqs, module.exponent_cdf, module.mantissa_freqs, module.mantissa_cdf = _compress(
+        wk, tile_height, tile_width, uncoalesced_interleaving, keep_on_device, want_man_freqs=True)
     if r.success:
         module.exponent_compressed_weight = r.stream
         module.exponent_states = r.states
@@ -183,8 +191,6 @@ def rans_compress_module_weight_bf16(module: nn.Module, skip_mantissa=True, tile
         else:
             module.exponent_tile_offsets = r.tile_offsets
             module.exponent_tile_max_lens = r.tile_max_lens
-    else:
-        module.exponent_raw = exp if keep_on_device else exp.cpu()
     module.mantissa_raw = man if keep_on_device else man.cpu()
     module.compressed = "rans_bfloat16"
     del module.weight

@@ -177,6 +177,28 @@ int ci_encode_tiled_write(const uint8_t *d_plane, uint32_t K, uint32_t N, const 
                           uint32_t tile_h, uint32_t tile_w, const uint32_t *d_sizes, const uint32_t *d_tile_offsets,
                           const uint32_t *d_tile_max_lens, uint8_t *d_stream, uint64_t stream_len, ci_stream_t stream);
 
+/* One-pass encoder for 32-wide tiles, everything on the GPU up to the one wait for the stream's length.
+ *
+ * ci_compress_scratch_bytes: device scratch of a call; 0 = the tile width is not 32 (use the functions above).
+ * ci_compress_bf16: bf16 weight [K,N] -> tiled sign+mantissa bytes, initial states, stream sizes, tile offsets and
+ *   depths, packed {freq,cdf} table u32[256] and slot map u8[4096] on the device, frequencies and cumulative table
+ *   (and, when man_hist is not NULL, the sign+mantissa histogram, u64[256]) on the host.
+ * ci_compress_plane: the same from an exponent plane u8 [K,N] and given frequencies (host arrays of 256).
+ * Both fill *stream_len and SYNCHRONISE the stream; d_tables / d_slot_map may be NULL.
+ * ci_compress_pack: writes d_stream[stream_len] from the scratch and the arrays that call left; queued only. */
+size_t ci_compress_scratch_bytes(uint32_t K, uint32_t N, uint32_t tile_h, uint32_t tile_w);
+int ci_compress_bf16(const uint16_t *d_w, uint32_t K, uint32_t N, uint32_t tile_h, uint32_t tile_w, uint8_t *d_mantissa_tiled,
+                     uint32_t *d_states, uint32_t *d_sizes, uint32_t *d_tile_offsets, uint32_t *d_tile_max_lens,
+                     uint32_t *d_tables, uint8_t *d_slot_map, void *d_scratch, size_t scratch_bytes, uint16_t *freqs,
+                     uint16_t *cdf, uint64_t *man_hist, uint64_t *stream_len, ci_stream_t stream);
+int ci_compress_plane(const uint8_t *d_plane, uint32_t K, uint32_t N, const uint16_t *freqs, const uint16_t *cdf,
+                      uint32_t tile_h, uint32_t tile_w, uint32_t *d_states, uint32_t *d_sizes, uint32_t *d_tile_offsets,
+                      uint32_t *d_tile_max_lens, uint32_t *d_tables, uint8_t *d_slot_map, void *d_scratch,
+                      size_t scratch_bytes, uint64_t *stream_len, ci_stream_t stream);
+int ci_compress_pack(uint32_t K, uint32_t N, uint32_t tile_h, uint32_t tile_w, const uint32_t *d_sizes,
+                     const uint32_t *d_tile_offsets, const uint32_t *d_tile_max_lens, const void *d_scratch,
+                     size_t scratch_bytes, uint8_t *d_stream, uint64_t stream_len, ci_stream_t stream);
+
 /* Dense layout encoder (RansManager::compress_tiled_uncoalesced,
  * src/cuda/rans_ops.cu:74-203; kernel src/cuda/rans_kernels.cuh:7-74). */
 int ci_encode_dense_sizes(const uint8_t *d_plane, uint32_t K, uint32_t N, const uint16_t *freqs, const uint16_t *cdf,
@@ -214,7 +236,8 @@ size_t ci_linear_workspace_bytes(uint32_t M, uint32_t n_out, uint32_t K, uint32_
  * large M, the decompress + triton_matmul pair (comp_inference/triton_gemm.py:324-337).
  * d_workspace must hold ci_linear_workspace_bytes() bytes and must have been
  * zero-filled once when allocated; each call leaves it zeroed again.
- * split_k = 0 lets the library choose. */
+ * split_k is a hint for the shapes that only the generic split-K kernel takes, and for the prefill GEMM
+ * (0: the library's choice); the staged kernels split K by themselves. */
 int ci_linear(const ci_tiled_weight *w, const uint16_t *d_x, int64_t x_row_stride, uint32_t M, const uint16_t *d_bias,
               uint16_t *d_y, int64_t y_row_stride, void *d_workspace, size_t workspace_bytes, uint32_t split_k,
               ci_stream_t stream);

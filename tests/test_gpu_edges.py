@@ -34,3 +34,29 @@ def test_linear_dispatch_edges(K, N, th, M, split_k):
         bias=bias, SPLIT_K=split_k)
     assert _close(y, x.float() @ W.float() + bias.float())
     assert _lib.kernel_status(x.device) == 0
+
+
+# every split of the one-pass encoder (one / two columns a lane, one / two halves), odd and ragged sides, streams whose
+# length is no multiple of four symbols' worth of rows, a plane of one symbol, symbols of frequency one
+@pytest.mark.parametrize("K,N,th", [(2048, 4800, 64), (2050, 4800, 64), (1100, 2432, 128), (1000, 77, 128), (16, 1, 16),
+                                    (33, 64, 16), (2049, 130, 1024), (40, 62, 32)])
+@pytest.mark.parametrize("kind", ["normal", "wide", "constant"])
+def test_one_pass_encoder_matches_oracle(K, N, th, kind):
+    import numpy as np
+    import comp_inference_b200 as ci
+    from oracle import oracle as O
+    g = torch.Generator().manual_seed(K * 31 + N)
+    W = {"normal": lambda: torch.randn(K, N, generator=g) * 0.02,
+         "wide": lambda: torch.randn(K, N, generator=g) * 2.0 ** torch.randint(-100, 100, (K, N), generator=g),
+         "constant": lambda: torch.full((K, N), 1.5)}[kind]().to(torch.bfloat16)
+    c = ci.compress_weight_cuda(W.cuda(), th, 32)
+    o = O.compress_bf16(W.view(torch.uint16).numpy(), c["tile_height"], c["tile_width"])
+    host = lambda name: c[name].cpu().view(torch.uint8).numpy()
+    for name, want in (("rans_exp_stream", o.stream), ("rans_exp_states", o.states), ("rans_exp_tables", o.tables),
+                       ("rans_exp_slot_map", o.slot_map), ("rans_exp_tile_offsets", o.tile_offsets),
+                       ("rans_exp_tile_max_lens", o.tile_max_lens), ("rans_man_raw", o["mantissa"])):
+        assert np.array_equal(host(name), np.ascontiguousarray(want).view(np.uint8).reshape(-1)), name
+    plane, _ = ci.extract_exp_and_mantissa(W.cuda())
+    r = ci.ccore.RansManager().compress_tiled(plane, c["exponent_freqs"], c["exponent_cdf"], th, 32)
+    assert torch.equal(r.stream, c["rans_exp_stream"].cpu()) and torch.equal(r.output_sizes.view(torch.int32),
+                                                                            c["output_sizes"].cpu().view(torch.int32))
