@@ -72,11 +72,11 @@ __global__ void __launch_bounds__(512) k_exp_histogram(const uint16_t *__restric
 // ---------------------------------------------------------------- 2. tables
 
 __device__ __forceinline__ uint4 encoder_entry(uint32_t f, uint32_t start) {
-    // {m, start (+ 4095 where m stands for a division by one: it yields x - 1), 4096 - f | s << 16, first state too large}
-    if (f == 1) return make_uint4(0xFFFFFFFFu, start + 4095u, 4095u, 1u << 12);
+    // {m, start (+ 4095 where m stands for a division by one: it yields x - 1), (4096 - f) << 5 | s, first state too large}
+    if (f == 1) return make_uint4(0xFFFFFFFFu, start + 4095u, 4095u << 5, 1u << 12);
     const uint32_t s = 31 - __clz(f - 1);
     const uint32_t m = (uint32_t)(((1ull << (32 + s)) + f - 1) / f);
-    return make_uint4(m, start, (4096u - f) | (s << 16), f << 12);
+    return make_uint4(m, start, (4096u - f) << 5 | s, f << 12);
 }
 
 // One block.  hist != null: the frequency rule of ci_normalize_freqs; null: frequencies are in res already.
@@ -98,29 +98,49 @@ __global__ void __launch_bounds__(256) k_make_tables(const unsigned long long *h
         if (man_hist) res->man_hist[t] = man_hist[t];
         __syncthreads();
         if (warp == 0) {
-            // value << 8 | 255 - symbol: the largest key is the largest frequency, ties to the lowest symbol
-            uint32_t key[8], total = 0;
+            // A surplus goes to the largest frequency (ties: the lowest symbol).  A deficit is taken one unit at a time from
+            // whichever is largest then (comp_inference/comp_inference.py:204-227): that levels everything above some v
+            // down to v, and the units that are left come off the first symbols at that level.
+            uint32_t v[8], total = 0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const uint32_t v = s_f[lane * 8 + j];
-                key[j] = v << 8 | (255 - (lane * 8 + j));
-                total += v;
+                v[j] = s_f[lane * 8 + j];
+                total += v[j];
             }
             total = __reduce_add_sync(kFull, total);
-            int diff = 4096 - (int)total;
-            while (diff != 0) {                                 // comp_inference/comp_inference.py:204-227
-                uint32_t top = key[0];
+            if (total < 4096u) {
+                uint32_t top = 0;                               // value << 8 | 255 - symbol
 #pragma unroll
-                for (int j = 1; j < 8; ++j) top = max(top, key[j]);
+                for (int j = 0; j < 8; ++j) top = max(top, v[j] << 8 | (255 - (lane * 8 + j)));
                 top = __reduce_max_sync(kFull, top);
-                const int by = diff > 0 ? diff : -1;            // a surplus goes to the top symbol at once, a deficit unit by unit
+                if (lane == 0) s_f[255 - (top & 255u)] += 4096u - total;
+            } else if (total > 4096u) {
+                const uint32_t need = total - 4096u;
+                auto above = [&](uint32_t level) {
+                    uint32_t sum = 0;
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (key[j] == top) key[j] += (uint32_t)by << 8;
-                diff -= by;
+                    for (int j = 0; j < 8; ++j) sum += v[j] > level ? v[j] - level : 0u;
+                    return __reduce_add_sync(kFull, sum);
+                };
+                uint32_t level = 0;                             // the smallest with above(level) <= need
+                for (uint32_t d = 4096; d; d >>= 1)
+                    if (above(level + d - 1) > need) level += d;
+                uint32_t left = need - above(level), at = 0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) at += v[j] >= level;
+                uint32_t rank = at;                             // symbols at the level in lower lanes
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t o = __shfl_up_sync(kFull, rank, d);
+                    if (lane >= d) rank += o;
+                }
+                rank -= at;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    uint32_t f = min(v[j], level);
+                    if (v[j] >= level && rank++ < left) --f;
+                    s_f[lane * 8 + j] = f;
+                }
             }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) s_f[lane * 8 + j] = key[j] >> 8;
         }
         __syncthreads();
         if (warp == 0) {
@@ -167,72 +187,76 @@ struct Enc32Args {
     const uint4 *table;
 };
 
-// One stream: state, the last bytes emitted (newest in the low byte), their number, and where the next word goes.
+// One stream: state, the last bytes emitted (newest in the low byte), their number, and its first word.
 struct Chain {
     uint32_t x, acc, n;
-    uint32_t *out, *end;
+    uint32_t *base;
 
-    __device__ __forceinline__ void emit() {
-        acc = __byte_perm(acc, x, 0x2104);                      // acc << 8 | x & 0xFF
-        x >>= 8;
-        if ((++n & 3u) == 0) {
-            if (out < end) *out = acc;
-            out += 64;
-        }
-    }
+    // Encodes one symbol.  Written with predicates: as branches the emission costs 20 of 44 instructions per symbol in
+    // reconvergence and 64-bit pointers.  A byte leaves about one symbol in three; a second one only before symbols of
+    // frequency below 16.  The slot of stream_words() words always suffices: every symbol multiplies the state by at
+    // most 4096 (1 + 1/16) and every byte divides it by 256.
     __device__ __forceinline__ void put(const uint4 e) {
-        if (x >= e.w) {
-            emit();
-            if (x >= e.w) emit();                               // only before symbols of frequency below 16
-        }
-        const uint32_t q = __umulhi(x, e.x) >> (e.z >> 16);
-        x = x + e.y + q * (e.z & 0xFFFFu);                      // x / f * 4096 + x % f + start
+        asm volatile(
+            "{\n\t.reg .pred p, q, r;\n\t.reg .u32 t;\n\t.reg .u64 a;\n\t"
+            "setp.ge.u32 p, %0, %4;\n\t"
+            "@p prmt.b32 %1, %1, %0, 0x2104;\n\t"             // acc << 8 | x & 0xFF
+            "@p shr.u32 %0, %0, 8;\n\t"
+            "@p add.u32 %2, %2, 1;\n\t"
+            "and.b32 t, %2, 3;\n\t"
+            "setp.eq.and.u32 q, t, 0, p;\n\t"
+            "@q mad.wide.u32 a, %2, 64, %3;\n\t"
+            "@q st.global.u32 [a+-256], %1;\n\t"
+            "setp.ge.u32 r, %0, %4;\n\t"
+            "@!r bra DONE;\n\t"
+            "prmt.b32 %1, %1, %0, 0x2104;\n\t"
+            "shr.u32 %0, %0, 8;\n\t"
+            "add.u32 %2, %2, 1;\n\t"
+            "and.b32 t, %2, 3;\n\t"
+            "setp.eq.u32 q, t, 0;\n\t"
+            "@q mad.wide.u32 a, %2, 64, %3;\n\t"
+            "@q st.global.u32 [a+-256], %1;\n\t"
+            "DONE:\n\t}"
+            : "+r"(x), "+r"(acc), "+r"(n)
+            : "l"(base), "r"(e.w)
+            : "memory");
+        const uint32_t q = __funnelshift_r(__umulhi(x, e.x), 0u, e.z);   // the shift is e.z mod 32
+        x = q * (e.z >> 5) + (x + e.y);                         // x / f * 4096 + x % f + start
     }
     __device__ __forceinline__ void finish() {
-        if ((n & 3u) && out < end) *out = acc << (8 * (4 - (n & 3u)));
+        if (n & 3u) base[(n >> 2) * 64] = acc << (8 * (4 - (n & 3u)));
     }
 };
 
-// COLS columns per lane (1, or 2 where rows of pairs are aligned and there are warps enough), HALVES of a tile per lane
-// (2: the top and bottom stream of a column interleaved; 1: one of them, which doubles the warps of a small matrix).
-// Rows are taken last first, four at a time, loaded one batch ahead of the chains.
-template <int COLS, int HALVES, bool PLANE>
-__global__ void __launch_bounds__(256) k_encode32(const __grid_constant__ Enc32Args a) {
+// One warp takes one half (top or bottom streams) of COLS neighbouring tiles, a lane one or two columns.  Rows are taken
+// last first, four at a time, loaded one batch ahead of the chains.  (Both halves in one lane, twice the independent
+// chains and half the warps, was slower: 95 to 141 us against 80 for 4096 x 11008.)
+template <int COLS, bool PLANE>
+__global__ void __launch_bounds__(256, 4) k_encode32(const __grid_constant__ Enc32Args a) {
     __shared__ uint4 s_tab[256];
     for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab[i] = a.table[i];
     __syncthreads();
-    const uint32_t lane = lane_id(), strips = (a.tiles_n + COLS - 1) / COLS;
-    const uint32_t per_row = strips * (3 - HALVES);
+    const uint32_t lane = lane_id(), per_row = (a.tiles_n + COLS - 1) / COLS * 2;
     const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (gw >= per_row * a.tiles_k) return;
-    const uint32_t tk = gw / per_row, rem = gw - tk * per_row;
-    const uint32_t strip = HALVES == 2 ? rem : rem >> 1, h0 = HALVES == 2 ? 0 : rem & 1;
+    const uint32_t tk = gw / per_row, rem = gw - tk * per_row, strip = rem >> 1, h = rem & 1;
     const uint32_t col = strip * (32 * COLS) + lane * COLS;     // first column of this lane
     const uint32_t tn = strip * COLS + (COLS == 2 ? lane >> 4 : 0), c = col & 31;
     const bool live = col < a.N, in_tile = tn < a.tiles_n;
     const size_t t = (size_t)tk * a.tiles_n + tn;
 
-    Chain z[HALVES][COLS];
+    Chain z[COLS];
 #pragma unroll
-    for (int h = 0; h < HALVES; ++h)
-#pragma unroll
-        for (int j = 0; j < COLS; ++j) {
-            z[h][j].x = kRansL;
-            z[h][j].acc = z[h][j].n = 0;
-            z[h][j].out = a.words + t * a.cap_words * 64 + (h0 + h) * 32 + c + j;
-            z[h][j].end = a.words + (t + 1) * a.cap_words * 64;
-        }
-    if (live) {
-        const uint32_t row0 = tk * a.th + h0 * a.half;
-        uint32_t rows[HALVES];
-#pragma unroll
-        for (int h = 0; h < HALVES; ++h) {
-            const uint32_t first = row0 + h * a.half;
-            rows[h] = first < a.K ? min(a.half, a.K - first) : 0u;
-        }
-        // entry of row i of half h: the symbols of the lane's columns
-        auto fetch = [&](int h, uint32_t i) -> uint32_t {
-            const size_t at = (size_t)(row0 + h * a.half + i) * a.N + col;
+    for (int j = 0; j < COLS; ++j) {
+        z[j].x = kRansL;
+        z[j].acc = z[j].n = 0;
+        z[j].base = a.words + t * a.cap_words * 64 + h * 32 + c + j;
+    }
+    const uint32_t row0 = tk * a.th + h * a.half;
+    if (live && row0 < a.K) {
+        const size_t first = (size_t)row0 * a.N + col;
+        auto fetch = [&](uint32_t i) -> uint32_t {              // row i of the half: the symbols of the lane's columns
+            const size_t at = first + (size_t)i * a.N;
             if constexpr (PLANE) {
                 const uint8_t *s = static_cast<const uint8_t *>(a.src) + at;
                 return COLS == 2 ? *reinterpret_cast<const uint16_t *>(s) : *s;
@@ -241,66 +265,49 @@ __global__ void __launch_bounds__(256) k_encode32(const __grid_constant__ Enc32A
                 return COLS == 2 ? *reinterpret_cast<const uint32_t *>(s) : *s;
             }
         };
-        uint8_t *man = a.mantissa + t * a.th * 32 + (size_t)h0 * a.half * 32 + c;
-        auto code = [&](int h, uint32_t i, uint32_t w) {
+        uint8_t *man = a.mantissa + t * a.th * 32 + (size_t)h * a.half * 32 + c;
+        auto code = [&](uint32_t i, uint32_t w) {
             if constexpr (PLANE) {
-                z[h][0].put(s_tab[w & 0xFFu]);
-                if constexpr (COLS == 2) z[h][1].put(s_tab[w >> 8]);
+                z[0].put(s_tab[w & 0xFFu]);
+                if constexpr (COLS == 2) z[1].put(s_tab[w >> 8]);
             } else {
                 const uint32_t m = ((w >> 8) & 0x00800080u) | (w & 0x007F007Fu);
-                uint8_t *dst = man + ((size_t)h * a.half + i) * 32;
+                uint8_t *dst = man + i * 32;
                 if constexpr (COLS == 2) *reinterpret_cast<uint16_t *>(dst) = (uint16_t)__byte_perm(m, 0u, 0x4420);
                 else *dst = (uint8_t)m;
-                z[h][0].put(s_tab[(w >> 7) & 0xFFu]);
-                if constexpr (COLS == 2) z[h][1].put(s_tab[(w >> 23) & 0xFFu]);
+                z[0].put(s_tab[(w >> 7) & 0xFFu]);
+                if constexpr (COLS == 2) z[1].put(s_tab[(w >> 23) & 0xFFu]);
             }
         };
-        // rows that one half has more than the other (the last tile row of a matrix), one at a time
-        const uint32_t both = HALVES == 2 ? min(rows[0], rows[HALVES - 1]) : rows[0];
-#pragma unroll
-        for (int h = 0; h < HALVES; ++h)
-            for (uint32_t i = rows[h]; i > both; --i) code(h, i - 1, fetch(h, i - 1));
-        uint32_t i = both;
-        for (; i & 3u; --i)
-#pragma unroll
-            for (int h = 0; h < HALVES; ++h) code(h, i - 1, fetch(h, i - 1));
+        uint32_t i = min(a.half, a.K - row0);
+        for (; i & 3u; --i) code(i - 1, fetch(i - 1));
         if (i) {
-            uint32_t w[HALVES][4], nx[HALVES][4];
+            uint32_t w[4], nx[4];
 #pragma unroll
-            for (int h = 0; h < HALVES; ++h)
-#pragma unroll
-                for (int r = 0; r < 4; ++r) w[h][r] = fetch(h, i - 1 - r);
+            for (int r = 0; r < 4; ++r) w[r] = fetch(i - 1 - r);
             for (; i; i -= 4) {
                 if (i > 4) {
 #pragma unroll
-                    for (int h = 0; h < HALVES; ++h)
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) nx[h][r] = fetch(h, i - 5 - r);
+                    for (int r = 0; r < 4; ++r) nx[r] = fetch(i - 5 - r);
                 }
 #pragma unroll
-                for (int r = 0; r < 4; ++r)
+                for (int r = 0; r < 4; ++r) code(i - 1 - r, w[r]);
 #pragma unroll
-                    for (int h = 0; h < HALVES; ++h) code(h, i - 1 - r, w[h][r]);
-#pragma unroll
-                for (int h = 0; h < HALVES; ++h)
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) w[h][r] = nx[h][r];
+                for (int r = 0; r < 4; ++r) w[r] = nx[r];
             }
         }
     }
     uint32_t deepest = 0;
 #pragma unroll
-    for (int h = 0; h < HALVES; ++h)
-#pragma unroll
-        for (int j = 0; j < COLS; ++j) {
-            if (in_tile) {
-                z[h][j].finish();
-                const size_t sid = t * 64 + (h0 + h) * 32 + c + j;
-                a.states[sid] = z[h][j].x;
-                a.sizes[sid] = z[h][j].n;
-            }
-            deepest = max(deepest, z[h][j].n);
+    for (int j = 0; j < COLS; ++j) {
+        if (in_tile) {
+            z[j].finish();
+            const size_t sid = t * 64 + h * 32 + c + j;
+            a.states[sid] = z[j].x;
+            a.sizes[sid] = z[j].n;
         }
+        deepest = max(deepest, z[j].n);
+    }
 #pragma unroll
     for (int d = COLS == 2 ? 8 : 16; d; d >>= 1) deepest = max(deepest, __shfl_xor_sync(kFull, deepest, d));
     if ((lane & (COLS == 2 ? 15 : 31)) == 0 && in_tile) atomicMax(a.max_lens + t, deepest);
@@ -308,37 +315,51 @@ __global__ void __launch_bounds__(256) k_encode32(const __grid_constant__ Enc32A
 
 // ---------------------------------------------------------------- 4. offsets
 
-// Exclusive scan of 64 x max_lens by one block, 4096 tiles a pass; the 64-bit total goes to the overflow check.
+// Exclusive scan of 64 x max_lens by one block, 16384 tiles a pass; the 64-bit total goes to the overflow check.
 __global__ void __launch_bounds__(1024) k_scan_tiles(const uint32_t *__restrict__ max_lens, uint32_t tiles,
                                                      uint32_t *__restrict__ offsets, EncResult *res) {
-    __shared__ unsigned long long s_warp[32];
+    __shared__ unsigned long long s_warp[33];
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     unsigned long long base = 0;
-    for (uint32_t first = 0; first < tiles; first += 4096) {
-        uint32_t v[4], at = first + 4 * t;
+    for (uint32_t first = 0; first < tiles; first += 16384) {
+        uint32_t v[4][4];                                       // tile first + 4096 k + 4 t + j
+        unsigned long long run, mine;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = at + j < tiles ? max_lens[at + j] * 64u : 0u;
-        const unsigned long long mine = (unsigned long long)v[0] + v[1] + v[2] + v[3];
-        unsigned long long run = mine;
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned long long o = __shfl_up_sync(kFull, run, d);
-            if (lane >= d) run += o;
-        }
-        if (lane == 31) s_warp[warp] = run;
-        __syncthreads();
-        unsigned long long before = 0, all = 0;
-        for (uint32_t i = 0; i < 32; ++i) {
-            if (i < warp) before += s_warp[i];
-            all += s_warp[i];
-        }
-        unsigned long long o = base + before + run - mine;
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t at = first + 4096 * k + 4 * t;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (at + j < tiles) offsets[at + j] = (uint32_t)o;
-            o += v[j];
+            for (int j = 0; j < 4; ++j) v[k][j] = at + j < tiles ? max_lens[at + j] * 64u : 0u;
         }
-        base += all;
-        __syncthreads();
+        for (int k = 0; k < 4 && first + 4096 * k < tiles; ++k) {
+            mine = (unsigned long long)v[k][0] + v[k][1] + v[k][2] + v[k][3];
+            run = mine;
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned long long o = __shfl_up_sync(kFull, run, d);
+                if (lane >= d) run += o;
+            }
+            if (lane == 31) s_warp[warp] = run;
+            __syncthreads();
+            if (warp == 0) {
+                const unsigned long long own = s_warp[lane];
+                unsigned long long w = own;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const unsigned long long o = __shfl_up_sync(kFull, w, d);
+                    if (lane >= d) w += o;
+                }
+                s_warp[lane] = w - own;
+                if (lane == 31) s_warp[32] = w;
+            }
+            __syncthreads();
+            unsigned long long o = base + s_warp[warp] + run - mine;
+            const uint32_t at = first + 4096 * k + 4 * t;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (at + j < tiles) offsets[at + j] = (uint32_t)o;
+                o += v[k][j];
+            }
+            base += s_warp[32];
+            __syncthreads();
+        }
     }
     if (t == 0) res->total = base;
 }
@@ -389,25 +410,22 @@ static EncResult *pinned_result() {
 
 static bool encode32_takes(const Geom &g) { return g.tw == 32 && g.th >= 16 && g.th % 16 == 0; }
 
-template <int COLS, int HALVES, bool PLANE>
+template <int COLS, bool PLANE>
 static int launch_encode32(const Enc32Args &a, cudaStream_t s) {
-    const uint32_t warps = ((a.tiles_n + COLS - 1) / COLS) * (3 - HALVES) * a.tiles_k;
-    k_encode32<COLS, HALVES, PLANE><<<(warps + 7) / 8, 256, 0, s>>>(a);
+    const uint32_t warps = (a.tiles_n + COLS - 1) / COLS * 2 * a.tiles_k;
+    k_encode32<COLS, PLANE><<<(warps + 7) / 8, 256, 0, s>>>(a);
     CI_LAUNCH_CHECK(k_encode32);
     return CI_OK;
 }
 
 template <bool PLANE>
 static int encode32(Enc32Args a, uint32_t *d_offsets, EncResult *d_res, uint64_t *stream_len, cudaStream_t s) {
-    // Two columns a lane halve the loads, stores and address arithmetic per symbol, but they and the interleaved
-    // halves also halve the warps: only where a multiprocessor keeps about 16 of them.
-    const uint32_t P = (uint32_t)sm_count(), strips = (a.tiles_n + 1) / 2 * a.tiles_k;
-    const bool pairs = a.N % 2 == 0 && (reinterpret_cast<uintptr_t>(a.src) & (PLANE ? 1u : 3u)) == 0;
+    // Two columns a lane halve the loads, stores and address arithmetic per symbol, but also the warps: only where a
+    // multiprocessor keeps 16 of them.
+    const bool aligned = a.N % 2 == 0 && (reinterpret_cast<uintptr_t>(a.src) & (PLANE ? 1u : 3u)) == 0;
+    const uint64_t warps2 = (uint64_t)(a.tiles_n + 1) / 2 * 2 * a.tiles_k;
     CI_CUDA(cudaMemsetAsync(a.max_lens, 0, (size_t)a.tiles_k * a.tiles_n * 4, s));
-    int rc;
-    if (pairs && strips >= 16 * P) rc = launch_encode32<2, 2, PLANE>(a, s);
-    else if (pairs && 2 * strips >= 16 * P) rc = launch_encode32<2, 1, PLANE>(a, s);
-    else rc = launch_encode32<1, 1, PLANE>(a, s);
+    int rc = aligned && warps2 >= 16ull * sm_count() ? launch_encode32<2, PLANE>(a, s) : launch_encode32<1, PLANE>(a, s);
     if (rc) return rc;
     k_scan_tiles<<<1, 1024, 0, s>>>(a.max_lens, a.tiles_k * a.tiles_n, d_offsets, d_res);
     CI_LAUNCH_CHECK(k_scan_tiles);
