@@ -29,13 +29,6 @@ struct Emb4Args {
     uint32_t out_vec;      // rows of the output can be written as 8-byte quads
 };
 
-__device__ __forceinline__ void e4_cp_async16(uint32_t dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void e4_cp_async_arrive(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 // What a task needs to know about its token: tile row, half, symbols to drop; valid = id inside the table.
 struct Tok {
     uint32_t tk, hsel, inner, rel;
@@ -87,9 +80,9 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
             const uint32_t mlj = __shfl_sync(kFull, ml, j), offj = __shfl_sync(kFull, off, j);
             const uint8_t *src = a.stream + offj + t.hsel * 32;
             for (uint32_t i = lane; i < mlj * 2; i += 32)
-                e4_cp_async16(dst + (i >> 1) * 128 + j * 32 + (i & 1) * 16, src + (size_t)(i >> 1) * 64 + (i & 1) * 16);
+                cp_async16(dst + (i >> 1) * 128 + j * 32 + (i & 1) * 16, src + (size_t)(i >> 1) * 64 + (i & 1) * 16);
         }
-        e4_cp_async_arrive(bar);
+        cp_async_arrive(bar);
     };
     // This lane's four initial states of a task (one 16-byte load) and its tile's depth.
     auto load_states = [&](uint64_t task, const Tok &t) {

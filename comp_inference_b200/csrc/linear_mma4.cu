@@ -41,9 +41,6 @@
 namespace ci {
 
 constexpr uint32_t kBar4Bytes = 512;         // up to 16 warps x (2 window stages + 2 mantissa chunks) x 8 B
-constexpr uint32_t kChunkRows = 16;          // rows of sign+mantissa bytes per chunk and segment
-constexpr uint32_t kSegPitch = kChunkRows * 32 + 32;   // the four segments of a chunk start 8 banks apart
-constexpr uint32_t kManBytes = 2 * 4 * kSegPitch;      // two chunks per warp
 constexpr uint32_t kMma4Warps = 16;          // x 32 threads x 128 registers = the register file
 
 struct Mma4Args {
@@ -58,14 +55,6 @@ struct Mma4Args {
     uint32_t x_step;       // elements from one row's activations k .. k+3 to k+4 .. k+7
     uint32_t *status;      // set non-zero if a wait ran out
 };
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-// The mbarrier gets one arrival when all cp.async issued so far by this thread have landed.
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
 
 // Packed bf16 pair (rows k, k+1) of column c of the lane from two table entries and the two
 // 4-column sign+mantissa words of those rows.
@@ -467,10 +456,8 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
         // ---- wait for the bytes (bounded) -------------------------------------
         {
             const uint32_t bar = bar_base + stage * 8, par = stage ? parity1 : parity0;
-            uint32_t ok = 0;
-            for (uint32_t it = 0; it < kWaitPolls && !ok; ++it) ok = mbar_try_wait(bar, par);
+            if (!mbar_wait(bar, par)) atomicExch(p.status, 1u);  // the result is invalid; the loop still ends
             if (stage) parity1 ^= 1; else parity0 ^= 1;
-            if (!ok) atomicExch(p.status, 1u);                  // the result is invalid; the loop still ends
         }
         z.start(st_s, first);
 
@@ -484,11 +471,7 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
             if (c + 1 < n_chunks) issue_man(t, c + 1, buf ^ 1);
             else if (t + 1 < hi) issue_man(t + 1, 0, buf ^ 1);
             if (c == 0 && p.stages == 2) next_unit();   // behind it: a chunk's arrival waits for older copies
-            {
-                uint32_t ok = 0;
-                for (uint32_t it = 0; it < kWaitPolls && !ok; ++it) ok = mbar_try_wait(man_bar + buf * 8, (chunk >> 1) & 1);
-                if (!ok) atomicExch(p.status, 1u);
-            }
+            if (!mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1)) atomicExch(p.status, 1u);
             z.clamp(win_s);
             uint32_t ms = man_s + (buf * 4 + q) * kSegPitch + gq * 4;
             const uint32_t end = min(blk + kChunkRows / 4, n_blocks);
@@ -575,10 +558,8 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     // tensor-parallel shard, say -- is latency bound and finishes sooner with the shorter units
     // (measured cross-over: 4096 x 2048 at tile height 128).  The two-streams kernel takes tiles of up to 256 rows.
     if (g.th <= 256 && p.total < P * CI_MMA4_MIN_UNITS) return 1;
-    // One CTA per multiprocessor, the units dealt out in equal runs (they differ by one at most).  The time of a round of
-    // units grows as 3.4 + 0.75 x warps us at 64 symbols per stream (measured for 11 to 16 warps; one warp alone on its
-    // scheduler takes about twice the constant), so the warp count decides how well the last round is filled: 4096 x 22016
-    // runs in five rounds of 15 warps, 79 us, against 90 for 14 warps or 11.  A second window per warp, which hides the
+    // One CTA per multiprocessor, the units dealt out in equal runs (they differ by one at most).  The warp count decides
+    // how well the last round is filled: 4096 x 22016 runs in five rounds of 15 warps, 82 us, against 90 for 14 or 11.  A second window per warp, which hides the
     // copies of the next unit, is worth 2 %: less than a warp that would not fit beside it.
     uint32_t warps = 0;
     double best = 0.0;
@@ -587,7 +568,7 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
         if (w_max > kMma4Warps) w_max = kMma4Warps;
         for (uint32_t w = 1; w <= w_max; ++w) {
             const uint64_t rounds = (p.total + (uint64_t)P * w - 1) / ((uint64_t)P * w);
-            const double round = w < 5 ? 7.15 : 3.4 + 0.75 * w, cost = (double)rounds * round * (stages == 1 ? 1.02 : 1.0);
+            const double cost = (double)rounds * round_cost(w) * (stages == 1 ? 1.02 : 1.0);
             if (warps == 0 || cost < best) { best = cost; warps = w; p.stages = stages; }
         }
     }

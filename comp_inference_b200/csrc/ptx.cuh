@@ -33,6 +33,13 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// The mbarrier gets one arrival when all cp.async issued so far by this thread have landed.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
@@ -136,9 +143,10 @@ __device__ __forceinline__ void renorm_fast(uint32_t &state, uint32_t &pos) {
 // step() decodes one symbol of each stream and returns the table entries.  The next byte of every stream is loaded
 // before it is known to be needed (its address does not depend on the new state, and some lane needs it on nearly
 // every step), which takes one shared-memory latency off the decode chain; about one symbol in three merges it, under
-// a predicate.  A second byte is needed only after a symbol of frequency below 16: the warp tests for it with one vote.
-// The whole renormalisation is one asm block so that the rare branch updates the registers in place; with the branch in
-// C++ the compiler copies all eight of them on the common path (2 of 22 instructions per symbol).
+// a predicate.  A second byte is needed only after a symbol of frequency below 16: one test for the four streams, one
+// branch.  The whole renormalisation is one asm block so that the rare branch updates the registers in place; with the
+// branch in C++ the compiler copies all eight of them on the common path (2 of 22 instructions per symbol).  A warp vote in
+// front of the branch made the stand-alone decoder 3 % slower and the fused linear no faster.
 struct Quad {
     uint32_t s[4], p[4];                                        // states, shared addresses of the next bytes
 
@@ -173,8 +181,7 @@ struct Quad {
             "min.u32 m1, %2, %3;\n\t"
             "min.u32 m0, m0, m1;\n\t"
             "setp.lt.u32 r, m0, 65536;\n\t"
-            "vote.sync.any.pred r, r, 0xffffffff;\n\t"
-            "@!r bra.uni DONE;\n\t"
+            "@!r bra DONE;\n\t"
             "setp.lt.u32 p0, %0, 65536;\n\t"
             "setp.lt.u32 p1, %1, 65536;\n\t"
             "setp.lt.u32 p2, %2, 65536;\n\t"
@@ -205,6 +212,23 @@ struct Quad {
 __device__ __forceinline__ void sts_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
+
+// Every lane polls an mbarrier phase itself, bounded.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok = 0;
+    for (uint32_t it = 0; it < kWaitPolls && !ok; ++it) ok = mbar_try_wait(bar, parity);
+    return ok != 0;
+}
+
+// Sign+mantissa bytes on their way through a warp that decodes four segments (two tiles, both halves) at once: chunks of
+// kChunkRows rows of 32 bytes per segment, double buffered.  The segments of a chunk start 8 banks apart, so a row of
+// the warp's 128 columns is one conflict-free wavefront.
+constexpr uint32_t kChunkRows = 16;
+constexpr uint32_t kSegPitch = kChunkRows * 32 + 32;
+constexpr uint32_t kManBytes = 2 * 4 * kSegPitch;
+// Time of a round of units with w warps on a multiprocessor, us at 64 symbols per stream: measured for 11 to 16 warps;
+// a warp alone on its scheduler takes about twice the constant.
+inline double round_cost(uint32_t w) { return w < 5 ? 7.15 : 3.4 + 0.75 * w; }
 
 // Lane 0 polls an mbarrier phase, bounded; the verdict is broadcast to the warp.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
