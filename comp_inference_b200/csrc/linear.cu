@@ -453,6 +453,11 @@ using namespace ci;
 extern "C" {
 
 size_t ci_linear_workspace_bytes(uint32_t M, uint32_t n_out, uint32_t K, uint32_t tile_h) {
+    if (K == 0 && tile_h != 0) {                                // ci_linear_transposed
+        const size_t generic = workspace_bytes(M, n_out);
+        const size_t fast = (size_t)kTicketBytes * 4 + linear_t4_workspace_bytes(M, n_out, tile_h);
+        return generic > fast ? generic : fast;
+    }
     size_t small = workspace_bytes(M, n_out) + x_scratch_bytes(K);
     size_t big = (size_t)kTicketBytes * 4 + gemm_workspace_bytes(M, n_out, K, tile_h);    // prefill path, split-K partials
     return small > big ? small : big;
@@ -596,6 +601,15 @@ int ci_linear_transposed(const ci_tiled_weight *w, const uint16_t *d_x, int64_t 
     CI_REQUIRE(ldx >= (int64_t)w->N && ldy >= (int64_t)w->K, "row strides smaller than the row length");
     LinArgs a = base_args(w);
     CI_REQUIRE(a.g.tiles_k <= kTicketBytes, "too many row tiles for the ticket area");
+    cudaStream_t s = (cudaStream_t)stream;
+    a.bias = d_bias; a.ldx = ldx; a.ldy = ldy;
+    if (d_ws != nullptr && ws_bytes > (size_t)kTicketBytes * 4) {
+        a.tickets = reinterpret_cast<uint32_t *>(d_ws);
+        a.partial = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(d_ws) + kTicketBytes * 4);
+        a.x = d_x; a.y = d_y; a.M = M;
+        rc = launch_linear_t4(a, w->max_tile_len, ws_bytes - (size_t)kTicketBytes * 4, s);
+        if (rc <= 0) return rc;                                 // launched, or an error; 1: not its kind of weight
+    }
     // rows per pass limited by the per-warp shared-memory accumulators: tile_h * MT floats <= 4 KB
     uint32_t mt_cap = a.g.th <= 256 ? 4 : (a.g.th <= 512 ? 2 : 1);
     CI_REQUIRE(a.g.th <= 1024, "tile height %u above 1024 is not supported by the transposed linear", a.g.th);
@@ -616,8 +630,6 @@ int ci_linear_transposed(const ci_tiled_weight *w, const uint16_t *d_x, int64_t 
     }
     a.tickets = reinterpret_cast<uint32_t *>(d_ws);
     a.partial = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(d_ws) + kTicketBytes * 4);
-    a.bias = d_bias; a.ldx = ldx; a.ldy = ldy;
-    cudaStream_t s = (cudaStream_t)stream;
     for (uint32_t m0 = 0; m0 < M; m0 += mt_cap) {
         uint32_t mc = M - m0 < mt_cap ? M - m0 : mt_cap;
         a.x = d_x + (size_t)m0 * ldx;

@@ -131,6 +131,10 @@ int launch_linear_mma(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s);
 // Register-direct variant for 32-wide tiles and K a multiple of the tile height (linear_mma4.cu).
 int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s);
 
+// Transposed weight, 32-wide tiles (linear_t4.cu); same return convention.
+int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_capacity, cudaStream_t s);
+size_t linear_t4_workspace_bytes(uint32_t M, uint32_t V, uint32_t th);
+
 // tcgen05 decode-GEMM for many activation rows (gemm_sm100.cu); same return convention.
 // partial_capacity = bytes available behind a.partial for split-K partial sums.
 int launch_linear_gemm(const LinArgs &a, uint32_t max_tile_len, size_t partial_capacity, uint32_t split_k,

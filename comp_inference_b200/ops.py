@@ -89,7 +89,7 @@ def _linear_call(w, x2, M, n_out, bias, out, split_k, transposed):
     y = out.view(M, n_out) if out is not None else torch.empty((M, n_out), device=dev, dtype=torch.bfloat16)
     if y.dtype != torch.bfloat16 or y.stride(1) != 1:
         raise RuntimeError("out must be a bfloat16 tensor with unit inner stride")
-    nbytes = lib.ci_linear_workspace_bytes(M, n_out, 0 if transposed else w.K, 0 if transposed else w.tile_h)
+    nbytes = lib.ci_linear_workspace_bytes(M, n_out, 0 if transposed else w.K, w.tile_h)
     if M > 16 and not transposed and split_k > 1:               # an explicit split-K of the prefill GEMM: room for its partials
         nbytes = max(nbytes, (1 << 14) + min(int(split_k), 8) * M * n_out * 4)
     ws = _lib.workspace(dev, nbytes)
@@ -129,7 +129,7 @@ def fused_rans_linear_transposed_triton(x, compressed_data, initial_states, tabl
     x2 = _check_x(x, H)
     M = x2.shape[0]
     w, keep = _lib.tiled_weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens,
-                                mantissas, V, H, int(tile_k), int(tile_n))
+                                mantissas, V, H, int(tile_k), int(tile_n), want_max=True)
     y = _linear_call(w, x2, M, V, bias, out, 0, True)
     return out if out is not None else y.view(*x.shape[:-1], V)
 

@@ -226,7 +226,8 @@ int ci_decode_bf16_dense(const ci_dense_weight *w, uint16_t *d_out, ci_stream_t 
 /* ---- fused consumers ---------------------------------------------------- */
 
 /* Bytes of workspace ci_linear / ci_linear_transposed need for M activation
- * rows and n_out output features (0 is a valid answer). */
+ * rows and n_out output features (0 is a valid answer).  ci_linear: K and tile_h of the weight; ci_linear_transposed:
+ * K = 0 and tile_h of the weight (without tile_h the call still runs, on its slower kernel). */
 size_t ci_linear_workspace_bytes(uint32_t M, uint32_t n_out, uint32_t K, uint32_t tile_h);
 
 /* y[M,N] = x[M,K] . W[K,N] (+ bias[N]), W decoded on the fly and never written

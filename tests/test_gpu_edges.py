@@ -60,3 +60,38 @@ def test_one_pass_encoder_matches_oracle(K, N, th, kind):
     r = ci.ccore.RansManager().compress_tiled(plane, c["exponent_freqs"], c["exponent_cdf"], th, 32)
     assert torch.equal(r.stream, c["rans_exp_stream"].cpu()) and torch.equal(r.output_sizes.view(torch.int32),
                                                                             c["output_sizes"].cpu().view(torch.int32))
+
+
+# stored-transposed linear: rows that end inside a tile / a group of four tiles, a last column block that ends inside a
+# lane's quad, one and several passes over the activation rows, tall tiles (fewer sums fit), runs that cross groups
+@pytest.mark.parametrize("V,H,th,M", [(512, 64, 128, 1), (2000, 100, 128, 2), (1111, 33, 64, 3), (333, 250, 16, 8),
+                                      (5000, 128, 1024, 1), (4099, 96, 1024, 5), (777, 1030, 256, 9), (16000, 512, 128, 1),
+                                      (40, 16, 32, 17)])
+def test_transposed_linear_edges(V, H, th, M):
+    import comp_inference_b200 as ci
+    from comp_inference_b200 import _lib
+    W = _weight(V, H)
+    c = ci.compress_weight_cuda(W, th, 32)
+    x = torch.randn(M, H, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).cuda()
+    bias = torch.randn(V, generator=torch.Generator().manual_seed(V)).to(torch.bfloat16).cuda()
+    args = (c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"], c["rans_exp_slot_map"], (V, H),
+            c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"], c["tile_height"], c["tile_width"], c["rans_man_raw"])
+    y = ci.fused_rans_linear_transposed_triton(x, *args, bias=bias)
+    assert _close(y, x.float() @ W.float().t() + bias.float())
+    assert torch.equal(y, ci.fused_rans_linear_transposed_triton(x, *args, bias=bias))   # workspace left clean, same order
+    assert _lib.kernel_status(x.device) == 0
+
+
+# stand-alone decoder: a last tile row that is not whole, odd widths, tall tiles with one window, both planes
+@pytest.mark.parametrize("K,N,th", [(100, 64, 128), (2050, 96, 1024), (4096, 160, 1024), (1111, 77, 128), (513, 30, 256),
+                                    (48, 41, 16), (640, 2050, 64)])
+def test_decoder_edges(K, N, th):
+    import comp_inference_b200 as ci
+    W = _weight(K, N)
+    c = ci.compress_weight_cuda(W, th, 32)
+    args = (c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"], c["rans_exp_slot_map"])
+    tile = (c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"], c["tile_height"], c["tile_width"])
+    w = ci.rans_decompress_bf16(*args, (K, N), *tile, c["rans_man_raw"])
+    assert torch.equal(w.view(torch.int16), W.view(torch.int16))
+    plane = ci.rans_decomp_triton_tiled(*args, (K, N), *tile)
+    assert torch.equal(plane, ci.extract_exp_and_mantissa(W)[0])
