@@ -134,6 +134,23 @@ def load():
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native host extension (csrc/host.cpp), linked against the same library; raises RuntimeError if it is not there."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from .csrc import _ci_host
+        except ImportError as e:
+            raise RuntimeError("comp_inference_b200/csrc/_ci_host.so cannot be loaded: build it with "
+                               f"`python comp_inference_b200/csrc/build.py` ({e})") from None
+        _host = _ci_host
+    return _host
+
+
 def check(rc):
     if rc != 0:
         msg = load().ci_last_error().decode("utf-8", "replace")

@@ -1,0 +1,294 @@
+// Native host path of the calls a decode step makes once per layer: descriptor checks, workspace and decode-table
+// look-ups, output allocation and the launch, in one call from Python instead of some fifty interpreted steps and two
+// ctypes conversions.  Same checks and messages as the Python layer; anything rare (a workspace that has to grow, a table
+// that has to be prepared) is done by calling back into comp_inference_b200._lib, which stays the owner of those buffers.
+//
+// Measured, RansLinear.forward of a 512 x 4096 shard, one row, back to back: 25.5 us in Python, see the table in the
+// design notes for now; the kernel itself takes 5.6 us.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include <mutex>
+#include <unordered_map>
+
+#include "../../include/comp_inference_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = c10::optional<Tensor>;
+
+namespace {
+
+void check(int rc) {
+    if (rc != 0) throw std::runtime_error("comp_inference_b200: " + std::string(ci_last_error()) + " (code " + std::to_string(rc) + ")");
+}
+
+void require_cuda(const Tensor &t, const char *name) {
+    TORCH_CHECK(t.is_cuda(), name, " must be a CUDA tensor: this package has no CPU path");
+}
+
+py::object lib_attr(const char *name) { return py::module_::import("comp_inference_b200._lib").attr(name); }
+
+// Launches go to the current stream of the current device, as everywhere in this package.
+ci_stream_t stream() { return reinterpret_cast<ci_stream_t>(c10::cuda::getCurrentCUDAStream().stream()); }
+
+struct StreamKey {
+    int device;
+    void *stream;
+    bool operator==(const StreamKey &o) const { return device == o.device && stream == o.stream; }
+};
+struct StreamKeyHash {
+    size_t operator()(const StreamKey &k) const { return std::hash<void *>()(k.stream) * 31 + k.device; }
+};
+
+// Buffers owned by the Python layer, one per (device, stream), remembered here; a larger one is asked for when needed.
+// A remembered buffer stays valid: the Python layer never frees one it handed out.
+struct BufferCache {
+    std::mutex mutex;
+    std::unordered_map<StreamKey, Tensor, StreamKeyHash> map;
+
+    template <class Ask>
+    Tensor get(const Tensor &like, size_t bytes, Ask ask) {
+        const StreamKey key{(int)like.get_device(), stream()};
+        {
+            std::lock_guard<std::mutex> lock(mutex);
+            auto it = map.find(key);
+            if (it != map.end() && (size_t)it->second.nbytes() >= bytes) return it->second;
+        }
+        Tensor t = ask();
+        std::lock_guard<std::mutex> lock(mutex);
+        map[key] = t;
+        return t;
+    }
+};
+// never destroyed: at exit the allocator behind the tensors may be gone before them
+BufferCache &g_workspaces = *new BufferCache, &g_scratch = *new BufferCache;
+
+Tensor workspace(const Tensor &like, size_t bytes) {
+    return g_workspaces.get(like, bytes, [&] { return lib_attr("workspace")(like.device(), bytes).cast<Tensor>(); });
+}
+
+Tensor decode_scratch(const Tensor &like, int64_t K, int64_t N) {
+    Tensor t = g_scratch.get(like, (size_t)(K * N * 2), [&] {
+        return py::module_::import("comp_inference_b200.pytorch_runtime").attr("_decode_scratch")(like.device(), K, N).cast<Tensor>().view({-1});
+    });
+    return t.narrow(0, 0, K * N).view({K, N});
+}
+
+// The arrays of one compressed weight and its descriptor.
+struct Weight {
+    Tensor stream, states, tables, slot_map, offsets, lens, mantissa, lut;
+    ci_tiled_weight w;
+
+    bool matches(const Tensor &s, const Tensor &st, const Tensor &m, const Tensor &o, int64_t th, int64_t tw) const {
+        return s.data_ptr() == w.stream && st.data_ptr() == (const void *)w.states && m.data_ptr() == (const void *)w.mantissa &&
+               o.data_ptr() == (const void *)w.tile_offsets && (uint32_t)th == w.tile_h && (uint32_t)tw == w.tile_w;
+    }
+};
+
+Tensor as_u32(const Tensor &t, const char *name) {
+    require_cuda(t, name);
+    TORCH_CHECK(t.scalar_type() == at::kUInt32 || t.scalar_type() == at::kInt, name, " must be uint32 or int32, got torch.",
+                t.scalar_type());
+    return t.contiguous();
+}
+Tensor as_u8(const Tensor &t, const char *name) {
+    require_cuda(t, name);
+    TORCH_CHECK(t.scalar_type() == at::kByte, name, " must be uint8, got torch.", t.scalar_type());
+    return t.contiguous();
+}
+
+void fill(Weight &h, int64_t K, int64_t N, int64_t th, int64_t tw, uint32_t max_len) {
+    memset(&h.w, 0, sizeof h.w);
+    h.w.stream = (const uint8_t *)h.stream.data_ptr();
+    h.w.states = (const uint32_t *)h.states.data_ptr();
+    h.w.tables = (const uint32_t *)h.tables.data_ptr();
+    h.w.slot_map = (const uint8_t *)h.slot_map.data_ptr();
+    h.w.tile_offsets = (const uint32_t *)h.offsets.data_ptr();
+    h.w.tile_max_lens = (const uint32_t *)h.lens.data_ptr();
+    h.w.mantissa = h.mantissa.defined() ? (const uint8_t *)h.mantissa.data_ptr() : nullptr;
+    h.w.lut = h.lut.defined() ? (const uint32_t *)h.lut.data_ptr() : nullptr;
+    h.w.stream_len = (uint64_t)h.stream.numel();
+    h.w.K = (uint32_t)K;
+    h.w.N = (uint32_t)N;
+    h.w.tile_h = (uint32_t)th;
+    h.w.tile_w = (uint32_t)tw;
+    h.w.max_tile_len = max_len;
+}
+
+// What is derived from a weight's tables and depths (the prepared decode table, the deepest tile) is kept per tensor
+// objects, as in the Python layer: weak references, data pointers and versions tell whether an entry still holds.
+struct Ref {
+    c10::weak_intrusive_ptr<c10::TensorImpl> impl;
+    const void *data;
+    uint32_t version;
+    explicit Ref(const Tensor &t) : impl(t.getIntrusivePtr()), data(t.data_ptr()), version(t.is_inference() ? 0 : t._version()) {}
+    bool is(const Tensor &t) const {
+        return !impl.expired() && impl._unsafe_get_target() == t.unsafeGetTensorImpl() && data == t.data_ptr() &&
+               version == (t.is_inference() ? 0 : t._version());
+    }
+};
+struct Derived {
+    Ref tables, slot_map, lens;
+    Tensor lut;
+    uint32_t max_len;
+};
+std::mutex g_derived_mutex;
+std::unordered_map<const void *, Derived> &g_derived = *new std::unordered_map<const void *, Derived>;   // by tile_max_lens' impl
+
+Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables, const Tensor &slot_map, const Tensor &offsets,
+             const Tensor &lens, const OptTensor &mantissa, int64_t K, int64_t N, int64_t th, int64_t tw) {
+    Weight h;
+    h.stream = as_u8(stream_t, "compressed stream");
+    h.states = as_u32(states, "states");
+    h.tables = as_u32(tables, "tables");
+    h.slot_map = as_u8(slot_map, "slot_map");
+    h.offsets = as_u32(offsets, "tile_offsets");
+    h.lens = as_u32(lens, "tile_max_lens");
+    if (mantissa.has_value()) h.mantissa = as_u8(*mantissa, "mantissas");
+    if (th <= 0 || tw <= 0) throw py::value_error("tile sizes must be positive");
+    const int64_t tiles = ((K + th - 1) / th) * ((N + tw - 1) / tw);
+    if (h.states.numel() != tiles * 2 * tw)
+        throw py::value_error("Initial states size mismatch. Expected " + std::to_string(tiles * 2 * tw));
+    if (h.offsets.numel() != tiles || h.lens.numel() != tiles)
+        throw py::value_error("tile_offsets / tile_max_lens must have " + std::to_string(tiles) + " entries");
+    if (h.mantissa.defined() && h.mantissa.numel() < tiles * th * tw)
+        throw py::value_error("mantissa plane has " + std::to_string(h.mantissa.numel()) + " bytes, " +
+                              std::to_string(tiles * th * tw) + " expected");
+    uint32_t max_len = 0;
+    // a contiguous copy made above is a new object on every call: nothing to remember
+    if (h.tables.is_same(tables) && h.slot_map.is_same(slot_map) && h.lens.is_same(lens)) {
+        const void *key = lens.unsafeGetTensorImpl();
+        {
+            std::lock_guard<std::mutex> lock(g_derived_mutex);
+            auto it = g_derived.find(key);
+            if (it != g_derived.end() && it->second.lens.is(lens) && it->second.tables.is(tables) && it->second.slot_map.is(slot_map)) {
+                h.lut = it->second.lut;
+                max_len = it->second.max_len;
+            }
+        }
+        if (!h.lut.defined()) {
+            h.lut = lib_attr("prepared_lut")(tables, slot_map).cast<Tensor>();
+            max_len = lib_attr("max_tile_len")(lens).cast<uint32_t>();
+            std::lock_guard<std::mutex> lock(g_derived_mutex);
+            if (g_derived.size() > 4096) g_derived.clear();
+            g_derived.erase(key);
+            g_derived.emplace(key, Derived{Ref(tables), Ref(slot_map), Ref(lens), h.lut, max_len});
+        }
+    }
+    fill(h, K, N, th, tw, max_len);
+    return h;
+}
+
+// Activations as rows of K bf16 with unit stride, without touching a tensor that already is that.
+struct Rows {
+    Tensor keep;
+    const uint16_t *ptr;
+    int64_t ld, M;
+};
+Rows rows_of(const Tensor &x, int64_t K) {
+    TORCH_CHECK(x.scalar_type() == at::kBFloat16, "activations must be bfloat16, got torch.", x.scalar_type());
+    require_cuda(x, "x");
+    Rows r;
+    if (x.dim() >= 1 && x.size(-1) == K && x.is_contiguous()) {
+        r.keep = x;
+        r.ld = K;
+        r.M = x.numel() / K;
+    } else {
+        r.keep = x.reshape({-1, K});
+        if (r.keep.stride(1) != 1) r.keep = r.keep.contiguous();
+        r.ld = r.keep.stride(0);
+        r.M = r.keep.size(0);
+        if (r.M <= 1) r.ld = K;                                 // the stride of a single row means nothing
+    }
+    r.ptr = (const uint16_t *)r.keep.data_ptr();
+    return r;
+}
+
+std::vector<int64_t> out_shape(const Tensor &x, int64_t n) {
+    std::vector<int64_t> s(x.sizes().begin(), x.sizes().end());
+    if (s.empty()) s.push_back(n); else s.back() = n;
+    return s;
+}
+
+Tensor linear_call(const Weight &h, const Tensor &x, const OptTensor &bias, const OptTensor &out, int64_t split_k, bool transposed,
+                   int64_t prefill_rows) {
+    const int64_t K = transposed ? h.w.N : h.w.K, n_out = transposed ? h.w.K : h.w.N;
+    const Rows r = rows_of(x, K);
+    if (prefill_rows > 0 && r.M >= prefill_rows && !out.has_value()) {
+        // many rows: one stand-alone decode into a reused buffer, then a library GEMM (see RansLinear)
+        Tensor w = decode_scratch(x, h.w.K, h.w.N);
+        check(ci_decode_bf16(&h.w, (uint16_t *)w.data_ptr(), stream()));
+        Tensor x2 = r.keep.dim() == 2 ? r.keep : r.keep.view({r.M, K});
+        Tensor y = at::matmul(x2, transposed ? w.t() : w);
+        if (bias.has_value()) y.add_(*bias);
+        return y.view(out_shape(x, n_out));
+    }
+    Tensor y;
+    if (out.has_value()) {
+        y = out->view({r.M, n_out});
+        TORCH_CHECK(y.scalar_type() == at::kBFloat16 && y.stride(1) == 1, "out must be a bfloat16 tensor with unit inner stride");
+    } else {
+        y = at::empty(out_shape(x, n_out), x.options());
+        TORCH_CHECK(y.numel() == r.M * n_out, "activations of ", x.sizes(), " do not have ", K, " columns");
+    }
+    const uint16_t *b = nullptr;
+    Tensor keep_bias;
+    if (bias.has_value()) {
+        TORCH_CHECK(bias->scalar_type() == at::kBFloat16 && bias->numel() == n_out,
+                    "bias must be bfloat16 with one entry per output feature");
+        keep_bias = bias->contiguous();
+        b = (const uint16_t *)keep_bias.data_ptr();
+    }
+    size_t bytes = ci_linear_workspace_bytes((uint32_t)r.M, (uint32_t)n_out, transposed ? 0 : h.w.K, h.w.tile_h);
+    if (r.M > 16 && !transposed && split_k > 1)                 // an explicit split-K of the prefill GEMM: room for its partials
+        bytes = std::max(bytes, (size_t)(1 << 14) + (size_t)std::min<int64_t>(split_k, 8) * r.M * n_out * 4);
+    const Tensor ws = workspace(x, bytes);
+    const int64_t ldy = out.has_value() ? y.stride(0) : n_out;
+    check(transposed ? ci_linear_transposed(&h.w, r.ptr, r.ld, (uint32_t)r.M, b, (uint16_t *)y.data_ptr(), ldy, ws.data_ptr(),
+                                            ws.nbytes(), stream())
+                     : ci_linear(&h.w, r.ptr, r.ld, (uint32_t)r.M, b, (uint16_t *)y.data_ptr(), ldy, ws.data_ptr(), ws.nbytes(),
+                                 (uint32_t)split_k, stream()));
+    return out.has_value() ? *out : y;
+}
+
+Tensor embedding_call(const Weight &h, const Tensor &x, const OptTensor &out) {
+    require_cuda(x, "x");
+    const Tensor ids = x.to(at::kLong).contiguous();
+    const int64_t n = ids.numel(), N = h.w.N;
+    std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+    shape.push_back(N);
+    Tensor o;
+    int64_t ld = N;
+    if (out.has_value()) {
+        o = out->view({n, N});
+        TORCH_CHECK(o.scalar_type() == at::kBFloat16 && (n == 0 || o.stride(1) == 1),
+                    "out must be a bfloat16 tensor with unit inner stride");
+        if (n > 0) ld = o.stride(0);
+    } else {
+        o = at::empty(shape, x.options().dtype(at::kBFloat16));
+    }
+    check(ci_embedding(&h.w, (const int64_t *)ids.data_ptr(), (uint64_t)n, (uint16_t *)o.data_ptr(), ld, stream()));
+    return o.view(shape);
+}
+
+Tensor decode_call(const Weight &h, bool bf16) {
+    Tensor o = at::empty({h.w.K, h.w.N}, h.stream.options().dtype(bf16 ? at::kBFloat16 : at::kByte));
+    check(bf16 ? ci_decode_bf16(&h.w, (uint16_t *)o.data_ptr(), stream()) : ci_decode_plane(&h.w, (uint8_t *)o.data_ptr(), stream()));
+    return o;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_ci_host, m) {
+    py::class_<Weight>(m, "Weight", "Descriptor of a compressed weight and the tensors it points into")
+        .def(py::init(&tiled), py::arg("stream"), py::arg("states"), py::arg("tables"), py::arg("slot_map"), py::arg("tile_offsets"),
+             py::arg("tile_max_lens"), py::arg("mantissas"), py::arg("K"), py::arg("N"), py::arg("tile_h"), py::arg("tile_w"))
+        .def("matches", &Weight::matches)
+        .def("linear", &linear_call, py::arg("x"), py::arg("bias") = py::none(), py::arg("out") = py::none(), py::arg("split_k") = 0,
+             py::arg("transposed") = false, py::arg("prefill_rows") = 0)
+        .def("embedding", &embedding_call, py::arg("x"), py::arg("out") = py::none())
+        .def("decode", &decode_call, py::arg("bf16"));
+}

@@ -105,7 +105,8 @@ __device__ __forceinline__ void group4(uint32_t (&b)[4][2], Quad &z, uint32_t lu
 // Every lane still runs the full warp-wide loop.  A lane whose segment has n_my < n_groups 4-row groups reads
 // zeros instead of activations from group n_my on, and -- so that what it multiplies by those zeros stays a
 // finite number -- starts its stream over whenever it has used it up (a lane without a segment decodes the top
-// half of the upper tile, which always exists).  Its products are exact zeros.
+// half of the upper tile, which always exists).  Its products are exact zeros.  Where K ends inside a group of four, the
+// weights decoded past the end of the stream are masked to zero (the activations there are zero already).
 __device__ __align__(16) uint16_t g_zero_activations[256];     // 64 per unit are read, 8 more are prefetched
 template <bool HI, bool RAGGED>
 __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid_constant__ Mma4Args p) {
@@ -413,15 +414,18 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
         }
         // Blocks of this lane's segment that exist (n_my) and of the stream it decodes (len); see the kernel's header.
         uint32_t n_my = n_blocks, len = n_blocks;
+        uint32_t cut = 0;                                       // rows of the stream's last group, 0 = all four
         uint32_t tsel_d = tsel, hsel_d = hsel;                  // the segment whose stream this lane decodes
         if (RAGGED && pk == ragged_pk) {
             const uint32_t r0 = (2 * pk + tsel) * g.th;
             const uint32_t rows_t = r0 < g.K ? min(g.th, g.K - r0) : 0u;
             const uint32_t seg = rows_t > hsel * g.half ? min(g.half, rows_t - hsel * g.half) : 0u;
-            n_my = len = seg >> 2;
+            n_my = len = (seg + 3) >> 2;
+            cut = seg & 3;
             if (seg == 0) {                                     // nothing of its own: the upper tile's top half stands in
                 tsel_d = hsel_d = 0;
-                len = min(g.half, g.K - 2 * pk * g.th) >> 2;
+                len = (min(g.half, g.K - 2 * pk * g.th) + 3) >> 2;
+                cut = min(g.half, g.K - 2 * pk * g.th) & 3;
             }
         }
         const uint32_t krow = (2 * pk + tsel) * g.th + hsel * g.half;
@@ -485,6 +489,15 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
                 // converged and drops the divergence checks (and the register copies they need) of the votes.
                 mma4<HI>(acc, wb, xf);
                 group4(wb, z, lut_s, m);
+                if constexpr (RAGGED) {
+                    if (cut != 0 && left == 1) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            wb[i][0] &= cut == 1 ? 0xFFFFu : 0xFFFFFFFFu;
+                            wb[i][1] &= cut == 3 ? 0xFFFFu : 0u;
+                        }
+                    }
+                }
                 xf[0] = v0.x; xf[1] = v0.y; xf[2] = v1.x; xf[3] = v1.y;
                 ms += 128;
                 xp0 += xs;
@@ -514,30 +527,42 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     flush(cur_grp);
 }
 
-// x[M][K] -> scratch[K / 4][M][4].  A warp's activation load reads four consecutive k of every row: from rows K elements
+// x[M][K] -> scratch[ceil(K / 4)][M][4], zeros beyond K.  A warp's activation load reads four consecutive k of every row: from rows K elements
 // apart that is a cache line, and a wavefront of the load pipe, per row and segment (32 a load for 8 rows, 60 % of the
 // kernel's pipe time at 16 rows); in this order a segment's rows are neighbours.
-__global__ void __launch_bounds__(256) k_interleave_x(const uint16_t *__restrict__ x, int64_t ldx, uint32_t M, uint32_t quads,
-                                                      uint2 *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_interleave_x(const uint16_t *__restrict__ x, int64_t ldx, uint32_t M, uint32_t K,
+                                                      uint32_t aligned, uint2 *__restrict__ out) {
     asm volatile("griddepcontrol.wait;" ::: "memory");          // the activations may be the previous kernel's product
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t k4 = blockIdx.x * 256 + threadIdx.x;
-    if (k4 >= quads) return;
-    for (uint32_t m = blockIdx.y; m < M; m += gridDim.y)
-        out[(size_t)k4 * M + m] = __ldg(reinterpret_cast<const uint2 *>(x + (size_t)m * ldx) + k4);
+    if (4 * k4 >= K) return;
+    for (uint32_t m = blockIdx.y; m < M; m += gridDim.y) {
+        const uint16_t *src = x + (size_t)m * ldx + 4 * k4;
+        uint2 v = make_uint2(0u, 0u);
+        if (aligned) {
+            v = __ldg(reinterpret_cast<const uint2 *>(src));
+        } else {
+            const uint32_t n = K - 4 * k4;
+            v.x = __ldg(src) | (n > 1 ? (uint32_t)__ldg(src + 1) << 16 : 0u);
+            v.y = (n > 2 ? (uint32_t)__ldg(src + 2) : 0u) | (n > 3 ? (uint32_t)__ldg(src + 3) << 16 : 0u);
+        }
+        out[(size_t)k4 * M + m] = v;
+    }
 }
 
 // ------------------------------------------------------------------------ host
 
 int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) {
     const Geom &g = a.g;
-    // 16-symbol-aligned streams; K a multiple of 8 (the loop decodes and multiplies two groups of four rows per
-    // pass); the last pair of tile rows may lack its lower tile and either tile may be short
-    if (g.tw != 32 || g.th % 16 != 0 || g.K % 8 != 0 || a.M > 16 || max_tile_len == 0) return 1;
+    // 16-symbol-aligned streams; the last pair of tile rows may lack its lower tile and either tile may be short
+    if (g.tw != 32 || g.th % 16 != 0 || a.M > 16 || max_tile_len == 0) return 1;
     if ((reinterpret_cast<uintptr_t>(a.stream) & 15u) || (reinterpret_cast<uintptr_t>(a.mantissa) & 15u) ||
         (reinterpret_cast<uintptr_t>(a.states) & 15u))
         return 1;
-    if ((reinterpret_cast<uintptr_t>(a.x) & 7u) || (a.ldx & 3)) return 1;      // activations are read as 8-byte quads
+    // activations are read as 8-byte quads: where they are not that, the reordering kernel makes them so
+    const bool quads_ok = (reinterpret_cast<uintptr_t>(a.x) & 7u) == 0 && (a.ldx & 3) == 0 && g.K % 4 == 0;
+    if (!quads_ok && a.x_scratch == nullptr && !a.dry_run) return 1;
+    if (!quads_ok && a.ar.world > 1) return 1;                  // every rank has to take the same kernel: only plain cases
     int dev = 0, max_smem = 0;
     CI_CUDA(cudaGetDevice(&dev));
     CI_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -600,11 +625,11 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     cfg.numAttrs = 1;
     // The extra launch takes 2.7 us and saves about 1.7e-8 us per activation row and weight, where the multiprocessors are
     // busy at all: it pays from 1.6e8 of them (4096 x 22016: 119 -> 90 us at 16 rows, 94 -> 85 at 8, 87 -> 85 at 4).
-    if (a.x_scratch != nullptr && a.M >= 3 && p.total >= 6 * P && (uint64_t)a.M * g.K * g.N >= 160000000ull) {
-        const uint32_t quads = g.K / 4;
-        cfg.gridDim = dim3((quads + 255) / 256, a.M);
+    if (!quads_ok || (a.x_scratch != nullptr && a.M >= 3 && p.total >= 6 * P && (uint64_t)a.M * g.K * g.N >= 160000000ull)) {
+        cfg.gridDim = dim3((g.K / 4 + 256) / 256, a.M);
         cfg.blockDim = dim3(256);
-        CI_CUDA(cudaLaunchKernelEx(&cfg, k_interleave_x, a.x, a.ldx, a.M, quads, reinterpret_cast<uint2 *>(a.x_scratch)));
+        CI_CUDA(cudaLaunchKernelEx(&cfg, k_interleave_x, a.x, a.ldx, a.M, g.K, (uint32_t)quads_ok,
+                                   reinterpret_cast<uint2 *>(a.x_scratch)));
         p.a.x = a.x_scratch;
         p.a.ldx = 4;
         p.x_step = 4 * a.M;

@@ -41,12 +41,8 @@ def _bias(bias, n):
 def rans_decomp_triton_tiled(compressed_streams, initial_states, tables, slot_map, output_shape, tile_offsets,
                              tile_max_lens, tile_k=1024, tile_n=32):
     """Exponent plane uint8 [K,N] of a tiled stream."""
-    K, N = int(output_shape[0]), int(output_shape[1])
-    w, keep = _lib.tiled_weight(compressed_streams, initial_states, tables, slot_map, tile_offsets, tile_max_lens,
-                                None, K, N, int(tile_k), int(tile_n), want_max=True)
-    out = torch.empty((K, N), device=compressed_streams.device, dtype=torch.uint8)
-    _lib.check(_lib.load().ci_decode_plane(w, _lib.ptr(out), _lib.stream()))
-    return out
+    return _lib.host().Weight(compressed_streams, initial_states, tables, slot_map, tile_offsets, tile_max_lens, None,
+                              int(output_shape[0]), int(output_shape[1]), int(tile_k), int(tile_n)).decode(False)
 
 
 def rans_decomp_triton(compressed_streams, initial_states, tables, slot_map, stream_sizes, output_shape):
@@ -75,12 +71,8 @@ def rans_decompress_bf16(compressed_streams, initial_states, tables, slot_map, w
                          tile_max_lens, tile_k, tile_n, mantissas):
     """Whole weight as bfloat16 [K,N] in one kernel: the decode + uninterleave + reconstruct
     chain of rans_decompress_module_weight_bf16 (comp_inference/comp_inference.py:633-711)."""
-    K, N = int(weight_shape[0]), int(weight_shape[1])
-    w, keep = _lib.tiled_weight(compressed_streams, initial_states, tables, slot_map, tile_offsets, tile_max_lens,
-                                mantissas, K, N, int(tile_k), int(tile_n), want_max=True)
-    out = torch.empty((K, N), device=compressed_streams.device, dtype=torch.bfloat16)
-    _lib.check(_lib.load().ci_decode_bf16(w, _lib.ptr(out), _lib.stream()))
-    return out
+    return _lib.host().Weight(compressed_streams, initial_states, tables, slot_map, tile_offsets, tile_max_lens, mantissas,
+                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n)).decode(True)
 
 
 def _linear_call(w, x2, M, n_out, bias, out, split_k, transposed):
@@ -112,42 +104,25 @@ def fused_rans_linear_triton(x, compressed_data, initial_states, tables, slot_ma
     and split-K partials live in this package's own fp32 workspace (the reference's is a bf16 buffer
     of another size).  ``SPLIT_K`` is honoured up to 16; 0 lets the library choose.
     """
-    K, N = int(weight_shape[0]), int(weight_shape[1])
-    x2 = _check_x(x, K)
-    M = x2.shape[0]
-    w, keep = _lib.tiled_weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens,
-                                mantissas, K, N, int(tile_k), int(tile_n), want_max=True)
-    y = _linear_call(w, x2, M, N, bias, out, SPLIT_K, False)
-    return out if out is not None else y.view(*x.shape[:-1], N)
+    return _lib.host().Weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens, mantissas,
+                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n)).linear(
+        x, bias, out, int(SPLIT_K))
 
 
 def fused_rans_linear_transposed_triton(x, compressed_data, initial_states, tables, slot_map, weight_shape,
                                         tile_offsets, tile_max_lens, tile_k, tile_n, mantissas, workspace=None,
                                         bias=None, out=None, SPLIT_K=8):
     """y[..., V] = x[..., H] . W[V, H]^T for a weight stored [V, H] (LM head / tied embedding)."""
-    V, H = int(weight_shape[0]), int(weight_shape[1])
-    x2 = _check_x(x, H)
-    M = x2.shape[0]
-    w, keep = _lib.tiled_weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens,
-                                mantissas, V, H, int(tile_k), int(tile_n), want_max=True)
-    y = _linear_call(w, x2, M, V, bias, out, 0, True)
-    return out if out is not None else y.view(*x.shape[:-1], V)
+    return _lib.host().Weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens, mantissas,
+                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n)).linear(
+        x, bias, out, 0, True)
 
 
 def fused_rans_embedding_triton(x, compressed_data, initial_states, tables, slot_map, weight_shape, tile_offsets,
                                 tile_max_lens, tile_k, tile_n, mantissas, out=None):
     """out[..., :] = W[x[...], :]; ids outside [0, K) give zero rows."""
-    K, N = int(weight_shape[0]), int(weight_shape[1])
-    _lib.require_cuda(x, "x")
-    ids = x.reshape(-1).to(torch.int64).contiguous()
-    n = ids.numel()
-    w, keep = _lib.tiled_weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens,
-                                mantissas, K, N, int(tile_k), int(tile_n), want_max=True)
-    o = out.view(n, N) if out is not None else torch.empty((n, N), device=x.device, dtype=torch.bfloat16)
-    if o.dtype != torch.bfloat16 or (n > 0 and o.stride(1) != 1):
-        raise RuntimeError("out must be a bfloat16 tensor with unit inner stride")
-    _lib.check(_lib.load().ci_embedding(w, _lib.ptr(ids), n, _lib.ptr(o), o.stride(0) if n else N, _lib.stream()))
-    return o.view(*x.shape, N)
+    return _lib.host().Weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens, mantissas,
+                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n)).embedding(x, out)
 
 
 # ---- dense ("uncoalesced") layout ------------------------------------------------

@@ -58,6 +58,7 @@ class _RansBase(nn.Module):
         before a CUDA graph is captured.  Subclasses add their own one-time work."""
         if self.rans_exp_stream.is_cuda and self.rans_exp_states.numel():
             self._weight(*self._stored_shape())
+            self._native()
         return self
 
     _handle = None
@@ -74,6 +75,19 @@ class _RansBase(nn.Module):
                                         int(self.tile_n), want_max=True)
             self._handle = (key, w, keep)
         return self._handle[1]
+
+    _native_handle = None
+
+    def _native(self):
+        """The same descriptor for the native host path (_lib.host()); rebuilt only if a buffer was replaced."""
+        b, h = self._buffers, self._native_handle
+        if h is None or not h.matches(b["rans_exp_stream"], b["rans_exp_states"], b["rans_man_raw"],
+                                      b["rans_exp_tile_offsets"], self.tile_k, self.tile_n):
+            h = _lib.host().Weight(b["rans_exp_stream"], b["rans_exp_states"], b["rans_exp_tables"], b["rans_exp_slot_map"],
+                                   b["rans_exp_tile_offsets"], b["rans_exp_tile_max_lens"], b["rans_man_raw"],
+                                   *self._stored_shape(), int(self.tile_k), int(self.tile_n))
+            self.__dict__["_native_handle"] = h
+        return h
 
 
 _scratch = {}
@@ -92,19 +106,6 @@ def _decode_scratch(device, K, N):
         buf = torch.empty(K * N, dtype=torch.bfloat16, device=device)
         _scratch[key] = buf
     return buf[:K * N].view(K, N)
-
-
-def _decode_then_gemm(w_desc, K, N, x2, bias=None, transposed=False):
-    """x2 [M, K] times the compressed weight behind ``w_desc``: one stand-alone decode into the device's scratch
-    buffer, then a library GEMM.  ``transposed``: the weight is stored [N, K] (the LM head's stored layout) and
-    the GEMM reads it as its transpose."""
-    rows, cols = (N, K) if transposed else (K, N)
-    w = _decode_scratch(x2.device, rows, cols)
-    _lib.check(_lib.load().ci_decode_bf16(w_desc, _lib.ptr(w), _lib.stream()))
-    y = torch.matmul(x2, w.t() if transposed else w)
-    if bias is not None:
-        y += bias
-    return y
 
 
 class RansLinear(_RansBase):
@@ -139,13 +140,9 @@ class RansLinear(_RansBase):
         return self.in_features, self.out_features
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        K, N = self.in_features, self.out_features
-        x2 = ops._check_x(x, K)
-        if self.prefill_policy != "fused" and x2.shape[0] >= max(self.prefill_rows, 17):
-            return _decode_then_gemm(self._weight(K, N), K, N, x2, self.bias).view(*x.shape[:-1], N)
-        y = ops._linear_call(self._weight(K, N), x2, x2.shape[0], N, self.bias, None,
-                             self.split_k if self.split_k > 1 else 0, False)
-        return y.view(*x.shape[:-1], N)
+        # up to 16 rows the fused kernels; more: stand-alone decode + library GEMM, or the fused decode-GEMM
+        return self._native().linear(x, self.bias, None, self.split_k if self.split_k > 1 else 0, False,
+                                     0 if self.prefill_policy == "fused" else max(self.prefill_rows, 17))
 
 
 class RansFusedLinear(RansLinear):
@@ -235,22 +232,18 @@ class RansLMHead(_RansBase):
                                         c["rans_exp_slot_map"], c["rans_exp_tile_offsets"],
                                         c["rans_exp_tile_max_lens"], c["rans_man_raw"], H, V, int(c["tile_height"]),
                                         int(c["tile_width"]), want_max=True)
-            self._twin = (key, w, keep, c)
+            native = _lib.host().Weight(c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"],
+                                        c["rans_exp_slot_map"], c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"],
+                                        c["rans_man_raw"], H, V, int(c["tile_height"]), int(c["tile_width"]))
+            self._twin = (key, w, keep, c, native)
         return self._twin[1]
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        V, H = self.out_features, self.in_features
-        x2 = ops._check_x(x, H)
-        if self.prefill_policy != "fused" and x2.shape[0] >= max(self.prefill_rows, 17):   # logits of a whole prompt
-            if self.fast_twin:
-                y = _decode_then_gemm(self._twin_weight(), H, V, x2)
-            else:
-                y = _decode_then_gemm(self._weight(V, H), H, V, x2, transposed=True)
-        elif self.fast_twin:
-            y = ops._linear_call(self._twin_weight(), x2, x2.shape[0], V, None, None, 0, False)
-        else:
-            y = ops._linear_call(self._weight(V, H), x2, x2.shape[0], V, None, None, 0, True)
-        return y.view(*x.shape[:-1], V)
+        rows = 0 if self.prefill_policy == "fused" else max(self.prefill_rows, 17)   # from here on: logits of a whole prompt
+        if self.fast_twin:
+            self._twin_weight()
+            return self._twin[4].linear(x, None, None, 0, False, rows)
+        return self._native().linear(x, None, None, 0, True, rows)
 
 
 class RansEmbedding(_RansBase):
@@ -266,12 +259,7 @@ class RansEmbedding(_RansBase):
         return self.num_embeddings, self.embedding_dim
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        V, H = self.num_embeddings, self.embedding_dim
-        ids = _lib.require_cuda(x, "x").reshape(-1).to(torch.int64).contiguous()
-        out = torch.empty((ids.numel(), H), device=x.device, dtype=torch.bfloat16)
-        _lib.check(_lib.load().ci_embedding(self._weight(V, H), _lib.ptr(ids), ids.numel(), _lib.ptr(out), H,
-                                            _lib.stream()))
-        return out.view(*x.shape, H)
+        return self._native().embedding(x)
 
 
 def prepare_model(model):
@@ -512,10 +500,10 @@ class RansVocabParallelLMHead(nn.Module):
         del w, sub
         self._c = ci_mod.compress_weight_cuda(mine, *twin_tile)
         del mine
-        self._w, self._keep = _lib.tiled_weight(
-            self._c["rans_exp_stream"], self._c["rans_exp_states"], self._c["rans_exp_tables"],
-            self._c["rans_exp_slot_map"], self._c["rans_exp_tile_offsets"], self._c["rans_exp_tile_max_lens"],
-            self._c["rans_man_raw"], H, per, int(self._c["tile_height"]), int(self._c["tile_width"]), want_max=True)
+        self._w = _lib.host().Weight(
+            self._c["rans_exp_stream"], self._c["rans_exp_states"], self._c["rans_exp_tables"], self._c["rans_exp_slot_map"],
+            self._c["rans_exp_tile_offsets"], self._c["rans_exp_tile_max_lens"], self._c["rans_man_raw"], H, per,
+            int(self._c["tile_height"]), int(self._c["tile_width"]))
         self.per_rank = per
 
     def prepare(self):
@@ -526,10 +514,7 @@ class RansVocabParallelLMHead(nn.Module):
         H, V = self.in_features, self.out_features
         x2 = ops._check_x(x, H)
         M = x2.shape[0]
-        if M >= 17:                                             # a whole prompt: decode once, library GEMM
-            y = _decode_then_gemm(self._w, H, self.per_rank, x2)
-        else:
-            y = ops._linear_call(self._w, x2, M, self.per_rank, None, None, 0, False)
+        y = self._w.linear(x2, None, None, 0, False, 17)         # a whole prompt: decode once, library GEMM
         if self.gather is not None:
             full = self.gather(y)
         else:

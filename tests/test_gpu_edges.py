@@ -19,7 +19,10 @@ def _close(y, ref, tol=1e-2):
 # twice / once per warp; many units per multiprocessor with 9..16 rows: activations reordered first
 @pytest.mark.parametrize("K,N,th,M", [(1024, 256, 512, 1), (1536, 96, 512, 3), (2056, 64, 1024, 2), (3000, 96, 1024, 16),
                                       (4096, 64, 1024, 9), (768, 2048, 256, 1), (600, 132, 512, 5),
-                                      (2048, 8192, 128, 16), (2056, 8196, 128, 11), (4096, 8192, 64, 5)])
+                                      (2048, 8192, 128, 16), (2056, 8196, 128, 11), (4096, 8192, 64, 5),
+                                      # K ends inside a group of four rows, in every quarter of a pair of tiles
+                                      (2050, 4096, 128, 1), (2113, 4099, 128, 4), (2177, 4097, 128, 2), (2247, 4096, 128, 16),
+                                      (1027, 64, 1024, 1), (1537, 32, 1024, 3), (3070, 40, 1024, 9), (4095, 64, 512, 1)])
 @pytest.mark.parametrize("split_k", [0, 8])
 def test_linear_dispatch_edges(K, N, th, M, split_k):
     import comp_inference_b200 as ci
