@@ -22,7 +22,7 @@
 namespace ci {
 
 constexpr uint32_t kDec4Warps = 16;
-constexpr uint32_t kDec4BarBytes = 512;      // up to 16 warps x (2 window stages + 2 mantissa chunks) x 8 B
+constexpr uint32_t kDec4BarBytes = 640;      // up to 16 warps x (2 window stages + 2 mantissa chunks) x 8 B
 
 struct Dec4Args {
     DecArgs a;
@@ -46,6 +46,8 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     // (state << 2 & 0x3FFC) | base, without an addition.
     const uint32_t lut_s = (smem_s + kLutBytes - 1) & ~(kLutBytes - 1);
     uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + (lut_s - smem_s));
+    const uint32_t lut_bar = lut_s + kLutBytes + kDec4BarBytes - 16;
+    start_lut(lut_s, lut_bar, a.lut);
     const uint32_t man_s = lut_s + kLutBytes + kDec4BarBytes + (BF16 ? warp * kManBytes : 0);
     const uint32_t wbase_s = lut_s + kLutBytes + kDec4BarBytes + (BF16 ? W * kManBytes : 0) + warp * p.stages * p.stage_bytes;
     const uint32_t bar_base = lut_s + kLutBytes + warp * 32, man_bar = bar_base + 16;
@@ -82,10 +84,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         }
     };
 
-    auto issue = [&](uint32_t u, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
-        uint32_t tk, tp, t0;
-        bool two;
-        unit_tiles(u, tk, tp, t0, two);
+    auto issue = [&](uint32_t t0, bool two, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
         const uint32_t bar = bar_base + stage * 8;
         const uint32_t dst = wbase_s + stage * p.stage_bytes;
         if (ml0 > p.cap_rows || ml1 > p.cap_rows) ml0 = ml1 = 0;   // metadata disagrees with the declared maximum
@@ -99,11 +98,9 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         for (uint32_t i = lane; i < ml1 * 4; i += 32) cp_async16(dst + (i >> 2) * 128 + 64 + (i & 3) * 16, s1 + i * 16);
         cp_async_arrive(bar);
     };
-    // Sign+mantissa rows [kChunkRows * c, + kChunkRows) of unit u's segments (left A, left B, right A, right B).
-    auto issue_man = [&](uint32_t u, uint32_t c, uint32_t buf) {
-        uint32_t tk, tp, t0;
-        bool two;
-        unit_tiles(u, tk, tp, t0, two);
+    // Sign+mantissa rows [kChunkRows * c, + kChunkRows) of the segments (left A, left B, right A, right B) of the unit whose
+    // first tile is t0.
+    auto issue_man = [&](uint32_t t0, bool two, uint32_t c, uint32_t buf) {
         const uint8_t *src = a.mantissa + (size_t)t0 * (2 * seg_bytes) + c * (kChunkRows * 32) + lane * 16;
         const uint32_t dst = man_s + buf * (4 * kSegPitch) + lane * 16;
         if (c * kChunkRows + (lane >> 1) < g.half) {
@@ -128,25 +125,26 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     load_desc();
     uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
     uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
+    uint32_t tk = 0, tp = 0, t0 = 0;                            // of unit t
+    bool two = false;
     if (gw < p.total) {
-        issue(gw, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
-        if (BF16) issue_man(gw, 0, 0);
+        unit_tiles(gw, tk, tp, t0, two);
+        issue(t0, two, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
+        if (BF16) issue_man(t0, two, 0, 0);
     }
-    load_lut(s_lut, a.lut, a.tables, a.slot_map);
+    if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
     // Only the weight was touched so far.  With programmatic dependent launch the output buffer may still
     // be in use by the previous kernel of the stream: wait for it, then let the next launch begin.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+    (void)wait_lut(lut_bar, a.lut);
     const uint32_t n_chunks = (g.half + kChunkRows - 1) / kChunkRows;
     uint32_t parity0 = 0, parity1 = 0, stage = 0, li = 0, chunk = 0;
     Quad z;
 
     for (uint32_t t = gw; t < p.total; t += n_warps, ++li) {
-        uint32_t tk, tp, t0;
-        bool two;
-        unit_tiles(t, tk, tp, t0, two);
         const bool tile_live = tsel == 0 || two;
         const uint32_t col0 = 64 * tp + 4 * quad;               // first of this lane's four columns
         const uint32_t cols = tile_live && col0 < g.N ? min(4u, g.N - col0) : 0u;
@@ -154,6 +152,9 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         uint32_t rows_left = cols == 0 ? 0u : !EDGE ? 0xFFFFFFFFu : row < g.K ? min(g.half, g.K - row) : 0u;
         const uint32_t ml = tsel ? nx_ml1 : nx_ml0;
         const bool more = (uint64_t)t + n_warps < p.total;
+        uint32_t n_tk = 0, n_tp = 0, n_t0 = 0;                  // of unit t + n_warps
+        bool n_two = false;
+        if (more) unit_tiles(t + n_warps, n_tk, n_tp, n_t0, n_two);
         auto next_unit = [&]() {
             if (!more) return;
             if (li + 1 - dbase == 32) {
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
             nx_ml0 = __shfl_sync(kFull, d_ml0, j);
             nx_off1 = __shfl_sync(kFull, d_off1, j);
             nx_ml1 = __shfl_sync(kFull, d_ml1, j);
-            issue(t + n_warps, p.stages == 2 ? stage ^ 1 : 0u, nx_off0, nx_ml0, nx_off1, nx_ml1);
+            issue(n_t0, n_two, p.stages == 2 ? stage ^ 1 : 0u, nx_off0, nx_ml0, nx_off1, nx_ml1);
         };
 
         const uint32_t win_s = wbase_s + stage * p.stage_bytes;
@@ -183,8 +184,8 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
             const uint32_t buf = chunk & 1;
             __syncwarp();                                       // every lane is done with the other buffers
             if (BF16) {
-                if (c + 1 < n_chunks) issue_man(t, c + 1, buf ^ 1);
-                else if (more) issue_man(t + n_warps, 0, buf ^ 1);
+                if (c + 1 < n_chunks) issue_man(t0, two, c + 1, buf ^ 1);
+                else if (more) issue_man(n_t0, n_two, 0, buf ^ 1);
             }
             if (c == 0 && p.stages == 2) next_unit();           // behind it: a chunk's arrival waits for older copies
             if (BF16) (void)mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1);
@@ -240,6 +241,10 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
             __syncwarp();                                       // every lane is done with the only window
             next_unit();
         }
+        tk = n_tk;
+        tp = n_tp;
+        t0 = n_t0;
+        two = n_two;
     }
 }
 

@@ -18,7 +18,7 @@
 namespace ci {
 
 constexpr uint32_t kEmb4Warps = 16;
-constexpr uint32_t kEmb4BarBytes = 256;
+constexpr uint32_t kEmb4BarBytes = 384;
 
 struct Emb4Args {
     EmbArgs a;
@@ -45,6 +45,8 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
     // (state << 2 & 0x3FFC) | base, without an addition.
     const uint32_t lut_s = (smem_s + kLutBytes - 1) & ~(kLutBytes - 1);
     uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + (lut_s - smem_s));
+    const uint32_t lut_bar = lut_s + kLutBytes + kEmb4BarBytes - 16;
+    start_lut(lut_s, lut_bar, a.lut);
     const uint32_t wbase_s = lut_s + kLutBytes + kEmb4BarBytes + warp * 2 * p.stage_bytes;
     const uint32_t bar_base = lut_s + kLutBytes + warp * 16;
     const uint64_t gw = (uint64_t)blockIdx.x * W + warp, n_warps = (uint64_t)gridDim.x * W;
@@ -100,13 +102,14 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
     }
     __syncwarp();
 
-    load_lut(s_lut, a.lut, a.tables, a.slot_map);
+    if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
     // The ids (and the output buffer) may be products of the previous kernel of the stream: with
     // programmatic dependent launch wait for it here, after the table load that does not depend on it.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+    (void)wait_lut(lut_bar, a.lut);
     // ---- fill the pipeline: task t = gw, t + n_warps, t + 2 n_warps; id of t + 3 n_warps -----------------
     int64_t id0 = load_id(gw), id1 = load_id(gw + n_warps), id2 = load_id(gw + 2 * n_warps);
     Tok tc = parse(gw, id0), tn1 = parse(gw + n_warps, id1), tn2 = parse(gw + 2 * n_warps, id2);

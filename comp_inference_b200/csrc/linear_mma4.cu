@@ -40,7 +40,7 @@
 
 namespace ci {
 
-constexpr uint32_t kBar4Bytes = 512;         // up to 16 warps x (2 window stages + 2 mantissa chunks) x 8 B
+constexpr uint32_t kBar4Bytes = 640;         // up to 16 warps x (2 window stages + 2 mantissa chunks) x 8 B
 constexpr uint32_t kMma4Warps = 16;          // x 32 threads x 128 registers = the register file
 
 struct Mma4Args {
@@ -119,6 +119,8 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     // (state << 2 & 0x3FFC) | base: one shift and one three-input logic operation, no addition.
     const uint32_t lut_s = (smem_s + kLutBytes - 1) & ~(kLutBytes - 1);
     uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + (lut_s - smem_s));
+    const uint32_t lut_bar = lut_s + kLutBytes + kBar4Bytes - 16;
+    start_lut(lut_s, lut_bar, a.lut);
     const uint32_t wbase_s = lut_s + kLutBytes + kBar4Bytes + W * kManBytes + warp * p.stages * p.stage_bytes;
     const uint32_t man_s = lut_s + kLutBytes + kBar4Bytes + warp * kManBytes;
     const uint32_t bar_base = lut_s + kLutBytes + warp * 32, man_bar = bar_base + 16;
@@ -129,8 +131,8 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     const uint32_t tsel = q >> 1, hsel = q & 1;                 // upper / lower tile, top / bottom half
 
     const uint32_t gw = blockIdx.x * W + warp;                  // this warp's rank in the grid
-    const uint32_t lo = gw < p.slots ? (uint32_t)((uint64_t)gw * p.total / p.slots) : p.total;
-    const uint32_t hi = gw < p.slots ? (uint32_t)((uint64_t)(gw + 1) * p.total / p.slots) : p.total;
+    const uint32_t lo = gw < p.slots ? gw * p.total / p.slots : p.total;       // slots * total fits 32 bits
+    const uint32_t hi = gw < p.slots ? (gw + 1) * p.total / p.slots : p.total;
 
     // Byte ranges of this warp's units, 32 at a time: lane j holds unit dbase + j.
     uint32_t d_off0 = 0, d_ml0 = 0, d_off1 = 0, d_ml1 = 0, dbase = lo;
@@ -149,9 +151,8 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
         }
     };
 
-    // Starts every copy of unit u into `stage` (whole warp).
-    auto issue = [&](uint32_t u, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
-        const uint32_t grp = u / p.pairs_k, pk = u - grp * p.pairs_k;
+    // Starts every copy of the unit (grp, pk) into `stage` (whole warp).
+    auto issue = [&](uint32_t grp, uint32_t pk, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
         const uint32_t t0 = (2 * pk) * g.tiles_n + grp;
         const bool two = 2 * pk + 1 < g.tiles_k;
         const uint32_t bar = bar_base + stage * 8;
@@ -173,15 +174,18 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
         cp_async_arrive(bar);
     };
 
-    // Sign+mantissa rows [kChunkRows * c, + kChunkRows) of the four segments of unit u into chunk buffer `buf`.
-    auto issue_man = [&](uint32_t u, uint32_t c, uint32_t buf) {
-        const uint32_t grp = u / p.pairs_k, pk = u - grp * p.pairs_k;
-        const uint8_t *src = a.mantissa + ((size_t)2 * pk * g.tiles_n + grp) * (2 * seg_bytes) + c * (kChunkRows * 32) + lane * 16;
+    // Sign+mantissa bytes of a unit's upper tile, this lane's 16-byte piece of every chunk row pair.
+    auto man_of = [&](uint32_t grp, uint32_t pk) {
+        return a.mantissa + ((size_t)2 * pk * g.tiles_n + grp) * (2 * seg_bytes) + lane * 16;
+    };
+    // Rows [kChunkRows * c, + kChunkRows) of the four segments of a unit into chunk buffer `buf`; src: man_of the unit.
+    auto issue_man = [&](const uint8_t *src, bool two, uint32_t c, uint32_t buf) {
         const uint32_t dst = man_s + buf * (4 * kSegPitch) + lane * 16;
         if (c * kChunkRows + (lane >> 1) < g.half) {
+            src += c * (kChunkRows * 32);
             cp_async16(dst, src);
             cp_async16(dst + kSegPitch, src + seg_bytes);
-            if (2 * pk + 1 < g.tiles_k) {
+            if (two) {
                 src += (size_t)g.tiles_n * (2 * seg_bytes);
                 cp_async16(dst + 2 * kSegPitch, src);
                 cp_async16(dst + 3 * kSegPitch, src + seg_bytes);
@@ -201,11 +205,12 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     load_desc();
     uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
     uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
+    uint32_t grp = lo / p.pairs_k, pk = lo - grp * p.pairs_k;   // of unit t
     if (lo < hi) {
-        issue(lo, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
-        issue_man(lo, 0, 0);
+        issue(grp, pk, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
+        issue_man(man_of(grp, pk), 2 * pk + 1 < g.tiles_k, 0, 0);
     }
-    load_lut(s_lut, a.lut, a.tables, a.slot_map);
+    if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
     // Everything above touches only the weight, which no kernel writes.  When this launch was allowed to
     // start before its predecessor in the stream has finished (programmatic dependent launch), wait here
@@ -213,6 +218,7 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     // its own preamble while this grid works.  Both are no-ops in an ordinary launch.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!wait_lut(lut_bar, a.lut)) atomicExch(p.status, 1u);
     if (lo >= hi) return;                                       // no CTA-wide synchronisation below this line
     const bool fused_ar = a.ar.world > 1;                       // row-parallel: exchange the sums with the peers here
     const uint32_t ar_seq = fused_ar ? fuse_seq(a.ar) : 0u;
@@ -228,7 +234,7 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     // Writes the finished (or partial) sums of column group grp.  After a lane exchange (below) a lane
     // works on rows gq and gq + 8 of the activation batch, columns 8q .. 8q+7 of the group.
     auto flush = [&](uint32_t grp) {
-        auto warp_of = [&](uint32_t u) { return (uint32_t)(((uint64_t)(u + 1) * p.slots - 1) / p.total); };
+        auto warp_of = [&](uint32_t u) { return ((u + 1) * p.slots - 1) / p.total; };
         const uint32_t first_w = warp_of(grp * p.pairs_k), last_w = warp_of((grp + 1) * p.pairs_k - 1);
         const uint32_t count = last_w - first_w + 1;
         const uint32_t n0 = grp * 32 + 8 * q;
@@ -397,7 +403,7 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     const uint16_t *x0 = a.x + (size_t)min(gq, m_last) * a.ldx;
     const uint16_t *x1 = a.x + (size_t)min(gq + 8, m_last) * a.ldx;
     uint32_t parity0 = 0, parity1 = 0, stage = 0;
-    uint32_t cur_grp = lo / p.pairs_k;
+    uint32_t cur_grp = grp;
     zero_acc();
     const uint32_t n_blocks = g.half / 4;                       // blocks of four symbols per stream
     const uint32_t n_chunks = (g.half + kChunkRows - 1) / kChunkRows;
@@ -406,7 +412,10 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
 
     Quad z;
     for (uint32_t t = lo; t < hi; ++t) {
-        const uint32_t grp = t / p.pairs_k, pk = t - grp * p.pairs_k;
+        const bool wrap = pk + 1 == p.pairs_k;
+        const uint32_t n_grp = grp + wrap, n_pk = wrap ? 0u : pk + 1;   // of unit t + 1
+        const uint8_t *man = man_of(grp, pk);
+        const bool two = 2 * pk + 1 < g.tiles_k;
         if (grp != cur_grp) {
             flush(cur_grp);
             zero_acc();
@@ -447,7 +456,7 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
             nx_ml0 = __shfl_sync(kFull, d_ml0, j);
             nx_off1 = __shfl_sync(kFull, d_off1, j);
             nx_ml1 = __shfl_sync(kFull, d_ml1, j);
-            issue(t + 1, p.stages == 1 ? 0u : stage ^ 1, nx_off0, nx_ml0, nx_off1, nx_ml1);
+            issue(n_grp, n_pk, p.stages == 1 ? 0u : stage ^ 1, nx_off0, nx_ml0, nx_off1, nx_ml1);
         };
         __syncwarp();
 
@@ -472,8 +481,8 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
         for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
             const uint32_t buf = chunk & 1;
             __syncwarp();                                       // every lane is done with the other chunk buffer
-            if (c + 1 < n_chunks) issue_man(t, c + 1, buf ^ 1);
-            else if (t + 1 < hi) issue_man(t + 1, 0, buf ^ 1);
+            if (c + 1 < n_chunks) issue_man(man, two, c + 1, buf ^ 1);
+            else if (t + 1 < hi) issue_man(man_of(n_grp, n_pk), 2 * n_pk + 1 < g.tiles_k, 0, buf ^ 1);
             if (c == 0 && p.stages == 2) next_unit();   // behind it: a chunk's arrival waits for older copies
             if (!mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1)) atomicExch(p.status, 1u);
             z.clamp(win_s);
@@ -523,6 +532,8 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
         } else {
             stage ^= 1;
         }
+        grp = n_grp;
+        pk = n_pk;
     }
     flush(cur_grp);
 }
@@ -602,6 +613,7 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     uint32_t blocks = (p.total + warps - 1) / warps;
     if (blocks > P) blocks = P;
     p.slots = blocks * warps < p.total ? blocks * warps : p.total;
+    if ((uint64_t)p.slots * (p.total + 1) >> 32) return 1;      // 1.8 million units
     p.y_vec = ((reinterpret_cast<uintptr_t>(a.y) & 15u) == 0 && (a.ldy & 7) == 0) ? 1u : 0u;
     p.x_step = 4;
     p.status = a.tickets + (kTicketBytes - 1);

@@ -23,7 +23,7 @@
 namespace ci {
 
 constexpr uint32_t kT4Warps = 16;
-constexpr uint32_t kT4BarBytes = 512;        // up to 16 warps x (2 window stages + 2 chunks) x 8 B
+constexpr uint32_t kT4BarBytes = 640;        // up to 16 warps x (2 window stages + 2 chunks) x 8 B
 constexpr uint32_t kT4SegPitch = kChunkRows * 16 + 16;       // eight segments of a chunk, 4 banks apart
 constexpr uint32_t kT4ManBytes = 2 * 8 * kT4SegPitch;
 
@@ -48,6 +48,8 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     const uint32_t smem_s = smem_u32(smem);
     const uint32_t lut_s = (smem_s + kLutBytes - 1) & ~(kLutBytes - 1);    // see linear_mma4.cu
     uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + (lut_s - smem_s));
+    const uint32_t lut_bar = lut_s + kLutBytes + kT4BarBytes - 16;
+    start_lut(lut_s, lut_bar, a.lut);
     const uint32_t bar_base = lut_s + kLutBytes + warp * 32, man_bar = bar_base + 16;
     const uint32_t man_s = lut_s + kLutBytes + kT4BarBytes + warp * kT4ManBytes;
     const uint32_t acc0_s = lut_s + kLutBytes + kT4BarBytes + W * kT4ManBytes, acc_s = acc0_s + warp * p.acc_bytes;
@@ -137,11 +139,12 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
         issue(u, 0, off, ml);
         issue_man(u, 0, 0);
     }
-    load_lut(s_lut, a.lut, a.tables, a.slot_map);
+    if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");          // everything above touched only the weight
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+    if (!wait_lut(lut_bar, a.lut)) atomicExch(p.status, 1u);
     const bool live_m = MT == 8 ? 2 * q < a.M : q == 0;         // lanes whose two D columns are activation rows
     const uint32_t n_chunks = (g.half + kChunkRows - 1) / kChunkRows;
     uint32_t parity0 = 0, parity1 = 0, stage = 0, chunk = 0;

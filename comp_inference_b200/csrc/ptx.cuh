@@ -220,6 +220,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// The decode table into shared memory at lut_s: a prepared one by one bulk copy that nobody waits for until the first
+// look-up (start_lut by thread 0 before the CTA's first barrier, wait_lut by every thread behind it), otherwise built on
+// the spot.
+__device__ __forceinline__ void start_lut(uint32_t lut_s, uint32_t bar, const uint32_t *lut) {
+    if (threadIdx.x == 0 && lut != nullptr) {
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_proxy();
+        mbar_expect_tx(bar, kLutBytes);
+        bulk_load(lut_s, lut, kLutBytes, bar);
+    }
+}
+__device__ __forceinline__ bool wait_lut(uint32_t bar, const uint32_t *lut) { return lut == nullptr || mbar_wait(bar, 0); }
+
 // Sign+mantissa bytes on their way through a warp that decodes four segments (two tiles, both halves) at once: chunks of
 // kChunkRows rows of 32 bytes per segment, double buffered.  The segments of a chunk start 8 banks apart, so a row of
 // the warp's 128 columns is one conflict-free wavefront.
