@@ -8,31 +8,30 @@
 // columns 4l .. 4l+3 of the strip.  The four 32-byte-wide half slices of the tiles' byte blocks are
 // copied by cp.async side by side into a window of 128-byte rows, which gives every lane a word column
 // (a shared-memory bank) of its own, so the renormalisation byte loads never conflict; the row's four
-// weights leave as one 8-byte store.  The pipeline is three tasks deep so that no dependent global load
-// (id -> tile metadata -> byte block) is ever waited for: ids are read three tasks ahead, tile offsets and
-// depths two ahead, the byte blocks and initial states one ahead into the other half of a per-warp double
-// buffer.
+// weights leave as one 8-byte store.  Only the rows a stream can reach are copied: two bytes a symbol at most.
+//
+// At the tile heights that suit gathers only a few symbols are decoded per task, so what bounds the kernel is the work
+// around them.  A warp therefore takes a run of consecutive tasks: eight at a time their ids are read and their tiles'
+// offsets and depths fetched, one tile per lane, while the eight before them are worked off; a task then costs two
+// shuffles for its lane's own tile, and no division.  Byte windows, initial states and the row's sign+mantissa bytes are
+// fetched one task ahead.  Measured, 4096 ids of 32000 x 4096 at tile height 16: 148 us with one task at a time,
+// divisions in 64 bits and eight shuffles per task -> see the table in the design notes.
 #include "embedding.cuh"
 #include "ptx.cuh"
 
 namespace ci {
 
-constexpr uint32_t kEmb4Warps = 16;
-constexpr uint32_t kEmb4BarBytes = 384;
+constexpr uint32_t kEmb4Warps = 24;          // x 32 threads x 80 registers
+constexpr uint32_t kEmb4BarBytes = 512;      // up to 24 warps x 2 stages x 8 B, the table's barrier
 
 struct Emb4Args {
     EmbArgs a;
     uint32_t cap_rows;     // rows of a byte window (>= every tile_max_len)
     uint32_t stage_bytes;
+    uint32_t stages;       // windows per warp: 2, or 1 for tall tiles
     uint32_t blocks_n;     // 128-column blocks per row = ceil(tiles_n / 4)
-    uint64_t total;        // tasks
+    uint32_t total;        // tasks, the column block running fastest
     uint32_t out_vec;      // rows of the output can be written as 8-byte quads
-};
-
-// What a task needs to know about its token: tile row, half, symbols to drop; valid = id inside the table.
-struct Tok {
-    uint32_t tk, hsel, inner, rel;
-    bool valid;
 };
 
 __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_constant__ Emb4Args p) {
@@ -47,155 +46,133 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
     uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + (lut_s - smem_s));
     const uint32_t lut_bar = lut_s + kLutBytes + kEmb4BarBytes - 16;
     start_lut(lut_s, lut_bar, a.lut);
-    const uint32_t wbase_s = lut_s + kLutBytes + kEmb4BarBytes + warp * 2 * p.stage_bytes;
+    const uint32_t wbase_s = lut_s + kLutBytes + kEmb4BarBytes + warp * p.stages * p.stage_bytes;
     const uint32_t bar_base = lut_s + kLutBytes + warp * 16;
-    const uint64_t gw = (uint64_t)blockIdx.x * W + warp, n_warps = (uint64_t)gridDim.x * W;
+    const uint32_t gw = blockIdx.x * W + warp, n_warps = gridDim.x * W;
+    const uint32_t lo = (uint32_t)((uint64_t)gw * p.total / n_warps), hi = (uint32_t)((uint64_t)(gw + 1) * p.total / n_warps);
     const uint32_t tsel = lane >> 3, quad = lane & 7;           // tile of the block, column quad inside it
-
-    auto parse = [&](uint64_t task, int64_t id) {
-        Tok t;
-        t.valid = task < p.total && id >= 0 && id < (int64_t)g.K;
-        const uint32_t row = t.valid ? (uint32_t)id : 0u;
-        t.tk = row / g.th;
-        t.rel = row - t.tk * g.th;
-        t.hsel = t.rel >= g.half ? 1u : 0u;
-        t.inner = t.rel - t.hsel * g.half;
-        return t;
-    };
-    auto load_id = [&](uint64_t task) -> int64_t { return task < p.total ? __ldg(a.ids + task / p.blocks_n) : -1; };
-    // Lanes 0..3 fetch offset and depth of the block's four tiles (zero for a tile beyond the matrix).
-    auto load_meta = [&](uint64_t task, const Tok &t, uint32_t &off, uint32_t &ml) {
-        off = ml = 0;
-        const uint32_t tn = (uint32_t)(task % p.blocks_n) * 4 + lane;
-        if (t.valid && lane < 4 && tn < g.tiles_n) {
-            const size_t tile = (size_t)t.tk * g.tiles_n + tn;
-            off = __ldg(a.tile_offsets + tile);
-            ml = __ldg(a.tile_max_lens + tile);
-        }
-    };
-    // Copies the token's half slice (32 bytes of every row) of the four tiles into `stage`.
-    auto issue = [&](const Tok &t, uint32_t off, uint32_t ml, uint32_t stage) {
-        const uint32_t bar = bar_base + stage * 8, dst = wbase_s + stage * p.stage_bytes;
-        if (ml > p.cap_rows) ml = 0;                            // metadata disagrees with the declared maximum
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            const uint32_t mlj = __shfl_sync(kFull, ml, j), offj = __shfl_sync(kFull, off, j);
-            const uint8_t *src = a.stream + offj + t.hsel * 32;
-            for (uint32_t i = lane; i < mlj * 2; i += 32)
-                cp_async16(dst + (i >> 1) * 128 + j * 32 + (i & 1) * 16, src + (size_t)(i >> 1) * 64 + (i & 1) * 16);
-        }
-        cp_async_arrive(bar);
-    };
-    // This lane's four initial states of a task (one 16-byte load) and its tile's depth.
-    auto load_states = [&](uint64_t task, const Tok &t) {
-        uint4 s = make_uint4(kRansL, kRansL, kRansL, kRansL);
-        const uint32_t tn = (uint32_t)(task % p.blocks_n) * 4 + tsel;
-        if (t.valid && tn < g.tiles_n)
-            s = __ldg(reinterpret_cast<const uint4 *>(a.states + ((size_t)t.tk * g.tiles_n + tn) * 64 + t.hsel * 32 + quad * 4));
-        return s;
-    };
 
     if (lane == 0) {
         mbar_init(bar_base, 32);                                // one arrival per lane when its copies have landed
         mbar_init(bar_base + 8, 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncwarp();
-
     if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
     // The ids (and the output buffer) may be products of the previous kernel of the stream: with
     // programmatic dependent launch wait for it here, after the table load that does not depend on it.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-
     (void)wait_lut(lut_bar, a.lut);
-    // ---- fill the pipeline: task t = gw, t + n_warps, t + 2 n_warps; id of t + 3 n_warps -----------------
-    int64_t id0 = load_id(gw), id1 = load_id(gw + n_warps), id2 = load_id(gw + 2 * n_warps);
-    Tok tc = parse(gw, id0), tn1 = parse(gw + n_warps, id1), tn2 = parse(gw + 2 * n_warps, id2);
-    uint32_t offC, mlC, offN, mlN, offNN = 0, mlNN = 0;
-    load_meta(gw, tc, offC, mlC);
-    load_meta(gw + n_warps, tn1, offN, mlN);
-    int64_t id3 = load_id(gw + 3 * n_warps);
-    uint4 stC = load_states(gw, tc), stN = make_uint4(kRansL, kRansL, kRansL, kRansL);
-    if (gw < p.total) issue(tc, offC, mlC, 0);
+    if (lo >= hi) return;
 
-    uint32_t parity0 = 0, parity1 = 0, stage = 0;
-    uint32_t s0, s1, s2, s3, pos0, pos1, pos2, pos3;
-    auto renorm4 = [&](uint32_t y0, uint32_t y1, uint32_t y2, uint32_t y3) {
-        const uint32_t lowest = min(min(s0, s1), min(s2, s3));
-        renorm_first<128>(s0, pos0, y0);
-        renorm_first<128>(s1, pos1, y1);
-        renorm_first<128>(s2, pos2, y2);
-        renorm_first<128>(s3, pos3, y3);
-        if (__any_sync(kFull, lowest < 256u)) {                 // a second byte: only after a symbol of frequency < 16
-            renorm_fast<128>(s0, pos0);
-            renorm_fast<128>(s1, pos1);
-            renorm_fast<128>(s2, pos2);
-            renorm_fast<128>(s3, pos3);
+    // A batch of eight tasks from `first` on: lane l holds what tile l % 4 of task first + l / 4 needs.
+    struct Batch {
+        uint32_t ti, cb;       // token and column block of the lane's task
+        uint32_t row;          // its row of the table; ~0 when the id is outside
+        uint32_t off, ml;      // the lane's tile: byte offset, depth (0 for a tile that is not read)
+    };
+    auto load_ids = [&](uint32_t first, Batch &b) {
+        const uint32_t t = min(first + (lane >> 2), hi - 1);
+        b.ti = t / p.blocks_n;
+        b.cb = t - b.ti * p.blocks_n;
+        const int64_t id = __ldg(a.ids + b.ti);
+        b.row = id >= 0 && id < (int64_t)g.K ? (uint32_t)id : 0xFFFFFFFFu;
+    };
+    auto load_tiles = [&](Batch &b) {
+        const uint32_t tn = b.cb * 4 + (lane & 3);
+        b.off = b.ml = 0;
+        if (b.row != 0xFFFFFFFFu && tn < g.tiles_n) {
+            const size_t tile = (size_t)(b.row / g.th) * g.tiles_n + tn;
+            b.off = __ldg(a.tile_offsets + tile);
+            b.ml = __ldg(a.tile_max_lens + tile);
         }
+        if (b.ml > p.cap_rows) b.ml = 0;                        // metadata disagrees with the declared maximum
     };
 
-    for (uint64_t t = gw; t < p.total; t += n_warps) {
-        const uint32_t cb = (uint32_t)(t % p.blocks_n);
-        const uint64_t ti = t / p.blocks_n;
-        const uint32_t tn = cb * 4 + tsel, col0 = tn * 32 + quad * 4;
-        const bool tile_live = tc.valid && tn < g.tiles_n;
-        const uint32_t ml = __shfl_sync(kFull, mlC, tsel);
-        // sign+mantissa bytes of the wanted row of this lane's four columns: in flight during the decode
-        uint32_t man = 0;
-        if (tile_live)
-            man = __ldg(reinterpret_cast<const uint32_t *>(a.mantissa + ((size_t)tc.tk * g.tiles_n + tn) * (g.th * 32) +
-                                                           (size_t)tc.rel * 32 + quad * 4));
-        __syncwarp();                                           // every lane is done with the other stage
-        // next task: copies and states; the task after: metadata; the one after that: its id
-        load_meta(t + 2 * n_warps, tn2, offNN, mlNN);
-        const int64_t id4 = load_id(t + 4 * n_warps);
-        if (t + n_warps < p.total) {
-            issue(tn1, offN, mlN, stage ^ 1);
-            stN = load_states(t + n_warps, tn1);
+    // What the lane knows about one task.
+    struct Task {
+        uint32_t ti, cb, inner, ml;
+        bool live;             // the id is inside the table and so is the lane's tile
+        uint4 states;
+        uint32_t man;
+    };
+    // Task k of the batch: its copies into `stage`, its states and sign+mantissa bytes.
+    auto open = [&](const Batch &b, uint32_t k, uint32_t stage, Task &t) {
+        const uint32_t src_lane = 4 * k + tsel;
+        t.ti = __shfl_sync(kFull, b.ti, 4 * k);
+        t.cb = __shfl_sync(kFull, b.cb, 4 * k);
+        const uint32_t row = __shfl_sync(kFull, b.row, 4 * k), off = __shfl_sync(kFull, b.off, src_lane);
+        t.ml = __shfl_sync(kFull, b.ml, src_lane);
+        const uint32_t tn = t.cb * 4 + tsel;
+        t.live = row != 0xFFFFFFFFu && tn < g.tiles_n;
+        const uint32_t tk = row / g.th, rel = row - tk * g.th, h = rel >= g.half ? 1u : 0u;
+        t.inner = t.live ? rel - h * g.half : 0u;
+        t.states = make_uint4(kRansL, kRansL, kRansL, kRansL);
+        t.man = 0;
+        if (t.live) {
+            const size_t tile = (size_t)tk * g.tiles_n + tn;
+            t.states = __ldg(reinterpret_cast<const uint4 *>(a.states + tile * 64 + h * 32 + quad * 4));
+            t.man = __ldg(reinterpret_cast<const uint32_t *>(a.mantissa + tile * (g.th * 32) + rel * 32 + quad * 4));
+            // eight lanes a tile: pieces of 16 bytes, two a row, from the last row upwards
+            const uint32_t rows = min(t.ml, 2 * t.inner + 2), skip = t.ml - rows;
+            const uint8_t *src = a.stream + off + h * 32 + (size_t)(skip + (quad >> 1)) * 64 + (quad & 1) * 16;
+            const uint32_t dst = wbase_s + stage * p.stage_bytes + (skip + (quad >> 1)) * 128 + tsel * 32 + (quad & 1) * 16;
+            for (uint32_t i = quad >> 1; i < rows; i += 4) cp_async16(dst + (i - (quad >> 1)) * 128, src + (size_t)(i - (quad >> 1)) * 64);
         }
+        cp_async_arrive(bar_base + stage * 8);
+    };
 
-        const uint32_t win_s = wbase_s + stage * p.stage_bytes;
-        pos0 = win_s + tsel * 32 + quad * 4;
-        if (tile_live && ml >= 1 && ml <= p.cap_rows) pos0 += (ml - 1) * 128;
-        pos1 = pos0 + 1;
-        pos2 = pos0 + 2;
-        pos3 = pos0 + 3;
-        {
-            const uint32_t bar = bar_base + stage * 8, par = stage ? parity1 : parity0;
-            uint32_t ok = 0;
-            if (lane == 0)
-                for (uint32_t it = 0; it < kWaitPolls && !ok; ++it) ok = mbar_try_wait(bar, par);
-            ok = __shfl_sync(kFull, ok, 0);
-            if (stage) parity1 ^= 1; else parity0 ^= 1;
-            (void)mbar_try_wait(bar, par);                      // each lane observes the completed phase itself
-            if (!ok) {                                          // give up on this task: zero row, keep the pipeline moving
-                s0 = s1 = s2 = s3 = kRansL;
-            } else {
-                s0 = stC.x; s1 = stC.y; s2 = stC.z; s3 = stC.w;
+    Batch cur, nxt;
+    load_ids(lo, cur);
+    load_tiles(cur);
+    Task t, n;
+    open(cur, 0, 0, t);
+    uint32_t parity0 = 0, parity1 = 0, stage = 0;
+    for (uint32_t first = lo; first < hi; first += 8) {
+        const bool more = first + 8 < hi;
+        const uint32_t count = min(8u, hi - first);
+        if (more) load_ids(first + 8, nxt);
+#pragma unroll 1
+        for (uint32_t k = 0; k < count; ++k) {
+            if (k == 2 && more) load_tiles(nxt);                // two tasks after its ids were asked for
+            const bool last = k + 1 == count;
+            __syncwarp();                                       // every lane is done with the other window
+            if (p.stages == 2) {
+                if (!last) open(cur, k + 1, stage ^ 1, n);
+                else if (more) open(nxt, 0, stage ^ 1, n);
             }
-            if (ok && tc.valid) {
-#pragma unroll 4
-                for (uint32_t i = 0; i < tc.inner; ++i) {        // the rows above the wanted one
-                    const uint32_t y0 = lds_u8(pos0), y1 = lds_u8(pos1), y2 = lds_u8(pos2), y3 = lds_u8(pos3);
-                    (void)decode_aligned(s0, lut_s);
-                    (void)decode_aligned(s1, lut_s);
-                    (void)decode_aligned(s2, lut_s);
-                    (void)decode_aligned(s3, lut_s);
-                    renorm4(y0, y1, y2, y3);
-                }
+            const uint32_t win_s = wbase_s + stage * p.stage_bytes;
+            const bool ok = mbar_wait(bar_base + stage * 8, stage ? parity1 : parity0);
+            if (stage) parity1 ^= 1; else parity0 ^= 1;
+            Quad z;
+            z.s[0] = t.states.x;
+            z.s[1] = t.states.y;
+            z.s[2] = t.states.z;
+            z.s[3] = t.states.w;
+            const uint32_t start = win_s + tsel * 32 + quad * 4 + (t.ml ? (t.ml - 1) * 128 : 0u);
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) z.p[j] = start + j;
+            // The rows above the wanted one.  Lanes without a tile run along on whatever is in the window.
+            const uint32_t drop = __shfl_sync(kFull, t.inner, 0);
+#pragma unroll 1
+            for (uint32_t i = 0; i < drop; ++i) {
+                uint32_t e[4];
+                z.step(lut_s, e);
+                if ((i & 15) == 15) z.clamp(win_s);
             }
             uint32_t w01 = 0, w23 = 0;
-            if (ok && tile_live) {
-                const uint32_t e0 = lds_u32(((s0 << 2) & (kProbMask << 2)) | lut_s), e1 = lds_u32(((s1 << 2) & (kProbMask << 2)) | lut_s);
-                const uint32_t e2 = lds_u32(((s2 << 2) & (kProbMask << 2)) | lut_s), e3 = lds_u32(((s3 << 2) & (kProbMask << 2)) | lut_s);
+            if (ok && t.live) {
+                const uint32_t mask = (kProbScale - 1) << 2;
+                const uint32_t e0 = lds_u32(((z.s[0] << 2) & mask) | lut_s), e1 = lds_u32(((z.s[1] << 2) & mask) | lut_s);
+                const uint32_t e2 = lds_u32(((z.s[2] << 2) & mask) | lut_s), e3 = lds_u32(((z.s[3] << 2) & mask) | lut_s);
                 const uint32_t a01 = __byte_perm(e0, e1, 0x6521), a23 = __byte_perm(e2, e3, 0x6521);
-                w01 = ((a01 << 3) & 0x7F807F80u) | (__byte_perm(man, 0u, 0x1100) & 0x807F807Fu);
-                w23 = ((a23 << 3) & 0x7F807F80u) | (__byte_perm(man, 0u, 0x3322) & 0x807F807Fu);
+                w01 = ((a01 << 3) & 0x7F807F80u) | (__byte_perm(t.man, 0u, 0x1100) & 0x807F807Fu);
+                w23 = ((a23 << 3) & 0x7F807F80u) | (__byte_perm(t.man, 0u, 0x3322) & 0x807F807Fu);
             }
+            const uint32_t col0 = t.cb * 128 + tsel * 32 + quad * 4;
             if (col0 < g.N) {
-                uint16_t *dst = a.out + ti * a.ldo + col0;
+                uint16_t *dst = a.out + (size_t)t.ti * a.ldo + col0;
                 if (p.out_vec && col0 + 4 <= g.N) {
                     *reinterpret_cast<uint2 *>(dst) = make_uint2(w01, w23);
                 } else {
@@ -205,16 +182,16 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
                         if (col0 + c < g.N) dst[c] = (uint16_t)v[c];
                 }
             }
+            if (p.stages == 2) {
+                stage ^= 1;
+            } else {
+                __syncwarp();                                   // every lane is done with the only window
+                if (!last) open(cur, k + 1, 0, n);
+                else if (more) open(nxt, 0, 0, n);
+            }
+            t = n;
         }
-        // rotate the pipeline
-        tc = tn1;
-        tn1 = tn2;
-        tn2 = parse(t + 3 * n_warps, id3);
-        id3 = id4;
-        offC = offN; mlC = mlN;
-        offN = offNN; mlN = mlNN;
-        stC = stN;
-        stage ^= 1;
+        cur = nxt;
     }
 }
 
@@ -226,7 +203,6 @@ int launch_embedding4(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t s) {
     if ((reinterpret_cast<uintptr_t>(a.stream) & 15u) || (reinterpret_cast<uintptr_t>(a.states) & 15u) ||
         (reinterpret_cast<uintptr_t>(a.mantissa) & 3u))
         return 1;
-    if (g.th * 128u > kLutBytes) return 1;                      // see the note on stream cursors in ptx.cuh
     int dev = 0, max_smem = 0;
     CI_CUDA(cudaGetDevice(&dev));
     CI_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -235,29 +211,36 @@ int launch_embedding4(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t s) {
     p.cap_rows = max_tile_len;
     p.stage_bytes = (p.cap_rows * 128u + 127u) & ~127u;
     p.blocks_n = (g.tiles_n + 3) / 4;
-    p.total = a.n_ids * p.blocks_n;
     p.out_vec = ((reinterpret_cast<uintptr_t>(a.out) & 7u) == 0 && (a.ldo & 3) == 0) ? 1u : 0u;
     const uint32_t fixed = 2 * kLutBytes + kEmb4BarBytes;           // up to one table size is lost to the table's alignment
-    const uint32_t warp_bytes = 2 * p.stage_bytes;
-    if ((uint32_t)max_smem < fixed + 4 * warp_bytes) return 1;
-    uint32_t warps = ((uint32_t)max_smem - fixed) / warp_bytes;
-    if (warps > kEmb4Warps) warps = kEmb4Warps;
-    uint64_t blocks = (p.total + warps - 1) / warps;
-    const uint64_t P = (uint64_t)sm_count();
-    if (blocks > P) blocks = P;
+    const uint32_t room = (uint32_t)max_smem - fixed;
+    if (room < p.stage_bytes) return 1;
+    p.stages = room / (2 * p.stage_bytes) >= 12 ? 2 : 1;        // a deep window is worth doubling while 12 warps still fit
+    uint32_t w_max = room / (p.stages * p.stage_bytes);
+    if (w_max > kEmb4Warps) w_max = kEmb4Warps;
     static SmemLimit lim = {};
     if (int rc = ensure_smem_limit(lim, (const void *)k_embedding4, (size_t)max_smem)) return rc;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(warps * 32);
-    cfg.dynamicSmemBytes = fixed + (size_t)warps * warp_bytes;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CI_CUDA(cudaLaunchKernelEx(&cfg, k_embedding4, p));
+    const uint32_t P = (uint32_t)sm_count();
+    const uint64_t ids_per_launch = 0x40000000ull / p.blocks_n;     // task numbers fit 32 bits
+    for (uint64_t i0 = 0; i0 < a.n_ids; i0 += ids_per_launch) {
+        const uint64_t n = a.n_ids - i0 < ids_per_launch ? a.n_ids - i0 : ids_per_launch;
+        p.a.ids = a.ids + i0;
+        p.a.out = a.out + i0 * a.ldo;
+        p.total = (uint32_t)(n * p.blocks_n);
+        uint32_t blocks = p.total < P ? p.total : P, warps = (p.total + blocks - 1) / blocks;
+        if (warps > w_max) warps = w_max;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(warps * 32);
+        cfg.dynamicSmemBytes = fixed + (size_t)warps * p.stages * p.stage_bytes;
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        CI_CUDA(cudaLaunchKernelEx(&cfg, k_embedding4, p));
+    }
     return CI_OK;
 }
 

@@ -98,3 +98,18 @@ def test_decoder_edges(K, N, th):
     assert torch.equal(w.view(torch.int16), W.view(torch.int16))
     plane = ci.rans_decomp_triton_tiled(*args, (K, N), *tile)
     assert torch.equal(plane, ci.extract_exp_and_mantissa(W)[0])
+
+
+# row gather: every row of small tables (each position inside a half tile), ids outside, one id, more ids than warps,
+# tall tiles (one window per warp), odd widths
+@pytest.mark.parametrize("V,H,th,n", [(96, 128, 16, 300), (300, 4096, 16, 1), (257, 100, 128, 257), (3000, 64, 1024, 500),
+                                      (2048, 1030, 1024, 40), (640, 320, 64, 5000), (64, 33, 32, 70)])
+def test_embedding_edges(V, H, th, n):
+    import comp_inference_b200 as ci
+    W = _weight(V, H)
+    c = ci.compress_weight_cuda(W, th, 32)
+    m = ci.RansEmbedding(V, H, c["tile_height"], c["tile_width"]).load_compressed(c).prepare()
+    ids = torch.arange(n, device="cuda") % (V + 2) - 1
+    want = torch.where(((ids >= 0) & (ids < V))[:, None], W[ids.clamp(0, V - 1)].float(), torch.zeros((), device="cuda"))
+    assert torch.equal(m(ids).float(), want)
+    assert torch.equal(m(ids.view(1, -1).to(torch.int32))[0].float(), want)
