@@ -4,7 +4,6 @@ GPU through libci_b200.so.  Inputs may live on the CPU (the reference's scripts
 pass CPU tensors); they are moved to the current CUDA device, results come back
 on the device the reference would have left them on.
 """
-import ctypes as C
 from typing import Tuple
 
 import numpy as np
@@ -98,26 +97,20 @@ def _compress(w, tile_height, tile_width, uncoalesced, keep_on_device, want_man_
     th, tw = ccore.effective_tile(K, N, int(tile_height), int(tile_width))
     tk, tn = -(-K // th), -(-N // tw)
     dev, lib = w.device, _lib.load()
-    man = torch.empty(tk * tn * th * tw, dtype=torch.uint8, device=dev)
     mfreqs = mcdf = None
     if not uncoalesced and lib.ci_compress_scratch_bytes(K, N, th, tw):
         # 32-wide tiles: histogram, tables, split and encoder in one queue with one wait
-        a = ccore.tiled_arrays(K, N, th, tw, dev)
-        freqs, cdf = np.empty(256, np.uint16), np.empty(256, np.uint16)
-        mhist = np.empty(256, np.uint64) if want_man_freqs else None
-        n = C.c_uint64(0)
-        _lib.check(lib.ci_compress_bf16(_lib.ptr(w), K, N, th, tw, _lib.ptr(man), *a.pointers, freqs.ctypes.data,
-                                        cdf.ctypes.data, mhist.ctypes.data if want_man_freqs else None, C.byref(n),
-                                        _lib.stream()))
-        a.pack(n.value)
+        stream, states, sizes, tables, slot_map, offsets, lens, man, freqs, cdf, mhist = _lib.host().compress(
+            w, th, tw, want_man_freqs)
         if want_man_freqs:
-            mfreqs, mcdf = _normalize(mhist)
+            mfreqs, mcdf = _normalize(mhist.numpy())
         mv = (lambda t: t) if keep_on_device else (lambda t: t.cpu())
         r = ccore.TiledTensorCompressResult(
-            success=True, stream=mv(a.stream), states=mv(a.states), tables=mv(a.tables), slot_map=mv(a.slot_map),
-            output_sizes=mv(a.sizes), num_streams=tk * tn * 2 * tw, stream_len=int(n.value), tile_offsets=mv(a.offsets),
-            tile_max_lens=mv(a.max_lens), num_tiles_n=tn, num_tiles_k=tk, tile_height=th, tile_width=tw)
-        return r, man, torch.from_numpy(freqs), torch.from_numpy(cdf), mfreqs, mcdf
+            success=True, stream=mv(stream), states=mv(states), tables=mv(tables), slot_map=mv(slot_map),
+            output_sizes=mv(sizes), num_streams=tk * tn * 2 * tw, stream_len=stream.numel(), tile_offsets=mv(offsets),
+            tile_max_lens=mv(lens), num_tiles_n=tn, num_tiles_k=tk, tile_height=th, tile_width=tw)
+        return r, man, freqs, cdf, mfreqs, mcdf
+    man = torch.empty(tk * tn * th * tw, dtype=torch.uint8, device=dev)
     exp = torch.empty((K, N), dtype=torch.uint8, device=dev)
     hist = torch.empty((2, 256), dtype=torch.int64, device=dev)
     _lib.check(lib.ci_split_bf16(_lib.ptr(w), K, N, th, tw, _lib.ptr(exp), _lib.ptr(man), _lib.ptr(hist[0]),

@@ -280,6 +280,39 @@ Tensor decode_call(const Weight &h, bool bf16) {
     return o;
 }
 
+// bf16 [K,N] -> the package arrays of the one-pass encoder (32-wide tiles).  Returns (stream, states, sizes, tables,
+// slot_map, offsets, max_lens, mantissas, freqs, cdf, man_hist or None); freqs, cdf, man_hist on the host.
+py::tuple compress(const Tensor &w, int64_t th, int64_t tw, bool want_man_hist) {
+    require_cuda(w, "weight");
+    TORCH_CHECK(w.scalar_type() == at::kBFloat16 && w.dim() == 2 && w.is_contiguous(), "expected a contiguous 2-D bfloat16 tensor");
+    const int64_t K = w.size(0), N = w.size(1), tiles = ((K + th - 1) / th) * ((N + tw - 1) / tw);
+    const auto u8 = w.options().dtype(at::kByte), u32 = w.options().dtype(at::kUInt32);
+    const auto u16 = at::TensorOptions().dtype(at::kUInt16);
+    Tensor states = at::empty({tiles * 2 * tw}, u32), sizes = at::empty({tiles * 2 * tw}, u32), offsets = at::empty({tiles}, u32);
+    Tensor lens = at::empty({tiles}, u32), tables = at::empty({256}, u32), slot_map = at::empty({4096}, u8);
+    Tensor man = at::empty({tiles * th * tw}, u8), freqs = at::empty({256}, u16), cdf = at::empty({256}, u16), man_hist;
+    if (want_man_hist) man_hist = at::empty({256}, at::TensorOptions().dtype(at::kLong));
+    const size_t bytes = ci_compress_scratch_bytes((uint32_t)K, (uint32_t)N, (uint32_t)th, (uint32_t)tw);
+    Tensor scratch = at::empty({(int64_t)bytes}, u8), stream_t;
+    uint64_t n = 0;
+    int rc;
+    {
+        py::gil_scoped_release release;                         // waits for the device
+        rc = ci_compress_bf16((const uint16_t *)w.data_ptr(), (uint32_t)K, (uint32_t)N, (uint32_t)th, (uint32_t)tw,
+                              (uint8_t *)man.data_ptr(), (uint32_t *)states.data_ptr(), (uint32_t *)sizes.data_ptr(),
+                              (uint32_t *)offsets.data_ptr(), (uint32_t *)lens.data_ptr(), (uint32_t *)tables.data_ptr(),
+                              (uint8_t *)slot_map.data_ptr(), scratch.data_ptr(), bytes, (uint16_t *)freqs.data_ptr(),
+                              (uint16_t *)cdf.data_ptr(), want_man_hist ? (uint64_t *)man_hist.data_ptr() : nullptr, &n, stream());
+    }
+    check(rc);
+    stream_t = at::empty({(int64_t)n}, u8);
+    check(ci_compress_pack((uint32_t)K, (uint32_t)N, (uint32_t)th, (uint32_t)tw, (const uint32_t *)sizes.data_ptr(),
+                           (const uint32_t *)offsets.data_ptr(), (const uint32_t *)lens.data_ptr(), scratch.data_ptr(), bytes,
+                           (uint8_t *)stream_t.data_ptr(), n, stream()));
+    return py::make_tuple(stream_t, states, sizes, tables, slot_map, offsets, lens, man, freqs, cdf,
+                          want_man_hist ? py::cast(man_hist) : py::none());
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_ci_host, m) {
@@ -291,4 +324,5 @@ PYBIND11_MODULE(_ci_host, m) {
              py::arg("transposed") = false, py::arg("prefill_rows") = 0)
         .def("embedding", &embedding_call, py::arg("x"), py::arg("out") = py::none())
         .def("decode", &decode_call, py::arg("bf16"));
+    m.def("compress", &compress, py::arg("weight"), py::arg("tile_h"), py::arg("tile_w"), py::arg("want_man_hist"));
 }
