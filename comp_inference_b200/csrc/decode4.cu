@@ -21,8 +21,8 @@
 
 namespace ci {
 
-constexpr uint32_t kDec4Warps = 16;
-constexpr uint32_t kDec4BarBytes = 640;      // up to 16 warps x (2 window stages + 2 mantissa chunks) x 8 B
+constexpr uint32_t kDec4Warps = 21;          // x 32 threads x 96 registers
+constexpr uint32_t kDec4BarBytes = 768;      // up to 21 warps x (2 window stages + 2 mantissa chunks) x 8 B, the table's
 
 struct Dec4Args {
     DecArgs a;
@@ -56,7 +56,8 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
 
     const uint32_t quad = lane >> 1, hsel = lane & 1;           // column quad of the 64-column strip, stream half
     const uint32_t tsel = quad >> 3;                            // left / right tile
-    const uint32_t gw = blockIdx.x * W + warp, n_warps = gridDim.x * W;
+    // Rank in the grid, the CTA running fastest: what the last round lacks, it lacks on every multiprocessor alike.
+    const uint32_t gw = warp * gridDim.x + blockIdx.x, n_warps = gridDim.x * W;
 
     // Unit u = (tile row, tile pair), the pair running fastest: warps that run at the same time write
     // neighbouring pieces of the same output rows.
@@ -203,8 +204,8 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
                     const bool store = EDGE ? i < rows_left : rows_left != 0;
                     if (BF16) {
                         const uint32_t m = lds_u32(ms + i * 32);
-                        const uint32_t w01 = ((a01 << 3) & 0x7F807F80u) | (__byte_perm(m, 0u, 0x1100) & 0x807F807Fu);
-                        const uint32_t w23 = ((a23 << 3) & 0x7F807F80u) | (__byte_perm(m, 0u, 0x3322) & 0x807F807Fu);
+                        const uint32_t w01 = exp_or_man(a01 << 3, __byte_perm(m, 0u, 0x1100));
+                        const uint32_t w23 = exp_or_man(a23 << 3, __byte_perm(m, 0u, 0x3322));
                         if (store) {
                             if (!EDGE) {
                                 *reinterpret_cast<uint2 *>(o8) = make_uint2(w01, w23);
@@ -294,8 +295,7 @@ int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
         uint32_t w_max = room / (stages * p.stage_bytes + man_bytes);
         if (w_max > kDec4Warps) w_max = kDec4Warps;
         for (uint32_t w = 1; w <= w_max; ++w) {
-            const uint64_t rounds = (p.total + (uint64_t)P * w - 1) / ((uint64_t)P * w);
-            const double cost = (double)rounds * round_cost(w) * (stages == 1 ? 1.02 : 1.0);
+            const double cost = run_cost((p.total + P - 1) / P, w, 0.9) * (stages == 1 ? 1.02 : 1.0);
             if (warps == 0 || cost < best) { best = cost; warps = w; p.stages = stages; }
         }
     }

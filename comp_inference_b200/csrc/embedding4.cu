@@ -167,8 +167,8 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
                 const uint32_t e0 = lds_u32(((z.s[0] << 2) & mask) | lut_s), e1 = lds_u32(((z.s[1] << 2) & mask) | lut_s);
                 const uint32_t e2 = lds_u32(((z.s[2] << 2) & mask) | lut_s), e3 = lds_u32(((z.s[3] << 2) & mask) | lut_s);
                 const uint32_t a01 = __byte_perm(e0, e1, 0x6521), a23 = __byte_perm(e2, e3, 0x6521);
-                w01 = ((a01 << 3) & 0x7F807F80u) | (__byte_perm(t.man, 0u, 0x1100) & 0x807F807Fu);
-                w23 = ((a23 << 3) & 0x7F807F80u) | (__byte_perm(t.man, 0u, 0x3322) & 0x807F807Fu);
+                w01 = exp_or_man(a01 << 3, __byte_perm(t.man, 0u, 0x1100));
+                w23 = exp_or_man(a23 << 3, __byte_perm(t.man, 0u, 0x3322));
             }
             const uint32_t col0 = t.cb * 128 + tsel * 32 + quad * 4;
             if (col0 < g.N) {

@@ -380,7 +380,7 @@ static LinArgs base_args(const ci_tiled_weight *w) {
 static size_t workspace_bytes(uint32_t M, uint32_t n_out) {
     uint32_t mt = M < 16 ? M : 16;
     size_t split = (size_t)kMaxSplits * mt * n_out * sizeof(float);
-    size_t slots = (size_t)sm_count() * 16 + (n_out + 31) / 32 + 2;
+    size_t slots = (size_t)sm_count() * 24 + (n_out + 31) / 32 + 2;
     size_t streamk = slots * mt * 32 * sizeof(float);
     return (size_t)kTicketBytes * 4 + (split > streamk ? split : streamk);
 }

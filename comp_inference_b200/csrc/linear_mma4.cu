@@ -40,8 +40,9 @@
 
 namespace ci {
 
-constexpr uint32_t kBar4Bytes = 640;         // up to 16 warps x (2 window stages + 2 mantissa chunks) x 8 B
+constexpr uint32_t kBar4Bytes = 768;         // up to 21 warps x (2 window stages + 2 mantissa chunks) x 8 B, the table's
 constexpr uint32_t kMma4Warps = 16;          // x 32 threads x 128 registers = the register file
+constexpr uint32_t kMma4ManyWarps = 21;      // with 96 registers (some spilled): where it saves a round of units
 
 struct Mma4Args {
     LinArgs a;
@@ -64,9 +65,7 @@ __device__ __forceinline__ uint32_t weight_pair4(uint32_t e_lo, uint32_t e_hi, u
     // place in a bf16 pair; whatever else the shift drags along is masked out by the bit-select.
     const uint32_t ee = __byte_perm(e_lo, e_hi, 0x6521) << 3;
     const uint32_t vv = __byte_perm(m_lo, m_hi, 0x4400 + 0x1111 * C);
-    uint32_t w;                                                 // bit-select in one instruction
-    asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(w) : "r"(ee), "r"(vv), "n"(0x7F807F80));
-    return w;
+    return exp_or_man(ee, vv);
 }
 
 // Four symbols of each of the lane's streams -> four packed weight pairs per column -> tensor core.
@@ -108,8 +107,8 @@ __device__ __forceinline__ void group4(uint32_t (&b)[4][2], Quad &z, uint32_t lu
 // half of the upper tile, which always exists).  Its products are exact zeros.  Where K ends inside a group of four, the
 // weights decoded past the end of the stream are masked to zero (the activations there are zero already).
 __device__ __align__(16) uint16_t g_zero_activations[256];     // 64 per unit are read, 8 more are prefetched
-template <bool HI, bool RAGGED>
-__global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid_constant__ Mma4Args p) {
+template <bool HI, bool RAGGED, uint32_t MAX_WARPS>
+__global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_constant__ Mma4Args p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const LinArgs &a = p.a;
     const Geom &g = a.g;
@@ -130,7 +129,9 @@ __global__ void __launch_bounds__(kMma4Warps * 32, 1) k_linear_mma4(const __grid
     const uint32_t gq = lane >> 2, q = lane & 3;                // column quad and row segment of this lane
     const uint32_t tsel = q >> 1, hsel = q & 1;                 // upper / lower tile, top / bottom half
 
-    const uint32_t gw = blockIdx.x * W + warp;                  // this warp's rank in the grid
+    // This warp's rank in the grid.  Runs differ by one unit in a regular pattern along the ranks: counted through one
+    // scheduler's warps (warp % 4) after the other, so that the longer runs do not all meet on the same ones.
+    const uint32_t gw = blockIdx.x * W + (warp & 3) * (W >> 2) + min(warp & 3, W & 3) + (warp >> 2);
     const uint32_t lo = gw < p.slots ? gw * p.total / p.slots : p.total;       // slots * total fits 32 bits
     const uint32_t hi = gw < p.slots ? (gw + 1) * p.total / p.slots : p.total;
 
@@ -595,17 +596,20 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     // (measured cross-over: 4096 x 2048 at tile height 128).  The two-streams kernel takes tiles of up to 256 rows.
     if (g.th <= 256 && p.total < P * CI_MMA4_MIN_UNITS) return 1;
     // One CTA per multiprocessor, the units dealt out in equal runs (they differ by one at most).  The warp count decides
-    // how well the last round is filled: 4096 x 22016 runs in five rounds of 15 warps, 82 us, against 90 for 14 or 11.  A second window per warp, which hides the
-    // copies of the next unit, is worth 2 %: less than a warp that would not fit beside it.
+    // how well the last round is filled: 11008 x 4096 takes two rounds of 19 warps (41.5 us) or three of 13 (46.7),
+    // 4096 x 22016 five of 15 or 16 (77) instead of six of 14 (86).  A second window per warp, which hides the copies of
+    // the next unit, is worth 2 %: less than a warp that would not fit beside it.
     uint32_t warps = 0;
+    bool many = false;
     double best = 0.0;
+    const uint32_t units = (p.total + P - 1) / P;
     for (uint32_t stages = 2; stages >= 1; --stages) {
         uint32_t w_max = room / (stages * p.stage_bytes + kManBytes);
-        if (w_max > kMma4Warps) w_max = kMma4Warps;
+        if (w_max > kMma4ManyWarps) w_max = kMma4ManyWarps;
         for (uint32_t w = 1; w <= w_max; ++w) {
-            const uint64_t rounds = (p.total + (uint64_t)P * w - 1) / ((uint64_t)P * w);
-            const double cost = (double)rounds * round_cost(w) * (stages == 1 ? 1.02 : 1.0);
-            if (warps == 0 || cost < best) { best = cost; warps = w; p.stages = stages; }
+            const bool m = w > kMma4Warps;                      // more spilled registers with a second set of accumulators
+            const double cost = run_cost(units, w, 0.9) * (stages == 1 ? 1.02 : 1.0) * (m && a.M > 8 ? 1.12 : 1.0);
+            if (warps == 0 || cost < best) { best = cost; warps = w; many = m; p.stages = stages; }
         }
     }
     if (warps == 0 || (g.th <= 256 && warps < 4)) return 1;
@@ -620,10 +624,13 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     if (a.dry_run) return CI_OK;                                // qualification only
 
     const bool ragged = g.K % (2 * g.th) != 0;
-    static void (*const kernels[4])(Mma4Args) = {k_linear_mma4<false, false>, k_linear_mma4<true, false>,
-                                                  k_linear_mma4<false, true>, k_linear_mma4<true, true>};
-    static SmemLimit lim[4] = {};
-    const int which = (a.M > 8) + 2 * ragged;
+    static void (*const kernels[8])(Mma4Args) = {
+        k_linear_mma4<false, false, kMma4Warps>,     k_linear_mma4<true, false, kMma4Warps>,
+        k_linear_mma4<false, true, kMma4Warps>,      k_linear_mma4<true, true, kMma4Warps>,
+        k_linear_mma4<false, false, kMma4ManyWarps>, k_linear_mma4<true, false, kMma4ManyWarps>,
+        k_linear_mma4<false, true, kMma4ManyWarps>,  k_linear_mma4<true, true, kMma4ManyWarps>};
+    static SmemLimit lim[8] = {};
+    const int which = (a.M > 8) + 2 * ragged + 4 * many;
     void (*kernel)(Mma4Args) = kernels[which];
     if (int rc = ensure_smem_limit(lim[which], (const void *)kernel, (size_t)max_smem)) return rc;
     // Programmatic dependent launch: the grid may be scheduled while the previous kernel of the stream

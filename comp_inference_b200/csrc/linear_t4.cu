@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
                             z.step(lut_s, e);
                             const uint32_t m = lds_u32(ms + (i + k) * 16);
                             const uint32_t e01 = __byte_perm(e[0], e[1], 0x6521) << 3, e23 = __byte_perm(e[2], e[3], 0x6521) << 3;
-                            w[k] = (e01 & 0x7F807F80u) | (__byte_perm(m, 0u, 0x1100) & 0x807F807Fu);
-                            w[2 + k] = (e23 & 0x7F807F80u) | (__byte_perm(m, 0u, 0x3322) & 0x807F807Fu);
+                            w[k] = exp_or_man(e01, __byte_perm(m, 0u, 0x1100));
+                            w[2 + k] = exp_or_man(e23, __byte_perm(m, 0u, 0x3322));
                         }
                         mma_bf16(d, w, xb[0], xb[1]);
                         if (live_m) {
@@ -327,8 +327,8 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
             uint32_t w_max = room / warp_bytes;
             if (w_max > kT4Warps) w_max = kT4Warps;
             for (uint32_t w = 1; w <= w_max; ++w) {
-                const uint64_t per_cta = (p.total + blocks - 1) / blocks, rounds = (per_cta + w - 1) / w;
-                const double cost = (double)((a.M + mt - 1) / mt) * rounds * round_cost(w) * (stages == 1 ? 1.02 : 1.0);
+                const double cost = (double)((a.M + mt - 1) / mt) * run_cost((p.total + blocks - 1) / blocks, w, 0.0) *
+                                    (stages == 1 ? 1.02 : 1.0);
                 if (warps == 0 || cost < best) {
                     best = cost;
                     warps = w;

@@ -67,6 +67,13 @@ __device__ __forceinline__ uint32_t weight_pair(uint32_t e_lo, uint32_t e_hi, ui
     return (ee & 0x7F807F80u) | (vv & 0x807F807Fu);
 }
 
+// Exponent bits of a packed bf16 pair from ee, the rest from vv: a bit-select, which the compiler makes two instructions of.
+__device__ __forceinline__ uint32_t exp_or_man(uint32_t ee, uint32_t vv) {
+    uint32_t w;
+    asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(w) : "r"(ee), "r"(vv), "n"(0x7F807F80));
+    return w;
+}
+
 __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
@@ -240,9 +247,19 @@ __device__ __forceinline__ bool wait_lut(uint32_t bar, const uint32_t *lut) { re
 constexpr uint32_t kChunkRows = 16;
 constexpr uint32_t kSegPitch = kChunkRows * 32 + 32;
 constexpr uint32_t kManBytes = 2 * 4 * kSegPitch;
-// Time of a round of units with w warps on a multiprocessor, us at 64 symbols per stream: measured for 11 to 16 warps;
-// a warp alone on its scheduler takes about twice the constant.
-inline double round_cost(uint32_t w) { return w < 5 ? 7.15 : 3.4 + 0.75 * w; }
+// Cost model of the persistent kernels' launches, in us at 64 symbols per stream.  A round of units -- every one of w warps
+// takes one -- lasts 3.6 + 0.75 x warps, where a scheduler with a warp more than the others counts half (measured in full
+// rounds of the fused linear: 12 warps 12.7, 14 14.8, 16 15.6; up to four warps have a scheduler each and take 7.2).
+// `extra` is what a round of more than 16 warps costs on top, where they have fewer registers or a pipe is full already.
+inline double round_cost(uint32_t w, double extra) {
+    if (w <= 4) return 7.2;
+    return 3.6 + 0.375 * (w + (w + 3) / 4 * 4) + (w > 16 ? extra : 0.0);
+}
+// `units` units on a multiprocessor with w warps: full rounds, then what is left on fewer warps.
+inline double run_cost(uint32_t units, uint32_t w, double extra) {
+    const double tail = units % w ? round_cost(units % w, extra) : 0.0;
+    return (units / w) * round_cost(w, extra) + tail;
+}
 
 // Lane 0 polls an mbarrier phase, bounded; the verdict is broadcast to the warp.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
