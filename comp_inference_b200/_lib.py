@@ -66,6 +66,7 @@ SIGNATURES = {
     "ci_compress_plane": (C.c_int, [_V, C.c_uint32, C.c_uint32, _V, _V, C.c_uint32, C.c_uint32] + [_V] * 7 +
                           [C.c_size_t, u64p, _S]),
     "ci_compress_pack": (C.c_int, [C.c_uint32] * 4 + [_V] * 4 + [C.c_size_t, _V, C.c_uint64, _S]),
+    "ci_build_entry_points": (C.c_int, [C.POINTER(TiledWeight), C.c_uint32, _V, _V, _V, _V, _S]),
     "ci_decode_plane": (C.c_int, [C.POINTER(TiledWeight), _V, _S]),
     "ci_decode_bf16": (C.c_int, [C.POINTER(TiledWeight), _V, _S]),
     "ci_decode_plane_dense": (C.c_int, [C.POINTER(DenseWeight), _V, _S]),

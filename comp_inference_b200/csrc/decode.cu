@@ -268,6 +268,24 @@ using namespace ci;
 
 extern "C" {
 
+int ci_build_entry_points(const ci_tiled_weight *w, uint32_t step, uint32_t *d_states, uint16_t *d_rows, uint32_t *d_spans,
+                          uint32_t *d_cap, ci_stream_t stream) {
+    int rc = check_weight(w, false);
+    if (rc) return rc;
+    CI_REQUIRE(d_states && d_rows && d_spans && d_cap, "null pointer");
+    CI_REQUIRE(w->tile_w == 32 && step >= 16 && step % 16 == 0 && w->tile_h % (2 * step) == 0 && w->tile_h <= 65536,
+               "no entry points every %u rows for %u x %u tiles", step, w->tile_h, w->tile_w);
+    CI_REQUIRE(w->max_tile_len != 0, "max_tile_len must be known");
+    CI_REQUIRE((reinterpret_cast<uintptr_t>(d_states) & 15u) == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15u) == 0,
+               "entry arrays must be 16-byte aligned");
+    rc = build_entry_points(make_args(w), w->max_tile_len, step, d_states, d_rows, d_spans, d_cap, (cudaStream_t)stream);
+    if (rc == 1) {
+        set_error("this weight does not qualify for the staged decoder (alignment, depth of its tiles)");
+        return CI_E_INVALID;
+    }
+    return rc;
+}
+
 int ci_decode_plane(const ci_tiled_weight *w, uint8_t *d_out, ci_stream_t stream) {
     return decode_tiled<false>(w, d_out, (cudaStream_t)stream);
 }

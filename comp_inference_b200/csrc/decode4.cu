@@ -31,11 +31,16 @@ struct Dec4Args {
     uint32_t stages;       // windows per warp
     uint32_t pairs_n;      // tile pairs per tile row = ceil(tiles_n / 2)
     uint32_t total;        // units
+    uint32_t step, subs;   // INDEX: rows between entry points, entry points per half tile
+    uint32_t *entry_states;
+    uint16_t *entry_rows;
 };
 
+// INDEX: nothing is stored but the decoder's state every `step` symbols, and for every stream the rows of its byte block
+// that are left then.
 // EDGE: the last tile row is not whole (rows beyond K are decoded to garbage and not stored), or output rows cannot be
 // written as aligned quads (N or the address is odd).
-template <bool BF16, bool EDGE>
+template <bool BF16, bool EDGE, bool INDEX>
 __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_constant__ Dec4Args p, void *out) {
     extern __shared__ __align__(128) uint8_t smem[];
     const DecArgs &a = p.a;
@@ -190,6 +195,17 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
             }
             if (c == 0 && p.stages == 2) next_unit();           // behind it: a chunk's arrival waits for older copies
             if (BF16) (void)mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1);
+            if constexpr (INDEX) {
+                if (c * kChunkRows % p.step == 0 && tile_live) {
+                    const size_t at = (((size_t)t0 + tsel) * p.subs + c * kChunkRows / p.step) * 64 + hsel * 32 + (quad & 7) * 4;
+                    const uint32_t below = win_s + tsel * 64 + hsel * 32 + (quad & 7) * 4 - 128;
+                    *reinterpret_cast<uint4 *>(p.entry_states + at) = make_uint4(z.s[0], z.s[1], z.s[2], z.s[3]);
+                    uint32_t left[4];                           // a used-up stream's cursor was clamped to the window: none or one
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) left[j] = z.p[j] > below + j ? (z.p[j] - below - j) >> 7 : 0u;
+                    *reinterpret_cast<uint2 *>(p.entry_rows + at) = make_uint2(left[0] | left[1] << 16, left[2] | left[3] << 16);
+                }
+            }
             z.clamp(win_s);
             uint32_t ms = man_s + (buf * 4 + tsel * 2 + hsel) * kSegPitch + (quad & 7) * 4;
             const uint32_t n = min(kChunkRows, g.half - c * kChunkRows);
@@ -201,6 +217,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
                     z.step(lut_s, e);
                     // bits 8..23 of two entries side by side: the symbols sit at bits 4..11 / 20..27
                     const uint32_t a01 = __byte_perm(e[0], e[1], 0x6521), a23 = __byte_perm(e[2], e[3], 0x6521);
+                    if constexpr (INDEX) continue;
                     const bool store = EDGE ? i < rows_left : rows_left != 0;
                     if (BF16) {
                         const uint32_t m = lds_u32(ms + i * 32);
@@ -249,13 +266,33 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     }
 }
 
+// One warp per tile: rows [lowest, lowest + depth) of the byte block that the symbols from an entry point to the next touch,
+// and every stream's next byte relative to that.  rows: in, bytes left; out, the index of the next byte in the span.
+__global__ void __launch_bounds__(256) k_entry_spans(uint16_t *rows, uint32_t *spans, uint32_t tiles, uint32_t subs, uint32_t *cap) {
+    const uint32_t t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = lane_id();
+    if (t >= tiles) return;
+    uint32_t *r = reinterpret_cast<uint32_t *>(rows + (size_t)t * subs * 64) + lane;     // two streams a lane
+    uint32_t cur = r[0], deepest = 0;
+    for (uint32_t s = 0; s < subs; ++s) {
+        const uint32_t nxt = s + 1 < subs ? r[(s + 1) * 32] : 0u;
+        const uint32_t hi = __reduce_max_sync(kFull, max(cur & 0xFFFFu, cur >> 16));
+        const uint32_t lo = min(hi, __reduce_min_sync(kFull, min(nxt & 0xFFFFu, nxt >> 16)));
+        auto rel = [&](uint32_t left) { return left > lo + 1 ? left - 1 - lo : 0u; };
+        r[s * 32] = rel(cur & 0xFFFFu) | rel(cur >> 16) << 16;
+        if (lane == 0) spans[(size_t)t * subs + s] = lo | (hi - lo) << 16;
+        deepest = max(deepest, hi - lo);
+        cur = nxt;
+    }
+    if (lane == 0) atomicMax(cap, deepest);
+}
+
 // ------------------------------------------------------------------------ host
 
-template <bool BF16, bool EDGE>
+template <bool BF16, bool EDGE, bool INDEX>
 static int launch_dec4(const Dec4Args &p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, void *out,
                        cudaStream_t s) {
     static SmemLimit lim = {};
-    if (int rc = ensure_smem_limit(lim, (const void *)k_decode4<BF16, EDGE>, (size_t)max_smem)) return rc;
+    if (int rc = ensure_smem_limit(lim, (const void *)k_decode4<BF16, EDGE, INDEX>, (size_t)max_smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(warps * 32);
@@ -266,12 +303,31 @@ static int launch_dec4(const Dec4Args &p, uint32_t blocks, uint32_t warps, size_
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CI_CUDA(cudaLaunchKernelEx(&cfg, k_decode4<BF16, EDGE>, p, out));
+    CI_CUDA(cudaLaunchKernelEx(&cfg, k_decode4<BF16, EDGE, INDEX>, p, out));
+    return CI_OK;
+}
+
+static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t step, uint32_t *entry_states,
+                   uint16_t *entry_rows, cudaStream_t s);
+
+int build_entry_points(const DecArgs &a, uint32_t max_tile_len, uint32_t step, uint32_t *d_states, uint16_t *d_rows,
+                       uint32_t *d_spans, uint32_t *d_cap, cudaStream_t s) {
+    const int rc = decode4(a, max_tile_len, false, nullptr, step, d_states, d_rows, s);
+    if (rc) return rc;
+    CI_CUDA(cudaMemsetAsync(d_cap, 0, sizeof(uint32_t), s));
+    const uint32_t tiles = a.g.tiles_k * a.g.tiles_n;
+    k_entry_spans<<<(tiles + 7) / 8, 256, 0, s>>>(d_rows, d_spans, tiles, a.g.half / step, d_cap);
+    CI_LAUNCH_CHECK(k_entry_spans);
     return CI_OK;
 }
 
 // Returns CI_OK when it launched, 1 when the tensor does not qualify, < 0 on error.
 int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, cudaStream_t s) {
+    return decode4(a, max_tile_len, bf16, out, 0, nullptr, nullptr, s);
+}
+
+static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t step, uint32_t *entry_states,
+                   uint16_t *entry_rows, cudaStream_t s) {
     const Geom &g = a.g;
     if (g.tw != 32 || g.th % 16 != 0 || max_tile_len == 0) return 1;
     if (!a.stream_aligned || (reinterpret_cast<uintptr_t>(a.states) & 15u)) return 1;
@@ -285,6 +341,10 @@ int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     p.stage_bytes = (p.cap_rows * 128u + 512u + 127u) & ~127u;
     p.pairs_n = (g.tiles_n + 1) / 2;
     p.total = g.tiles_k * p.pairs_n;
+    p.step = step;
+    p.subs = step ? g.half / step : 0;
+    p.entry_states = entry_states;
+    p.entry_rows = entry_rows;
     const uint32_t fixed = 2 * kLutBytes + kDec4BarBytes;           // up to one table size is lost to the table's alignment
     const uint32_t room = (uint32_t)max_smem - fixed, man_bytes = bf16 ? kManBytes : 0u;
     // As in the fused linear: the warp count with the cheapest rounds; a second window where it costs no warp that pays.
@@ -304,10 +364,11 @@ int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     if (blocks > P) blocks = P;
     const size_t smem = fixed + (size_t)warps * (p.stages * p.stage_bytes + man_bytes);
     const bool edge = g.K % g.th != 0 || g.N % 4 != 0 || (reinterpret_cast<uintptr_t>(out) & (bf16 ? 7u : 3u)) != 0;
-    if (bf16) return edge ? launch_dec4<true, true>(p, blocks, warps, smem, max_smem, out, s)
-                          : launch_dec4<true, false>(p, blocks, warps, smem, max_smem, out, s);
-    return edge ? launch_dec4<false, true>(p, blocks, warps, smem, max_smem, out, s)
-                : launch_dec4<false, false>(p, blocks, warps, smem, max_smem, out, s);
+    if (step) return launch_dec4<false, false, true>(p, blocks, warps, smem, max_smem, nullptr, s);
+    if (bf16) return edge ? launch_dec4<true, true, false>(p, blocks, warps, smem, max_smem, out, s)
+                          : launch_dec4<true, false, false>(p, blocks, warps, smem, max_smem, out, s);
+    return edge ? launch_dec4<false, true, false>(p, blocks, warps, smem, max_smem, out, s)
+                : launch_dec4<false, false, false>(p, blocks, warps, smem, max_smem, out, s);
 }
 
 }  // namespace ci

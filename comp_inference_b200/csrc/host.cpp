@@ -77,9 +77,18 @@ Tensor decode_scratch(const Tensor &like, int64_t K, int64_t N) {
     return t.narrow(0, 0, K * N).view({K, N});
 }
 
+// Entry points into the streams of tall tiles (ci_build_entry_points): every kEntryStep rows, the length of a half tile of
+// the heights the kernels run best at.
+constexpr int64_t kEntryStep = 64;
+struct Entries {
+    Tensor states, rows, spans;
+    uint32_t cap = 0;
+};
+
 // The arrays of one compressed weight and its descriptor.
 struct Weight {
     Tensor stream, states, tables, slot_map, offsets, lens, mantissa, lut;
+    Entries entries;
     ci_tiled_weight w;
 
     bool matches(const Tensor &s, const Tensor &st, const Tensor &m, const Tensor &o, int64_t th, int64_t tw) const {
@@ -134,12 +143,13 @@ struct Derived {
     Ref tables, slot_map, lens;
     Tensor lut;
     uint32_t max_len;
+    Entries entries;
 };
 std::mutex g_derived_mutex;
 std::unordered_map<const void *, Derived> &g_derived = *new std::unordered_map<const void *, Derived>;   // by tile_max_lens' impl
 
 Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables, const Tensor &slot_map, const Tensor &offsets,
-             const Tensor &lens, const OptTensor &mantissa, int64_t K, int64_t N, int64_t th, int64_t tw) {
+             const Tensor &lens, const OptTensor &mantissa, int64_t K, int64_t N, int64_t th, int64_t tw, bool entries) {
     Weight h;
     h.stream = as_u8(stream_t, "compressed stream");
     h.states = as_u32(states, "states");
@@ -158,6 +168,7 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
         throw py::value_error("mantissa plane has " + std::to_string(h.mantissa.numel()) + " bytes, " +
                               std::to_string(tiles * th * tw) + " expected");
     uint32_t max_len = 0;
+    bool keep = false;
     // a contiguous copy made above is a new object on every call: nothing to remember
     if (h.tables.is_same(tables) && h.slot_map.is_same(slot_map) && h.lens.is_same(lens)) {
         const void *key = lens.unsafeGetTensorImpl();
@@ -167,18 +178,48 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
             if (it != g_derived.end() && it->second.lens.is(lens) && it->second.tables.is(tables) && it->second.slot_map.is(slot_map)) {
                 h.lut = it->second.lut;
                 max_len = it->second.max_len;
+                h.entries = it->second.entries;
             }
         }
         if (!h.lut.defined()) {
             h.lut = lib_attr("prepared_lut")(tables, slot_map).cast<Tensor>();
             max_len = lib_attr("max_tile_len")(lens).cast<uint32_t>();
-            std::lock_guard<std::mutex> lock(g_derived_mutex);
-            if (g_derived.size() > 4096) g_derived.clear();
-            g_derived.erase(key);
-            g_derived.emplace(key, Derived{Ref(tables), Ref(slot_map), Ref(lens), h.lut, max_len});
+            keep = true;
         }
     }
     fill(h, K, N, th, tw, max_len);
+    const bool tall = entries && h.lut.defined() && tw == 32 && th > 2 * kEntryStep && th % (2 * kEntryStep) == 0 && th <= 65536 &&
+                      (reinterpret_cast<uintptr_t>(h.w.stream) & 15u) == 0 && (reinterpret_cast<uintptr_t>(h.w.states) & 15u) == 0;
+    if (tall && !h.entries.states.defined() && max_len != 0) {
+        Entries e;
+        const int64_t n = tiles * (th / 2 / kEntryStep);
+        e.states = at::empty({n * 64}, h.states.options());
+        e.rows = at::empty({n * 64}, h.states.options().dtype(at::kShort));
+        e.spans = at::empty({n}, h.states.options());
+        Tensor cap = at::empty({1}, h.states.options().dtype(at::kInt));
+        check(ci_build_entry_points(&h.w, kEntryStep, (uint32_t *)e.states.data_ptr(), (uint16_t *)e.rows.data_ptr(),
+                                    (uint32_t *)e.spans.data_ptr(), (uint32_t *)cap.data_ptr(), stream()));
+        e.cap = std::max<uint32_t>(1, (uint32_t)cap.item<int32_t>());
+        h.entries = e;
+        keep = true;
+    }
+    if (tall && h.entries.states.defined()) {
+        h.w.entry_step = kEntryStep;
+        h.w.entry_states = (const uint32_t *)h.entries.states.data_ptr();
+        h.w.entry_rows = (const uint16_t *)h.entries.rows.data_ptr();
+        h.w.entry_spans = (const uint32_t *)h.entries.spans.data_ptr();
+        h.w.entry_cap = h.entries.cap;
+    }
+    if (keep) {
+        std::lock_guard<std::mutex> lock(g_derived_mutex);
+        // what belongs to weights that are gone goes with the next new one
+        for (auto it = g_derived.begin(); it != g_derived.end();)
+            it = it->second.lens.impl.expired() || it->second.tables.impl.expired() ? g_derived.erase(it) : std::next(it);
+        if (g_derived.size() > 4096) g_derived.clear();
+        const void *key = lens.unsafeGetTensorImpl();
+        g_derived.erase(key);
+        g_derived.emplace(key, Derived{Ref(tables), Ref(slot_map), Ref(lens), h.lut, max_len, h.entries});
+    }
     return h;
 }
 
@@ -318,7 +359,7 @@ py::tuple compress(const Tensor &w, int64_t th, int64_t tw, bool want_man_hist) 
 PYBIND11_MODULE(_ci_host, m) {
     py::class_<Weight>(m, "Weight", "Descriptor of a compressed weight and the tensors it points into")
         .def(py::init(&tiled), py::arg("stream"), py::arg("states"), py::arg("tables"), py::arg("slot_map"), py::arg("tile_offsets"),
-             py::arg("tile_max_lens"), py::arg("mantissas"), py::arg("K"), py::arg("N"), py::arg("tile_h"), py::arg("tile_w"))
+             py::arg("tile_max_lens"), py::arg("mantissas"), py::arg("K"), py::arg("N"), py::arg("tile_h"), py::arg("tile_w"), py::arg("entries") = false)
         .def("matches", &Weight::matches)
         .def("linear", &linear_call, py::arg("x"), py::arg("bias") = py::none(), py::arg("out") = py::none(), py::arg("split_k") = 0,
              py::arg("transposed") = false, py::arg("prefill_rows") = 0)

@@ -372,6 +372,13 @@ static LinArgs base_args(const ci_tiled_weight *w) {
     a.tile_max_lens = w->tile_max_lens; a.lut = w->lut; a.slot_map = w->slot_map; a.mantissa = w->mantissa;
     a.g = make_geom(w->K, w->N, w->tile_h, w->tile_w);
     a.stream_aligned = (reinterpret_cast<uintptr_t>(w->stream) & 15u) == 0;
+    if (w->entry_step != 0) {
+        a.entry_step = w->entry_step;
+        a.entry_cap = w->entry_cap;
+        a.entry_states = w->entry_states;
+        a.entry_rows = w->entry_rows;
+        a.entry_spans = w->entry_spans;
+    }
     return a;
 }
 

@@ -28,6 +28,10 @@ struct LinArgs {
     uint32_t *tickets;   // [items along the non-reduced dimension]
     float *partial;      // [splits][M][n_out]
     ArFuse ar;           // ar.world > 1: all-reduce the output over the ranks inside the kernel (M <= 2)
+    // entry points into the streams of tall tiles (ci_build_entry_points), step 0: none
+    uint32_t entry_step, entry_cap;
+    const uint32_t *entry_states, *entry_spans;
+    const uint16_t *entry_rows;
     uint32_t dry_run;    // launchers stop before the launch: "would this weight take the staged route?"
 };
 

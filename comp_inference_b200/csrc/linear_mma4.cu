@@ -51,6 +51,9 @@ struct Mma4Args {
     uint32_t slots;        // warps of the grid: warp i takes units [i * total / slots, (i + 1) * total / slots)
     uint32_t total;        // units in the matrix
     uint32_t pairs_k;      // tile-row pairs = ceil(tiles_k / 2)
+    uint32_t subs;         // units per pair: 1, or the entry points per half tile
+    uint32_t step;         // rows of a segment in a unit: half a tile, or the rows between entry points
+    uint32_t per_group;    // units of a column group = pairs_k * subs
     uint32_t stages;       // byte windows per warp: 2, or 1 where tall tiles leave no room for two
     uint32_t y_vec;        // outputs can be written as 16-byte rows of eight
     uint32_t x_step;       // elements from one row's activations k .. k+3 to k+4 .. k+7
@@ -99,15 +102,16 @@ __device__ __forceinline__ void group4(uint32_t (&b)[4][2], Quad &z, uint32_t lu
     }
 }
 
-// RAGGED: K is not a whole number of tile pairs, so the last unit of a column group lacks its lower tile or ends
+// RAGGED: K is not a whole number of tile pairs, so the last units of a column group lack their lower tile or end
 // inside a tile (an instantiation of its own: the common case carries none of the bookkeeping in its registers).
-// Every lane still runs the full warp-wide loop.  A lane whose segment has n_my < n_groups 4-row groups reads
-// zeros instead of activations from group n_my on, and -- so that what it multiplies by those zeros stays a
-// finite number -- starts its stream over whenever it has used it up (a lane without a segment decodes the top
-// half of the upper tile, which always exists).  Its products are exact zeros.  Where K ends inside a group of four, the
-// weights decoded past the end of the stream are masked to zero (the activations there are zero already).
-__device__ __align__(16) uint16_t g_zero_activations[256];     // 64 per unit are read, 8 more are prefetched
-template <bool HI, bool RAGGED, uint32_t MAX_WARPS>
+// Every lane still runs the full warp-wide loop.  A lane whose segment has n_my < n_blocks 4-row groups reads zeros instead
+// of activations from group n_my on, and what it decodes past the end of its stream is masked to zero.
+//
+// ENTRY: a unit is not a pair of whole tiles but the rows between two entry points of it (tall tiles: 512 symbols are one
+// serial chain).  The states and cursors of its streams come from the index, its window holds just the rows of the byte
+// blocks that those symbols touch.  4096 x 4096 at tile height 1024, one row: 63 us -> see the table in the design notes.
+__device__ __align__(16) uint16_t g_zero_activations[256];
+template <bool HI, bool RAGGED, bool ENTRY, uint32_t MAX_WARPS>
 __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_constant__ Mma4Args p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const LinArgs &a = p.a;
@@ -135,25 +139,33 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     const uint32_t lo = gw < p.slots ? gw * p.total / p.slots : p.total;       // slots * total fits 32 bits
     const uint32_t hi = gw < p.slots ? (gw + 1) * p.total / p.slots : p.total;
 
+    const uint32_t subs = ENTRY ? p.subs : 1u, step = ENTRY ? p.step : g.half;
+
     // Byte ranges of this warp's units, 32 at a time: lane j holds unit dbase + j.
     uint32_t d_off0 = 0, d_ml0 = 0, d_off1 = 0, d_ml1 = 0, dbase = lo;
     auto load_desc = [&]() {
         const uint32_t u = dbase + lane;
         if (u >= hi) return;
-        const uint32_t grp = u / p.pairs_k, pk = u - grp * p.pairs_k;
+        const uint32_t grp = u / p.per_group, v = u - grp * p.per_group, pk = v / subs, sub = v - pk * subs;
         const uint32_t t0 = (2 * pk) * g.tiles_n + grp;
-        d_off0 = __ldg(a.tile_offsets + t0);
-        d_ml0 = __ldg(a.tile_max_lens + t0);
+        auto range = [&](uint32_t t, uint32_t &off, uint32_t &ml) {
+            off = __ldg(a.tile_offsets + t);
+            if constexpr (ENTRY) {
+                const uint32_t span = __ldg(a.entry_spans + (size_t)t * subs + sub);   // first row | rows << 16
+                off += (span & 0xFFFFu) * 64;
+                ml = span >> 16;
+            } else {
+                ml = __ldg(a.tile_max_lens + t);
+            }
+        };
+        range(t0, d_off0, d_ml0);
         d_off1 = 0;
         d_ml1 = 0;
-        if (2 * pk + 1 < g.tiles_k) {
-            d_off1 = __ldg(a.tile_offsets + t0 + g.tiles_n);
-            d_ml1 = __ldg(a.tile_max_lens + t0 + g.tiles_n);
-        }
+        if (2 * pk + 1 < g.tiles_k) range(t0 + g.tiles_n, d_off1, d_ml1);
     };
 
-    // Starts every copy of the unit (grp, pk) into `stage` (whole warp).
-    auto issue = [&](uint32_t grp, uint32_t pk, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
+    // Starts every copy of the unit (grp, pk, sub) into `stage` (whole warp).
+    auto issue = [&](uint32_t grp, uint32_t pk, uint32_t sub, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
         const uint32_t t0 = (2 * pk) * g.tiles_n + grp;
         const bool two = 2 * pk + 1 < g.tiles_k;
         const uint32_t bar = bar_base + stage * 8;
@@ -164,9 +176,20 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
         }
         if (lane == 0) {
             fence_async_proxy();
-            mbar_expect_tx(bar, two ? 512u : 256u);
-            bulk_load(dst + st_off, a.states + (size_t)t0 * 64, 256, bar);
-            if (two) bulk_load(dst + st_off + 256, a.states + ((size_t)t0 + g.tiles_n) * 64, 256, bar);
+            if constexpr (ENTRY) {
+                const size_t e0 = ((size_t)t0 * subs + sub) * 64, e1 = e0 + (size_t)g.tiles_n * subs * 64;
+                mbar_expect_tx(bar, two ? 768u : 384u);
+                bulk_load(dst + st_off, a.entry_states + e0, 256, bar);
+                bulk_load(dst + st_off + 512, a.entry_rows + e0, 128, bar);
+                if (two) {
+                    bulk_load(dst + st_off + 256, a.entry_states + e1, 256, bar);
+                    bulk_load(dst + st_off + 640, a.entry_rows + e1, 128, bar);
+                }
+            } else {
+                mbar_expect_tx(bar, two ? 512u : 256u);
+                bulk_load(dst + st_off, a.states + (size_t)t0 * 64, 256, bar);
+                if (two) bulk_load(dst + st_off + 256, a.states + ((size_t)t0 + g.tiles_n) * 64, 256, bar);
+            }
         }
         // byte blocks: 16-byte pieces, piece i of a tile = (row i / 4, quarter i % 4)
         const uint8_t *s0 = a.stream + off0, *s1 = a.stream + off1;
@@ -176,13 +199,13 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     };
 
     // Sign+mantissa bytes of a unit's upper tile, this lane's 16-byte piece of every chunk row pair.
-    auto man_of = [&](uint32_t grp, uint32_t pk) {
-        return a.mantissa + ((size_t)2 * pk * g.tiles_n + grp) * (2 * seg_bytes) + lane * 16;
+    auto man_of = [&](uint32_t grp, uint32_t pk, uint32_t sub) {
+        return a.mantissa + ((size_t)2 * pk * g.tiles_n + grp) * (2 * seg_bytes) + (ENTRY ? sub * step * 32 : 0u) + lane * 16;
     };
     // Rows [kChunkRows * c, + kChunkRows) of the four segments of a unit into chunk buffer `buf`; src: man_of the unit.
     auto issue_man = [&](const uint8_t *src, bool two, uint32_t c, uint32_t buf) {
         const uint32_t dst = man_s + buf * (4 * kSegPitch) + lane * 16;
-        if (c * kChunkRows + (lane >> 1) < g.half) {
+        if (c * kChunkRows + (lane >> 1) < step) {
             src += c * (kChunkRows * 32);
             cp_async16(dst, src);
             cp_async16(dst + kSegPitch, src + seg_bytes);
@@ -206,10 +229,14 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     load_desc();
     uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
     uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
-    uint32_t grp = lo / p.pairs_k, pk = lo - grp * p.pairs_k;   // of unit t
+    uint32_t grp = lo / p.per_group, pk = lo - grp * p.per_group, sub = 0;   // of unit t
+    if constexpr (ENTRY) {
+        sub = pk % subs;
+        pk /= subs;
+    }
     if (lo < hi) {
-        issue(grp, pk, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
-        issue_man(man_of(grp, pk), 2 * pk + 1 < g.tiles_k, 0, 0);
+        issue(grp, pk, sub, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
+        issue_man(man_of(grp, pk, sub), 2 * pk + 1 < g.tiles_k, 0, 0);
     }
     if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
@@ -236,7 +263,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     // works on rows gq and gq + 8 of the activation batch, columns 8q .. 8q+7 of the group.
     auto flush = [&](uint32_t grp) {
         auto warp_of = [&](uint32_t u) { return ((u + 1) * p.slots - 1) / p.total; };
-        const uint32_t first_w = warp_of(grp * p.pairs_k), last_w = warp_of((grp + 1) * p.pairs_k - 1);
+        const uint32_t first_w = warp_of(grp * p.per_group), last_w = warp_of((grp + 1) * p.per_group - 1);
         const uint32_t count = last_w - first_w + 1;
         const uint32_t n0 = grp * 32 + 8 * q;
         auto store_row = [&](uint32_t m, const float (&v)[8]) {
@@ -406,46 +433,37 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     uint32_t parity0 = 0, parity1 = 0, stage = 0;
     uint32_t cur_grp = grp;
     zero_acc();
-    const uint32_t n_blocks = g.half / 4;                       // blocks of four symbols per stream
-    const uint32_t n_chunks = (g.half + kChunkRows - 1) / kChunkRows;
+    const uint32_t n_blocks = step / 4;                         // blocks of four symbols per stream
+    const uint32_t n_chunks = (step + kChunkRows - 1) / kChunkRows;
     const uint32_t ragged_pk = (g.K % (2 * g.th)) ? p.pairs_k - 1 : 0xFFFFFFFFu;   // the unit index with rows beyond K
     uint32_t chunk = 0;                                         // sign+mantissa chunks consumed: buffer and phase parity
 
     Quad z;
     for (uint32_t t = lo; t < hi; ++t) {
-        const bool wrap = pk + 1 == p.pairs_k;
-        const uint32_t n_grp = grp + wrap, n_pk = wrap ? 0u : pk + 1;   // of unit t + 1
-        const uint8_t *man = man_of(grp, pk);
+        const bool last_sub = !ENTRY || sub + 1 == subs, wrap = last_sub && pk + 1 == p.pairs_k;
+        const uint32_t n_grp = grp + wrap, n_pk = wrap ? 0u : pk + last_sub, n_sub = last_sub ? 0u : sub + 1;   // of unit t + 1
+        const uint8_t *man = man_of(grp, pk, sub);
         const bool two = 2 * pk + 1 < g.tiles_k;
         if (grp != cur_grp) {
             flush(cur_grp);
             zero_acc();
             cur_grp = grp;
         }
-        // Blocks of this lane's segment that exist (n_my) and of the stream it decodes (len); see the kernel's header.
-        uint32_t n_my = n_blocks, len = n_blocks;
-        uint32_t cut = 0;                                       // rows of the stream's last group, 0 = all four
-        uint32_t tsel_d = tsel, hsel_d = hsel;                  // the segment whose stream this lane decodes
+        const uint32_t krow = (2 * pk + tsel) * g.th + hsel * g.half + (ENTRY ? sub * step : 0u);
+        // Blocks of this lane's segment that exist, and the rows of the last one (0 = all four); see the kernel's header.
+        uint32_t n_my = n_blocks, cut = 0;
         if (RAGGED && pk == ragged_pk) {
-            const uint32_t r0 = (2 * pk + tsel) * g.th;
-            const uint32_t rows_t = r0 < g.K ? min(g.th, g.K - r0) : 0u;
-            const uint32_t seg = rows_t > hsel * g.half ? min(g.half, rows_t - hsel * g.half) : 0u;
-            n_my = len = (seg + 3) >> 2;
+            const uint32_t seg = krow < g.K ? min(step, g.K - krow) : 0u;
+            n_my = (seg + 3) >> 2;
             cut = seg & 3;
-            if (seg == 0) {                                     // nothing of its own: the upper tile's top half stands in
-                tsel_d = hsel_d = 0;
-                len = (min(g.half, g.K - 2 * pk * g.th) + 3) >> 2;
-                cut = min(g.half, g.K - 2 * pk * g.th) & 3;
-            }
         }
-        const uint32_t krow = (2 * pk + tsel) * g.th + hsel * g.half;
         uint32_t xs = p.x_step;
         const uint16_t *xp0 = x0 + (size_t)(krow >> 2) * xs, *xp1 = x1 + (size_t)(krow >> 2) * xs;
         if (RAGGED && n_my == 0) {
             xp0 = xp1 = g_zero_activations;
             xs = 0;
         }
-        const uint32_t ml = (RAGGED ? tsel_d : tsel) ? nx_ml1 : nx_ml0;
+        const uint32_t ml = tsel ? nx_ml1 : nx_ml0;
         auto next_unit = [&]() {                                // every lane is done with the window it goes to
             if (t + 1 >= hi) return;
             if (t + 1 - dbase == 32) {
@@ -457,15 +475,15 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
             nx_ml0 = __shfl_sync(kFull, d_ml0, j);
             nx_off1 = __shfl_sync(kFull, d_off1, j);
             nx_ml1 = __shfl_sync(kFull, d_ml1, j);
-            issue(n_grp, n_pk, p.stages == 1 ? 0u : stage ^ 1, nx_off0, nx_ml0, nx_off1, nx_ml1);
+            issue(n_grp, n_pk, n_sub, p.stages == 1 ? 0u : stage ^ 1, nx_off0, nx_ml0, nx_off1, nx_ml1);
         };
         __syncwarp();
 
         // ---- this lane's four streams --------------------------------------
         const uint32_t win_s = wbase_s + stage * p.stage_bytes;
-        const uint32_t st_s = win_s + st_off + (RAGGED ? tsel_d : tsel) * 256 + ((RAGGED ? hsel_d : hsel) * 32 + gq * 4) * 4;
-        uint32_t first = win_s + (RAGGED ? tsel_d : tsel) * 64 + (RAGGED ? hsel_d : hsel) * 32 + gq * 4;
-        if (ml <= p.cap_rows) first += (ml - 1) * 128;          // last byte row; an empty tile starts one row below
+        const uint32_t st_s = win_s + st_off + tsel * 256 + (hsel * 32 + gq * 4) * 4;
+        uint32_t first = win_s + tsel * 64 + hsel * 32 + gq * 4;
+        if (!ENTRY && ml <= p.cap_rows) first += (ml - 1) * 128;   // last byte row; an empty tile starts one row below
 
         // ---- wait for the bytes (bounded) -------------------------------------
         {
@@ -474,16 +492,25 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
             if (stage) parity1 ^= 1; else parity0 ^= 1;
         }
         z.start(st_s, first);
+        if constexpr (ENTRY) {                                  // every stream has its own row of the window
+            const uint32_t rows_s = win_s + st_off + 512 + tsel * 128 + (hsel * 32 + gq * 4) * 2;
+            const uint32_t r01 = lds_u32(rows_s), r23 = lds_u32(rows_s + 4);
+            const uint32_t top = p.cap_rows - 1;
+            z.p[0] += min(r01 & 0xFFFFu, top) * 128;
+            z.p[1] += min(r01 >> 16, top) * 128;
+            z.p[2] += min(r23 & 0xFFFFu, top) * 128;
+            z.p[3] += min(r23 >> 16, top) * 128;
+        }
 
         uint32_t wb[4][2] = {};
         uint32_t xf[4] = {};                                     // the group before: its weights, its activations
-        uint32_t blk = 0, left = len;                           // left: blocks until this lane's stream is used up (RAGGED)
+        uint32_t blk = 0;
 #pragma unroll 1
         for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
             const uint32_t buf = chunk & 1;
             __syncwarp();                                       // every lane is done with the other chunk buffer
             if (c + 1 < n_chunks) issue_man(man, two, c + 1, buf ^ 1);
-            else if (t + 1 < hi) issue_man(man_of(n_grp, n_pk), 2 * n_pk + 1 < g.tiles_k, 0, buf ^ 1);
+            else if (t + 1 < hi) issue_man(man_of(n_grp, n_pk, n_sub), 2 * n_pk + 1 < g.tiles_k, 0, buf ^ 1);
             if (c == 0 && p.stages == 2) next_unit();   // behind it: a chunk's arrival waits for older copies
             if (!mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1)) atomicExch(p.status, 1u);
             z.clamp(win_s);
@@ -500,11 +527,12 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
                 mma4<HI>(acc, wb, xf);
                 group4(wb, z, lut_s, m);
                 if constexpr (RAGGED) {
-                    if (cut != 0 && left == 1) {
+                    const uint32_t n = blk + 1 < n_my ? 4u : blk >= n_my ? 0u : cut ? cut : 4u;   // rows of the block that exist
+                    if (n < 4) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            wb[i][0] &= cut == 1 ? 0xFFFFu : 0xFFFFFFFFu;
-                            wb[i][1] &= cut == 3 ? 0xFFFFu : 0u;
+                            wb[i][0] &= n == 0 ? 0u : n == 1 ? 0xFFFFu : 0xFFFFFFFFu;
+                            wb[i][1] &= n == 3 ? 0xFFFFu : 0u;
                         }
                     }
                 }
@@ -518,12 +546,6 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
                         xs = 0;
                     }
                 }
-                if constexpr (RAGGED) {
-                    if (--left == 0) {                          // stream used up: start it over (its products meet zeros)
-                        left = len;
-                        z.start(st_s, first);
-                    }
-                }
             }
         }
         mma4<HI>(acc, wb, xf);
@@ -535,6 +557,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
         }
         grp = n_grp;
         pk = n_pk;
+        sub = n_sub;
     }
     flush(cur_grp);
 }
@@ -580,13 +603,19 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     CI_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     Mma4Args p;
     p.a = a;
-    p.cap_rows = max_tile_len;
-    p.stage_bytes = (p.cap_rows * 128u + 512u + 127u) & ~127u;
+    const bool entry = a.entry_step != 0 && a.entry_cap != 0 && g.half > a.entry_step && g.half % a.entry_step == 0 &&
+                       a.entry_step % kChunkRows == 0 &&
+                       ((reinterpret_cast<uintptr_t>(a.entry_states) | reinterpret_cast<uintptr_t>(a.entry_rows)) & 15u) == 0;
+    p.cap_rows = entry ? a.entry_cap : max_tile_len;
+    p.stage_bytes = (p.cap_rows * 128u + (entry ? 768u : 512u) + 127u) & ~127u;
     const uint32_t fixed = 2 * kLutBytes + kBar4Bytes;         // up to one table size is lost to the table's alignment
     const uint32_t room = (uint32_t)max_smem - fixed;
     const uint32_t P = (uint32_t)sm_count();
     p.pairs_k = (g.tiles_k + 1) / 2;
-    p.total = g.groups * p.pairs_k;
+    p.step = entry ? a.entry_step : g.half;
+    p.subs = g.half / p.step;
+    p.per_group = p.pairs_k * p.subs;
+    p.total = g.groups * p.per_group;
 #ifndef CI_MMA4_MIN_UNITS
 #define CI_MMA4_MIN_UNITS 6
 #endif
@@ -594,7 +623,7 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     // That pays once the multiprocessors are saturated (about eight warps each); a small matrix -- a
     // tensor-parallel shard, say -- is latency bound and finishes sooner with the shorter units
     // (measured cross-over: 4096 x 2048 at tile height 128).  The two-streams kernel takes tiles of up to 256 rows.
-    if (g.th <= 256 && p.total < P * CI_MMA4_MIN_UNITS) return 1;
+    if (g.th <= 256 && !entry && p.total < P * CI_MMA4_MIN_UNITS) return 1;
     // One CTA per multiprocessor, the units dealt out in equal runs (they differ by one at most).  The warp count decides
     // how well the last round is filled: 11008 x 4096 takes two rounds of 19 warps (41.5 us) or three of 13 (46.7),
     // 4096 x 22016 five of 15 or 16 (77) instead of six of 14 (86).  A second window per warp, which hides the copies of
@@ -612,7 +641,7 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
             if (warps == 0 || cost < best) { best = cost; warps = w; many = m; p.stages = stages; }
         }
     }
-    if (warps == 0 || (g.th <= 256 && warps < 4)) return 1;
+    if (warps == 0 || (g.th <= 256 && !entry && warps < 4)) return 1;
     const uint32_t warp_bytes = p.stages * p.stage_bytes + kManBytes;
     uint32_t blocks = (p.total + warps - 1) / warps;
     if (blocks > P) blocks = P;
@@ -624,13 +653,14 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     if (a.dry_run) return CI_OK;                                // qualification only
 
     const bool ragged = g.K % (2 * g.th) != 0;
-    static void (*const kernels[8])(Mma4Args) = {
-        k_linear_mma4<false, false, kMma4Warps>,     k_linear_mma4<true, false, kMma4Warps>,
-        k_linear_mma4<false, true, kMma4Warps>,      k_linear_mma4<true, true, kMma4Warps>,
-        k_linear_mma4<false, false, kMma4ManyWarps>, k_linear_mma4<true, false, kMma4ManyWarps>,
-        k_linear_mma4<false, true, kMma4ManyWarps>,  k_linear_mma4<true, true, kMma4ManyWarps>};
-    static SmemLimit lim[8] = {};
-    const int which = (a.M > 8) + 2 * ragged + 4 * many;
+#define CI_MMA4_SET(E, W)                                                                                            \
+    k_linear_mma4<false, false, E, W>, k_linear_mma4<true, false, E, W>, k_linear_mma4<false, true, E, W>,           \
+        k_linear_mma4<true, true, E, W>
+    static void (*const kernels[16])(Mma4Args) = {CI_MMA4_SET(false, kMma4Warps), CI_MMA4_SET(false, kMma4ManyWarps),
+                                                  CI_MMA4_SET(true, kMma4Warps), CI_MMA4_SET(true, kMma4ManyWarps)};
+#undef CI_MMA4_SET
+    static SmemLimit lim[16] = {};
+    const int which = (a.M > 8) + 2 * ragged + 4 * many + 8 * entry;
     void (*kernel)(Mma4Args) = kernels[which];
     if (int rc = ensure_smem_limit(lim[which], (const void *)kernel, (size_t)max_smem)) return rc;
     // Programmatic dependent launch: the grid may be scheduled while the previous kernel of the stream

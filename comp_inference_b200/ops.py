@@ -105,7 +105,7 @@ def fused_rans_linear_triton(x, compressed_data, initial_states, tables, slot_ma
     of another size).  ``SPLIT_K`` is honoured up to 16; 0 lets the library choose.
     """
     return _lib.host().Weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens, mantissas,
-                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n)).linear(
+                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n), True).linear(
         x, bias, out, int(SPLIT_K))
 
 

@@ -77,6 +77,7 @@ class _RansBase(nn.Module):
         return self._handle[1]
 
     _native_handle = None
+    _entries = False                # whether the module's kernel uses entry points into the streams of tall tiles
 
     def _native(self):
         """The same descriptor for the native host path (_lib.host()); rebuilt only if a buffer was replaced."""
@@ -85,7 +86,7 @@ class _RansBase(nn.Module):
                                       b["rans_exp_tile_offsets"], self.tile_k, self.tile_n):
             h = _lib.host().Weight(b["rans_exp_stream"], b["rans_exp_states"], b["rans_exp_tables"], b["rans_exp_slot_map"],
                                    b["rans_exp_tile_offsets"], b["rans_exp_tile_max_lens"], b["rans_man_raw"],
-                                   *self._stored_shape(), int(self.tile_k), int(self.tile_n))
+                                   *self._stored_shape(), int(self.tile_k), int(self.tile_n), self._entries)
             self.__dict__["_native_handle"] = h
         return h
 
@@ -135,6 +136,8 @@ class RansLinear(_RansBase):
             self.register_buffer("bias", torch.empty(out_features, dtype=torch.bfloat16))
         else:
             self.bias = None
+
+    _entries = True
 
     def _stored_shape(self):
         return self.in_features, self.out_features

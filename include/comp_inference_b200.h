@@ -64,6 +64,11 @@ typedef struct ci_tiled_weight {
     uint32_t K, N;                 /* logical matrix                                    */
     uint32_t tile_h, tile_w;       /* tile_h % 16 == 0; tile_w a power of two <= 128   */
     uint32_t max_tile_len;         /* max over tile_max_lens if known, else 0           */
+    uint32_t entry_step;           /* 0, or rows between the entry points below (the fields behind are then read) */
+    const uint32_t *entry_states;  /* from ci_build_entry_points: [tiles][tile_h / 2 / entry_step][2 * tile_w] */
+    const uint16_t *entry_rows;    /* the same */
+    const uint32_t *entry_spans;   /* [tiles][tile_h / 2 / entry_step] */
+    uint32_t entry_cap;            /* deepest span */
     uint32_t reserved;
 } ci_tiled_weight;
 
@@ -222,6 +227,15 @@ int ci_decode_bf16(const ci_tiled_weight *w, uint16_t *d_out, ci_stream_t stream
 /* Dense-layout counterparts. */
 int ci_decode_plane_dense(const ci_dense_weight *w, uint8_t *d_out, ci_stream_t stream);
 int ci_decode_bf16_dense(const ci_dense_weight *w, uint16_t *d_out, ci_stream_t stream);
+
+/* Entry points of a weight with tall 32-wide tiles (tile_h / 2 a multiple of `step`, step a multiple of 16): the decoder
+ * state of every stream before rows 0, step, 2 step, ... of its half tile, where its next byte lies, and which rows of
+ * the tile's byte block those step symbols touch.  ci_linear and ci_embedding then enter a stream at these rows instead
+ * of decoding it from its start: a stream of tile_h / 2 symbols is one serial chain.  6 bytes per `step` symbols; the
+ * arrays hold tiles * (tile_h / 2 / step) * 64 entries (states, rows) and * 1 (spans); *d_cap receives the deepest span,
+ * for entry_cap.  Derived data, like the prepared decode table: build it once per weight.  Queued only. */
+int ci_build_entry_points(const ci_tiled_weight *w, uint32_t step, uint32_t *d_states, uint16_t *d_rows, uint32_t *d_spans,
+                          uint32_t *d_cap, ci_stream_t stream);
 
 /* ---- fused consumers ---------------------------------------------------- */
 
