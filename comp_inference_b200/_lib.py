@@ -69,6 +69,7 @@ SIGNATURES = {
     "ci_build_entry_points": (C.c_int, [C.POINTER(TiledWeight), C.c_uint32, _V, _V, _V, _V, _S]),
     "ci_decode_plane": (C.c_int, [C.POINTER(TiledWeight), _V, _S]),
     "ci_decode_bf16": (C.c_int, [C.POINTER(TiledWeight), _V, _S]),
+    "ci_decode_bf16_ld": (C.c_int, [C.POINTER(TiledWeight), _V, C.c_int64, _S]),
     "ci_decode_plane_dense": (C.c_int, [C.POINTER(DenseWeight), _V, _S]),
     "ci_decode_bf16_dense": (C.c_int, [C.POINTER(DenseWeight), _V, _S]),
     "ci_linear_workspace_bytes": (C.c_size_t, [C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32]),

@@ -219,17 +219,28 @@ static DecArgs make_args(const ci_tiled_weight *w) {
     a.tile_max_lens = w->tile_max_lens; a.lut = w->lut; a.slot_map = w->slot_map; a.mantissa = w->mantissa;
     a.g = make_geom(w->K, w->N, w->tile_h, w->tile_w);
     a.stream_aligned = (reinterpret_cast<uintptr_t>(w->stream) & 15u) == 0;
+    a.entry_step = w->entry_step;
+    if (a.entry_step != 0) {
+        a.entry_cap = w->entry_cap;
+        a.entry_states = w->entry_states;
+        a.entry_rows = w->entry_rows;
+        a.entry_spans = w->entry_spans;
+    }
     return a;
 }
 
 template <bool BF16>
-static int decode_tiled(const ci_tiled_weight *w, void *d_out, cudaStream_t s) {
+static int decode_tiled(const ci_tiled_weight *w, void *d_out, uint32_t ld, cudaStream_t s) {
     int rc = check_weight(w, BF16);
     if (rc) return rc;
     CI_REQUIRE(d_out != nullptr, "null output");
     DecArgs a = make_args(w);
-    rc = launch_decode4(a, w->max_tile_len, BF16, d_out, s);         // 32-wide tiles, whole tile rows
+    rc = launch_decode4(a, w->max_tile_len, BF16, d_out, ld ? ld : w->N, s);   // 32-wide tiles
     if (rc <= 0) return rc;
+    if (ld != 0 && ld != w->N) {
+        set_error("this weight does not qualify for the staged decoder, the only one that writes padded rows");
+        return CI_E_INVALID;
+    }
     rc = launch_decode_staged(a, w->max_tile_len, BF16, d_out, s);   // other staged shapes
     if (rc <= 0) return rc;
     uint32_t n_tasks = a.g.tiles_k * a.g.groups;
@@ -287,11 +298,16 @@ int ci_build_entry_points(const ci_tiled_weight *w, uint32_t step, uint32_t *d_s
 }
 
 int ci_decode_plane(const ci_tiled_weight *w, uint8_t *d_out, ci_stream_t stream) {
-    return decode_tiled<false>(w, d_out, (cudaStream_t)stream);
+    return decode_tiled<false>(w, d_out, 0, (cudaStream_t)stream);
 }
 int ci_decode_bf16(const ci_tiled_weight *w, uint16_t *d_out, ci_stream_t stream) {
-    return decode_tiled<true>(w, d_out, (cudaStream_t)stream);
+    return decode_tiled<true>(w, d_out, 0, (cudaStream_t)stream);
 }
+int ci_decode_bf16_ld(const ci_tiled_weight *w, uint16_t *d_out, int64_t ld, ci_stream_t stream) {
+    CI_REQUIRE(w != nullptr && ld >= (int64_t)w->N && ld <= 0xFFFFFFFFll, "row stride smaller than the row length");
+    return decode_tiled<true>(w, d_out, (uint32_t)ld, (cudaStream_t)stream);
+}
+
 int ci_decode_plane_dense(const ci_dense_weight *w, uint8_t *d_out, ci_stream_t stream) {
     return decode_dense<false>(w, d_out, (cudaStream_t)stream);
 }

@@ -31,16 +31,20 @@ struct Dec4Args {
     uint32_t stages;       // windows per warp
     uint32_t pairs_n;      // tile pairs per tile row = ceil(tiles_n / 2)
     uint32_t total;        // units
-    uint32_t step, subs;   // INDEX: rows between entry points, entry points per half tile
+    uint32_t ld;           // elements from one output row to the next
+    uint32_t vec;          // output rows can be written as aligned quads
+    uint32_t step, subs;   // INDEX, ENTRY: rows between entry points, entry points per half tile
     uint32_t *entry_states;
     uint16_t *entry_rows;
+    const uint32_t *entry_spans;
 };
 
+// ENTRY: units are the rows between two entry points of a tile pair, as in linear_mma4.cu.
 // INDEX: nothing is stored but the decoder's state every `step` symbols, and for every stream the rows of its byte block
 // that are left then.
 // EDGE: the last tile row is not whole (rows beyond K are decoded to garbage and not stored), or output rows cannot be
 // written as aligned quads (N or the address is odd).
-template <bool BF16, bool EDGE, bool INDEX>
+template <bool BF16, bool EDGE, bool INDEX, bool ENTRY>
 __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_constant__ Dec4Args p, void *out) {
     extern __shared__ __align__(128) uint8_t smem[];
     const DecArgs &a = p.a;
@@ -64,11 +68,18 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     // Rank in the grid, the CTA running fastest: what the last round lacks, it lacks on every multiprocessor alike.
     const uint32_t gw = warp * gridDim.x + blockIdx.x, n_warps = gridDim.x * W;
 
-    // Unit u = (tile row, tile pair), the pair running fastest: warps that run at the same time write
+    const uint32_t subs = ENTRY ? p.subs : 1u, step = ENTRY ? p.step : g.half;
+
+    // Unit u = (tile row, entry point, tile pair), the pair running fastest: warps that run at the same time write
     // neighbouring pieces of the same output rows.
-    auto unit_tiles = [&](uint32_t u, uint32_t &tk, uint32_t &tp, uint32_t &t0, bool &two) {
+    auto unit_tiles = [&](uint32_t u, uint32_t &tk, uint32_t &sub, uint32_t &tp, uint32_t &t0, bool &two) {
         tk = u / p.pairs_n;
         tp = u - tk * p.pairs_n;
+        sub = 0;
+        if constexpr (ENTRY) {
+            sub = tk % subs;
+            tk /= subs;
+        }
         t0 = tk * g.tiles_n + 2 * tp;
         two = 2 * tp + 1 < g.tiles_n;
     };
@@ -79,25 +90,42 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         const uint64_t u = (uint64_t)gw + (uint64_t)(dbase + lane) * n_warps;
         d_off0 = d_ml0 = d_off1 = d_ml1 = 0;
         if (u >= p.total) return;
-        uint32_t tk, tp, t0;
+        uint32_t tk, sub, tp, t0;
         bool two;
-        unit_tiles((uint32_t)u, tk, tp, t0, two);
-        d_off0 = __ldg(a.tile_offsets + t0);
-        d_ml0 = __ldg(a.tile_max_lens + t0);
-        if (two) {
-            d_off1 = __ldg(a.tile_offsets + t0 + 1);
-            d_ml1 = __ldg(a.tile_max_lens + t0 + 1);
-        }
+        unit_tiles((uint32_t)u, tk, sub, tp, t0, two);
+        auto range = [&](uint32_t t, uint32_t &off, uint32_t &ml) {
+            off = __ldg(a.tile_offsets + t);
+            if constexpr (ENTRY) {
+                const uint32_t span = __ldg(p.entry_spans + (size_t)t * subs + sub);   // first row | rows << 16
+                off += (span & 0xFFFFu) * 64;
+                ml = span >> 16;
+            } else {
+                ml = __ldg(a.tile_max_lens + t);
+            }
+        };
+        range(t0, d_off0, d_ml0);
+        if (two) range(t0 + 1, d_off1, d_ml1);
     };
 
-    auto issue = [&](uint32_t t0, bool two, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
+    auto issue = [&](uint32_t t0, uint32_t sub, bool two, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
         const uint32_t bar = bar_base + stage * 8;
         const uint32_t dst = wbase_s + stage * p.stage_bytes;
         if (ml0 > p.cap_rows || ml1 > p.cap_rows) ml0 = ml1 = 0;   // metadata disagrees with the declared maximum
         if (lane == 0) {
             fence_async_proxy();
-            mbar_expect_tx(bar, two ? 512u : 256u);
-            bulk_load(dst + st_off, a.states + (size_t)t0 * 64, two ? 512u : 256u, bar);   // the tiles are neighbours
+            if constexpr (ENTRY) {
+                const size_t e0 = ((size_t)t0 * subs + sub) * 64, e1 = e0 + (size_t)subs * 64;
+                mbar_expect_tx(bar, two ? 768u : 384u);
+                bulk_load(dst + st_off, p.entry_states + e0, 256, bar);
+                bulk_load(dst + st_off + 512, p.entry_rows + e0, 128, bar);
+                if (two) {
+                    bulk_load(dst + st_off + 256, p.entry_states + e1, 256, bar);
+                    bulk_load(dst + st_off + 640, p.entry_rows + e1, 128, bar);
+                }
+            } else {
+                mbar_expect_tx(bar, two ? 512u : 256u);
+                bulk_load(dst + st_off, a.states + (size_t)t0 * 64, two ? 512u : 256u, bar);   // the tiles are neighbours
+            }
         }
         const uint8_t *s0 = a.stream + off0, *s1 = a.stream + off1;
         for (uint32_t i = lane; i < ml0 * 4; i += 32) cp_async16(dst + (i >> 2) * 128 + (i & 3) * 16, s0 + i * 16);
@@ -106,10 +134,11 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     };
     // Sign+mantissa rows [kChunkRows * c, + kChunkRows) of the segments (left A, left B, right A, right B) of the unit whose
     // first tile is t0.
-    auto issue_man = [&](uint32_t t0, bool two, uint32_t c, uint32_t buf) {
-        const uint8_t *src = a.mantissa + (size_t)t0 * (2 * seg_bytes) + c * (kChunkRows * 32) + lane * 16;
+    auto issue_man = [&](uint32_t t0, uint32_t sub, bool two, uint32_t c, uint32_t buf) {
+        const uint8_t *src = a.mantissa + (size_t)t0 * (2 * seg_bytes) + (ENTRY ? sub * step * 32 : 0u) +
+                             c * (kChunkRows * 32) + lane * 16;
         const uint32_t dst = man_s + buf * (4 * kSegPitch) + lane * 16;
-        if (c * kChunkRows + (lane >> 1) < g.half) {
+        if (c * kChunkRows + (lane >> 1) < step) {
             cp_async16(dst, src);
             cp_async16(dst + kSegPitch, src + seg_bytes);
             if (two) {
@@ -131,12 +160,12 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     load_desc();
     uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
     uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
-    uint32_t tk = 0, tp = 0, t0 = 0;                            // of unit t
+    uint32_t tk = 0, sub = 0, tp = 0, t0 = 0;                   // of unit t
     bool two = false;
     if (gw < p.total) {
-        unit_tiles(gw, tk, tp, t0, two);
-        issue(t0, two, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
-        if (BF16) issue_man(t0, two, 0, 0);
+        unit_tiles(gw, tk, sub, tp, t0, two);
+        issue(t0, sub, two, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
+        if (BF16) issue_man(t0, sub, two, 0, 0);
     }
     if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
@@ -146,7 +175,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     (void)wait_lut(lut_bar, a.lut);
-    const uint32_t n_chunks = (g.half + kChunkRows - 1) / kChunkRows;
+    const uint32_t n_chunks = (step + kChunkRows - 1) / kChunkRows;
     uint32_t parity0 = 0, parity1 = 0, stage = 0, li = 0, chunk = 0;
     Quad z;
 
@@ -154,13 +183,13 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         const bool tile_live = tsel == 0 || two;
         const uint32_t col0 = 64 * tp + 4 * quad;               // first of this lane's four columns
         const uint32_t cols = tile_live && col0 < g.N ? min(4u, g.N - col0) : 0u;
-        const uint32_t row = tk * g.th + hsel * g.half;         // first row of this lane's streams
-        uint32_t rows_left = cols == 0 ? 0u : !EDGE ? 0xFFFFFFFFu : row < g.K ? min(g.half, g.K - row) : 0u;
+        const uint32_t row = tk * g.th + hsel * g.half + (ENTRY ? sub * step : 0u);   // first row of this lane's streams
+        uint32_t rows_left = cols == 0 ? 0u : !EDGE ? 0xFFFFFFFFu : row < g.K ? min(step, g.K - row) : 0u;
         const uint32_t ml = tsel ? nx_ml1 : nx_ml0;
         const bool more = (uint64_t)t + n_warps < p.total;
-        uint32_t n_tk = 0, n_tp = 0, n_t0 = 0;                  // of unit t + n_warps
+        uint32_t n_tk = 0, n_sub = 0, n_tp = 0, n_t0 = 0;       // of unit t + n_warps
         bool n_two = false;
-        if (more) unit_tiles(t + n_warps, n_tk, n_tp, n_t0, n_two);
+        if (more) unit_tiles(t + n_warps, n_tk, n_sub, n_tp, n_t0, n_two);
         auto next_unit = [&]() {
             if (!more) return;
             if (li + 1 - dbase == 32) {
@@ -172,26 +201,34 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
             nx_ml0 = __shfl_sync(kFull, d_ml0, j);
             nx_off1 = __shfl_sync(kFull, d_off1, j);
             nx_ml1 = __shfl_sync(kFull, d_ml1, j);
-            issue(n_t0, n_two, p.stages == 2 ? stage ^ 1 : 0u, nx_off0, nx_ml0, nx_off1, nx_ml1);
+            issue(n_t0, n_sub, n_two, p.stages == 2 ? stage ^ 1 : 0u, nx_off0, nx_ml0, nx_off1, nx_ml1);
         };
 
         const uint32_t win_s = wbase_s + stage * p.stage_bytes;
         const uint32_t st_s = win_s + st_off + tsel * 256 + (hsel * 32 + (quad & 7) * 4) * 4;
         uint32_t first = win_s + tsel * 64 + hsel * 32 + (quad & 7) * 4;
-        if (tile_live && ml <= p.cap_rows) first += (ml - 1) * 128;  // last byte row; an empty tile starts one row below
+        if (!ENTRY && tile_live && ml <= p.cap_rows) first += (ml - 1) * 128;  // last byte row; an empty tile starts one row below
         (void)mbar_wait(bar_base + stage * 8, stage ? parity1 : parity0);
         if (stage) parity1 ^= 1; else parity0 ^= 1;
         z.start(st_s, first);                                   // a tile that does not exist decodes what is in its place
+        if constexpr (ENTRY) {                                  // every stream has its own row of the window
+            const uint32_t rows_s = win_s + st_off + 512 + tsel * 128 + (hsel * 32 + (quad & 7) * 4) * 2;
+            const uint32_t r01 = lds_u32(rows_s), r23 = lds_u32(rows_s + 4), top = p.cap_rows - 1;
+            z.p[0] += min(r01 & 0xFFFFu, top) * 128;
+            z.p[1] += min(r01 >> 16, top) * 128;
+            z.p[2] += min(r23 & 0xFFFFu, top) * 128;
+            z.p[3] += min(r23 >> 16, top) * 128;
+        }
 
-        uint8_t *o8 = reinterpret_cast<uint8_t *>(out) + ((size_t)row * g.N + col0) * (BF16 ? 2 : 1);
-        const size_t o_pitch = (size_t)g.N * (BF16 ? 2 : 1);
+        uint8_t *o8 = reinterpret_cast<uint8_t *>(out) + ((size_t)row * p.ld + col0) * (BF16 ? 2 : 1);
+        const size_t o_pitch = (size_t)p.ld * (BF16 ? 2 : 1);
 #pragma unroll 1
         for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
             const uint32_t buf = chunk & 1;
             __syncwarp();                                       // every lane is done with the other buffers
             if (BF16) {
-                if (c + 1 < n_chunks) issue_man(t0, two, c + 1, buf ^ 1);
-                else if (more) issue_man(n_t0, n_two, 0, buf ^ 1);
+                if (c + 1 < n_chunks) issue_man(t0, sub, two, c + 1, buf ^ 1);
+                else if (more) issue_man(n_t0, n_sub, n_two, 0, buf ^ 1);
             }
             if (c == 0 && p.stages == 2) next_unit();           // behind it: a chunk's arrival waits for older copies
             if (BF16) (void)mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1);
@@ -208,7 +245,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
             }
             z.clamp(win_s);
             uint32_t ms = man_s + (buf * 4 + tsel * 2 + hsel) * kSegPitch + (quad & 7) * 4;
-            const uint32_t n = min(kChunkRows, g.half - c * kChunkRows);
+            const uint32_t n = min(kChunkRows, step - c * kChunkRows);
 #pragma unroll 1
             for (uint32_t r = 0; r < n; r += 4) {
 #pragma unroll
@@ -224,7 +261,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
                         const uint32_t w01 = exp_or_man(a01 << 3, __byte_perm(m, 0u, 0x1100));
                         const uint32_t w23 = exp_or_man(a23 << 3, __byte_perm(m, 0u, 0x3322));
                         if (store) {
-                            if (!EDGE) {
+                            if (!EDGE || (p.vec && cols == 4)) {
                                 *reinterpret_cast<uint2 *>(o8) = make_uint2(w01, w23);
                             } else {
                                 uint16_t *o = reinterpret_cast<uint16_t *>(o8);
@@ -237,7 +274,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
                     } else {
                         const uint32_t w = __byte_perm(a01 >> 4, a23 >> 4, 0x6420);
                         if (store) {
-                            if (!EDGE) {
+                            if (!EDGE || (p.vec && cols == 4)) {
                                 *reinterpret_cast<uint32_t *>(o8) = w;
                             } else {
                                 o8[0] = (uint8_t)w;
@@ -260,6 +297,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
             next_unit();
         }
         tk = n_tk;
+        sub = n_sub;
         tp = n_tp;
         t0 = n_t0;
         two = n_two;
@@ -288,11 +326,11 @@ __global__ void __launch_bounds__(256) k_entry_spans(uint16_t *rows, uint32_t *s
 
 // ------------------------------------------------------------------------ host
 
-template <bool BF16, bool EDGE, bool INDEX>
+template <bool BF16, bool EDGE, bool INDEX, bool ENTRY>
 static int launch_dec4(const Dec4Args &p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, void *out,
                        cudaStream_t s) {
     static SmemLimit lim = {};
-    if (int rc = ensure_smem_limit(lim, (const void *)k_decode4<BF16, EDGE, INDEX>, (size_t)max_smem)) return rc;
+    if (int rc = ensure_smem_limit(lim, (const void *)k_decode4<BF16, EDGE, INDEX, ENTRY>, (size_t)max_smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(warps * 32);
@@ -303,16 +341,16 @@ static int launch_dec4(const Dec4Args &p, uint32_t blocks, uint32_t warps, size_
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CI_CUDA(cudaLaunchKernelEx(&cfg, k_decode4<BF16, EDGE, INDEX>, p, out));
+    CI_CUDA(cudaLaunchKernelEx(&cfg, k_decode4<BF16, EDGE, INDEX, ENTRY>, p, out));
     return CI_OK;
 }
 
-static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t step, uint32_t *entry_states,
-                   uint16_t *entry_rows, cudaStream_t s);
+static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, uint32_t step,
+                   uint32_t *entry_states, uint16_t *entry_rows, cudaStream_t s);
 
 int build_entry_points(const DecArgs &a, uint32_t max_tile_len, uint32_t step, uint32_t *d_states, uint16_t *d_rows,
                        uint32_t *d_spans, uint32_t *d_cap, cudaStream_t s) {
-    const int rc = decode4(a, max_tile_len, false, nullptr, step, d_states, d_rows, s);
+    const int rc = decode4(a, max_tile_len, false, nullptr, a.g.N, step, d_states, d_rows, s);
     if (rc) return rc;
     CI_CUDA(cudaMemsetAsync(d_cap, 0, sizeof(uint32_t), s));
     const uint32_t tiles = a.g.tiles_k * a.g.tiles_n;
@@ -322,12 +360,12 @@ int build_entry_points(const DecArgs &a, uint32_t max_tile_len, uint32_t step, u
 }
 
 // Returns CI_OK when it launched, 1 when the tensor does not qualify, < 0 on error.
-int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, cudaStream_t s) {
-    return decode4(a, max_tile_len, bf16, out, 0, nullptr, nullptr, s);
+int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, cudaStream_t s) {
+    return decode4(a, max_tile_len, bf16, out, ld, 0, nullptr, nullptr, s);
 }
 
-static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t step, uint32_t *entry_states,
-                   uint16_t *entry_rows, cudaStream_t s) {
+static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, uint32_t step,
+                   uint32_t *entry_states, uint16_t *entry_rows, cudaStream_t s) {
     const Geom &g = a.g;
     if (g.tw != 32 || g.th % 16 != 0 || max_tile_len == 0) return 1;
     if (!a.stream_aligned || (reinterpret_cast<uintptr_t>(a.states) & 15u)) return 1;
@@ -337,14 +375,18 @@ static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     CI_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     Dec4Args p;
     p.a = a;
-    p.cap_rows = max_tile_len;
-    p.stage_bytes = (p.cap_rows * 128u + 512u + 127u) & ~127u;
+    const bool entry = bf16 && a.entry_step != 0 && a.entry_cap != 0 && g.half > a.entry_step && g.half % a.entry_step == 0 &&
+                       a.entry_step % kChunkRows == 0 &&
+                       ((reinterpret_cast<uintptr_t>(a.entry_states) | reinterpret_cast<uintptr_t>(a.entry_rows)) & 15u) == 0;
+    p.cap_rows = entry ? a.entry_cap : max_tile_len;
+    p.stage_bytes = (p.cap_rows * 128u + (entry ? 768u : 512u) + 127u) & ~127u;
     p.pairs_n = (g.tiles_n + 1) / 2;
-    p.total = g.tiles_k * p.pairs_n;
-    p.step = step;
-    p.subs = step ? g.half / step : 0;
-    p.entry_states = entry_states;
-    p.entry_rows = entry_rows;
+    p.step = entry ? a.entry_step : step;
+    p.subs = p.step ? g.half / p.step : 0;
+    p.total = g.tiles_k * p.pairs_n * (entry ? p.subs : 1u);
+    p.entry_states = entry ? const_cast<uint32_t *>(a.entry_states) : entry_states;
+    p.entry_rows = entry ? const_cast<uint16_t *>(a.entry_rows) : entry_rows;
+    p.entry_spans = a.entry_spans;
     const uint32_t fixed = 2 * kLutBytes + kDec4BarBytes;           // up to one table size is lost to the table's alignment
     const uint32_t room = (uint32_t)max_smem - fixed, man_bytes = bf16 ? kManBytes : 0u;
     // As in the fused linear: the warp count with the cheapest rounds; a second window where it costs no warp that pays.
@@ -363,12 +405,16 @@ static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     uint32_t blocks = (p.total + warps - 1) / warps;
     if (blocks > P) blocks = P;
     const size_t smem = fixed + (size_t)warps * (p.stages * p.stage_bytes + man_bytes);
-    const bool edge = g.K % g.th != 0 || g.N % 4 != 0 || (reinterpret_cast<uintptr_t>(out) & (bf16 ? 7u : 3u)) != 0;
-    if (step) return launch_dec4<false, false, true>(p, blocks, warps, smem, max_smem, nullptr, s);
-    if (bf16) return edge ? launch_dec4<true, true, false>(p, blocks, warps, smem, max_smem, out, s)
-                          : launch_dec4<true, false, false>(p, blocks, warps, smem, max_smem, out, s);
-    return edge ? launch_dec4<false, true, false>(p, blocks, warps, smem, max_smem, out, s)
-                : launch_dec4<false, false, false>(p, blocks, warps, smem, max_smem, out, s);
+    p.ld = ld;
+    p.vec = ld % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & (bf16 ? 7u : 3u)) == 0;
+    const bool edge = g.K % g.th != 0 || g.N % 4 != 0 || !p.vec;
+    if (step) return launch_dec4<false, false, true, false>(p, blocks, warps, smem, max_smem, nullptr, s);
+    if (entry) return edge ? launch_dec4<true, true, false, true>(p, blocks, warps, smem, max_smem, out, s)
+                           : launch_dec4<true, false, false, true>(p, blocks, warps, smem, max_smem, out, s);
+    if (bf16) return edge ? launch_dec4<true, true, false, false>(p, blocks, warps, smem, max_smem, out, s)
+                          : launch_dec4<true, false, false, false>(p, blocks, warps, smem, max_smem, out, s);
+    return edge ? launch_dec4<false, true, false, false>(p, blocks, warps, smem, max_smem, out, s)
+                : launch_dec4<false, false, false, false>(p, blocks, warps, smem, max_smem, out, s);
 }
 
 }  // namespace ci

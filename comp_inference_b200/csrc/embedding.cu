@@ -122,6 +122,13 @@ int ci_embedding(const ci_tiled_weight *w, const int64_t *d_ids, uint64_t n_ids,
     a.tile_max_lens = w->tile_max_lens; a.lut = w->lut; a.slot_map = w->slot_map; a.mantissa = w->mantissa;
     a.g = make_geom(w->K, w->N, w->tile_h, w->tile_w);
     a.ids = d_ids; a.n_ids = n_ids; a.out = d_out; a.ldo = ldo;
+    a.entry_step = w->entry_step;
+    if (a.entry_step != 0) {
+        a.entry_cap = w->entry_cap;
+        a.entry_states = w->entry_states;
+        a.entry_rows = w->entry_rows;
+        a.entry_spans = w->entry_spans;
+    }
     rc = launch_embedding4(a, w->max_tile_len, (cudaStream_t)stream);  // 32-wide tiles: four streams per lane
     if (rc <= 0) return rc;
     uint64_t tasks = n_ids * a.g.groups, blocks = (tasks + kEmbWarps - 1) / kEmbWarps, cap = (uint64_t)sm_count() * 8;

@@ -13,6 +13,10 @@ struct EmbArgs {
     uint64_t n_ids;
     uint16_t *out;
     int64_t ldo;
+    // entry points into the streams of tall tiles (ci_build_entry_points), step 0: none
+    uint32_t entry_step, entry_cap;
+    const uint32_t *entry_states, *entry_spans;
+    const uint16_t *entry_rows;
 };
 
 // Four-streams-per-lane gather for 32-wide tiles (embedding4.cu): CI_OK when launched, 1 when the

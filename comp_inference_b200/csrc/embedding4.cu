@@ -14,7 +14,7 @@
 // around them.  A warp therefore takes a run of consecutive tasks: eight at a time their ids are read and their tiles'
 // offsets and depths fetched, one tile per lane, while the eight before them are worked off; a task then costs two
 // shuffles for its lane's own tile, and no division.  Byte windows, initial states and the row's sign+mantissa bytes are
-// fetched one task ahead.  Measured, 4096 ids of 32000 x 4096 at tile height 16: 148 us with one task at a time,
+// fetched one task ahead.  Tall tiles are entered at the entry point before the row where the caller has them.  Measured, 4096 ids of 32000 x 4096 at tile height 16: 148 us with one task at a time,
 // divisions in 64 bits and eight shuffles per task -> see the table in the design notes.
 #include "embedding.cuh"
 #include "ptx.cuh"
@@ -32,8 +32,11 @@ struct Emb4Args {
     uint32_t blocks_n;     // 128-column blocks per row = ceil(tiles_n / 4)
     uint32_t total;        // tasks, the column block running fastest
     uint32_t out_vec;      // rows of the output can be written as 8-byte quads
+    uint32_t subs;         // ENTRY: entry points per half tile
 };
 
+// ENTRY: streams are entered at the entry point before the row (tall tiles), not at their start.
+template <bool ENTRY>
 __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_constant__ Emb4Args p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const EmbArgs &a = p.a;
@@ -83,9 +86,17 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
         const uint32_t tn = b.cb * 4 + (lane & 3);
         b.off = b.ml = 0;
         if (b.row != 0xFFFFFFFFu && tn < g.tiles_n) {
-            const size_t tile = (size_t)(b.row / g.th) * g.tiles_n + tn;
+            const uint32_t tk = b.row / g.th;
+            const size_t tile = (size_t)tk * g.tiles_n + tn;
             b.off = __ldg(a.tile_offsets + tile);
-            b.ml = __ldg(a.tile_max_lens + tile);
+            if constexpr (ENTRY) {
+                const uint32_t rel = b.row - tk * g.th, inner = rel >= g.half ? rel - g.half : rel;
+                const uint32_t span = __ldg(a.entry_spans + tile * p.subs + inner / a.entry_step);   // first row | rows << 16
+                b.off += (span & 0xFFFFu) * 64;
+                b.ml = span >> 16;
+            } else {
+                b.ml = __ldg(a.tile_max_lens + tile);
+            }
         }
         if (b.ml > p.cap_rows) b.ml = 0;                        // metadata disagrees with the declared maximum
     };
@@ -96,6 +107,7 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
         bool live;             // the id is inside the table and so is the lane's tile
         uint4 states;
         uint32_t man;
+        uint2 rows;            // ENTRY: next byte's row of every stream
     };
     // Task k of the batch: its copies into `stage`, its states and sign+mantissa bytes.
     auto open = [&](const Batch &b, uint32_t k, uint32_t stage, Task &t) {
@@ -112,10 +124,20 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
         t.man = 0;
         if (t.live) {
             const size_t tile = (size_t)tk * g.tiles_n + tn;
-            t.states = __ldg(reinterpret_cast<const uint4 *>(a.states + tile * 64 + h * 32 + quad * 4));
+            uint32_t rows;
+            if constexpr (ENTRY) {
+                const size_t e = (tile * p.subs + t.inner / a.entry_step) * 64 + h * 32 + quad * 4;
+                t.inner %= a.entry_step;
+                t.states = __ldg(reinterpret_cast<const uint4 *>(a.entry_states + e));
+                t.rows = __ldg(reinterpret_cast<const uint2 *>(a.entry_rows + e));
+                rows = t.ml;
+            } else {
+                t.states = __ldg(reinterpret_cast<const uint4 *>(a.states + tile * 64 + h * 32 + quad * 4));
+                rows = min(t.ml, 2 * t.inner + 2);
+            }
             t.man = __ldg(reinterpret_cast<const uint32_t *>(a.mantissa + tile * (g.th * 32) + rel * 32 + quad * 4));
             // eight lanes a tile: pieces of 16 bytes, two a row, from the last row upwards
-            const uint32_t rows = min(t.ml, 2 * t.inner + 2), skip = t.ml - rows;
+            const uint32_t skip = t.ml - rows;
             const uint8_t *src = a.stream + off + h * 32 + (size_t)(skip + (quad >> 1)) * 64 + (quad & 1) * 16;
             const uint32_t dst = wbase_s + stage * p.stage_bytes + (skip + (quad >> 1)) * 128 + tsel * 32 + (quad & 1) * 16;
             for (uint32_t i = quad >> 1; i < rows; i += 4) cp_async16(dst + (i - (quad >> 1)) * 128, src + (size_t)(i - (quad >> 1)) * 64);
@@ -150,9 +172,18 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
             z.s[1] = t.states.y;
             z.s[2] = t.states.z;
             z.s[3] = t.states.w;
-            const uint32_t start = win_s + tsel * 32 + quad * 4 + (t.ml ? (t.ml - 1) * 128 : 0u);
+            const uint32_t start = win_s + tsel * 32 + quad * 4 + (!ENTRY && t.ml ? (t.ml - 1) * 128 : 0u);
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j) z.p[j] = start + j;
+            if constexpr (ENTRY) {
+                const uint32_t top = p.cap_rows - 1;
+                if (t.live) {
+                    z.p[0] += min(t.rows.x & 0xFFFFu, top) * 128;
+                    z.p[1] += min(t.rows.x >> 16, top) * 128;
+                    z.p[2] += min(t.rows.y & 0xFFFFu, top) * 128;
+                    z.p[3] += min(t.rows.y >> 16, top) * 128;
+                }
+            }
             // The rows above the wanted one.  Lanes without a tile run along on whatever is in the window.
             const uint32_t drop = __shfl_sync(kFull, t.inner, 0);
 #pragma unroll 1
@@ -208,7 +239,10 @@ int launch_embedding4(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t s) {
     CI_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     Emb4Args p;
     p.a = a;
-    p.cap_rows = max_tile_len;
+    const bool entry = a.entry_step != 0 && a.entry_cap != 0 && g.half > a.entry_step && g.half % a.entry_step == 0 &&
+                       ((reinterpret_cast<uintptr_t>(a.entry_states) | reinterpret_cast<uintptr_t>(a.entry_rows)) & 15u) == 0;
+    p.cap_rows = entry ? a.entry_cap : max_tile_len;
+    p.subs = entry ? g.half / a.entry_step : 1u;
     p.stage_bytes = (p.cap_rows * 128u + 127u) & ~127u;
     p.blocks_n = (g.tiles_n + 3) / 4;
     p.out_vec = ((reinterpret_cast<uintptr_t>(a.out) & 7u) == 0 && (a.ldo & 3) == 0) ? 1u : 0u;
@@ -218,8 +252,9 @@ int launch_embedding4(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t s) {
     p.stages = room / (2 * p.stage_bytes) >= 12 ? 2 : 1;        // a deep window is worth doubling while 12 warps still fit
     uint32_t w_max = room / (p.stages * p.stage_bytes);
     if (w_max > kEmb4Warps) w_max = kEmb4Warps;
-    static SmemLimit lim = {};
-    if (int rc = ensure_smem_limit(lim, (const void *)k_embedding4, (size_t)max_smem)) return rc;
+    static SmemLimit lim[2] = {};
+    void (*const kernel)(Emb4Args) = entry ? k_embedding4<true> : k_embedding4<false>;
+    if (int rc = ensure_smem_limit(lim[entry], (const void *)kernel, (size_t)max_smem)) return rc;
     const uint32_t P = (uint32_t)sm_count();
     const uint64_t ids_per_launch = 0x40000000ull / p.blocks_n;     // task numbers fit 32 bits
     for (uint64_t i0 = 0; i0 < a.n_ids; i0 += ids_per_launch) {
@@ -239,7 +274,7 @@ int launch_embedding4(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t s) {
         at[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        CI_CUDA(cudaLaunchKernelEx(&cfg, k_embedding4, p));
+        CI_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
     }
     return CI_OK;
 }

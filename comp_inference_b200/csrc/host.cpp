@@ -260,10 +260,30 @@ Tensor linear_call(const Weight &h, const Tensor &x, const OptTensor &bias, cons
     const Rows r = rows_of(x, K);
     if (prefill_rows > 0 && r.M >= prefill_rows && !out.has_value()) {
         // many rows: one stand-alone decode into a reused buffer, then a library GEMM (see RansLinear)
-        Tensor w = decode_scratch(x, h.w.K, h.w.N);
-        check(ci_decode_bf16(&h.w, (uint16_t *)w.data_ptr(), stream()));
         Tensor x2 = r.keep.dim() == 2 ? r.keep : r.keep.view({r.M, K});
-        Tensor y = at::matmul(x2, transposed ? w.t() : w);
+        Tensor y;
+        const int64_t rows = (h.w.K + 7) / 8 * 8, cols = (h.w.N + 7) / 8 * 8;
+        if ((rows != h.w.K || cols != h.w.N) && h.w.tile_w == 32 && h.w.max_tile_len != 0) {
+            // Odd sizes: the library has only slow kernels for operands whose rows are not 16-byte aligned (3.5 times
+            // slower at 748 x 4873 x 13236), so the weight is decoded into padded rows and the activations are copied.
+            Tensor w = decode_scratch(x, rows, cols);
+            check(ci_decode_bf16_ld(&h.w, (uint16_t *)w.data_ptr(), cols, stream()));
+            if (rows != h.w.K) w.narrow(0, h.w.K, rows - h.w.K).zero_();
+            const int64_t Kp = transposed ? cols : rows;
+            if (transposed && cols != K) w.narrow(1, K, cols - K).zero_();
+            if (Kp != K || r.ld % 8) {
+                Tensor xp = at::empty({r.M, Kp}, x.options());
+                xp.narrow(1, 0, K).copy_(x2);
+                if (Kp != K) xp.narrow(1, K, Kp - K).zero_();
+                x2 = xp;
+            }
+            y = at::matmul(x2, transposed ? w.t() : w);
+            if (y.size(1) != n_out) y = y.narrow(1, 0, n_out).contiguous();
+        } else {
+            Tensor w = decode_scratch(x, h.w.K, h.w.N);
+            check(ci_decode_bf16(&h.w, (uint16_t *)w.data_ptr(), stream()));
+            y = at::matmul(x2, transposed ? w.t() : w);
+        }
         if (bias.has_value()) y.add_(*bias);
         return y.view(out_shape(x, n_out));
     }

@@ -122,7 +122,7 @@ def fused_rans_embedding_triton(x, compressed_data, initial_states, tables, slot
                                 tile_max_lens, tile_k, tile_n, mantissas, out=None):
     """out[..., :] = W[x[...], :]; ids outside [0, K) give zero rows."""
     return _lib.host().Weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens, mantissas,
-                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n)).embedding(x, out)
+                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n), True).embedding(x, out)
 
 
 # ---- dense ("uncoalesced") layout ------------------------------------------------

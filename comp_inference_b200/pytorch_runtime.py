@@ -258,6 +258,8 @@ class RansEmbedding(_RansBase):
         self.tile_k, self.tile_n = tile_k, tile_n
         self._register()
 
+    _entries = True
+
     def _stored_shape(self):
         return self.num_embeddings, self.embedding_dim
 

@@ -113,3 +113,20 @@ def test_embedding_edges(V, H, th, n):
     want = torch.where(((ids >= 0) & (ids < V))[:, None], W[ids.clamp(0, V - 1)].float(), torch.zeros((), device="cuda"))
     assert torch.equal(m(ids).float(), want)
     assert torch.equal(m(ids.view(1, -1).to(torch.int32))[0].float(), want)
+
+
+# prompts through the module: sizes whose rows the library cannot take aligned, tall tiles entered at entry points
+@pytest.mark.parametrize("K,N,th,M", [(1000, 776, 128, 20), (1001, 776, 128, 33), (1000, 777, 64, 17), (2305, 131, 1024, 65),
+                                      (3072, 512, 512, 40), (1024, 96, 1024, 18)])
+def test_prompt_edges(K, N, th, M):
+    import comp_inference_b200 as ci
+    W = _weight(K, N)
+    c = ci.compress_weight_cuda(W, th, 32)
+    m = ci.RansLinear(K, N, c["tile_height"], c["tile_width"], has_bias=True)
+    m.bias = torch.randn(N, generator=torch.Generator().manual_seed(N)).to(torch.bfloat16).cuda()
+    m.load_compressed(c).prepare()
+    x = torch.randn(2, M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).cuda()
+    for x in (x, x[:1, :, :].transpose(0, 1)):
+        y = m(x)
+        assert y.shape == (*x.shape[:-1], N) and y.is_contiguous()
+        assert _close(y, x.float() @ W.float() + m.bias.float())
