@@ -34,12 +34,15 @@ struct T4Args {
     uint32_t stages;       // windows per warp
     uint32_t acc_bytes;    // sums of a warp
     uint32_t cblocks;      // 16-column blocks per group
+    uint32_t subs, step;   // ENTRY: groups per four tiles, the rows of a segment in each; else 1, half a tile
     uint32_t total;        // units
     uint32_t *status;
 };
 
 // MT: sums per row in shared memory (1, 2 or 8 activation rows).
-template <int MT>
+// ENTRY: a group is the rows of four tiles between two entry points (see linear_mma4.cu), so its sums are those of a short
+// tile; without, a tall tile's sums and window leave room for three warps.
+template <int MT, bool ENTRY>
 __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_constant__ T4Args p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const LinArgs &a = p.a;
@@ -54,7 +57,8 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     const uint32_t man_s = lut_s + kLutBytes + kT4BarBytes + warp * kT4ManBytes;
     const uint32_t acc0_s = lut_s + kLutBytes + kT4BarBytes + W * kT4ManBytes, acc_s = acc0_s + warp * p.acc_bytes;
     const uint32_t wbase_s = acc0_s + W * p.acc_bytes + warp * p.stages * p.stage_bytes;
-    const uint32_t seg_acc = g.half * (MT * 4) + (MT == 8 ? 32 : MT * 4);  // bytes between the sums of two segments
+    const uint32_t subs = ENTRY ? p.subs : 1u, step = ENTRY ? p.step : g.half;
+    const uint32_t seg_acc = step * (MT * 4) + (MT == 8 ? 32 : MT * 4);  // bytes between the sums of two segments
     __shared__ uint32_t s_flag;
 
     const uint32_t sg = lane >> 2, q = lane & 3;                // row segment and column quad of this lane
@@ -78,10 +82,17 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     auto load_desc = [&](uint32_t u, uint32_t &off, uint32_t &ml) {
         off = ml = 0;
         if (u >= hi || lane >= 4) return;
-        const uint32_t grp = u / p.cblocks, ct = (u - grp * p.cblocks) >> 1, tk = 4 * grp + lane;
+        const uint32_t grp = u / p.cblocks, ct = (u - grp * p.cblocks) >> 1, tk = 4 * (grp / subs) + lane;
         if (tk >= g.tiles_k) return;
-        off = __ldg(a.tile_offsets + (size_t)tk * g.tiles_n + ct);
-        ml = __ldg(a.tile_max_lens + (size_t)tk * g.tiles_n + ct);
+        const size_t tile = (size_t)tk * g.tiles_n + ct;
+        off = __ldg(a.tile_offsets + tile);
+        if constexpr (ENTRY) {
+            const uint32_t span = __ldg(a.entry_spans + tile * subs + grp % subs);   // first row | rows << 16
+            off += (span & 0xFFFFu) * 64;
+            ml = span >> 16;
+        } else {
+            ml = __ldg(a.tile_max_lens + tile);
+        }
     };
     auto issue = [&](uint32_t u, uint32_t stage, uint32_t off, uint32_t ml) {
         const uint32_t hb = u % p.cblocks & 1, dst = wbase_s + stage * p.stage_bytes;
@@ -101,27 +112,33 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     auto issue_man = [&](uint32_t u, uint32_t c, uint32_t buf) {
         const uint32_t grp = u / p.cblocks, cb = u - grp * p.cblocks;
         const uint32_t row = lane & 15, h = lane >> 4;          // a lane copies one row of one half of every tile
-        if (c * kChunkRows + row < g.half) {
-            const uint8_t *src = a.mantissa + (((size_t)4 * grp * g.tiles_n + (cb >> 1)) * g.th + h * g.half + c * kChunkRows + row) * 32 +
+        if (c * kChunkRows + row < step) {
+            const uint32_t tk0 = 4 * (grp / subs), sub_row = ENTRY ? grp % subs * step : 0u;
+            const uint8_t *src = a.mantissa + (((size_t)tk0 * g.tiles_n + (cb >> 1)) * g.th + h * g.half + sub_row + c * kChunkRows + row) * 32 +
                                  (cb & 1) * 16;
             const uint32_t dst = man_s + (buf * 8 + h) * kT4SegPitch + row * 16;
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j)
-                if (4 * grp + j < g.tiles_k) cp_async16(dst + 2 * j * kT4SegPitch, src + (size_t)j * g.tiles_n * g.th * 32);
+                if (tk0 + j < g.tiles_k) cp_async16(dst + 2 * j * kT4SegPitch, src + (size_t)j * g.tiles_n * g.th * 32);
         }
         cp_async_arrive(man_bar + buf * 8);
     };
+    // The segment whose streams this lane decodes: its own, or, where the group has no such tile, the same half of the
+    // first one (real symbols; random ones would take the branch for a second byte at every step).
+    auto seg_of = [&](uint32_t grp) { return 4 * (grp / subs) + (sg >> 1) < g.tiles_k ? sg : sg & 1; };
     // Initial states of this lane's streams in unit u; a column beyond the matrix repeats the block's first one (its
     // weights are finite and meet zero activations).
-    auto load_states = [&](uint32_t u, uint32_t (&s)[4]) {
-        const uint32_t grp = u / p.cblocks, cb = u - grp * p.cblocks, tk = 4 * grp + (sg >> 1);
-        if (tk >= g.tiles_k) {
-            s[0] = s[1] = s[2] = s[3] = kRansL;
-            return;
-        }
-        const uint32_t *src = a.states + ((size_t)tk * g.tiles_n + (cb >> 1)) * 64 + (sg & 1) * 32 + (cb & 1) * 16;
+    auto load_states = [&](uint32_t u, uint32_t (&s)[4], uint32_t (&rows)[4]) {
+        const uint32_t grp = u / p.cblocks, cb = u - grp * p.cblocks, tk = 4 * (grp / subs) + (seg_of(grp) >> 1);
+        rows[0] = rows[1] = rows[2] = rows[3] = 0;
+        const size_t at = (((size_t)tk * g.tiles_n + (cb >> 1)) * subs + (ENTRY ? grp % subs : 0u)) * 64 + (sg & 1) * 32 + (cb & 1) * 16;
+        const uint32_t *src = (ENTRY ? a.entry_states : a.states) + at;
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) s[j] = __ldg(src + (cb * 16 + 4 * q + j < g.N ? 4 * q + j : 0u));
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t c = cb * 16 + 4 * q + j < g.N ? 4 * q + j : 0u;
+            s[j] = __ldg(src + c);
+            if constexpr (ENTRY) rows[j] = min((uint32_t)__ldg(a.entry_rows + at + c), p.cap_rows - 1);
+        }
     };
 
     if (lane == 0) {
@@ -146,7 +163,7 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
 
     if (!wait_lut(lut_bar, a.lut)) atomicExch(p.status, 1u);
     const bool live_m = MT == 8 ? 2 * q < a.M : q == 0;         // lanes whose two D columns are activation rows
-    const uint32_t n_chunks = (g.half + kChunkRows - 1) / kChunkRows;
+    const uint32_t n_chunks = (step + kChunkRows - 1) / kChunkRows;
     uint32_t parity0 = 0, parity1 = 0, stage = 0, chunk = 0;
     Quad z;
     for (uint32_t run = lo; run < hi; run = group_end(run)) {   // the CTA's runs: one per group it touches
@@ -155,7 +172,8 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
         __syncwarp();
         for (; u < end; u = nu, base = nbase, nu = u < hi ? advance(u, nbase) : hi) {
             const uint32_t cb = u - grp * p.cblocks, col = cb * 16 + 4 * q;
-            load_states(u, z.s);
+            uint32_t next_row[4];
+            load_states(u, z.s, next_row);
             uint32_t xb[2] = {0u, 0u};                          // activations of row sg, columns col .. col + 3
             if (sg < a.M) {
                 const uint16_t *x = a.x + (size_t)sg * a.ldx + col;
@@ -163,11 +181,11 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
                 for (uint32_t j = 0; j < 4; ++j)
                     if (col + j < g.N) xb[j >> 1] |= (uint32_t)__ldg(x + j) << (16 * (j & 1));
             }
-            const uint32_t my_ml = __shfl_sync(kFull, ml, sg >> 1);
+            const uint32_t sd = seg_of(grp), my_ml = __shfl_sync(kFull, ml, sd >> 1);
             const uint32_t win_s = wbase_s + stage * p.stage_bytes;
-            const uint32_t first = win_s + (my_ml <= p.cap_rows ? my_ml - 1 : 0u) * 128 + sg * 16;
+            const uint32_t first = win_s + (!ENTRY && my_ml <= p.cap_rows ? my_ml - 1 : 0u) * 128 + sd * 16;
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) z.p[j] = first + (col + j < g.N ? 4 * q + j : 0u);
+            for (uint32_t j = 0; j < 4; ++j) z.p[j] = first + next_row[j] * 128 + (col + j < g.N ? 4 * q + j : 0u);
             if (!mbar_wait(bar_base + stage * 8, stage ? parity1 : parity0)) atomicExch(p.status, 1u);
             if (stage) parity1 ^= 1; else parity0 ^= 1;
             auto next_unit = [&]() {
@@ -189,7 +207,7 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
                 if (!mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1)) atomicExch(p.status, 1u);
                 z.clamp(win_s);
                 uint32_t ms = man_s + (buf * 8 + sg) * kT4SegPitch + q * 4;
-                const uint32_t n = min(kChunkRows, g.half - c * kChunkRows);
+                const uint32_t n = min(kChunkRows, step - c * kChunkRows);
 #pragma unroll 1
                 for (uint32_t r = 0; r < n; r += 4) {
 #pragma unroll
@@ -239,32 +257,36 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
         }
         // ---- the group's sums of this CTA ------------------------------------------------------------------
         __syncthreads();
-        const uint32_t rows = 8 * g.half, first_cta = (uint32_t)(((uint64_t)(grp * p.cblocks + 1) * gridDim.x - 1) / p.total);
+        const uint32_t rows = 8 * step, first_cta = (uint32_t)(((uint64_t)(grp * p.cblocks + 1) * gridDim.x - 1) / p.total);
         const uint32_t last_cta = (uint32_t)(((uint64_t)min((grp + 1) * p.cblocks, p.total) * gridDim.x - 1) / p.total);
         const uint32_t count = last_cta - first_cta + 1;
-        const uint32_t v0 = grp * 4 * g.th;                     // segment s of the group = rows s * half of it
+        // row r of the group = row r % step of its segment r / step
+        auto out_row = [&](uint32_t r) {
+            const uint32_t seg = r / step;
+            return (4 * (grp / subs) * 2 + seg) * g.half + (ENTRY ? grp % subs * step : 0u) + r - seg * step;
+        };
         float *mine = a.partial + (size_t)(blockIdx.x + grp) * rows * a.M;
         for (uint32_t i = threadIdx.x; i < rows * a.M; i += blockDim.x) {
-            const uint32_t m = i / rows, r = i - m * rows, seg = r / g.half;
-            const uint32_t at = acc0_s + seg * seg_acc + (r - seg * g.half) * (MT * 4) + m * 4;
+            const uint32_t m = i / rows, r = i - m * rows, seg = r / step, v = out_row(r);
+            const uint32_t at = acc0_s + seg * seg_acc + (r - seg * step) * (MT * 4) + m * 4;
             float sum = 0.f;
             for (uint32_t w = 0; w < W; ++w) sum += __uint_as_float(lds_u32(at + w * p.acc_bytes));
             if (count > 1) {
                 mine[i] = sum;
-            } else if (v0 + r < g.K) {
-                if (a.bias) sum += load_bf16(a.bias + v0 + r);
-                a.y[(size_t)m * a.ldy + v0 + r] = float_to_bf16_bits(sum);
+            } else if (v < g.K) {
+                if (a.bias) sum += load_bf16(a.bias + v);
+                a.y[(size_t)m * a.ldy + v] = float_to_bf16_bits(sum);
             }
         }
         if (count > 1) {
             if (last_arrival(a.tickets + grp, count, &s_flag)) {
                 for (uint32_t i = threadIdx.x; i < rows * a.M; i += blockDim.x) {
-                    const uint32_t m = i / rows, r = i - m * rows;
-                    if (v0 + r >= g.K) continue;
+                    const uint32_t m = i / rows, v = out_row(i - m * rows);
+                    if (v >= g.K) continue;
                     float sum = 0.f;
                     for (uint32_t c = first_cta; c <= last_cta; ++c) sum += __ldcg(a.partial + (size_t)(c + grp) * rows * a.M + i);
-                    if (a.bias) sum += load_bf16(a.bias + v0 + r);
-                    a.y[(size_t)m * a.ldy + v0 + r] = float_to_bf16_bits(sum);
+                    if (a.bias) sum += load_bf16(a.bias + v);
+                    a.y[(size_t)m * a.ldy + v] = float_to_bf16_bits(sum);
                 }
                 if (threadIdx.x == 0) a.tickets[grp] = 0;       // ready for the next call
             }
@@ -275,10 +297,10 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
 
 // ------------------------------------------------------------------------ host
 
-template <int MT>
+template <int MT, bool ENTRY>
 static int launch_t4_pass(T4Args p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, cudaStream_t s) {
     static SmemLimit lim = {};
-    if (int rc = ensure_smem_limit(lim, (const void *)k_linear_t4<MT>, (size_t)max_smem - 1024)) return rc;
+    if (int rc = ensure_smem_limit(lim, (const void *)k_linear_t4<MT, ENTRY>, (size_t)max_smem - 1024)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(warps * 32);
@@ -289,7 +311,7 @@ static int launch_t4_pass(T4Args p, uint32_t blocks, uint32_t warps, size_t smem
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CI_CUDA(cudaLaunchKernelEx(&cfg, k_linear_t4<MT>, p));
+    CI_CUDA(cudaLaunchKernelEx(&cfg, k_linear_t4<MT, ENTRY>, p));
     return CI_OK;
 }
 
@@ -303,13 +325,17 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
     if (g.tw != 32 || g.th % 16 != 0 || max_tile_len == 0) return 1;
     if ((reinterpret_cast<uintptr_t>(a.stream) & 15u) || (reinterpret_cast<uintptr_t>(a.mantissa) & 15u)) return 1;
     if (partial_capacity < linear_t4_workspace_bytes(a.M, g.K, g.th)) return 1;
-    const uint32_t groups = (g.tiles_k + 3) / 4;
+    const bool entry = a.entry_step != 0 && a.entry_cap != 0 && g.half > a.entry_step && g.half % a.entry_step == 0 &&
+                       a.entry_step % kChunkRows == 0;
+    const uint32_t step = entry ? a.entry_step : g.half, subs = g.half / step, groups = (g.tiles_k + 3) / 4 * subs;
     if (groups >= kTicketBytes - 1) return 1;
     int dev = 0, max_smem = 0;
     CI_CUDA(cudaGetDevice(&dev));
     CI_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     T4Args p;
-    p.cap_rows = max_tile_len;
+    p.cap_rows = entry ? a.entry_cap : max_tile_len;
+    p.step = step;
+    p.subs = subs;
     p.stage_bytes = p.cap_rows * 128u;
     p.cblocks = (g.N + 15) / 16;
     p.total = groups * p.cblocks;
@@ -322,7 +348,7 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
     double best = 0.0;
     for (uint32_t mt = 1; mt <= 8; mt = mt == 2 ? 8 : mt * 2)
         for (uint32_t stages = 1; stages <= 2; ++stages) {
-            const uint32_t acc = (8 * (g.half * (mt * 4) + (mt == 8 ? 32 : mt * 4)) + 15) & ~15u;
+            const uint32_t acc = (8 * (step * (mt * 4) + (mt == 8 ? 32 : mt * 4)) + 15) & ~15u;
             const uint32_t warp_bytes = stages * p.stage_bytes + kT4ManBytes + acc;
             uint32_t w_max = room / warp_bytes;
             if (w_max > kT4Warps) w_max = kT4Warps;
@@ -345,9 +371,15 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
         p.a.x = a.x + (size_t)m0 * a.ldx;
         p.a.y = a.y + (size_t)m0 * a.ldy;
         p.a.M = a.M - m0 < rows_per_pass ? a.M - m0 : rows_per_pass;
-        const int rc = rows_per_pass == 1   ? launch_t4_pass<1>(p, blocks, warps, smem, max_smem, s)
-                       : rows_per_pass == 2 ? launch_t4_pass<2>(p, blocks, warps, smem, max_smem, s)
-                                            : launch_t4_pass<8>(p, blocks, warps, smem, max_smem, s);
+        int rc;
+        if (entry)
+            rc = rows_per_pass == 1   ? launch_t4_pass<1, true>(p, blocks, warps, smem, max_smem, s)
+                 : rows_per_pass == 2 ? launch_t4_pass<2, true>(p, blocks, warps, smem, max_smem, s)
+                                      : launch_t4_pass<8, true>(p, blocks, warps, smem, max_smem, s);
+        else
+            rc = rows_per_pass == 1   ? launch_t4_pass<1, false>(p, blocks, warps, smem, max_smem, s)
+                 : rows_per_pass == 2 ? launch_t4_pass<2, false>(p, blocks, warps, smem, max_smem, s)
+                                      : launch_t4_pass<8, false>(p, blocks, warps, smem, max_smem, s);
         if (rc) return rc;
     }
     return CI_OK;

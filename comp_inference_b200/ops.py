@@ -114,7 +114,7 @@ def fused_rans_linear_transposed_triton(x, compressed_data, initial_states, tabl
                                         bias=None, out=None, SPLIT_K=8):
     """y[..., V] = x[..., H] . W[V, H]^T for a weight stored [V, H] (LM head / tied embedding)."""
     return _lib.host().Weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens, mantissas,
-                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n)).linear(
+                              int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n), True).linear(
         x, bias, out, 0, True)
 
 

@@ -207,6 +207,7 @@ class RansLMHead(_RansBase):
         self._register()
 
     _twin = None
+    _entries = True
 
     def _stored_shape(self):
         return self.out_features, self.in_features
