@@ -309,6 +309,67 @@ static int launch_pdl(void (*kernel)(Args...), dim3 grid, dim3 block, size_t sme
     return CI_OK;
 }
 
+// ---------------------------------------------------------------- greedy step
+
+// One block per sequence: the token with the largest logit (a NaN is the largest, ties go to the lowest token, as
+// torch.argmax has it) becomes the input of the next step and joins the output; the block that finishes last advances
+// position and step count.  One launch for what took argmax, two additions, a copy and an indexed copy: 24 us of a step
+// of eight sequences over 32000 tokens.
+__global__ void __launch_bounds__(1024) k_greedy_step(const uint16_t *__restrict__ logits, int64_t ld, uint32_t V, uint32_t vec,
+                                                      int64_t *tok, int64_t *pos, int64_t *steps, int64_t *out, int64_t T,
+                                                      uint32_t *ticket) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ unsigned long long s_best[32];
+    const uint16_t *row = logits + (size_t)blockIdx.x * ld;
+    // order of floats as unsigned integers in the high word, the complement of the token in the low one
+    auto key = [](uint32_t bits, uint32_t i) {
+        uint32_t u = bits << 16;
+        u = (u & 0x7FFFFFFFu) > 0x7F800000u ? 0xFFFFFFFFu : u == 0x80000000u ? 0x80000000u : u & 0x80000000u ? ~u : u | 0x80000000u;
+        return (unsigned long long)u << 32 | (0xFFFFFFFFu - i);
+    };
+    unsigned long long best = 0;
+    if (vec) {
+        for (uint32_t i = threadIdx.x * 8; i < V; i += 8192) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(row + i);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+                const unsigned long long k = key(w[j >> 1] >> (16 * (j & 1)) & 0xFFFFu, i + j);
+                best = k > best ? k : best;
+            }
+        }
+    } else {
+        for (uint32_t i = threadIdx.x; i < V; i += 1024) {
+            const unsigned long long k = key(row[i], i);
+            best = k > best ? k : best;
+        }
+    }
+    for (int d = 16; d; d >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(kFull, best, d);
+        best = o > best ? o : best;
+    }
+    if ((threadIdx.x & 31) == 0) s_best[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    best = s_best[threadIdx.x];
+    for (int d = 16; d; d >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(kFull, best, d);
+        best = o > best ? o : best;
+    }
+    if (threadIdx.x == 0) {
+        const int64_t t = (int64_t)(0xFFFFFFFFu - (uint32_t)best), s = *steps + 1;
+        tok[blockIdx.x] = t;
+        if (s < T) out[(size_t)blockIdx.x * T + s] = t;
+        __threadfence();
+        if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
+            *ticket = 0;
+            *pos += 1;
+            *steps += 1;
+        }
+    }
+}
+
 }  // namespace ci
 
 using namespace ci;
@@ -401,6 +462,25 @@ int ci_silu_mul(const uint16_t *d_gate, int64_t ldg, const uint16_t *d_up, int64
     if (blocks > cap) blocks = cap;
     return launch_pdl(k_silu_mul, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, d_gate, ldg, d_up, ldu, rows,
                       cols, d_out, ldo);
+}
+
+int ci_greedy_step(const uint16_t *d_logits, int64_t ld, uint32_t B, uint32_t V, int64_t *d_tok, int64_t *d_pos, int64_t *d_steps,
+                   int64_t *d_out, int64_t T, uint32_t *d_ticket, ci_stream_t stream) {
+    CI_REQUIRE(d_logits && d_tok && d_pos && d_steps && d_out && d_ticket, "null pointer");
+    CI_REQUIRE(V > 0 && ld >= (int64_t)V, "row stride smaller than the vocabulary");
+    if (B == 0) return CI_OK;
+    const uint32_t vec = V % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(d_logits) & 15u) == 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(B);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CI_CUDA(cudaLaunchKernelEx(&cfg, k_greedy_step, d_logits, ld, V, vec, d_tok, d_pos, d_steps, d_out, T, d_ticket));
+    return CI_OK;
 }
 
 }  // extern "C"

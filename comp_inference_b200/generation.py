@@ -51,6 +51,7 @@ class LlamaGreedyRunner:
         self.pos = torch.zeros(1, dtype=torch.int64, device=self.device)
         self.out = torch.zeros(self.B, self.T, dtype=torch.int64, device=self.device)
         self.steps_done = torch.zeros(1, dtype=torch.int64, device=self.device)
+        self._ticket = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.logits = None
         self._graph = None
         self._graph_batch = None
@@ -130,10 +131,7 @@ class LlamaGreedyRunner:
             delta = mlp.down_proj(ops.silu_mul(mlp.gate_proj(x), mlp.up_proj(x)))
         x, h = ops.add_rmsnorm(delta, h, m.norm.weight, m.norm.variance_epsilon)
         self.logits = self.model.lm_head(x)
-        self.tok[:B] = self.logits.argmax(-1)
-        self.pos.add_(1)
-        self.steps_done.add_(1)
-        self.out[:B].index_copy_(1, self.steps_done, self.tok[:B].view(B, 1))
+        ops.greedy_step(self.logits, self.tok, pos, self.steps_done, self.out, self._ticket)
 
     def _decode_step(self, B):
         """Consumes self.tok (the token at position self.pos), produces the next one.  All shapes static."""

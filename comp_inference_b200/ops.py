@@ -276,3 +276,16 @@ def silu_mul(gate, up):
     _lib.check(_lib.load().ci_silu_mul(_lib.ptr(g2), g2.stride(0), _lib.ptr(u2), u2.stride(0), rows, cols, _lib.ptr(out),
                                        cols, _lib.stream()))
     return out.view(*gate.shape)
+
+
+def greedy_step(logits, tok, pos, steps_done, out, ticket):
+    """The end of a greedy decode step in one kernel: tok[b] = argmax of logits[b] (bf16 [B, V]), appended to
+    out[b, steps_done + 1]; pos and steps_done (one int64 each, on the device) grow by one.  ``ticket``: an int32 tensor
+    of one zero, left zero."""
+    l2 = _rows(logits)
+    B, V = l2.shape
+    if not (tok.is_contiguous() and out.is_contiguous() and out.shape[0] >= B and tok.numel() >= B):
+        raise RuntimeError("tok [B] and out [B, T] must be contiguous int64 tensors")
+    _lib.check(_lib.load().ci_greedy_step(_lib.ptr(l2), l2.stride(0), B, V, _lib.ptr(tok), _lib.ptr(pos),
+                                          _lib.ptr(steps_done), _lib.ptr(out), out.shape[1], _lib.ptr(ticket),
+                                          _lib.stream()))

@@ -354,6 +354,12 @@ int ci_encode_legacy_segments_write(const uint8_t *d_data, uint32_t rows, uint32
 
 /* ---- between the linears of a decode step ----------------------------------------- */
 
+/* The end of a greedy decode step: for each of B sequences the token with the largest of its V bf16 logits (rows ld apart;
+ * ties to the lowest token) goes to d_tok[b] and d_out[b * T + *d_steps + 1]; then *d_pos and *d_steps grow by one.
+ * d_ticket: one word, zero before the first call; every call leaves it zero. */
+int ci_greedy_step(const uint16_t *d_logits, int64_t ld, uint32_t B, uint32_t V, int64_t *d_tok, int64_t *d_pos, int64_t *d_steps,
+                   int64_t *d_out, int64_t T, uint32_t *d_ticket, ci_stream_t stream);
+
 /* The weightless steps of a Llama-style decode step, one launch each instead of the thirty-odd element-wise
  * launches of eager PyTorch; bf16 bits in and out, fp32 arithmetic.  No counterpart in the reference, which has
  * no decode loop of its own (tests/test_rans_pytorch_runtime.py:89-118 calls Hugging Face's generate).

@@ -130,3 +130,27 @@ def test_prompt_edges(K, N, th, M):
         y = m(x)
         assert y.shape == (*x.shape[:-1], N) and y.is_contiguous()
         assert _close(y, x.float() @ W.float() + m.bias.float())
+
+
+# end of a greedy step: ties, NaN, infinities, widths that are no multiple of eight, one and several sequences
+@pytest.mark.parametrize("B,V", [(1, 32000), (3, 101), (8, 4096), (5, 1), (2, 50257)])
+def test_greedy_step(B, V):
+    from comp_inference_b200 import ops
+    logits = torch.randn(B, V, generator=torch.Generator().manual_seed(V)).to(torch.bfloat16)
+    logits[0, V // 2:] = logits[0].max()
+    if B > 1:
+        logits[1, V // 3] = float("inf")
+        logits[B - 1] = -logits[B - 1].abs() if V > 1 else 0.0
+        logits[B - 1, V - 1] = -0.0
+    if B > 2:
+        logits[2, V // 5] = float("nan")
+    logits = logits.cuda()
+    tok, out = torch.zeros(B + 1, dtype=torch.int64, device="cuda"), torch.zeros(B + 1, 4, dtype=torch.int64, device="cuda")
+    pos, steps = torch.full((1,), 7, device="cuda"), torch.zeros(1, dtype=torch.int64, device="cuda")
+    ticket = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = logits.argmax(-1)
+    for i in range(1, 4):
+        ops.greedy_step(logits, tok, pos, steps, out, ticket)
+        assert torch.equal(tok[:B], want) and torch.equal(out[:B, i], want)
+        assert int(pos) == 7 + i and int(steps) == i and int(ticket) == 0
+    assert int(tok[B]) == 0 and int(out[B].sum()) == 0
