@@ -185,7 +185,20 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         const uint32_t cols = tile_live && col0 < g.N ? min(4u, g.N - col0) : 0u;
         const uint32_t row = tk * g.th + hsel * g.half + (ENTRY ? sub * step : 0u);   // first row of this lane's streams
         uint32_t rows_left = cols == 0 ? 0u : !EDGE ? 0xFFFFFFFFu : row < g.K ? min(step, g.K - row) : 0u;
-        const uint32_t ml = tsel ? nx_ml1 : nx_ml0;
+        // A lane without rows decodes the left tile's top half, and a stream that is used up before the unit's last row starts
+        // over: any real symbols will do, but past the end of a stream the symbols are rare ones, and every step would
+        // take the branch for a second byte.
+        uint32_t tsel_d = two ? tsel : 0u, hsel_d = hsel, len = 0xFFFFFFFFu;   // len: blocks of four rows, where short
+        bool empty = false;                                     // an entry point's unit may lie beyond K altogether
+        if (EDGE && (tk + 1) * g.th > g.K) {
+            const uint32_t top = row - hsel * g.half, top_rows = top < g.K ? min(step, g.K - top) : 0u;
+            const uint32_t own = row < g.K ? min(step, g.K - row) : 0u;
+            empty = top_rows == 0;
+            if (own == 0) hsel_d = 0;
+            len = ((own ? own : top_rows) + 3) >> 2;
+        }
+        uint32_t left = len;
+        const uint32_t ml = tsel_d ? nx_ml1 : nx_ml0;
         const bool more = (uint64_t)t + n_warps < p.total;
         uint32_t n_tk = 0, n_sub = 0, n_tp = 0, n_t0 = 0;       // of unit t + n_warps
         bool n_two = false;
@@ -205,20 +218,23 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         };
 
         const uint32_t win_s = wbase_s + stage * p.stage_bytes;
-        const uint32_t st_s = win_s + st_off + tsel * 256 + (hsel * 32 + (quad & 7) * 4) * 4;
-        uint32_t first = win_s + tsel * 64 + hsel * 32 + (quad & 7) * 4;
-        if (!ENTRY && tile_live && ml <= p.cap_rows) first += (ml - 1) * 128;  // last byte row; an empty tile starts one row below
+        const uint32_t st_s = win_s + st_off + tsel_d * 256 + (hsel_d * 32 + (quad & 7) * 4) * 4;
+        uint32_t first = win_s + tsel_d * 64 + hsel_d * 32 + (quad & 7) * 4;
+        if (!ENTRY && ml <= p.cap_rows) first += (ml - 1) * 128;  // last byte row; an empty tile starts one row below
         (void)mbar_wait(bar_base + stage * 8, stage ? parity1 : parity0);
         if (stage) parity1 ^= 1; else parity0 ^= 1;
-        z.start(st_s, first);                                   // a tile that does not exist decodes what is in its place
-        if constexpr (ENTRY) {                                  // every stream has its own row of the window
-            const uint32_t rows_s = win_s + st_off + 512 + tsel * 128 + (hsel * 32 + (quad & 7) * 4) * 2;
+        auto start_streams = [&]() {
+            z.start(st_s, first);
+            if constexpr (!ENTRY) return;
+            // every stream has its own row of the window
+            const uint32_t rows_s = win_s + st_off + 512 + tsel_d * 128 + (hsel_d * 32 + (quad & 7) * 4) * 2;
             const uint32_t r01 = lds_u32(rows_s), r23 = lds_u32(rows_s + 4), top = p.cap_rows - 1;
             z.p[0] += min(r01 & 0xFFFFu, top) * 128;
             z.p[1] += min(r01 >> 16, top) * 128;
             z.p[2] += min(r23 & 0xFFFFu, top) * 128;
             z.p[3] += min(r23 >> 16, top) * 128;
-        }
+        };
+        start_streams();
 
         uint8_t *o8 = reinterpret_cast<uint8_t *>(out) + ((size_t)row * p.ld + col0) * (BF16 ? 2 : 1);
         const size_t o_pitch = (size_t)p.ld * (BF16 ? 2 : 1);
@@ -245,7 +261,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
             }
             z.clamp(win_s);
             uint32_t ms = man_s + (buf * 4 + tsel * 2 + hsel) * kSegPitch + (quad & 7) * 4;
-            const uint32_t n = min(kChunkRows, step - c * kChunkRows);
+            const uint32_t n = EDGE && empty ? 0u : min(kChunkRows, step - c * kChunkRows);
 #pragma unroll 1
             for (uint32_t r = 0; r < n; r += 4) {
 #pragma unroll
@@ -287,7 +303,13 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
                     o8 += o_pitch;
                 }
                 ms += 128;
-                if (EDGE) rows_left = rows_left > 4 ? rows_left - 4 : 0u;
+                if (EDGE) {
+                    rows_left = rows_left > 4 ? rows_left - 4 : 0u;
+                    if (--left == 0) {
+                        left = len;
+                        start_streams();
+                    }
+                }
             }
         }
         if (p.stages == 2) {

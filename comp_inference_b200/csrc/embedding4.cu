@@ -103,21 +103,24 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
 
     // What the lane knows about one task.
     struct Task {
-        uint32_t ti, cb, inner, ml;
-        bool live;             // the id is inside the table and so is the lane's tile
+        uint32_t ti, cb, inner, ml, tsel;
+        bool live;             // the id is inside the table
         uint4 states;
         uint32_t man;
         uint2 rows;            // ENTRY: next byte's row of every stream
     };
     // Task k of the batch: its copies into `stage`, its states and sign+mantissa bytes.
     auto open = [&](const Batch &b, uint32_t k, uint32_t stage, Task &t) {
-        const uint32_t src_lane = 4 * k + tsel;
         t.ti = __shfl_sync(kFull, b.ti, 4 * k);
         t.cb = __shfl_sync(kFull, b.cb, 4 * k);
+        // a lane without a tile of its own decodes the block's first one along: real symbols, whose steps do not take the
+        // branch for a second byte
+        t.tsel = t.cb * 4 + tsel < g.tiles_n ? tsel : 0u;
+        const uint32_t src_lane = 4 * k + t.tsel;
         const uint32_t row = __shfl_sync(kFull, b.row, 4 * k), off = __shfl_sync(kFull, b.off, src_lane);
         t.ml = __shfl_sync(kFull, b.ml, src_lane);
-        const uint32_t tn = t.cb * 4 + tsel;
-        t.live = row != 0xFFFFFFFFu && tn < g.tiles_n;
+        const uint32_t tn = t.cb * 4 + t.tsel;
+        t.live = row != 0xFFFFFFFFu;
         const uint32_t tk = row / g.th, rel = row - tk * g.th, h = rel >= g.half ? 1u : 0u;
         t.inner = t.live ? rel - h * g.half : 0u;
         t.states = make_uint4(kRansL, kRansL, kRansL, kRansL);
@@ -140,7 +143,7 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
             const uint32_t skip = t.ml - rows;
             const uint8_t *src = a.stream + off + h * 32 + (size_t)(skip + (quad >> 1)) * 64 + (quad & 1) * 16;
             const uint32_t dst = wbase_s + stage * p.stage_bytes + (skip + (quad >> 1)) * 128 + tsel * 32 + (quad & 1) * 16;
-            for (uint32_t i = quad >> 1; i < rows; i += 4) cp_async16(dst + (i - (quad >> 1)) * 128, src + (size_t)(i - (quad >> 1)) * 64);
+            for (uint32_t i = t.tsel == tsel ? quad >> 1 : rows; i < rows; i += 4) cp_async16(dst + (i - (quad >> 1)) * 128, src + (size_t)(i - (quad >> 1)) * 64);
         }
         cp_async_arrive(bar_base + stage * 8);
     };
@@ -172,7 +175,7 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
             z.s[1] = t.states.y;
             z.s[2] = t.states.z;
             z.s[3] = t.states.w;
-            const uint32_t start = win_s + tsel * 32 + quad * 4 + (!ENTRY && t.ml ? (t.ml - 1) * 128 : 0u);
+            const uint32_t start = win_s + t.tsel * 32 + quad * 4 + (!ENTRY && t.ml ? (t.ml - 1) * 128 : 0u);
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j) z.p[j] = start + j;
             if constexpr (ENTRY) {
@@ -184,7 +187,7 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
                     z.p[3] += min(t.rows.y >> 16, top) * 128;
                 }
             }
-            // The rows above the wanted one.  Lanes without a tile run along on whatever is in the window.
+            // The rows above the wanted one.
             const uint32_t drop = __shfl_sync(kFull, t.inner, 0);
 #pragma unroll 1
             for (uint32_t i = 0; i < drop; ++i) {

@@ -105,7 +105,9 @@ __device__ __forceinline__ void group4(uint32_t (&b)[4][2], Quad &z, uint32_t lu
 // RAGGED: K is not a whole number of tile pairs, so the last units of a column group lack their lower tile or end
 // inside a tile (an instantiation of its own: the common case carries none of the bookkeeping in its registers).
 // Every lane still runs the full warp-wide loop.  A lane whose segment has n_my < n_blocks 4-row groups reads zeros instead
-// of activations from group n_my on, and what it decodes past the end of its stream is masked to zero.
+// of activations from group n_my on, and what it decodes past the end of its stream is masked to zero.  It starts its stream
+// over whenever that is used up, and a lane without a segment decodes the upper tile's top half: any real symbols will do,
+// but past the end of a stream the symbols are rare ones, and every step would take the branch for a second byte.
 //
 // ENTRY: a unit is not a pair of whole tiles but the rows between two entry points of it (tall tiles: 512 symbols are one
 // serial chain).  The states and cursors of its streams come from the index, its window holds just the rows of the byte
@@ -451,11 +453,20 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
         }
         const uint32_t krow = (2 * pk + tsel) * g.th + hsel * g.half + (ENTRY ? sub * step : 0u);
         // Blocks of this lane's segment that exist, and the rows of the last one (0 = all four); see the kernel's header.
-        uint32_t n_my = n_blocks, cut = 0;
-        if (RAGGED && pk == ragged_pk) {
+        uint32_t n_my = n_blocks, len = n_blocks, cut = 0;
+        uint32_t tsel_d = tsel, hsel_d = hsel;                  // the segment whose stream this lane decodes, its blocks: len
+        bool empty = false;                                     // an entry point's unit may lie beyond K altogether
+        const bool rag = RAGGED && pk == ragged_pk;             // the same for every lane: other units skip the bookkeeping
+        if (rag) {
             const uint32_t seg = krow < g.K ? min(step, g.K - krow) : 0u;
-            n_my = (seg + 3) >> 2;
+            n_my = len = (seg + 3) >> 2;
             cut = seg & 3;
+            const uint32_t top = 2 * pk * g.th + (ENTRY ? sub * step : 0u), top_rows = top < g.K ? min(step, g.K - top) : 0u;
+            empty = top_rows == 0;
+            if (seg == 0) {
+                tsel_d = hsel_d = 0;
+                len = (top_rows + 3) >> 2;
+            }
         }
         uint32_t xs = p.x_step;
         const uint16_t *xp0 = x0 + (size_t)(krow >> 2) * xs, *xp1 = x1 + (size_t)(krow >> 2) * xs;
@@ -463,7 +474,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
             xp0 = xp1 = g_zero_activations;
             xs = 0;
         }
-        const uint32_t ml = tsel ? nx_ml1 : nx_ml0;
+        const uint32_t ml = tsel_d ? nx_ml1 : nx_ml0;
         auto next_unit = [&]() {                                // every lane is done with the window it goes to
             if (t + 1 >= hi) return;
             if (t + 1 - dbase == 32) {
@@ -481,8 +492,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
 
         // ---- this lane's four streams --------------------------------------
         const uint32_t win_s = wbase_s + stage * p.stage_bytes;
-        const uint32_t st_s = win_s + st_off + tsel * 256 + (hsel * 32 + gq * 4) * 4;
-        uint32_t first = win_s + tsel * 64 + hsel * 32 + gq * 4;
+        const uint32_t st_s = win_s + st_off + tsel_d * 256 + (hsel_d * 32 + gq * 4) * 4;
+        uint32_t first = win_s + tsel_d * 64 + hsel_d * 32 + gq * 4;
         if (!ENTRY && ml <= p.cap_rows) first += (ml - 1) * 128;   // last byte row; an empty tile starts one row below
 
         // ---- wait for the bytes (bounded) -------------------------------------
@@ -491,20 +502,23 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
             if (!mbar_wait(bar, par)) atomicExch(p.status, 1u);  // the result is invalid; the loop still ends
             if (stage) parity1 ^= 1; else parity0 ^= 1;
         }
-        z.start(st_s, first);
-        if constexpr (ENTRY) {                                  // every stream has its own row of the window
-            const uint32_t rows_s = win_s + st_off + 512 + tsel * 128 + (hsel * 32 + gq * 4) * 2;
+        auto start_streams = [&]() {
+            z.start(st_s, first);
+            if constexpr (!ENTRY) return;
+            // every stream has its own row of the window
+            const uint32_t rows_s = win_s + st_off + 512 + tsel_d * 128 + (hsel_d * 32 + gq * 4) * 2;
             const uint32_t r01 = lds_u32(rows_s), r23 = lds_u32(rows_s + 4);
             const uint32_t top = p.cap_rows - 1;
             z.p[0] += min(r01 & 0xFFFFu, top) * 128;
             z.p[1] += min(r01 >> 16, top) * 128;
             z.p[2] += min(r23 & 0xFFFFu, top) * 128;
             z.p[3] += min(r23 >> 16, top) * 128;
-        }
+        };
+        start_streams();
 
         uint32_t wb[4][2] = {};
         uint32_t xf[4] = {};                                     // the group before: its weights, its activations
-        uint32_t blk = 0;
+        uint32_t blk = 0, left = len;                           // left: blocks until this lane's stream is used up
 #pragma unroll 1
         for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
             const uint32_t buf = chunk & 1;
@@ -515,7 +529,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
             if (!mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1)) atomicExch(p.status, 1u);
             z.clamp(win_s);
             uint32_t ms = man_s + (buf * 4 + q) * kSegPitch + gq * 4;
-            const uint32_t end = min(blk + kChunkRows / 4, n_blocks);
+            const uint32_t end = RAGGED && empty ? 0u : min(blk + kChunkRows / 4, n_blocks);
 #pragma unroll 1
             for (; blk < end; ++blk) {
                 const uint2 v0 = __ldg(reinterpret_cast<const uint2 *>(xp0));   // used by the mma at the end
@@ -526,7 +540,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
                 // converged and drops the divergence checks (and the register copies they need) of the votes.
                 mma4<HI>(acc, wb, xf);
                 group4(wb, z, lut_s, m);
-                if constexpr (RAGGED) {
+                if (rag) {
                     const uint32_t n = blk + 1 < n_my ? 4u : blk >= n_my ? 0u : cut ? cut : 4u;   // rows of the block that exist
                     if (n < 4) {
 #pragma unroll
@@ -540,10 +554,14 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
                 ms += 128;
                 xp0 += xs;
                 if constexpr (HI) xp1 += xs;
-                if constexpr (RAGGED) {
+                if (rag) {
                     if (blk + 1 == n_my) {                      // rows beyond K from the next block on
                         xp0 = xp1 = g_zero_activations;
                         xs = 0;
+                    }
+                    if (--left == 0) {
+                        left = len;
+                        start_streams();
                     }
                 }
             }
