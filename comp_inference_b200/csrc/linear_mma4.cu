@@ -692,7 +692,8 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     cfg.numAttrs = 1;
     // The extra launch takes 2.7 us and saves about 1.7e-8 us per activation row and weight, where the multiprocessors are
     // busy at all: it pays from 1.6e8 of them (4096 x 22016: 119 -> 90 us at 16 rows, 94 -> 85 at 8, 87 -> 85 at 4).
-    if (!quads_ok || (a.x_scratch != nullptr && a.M >= 3 && p.total >= 6 * P && (uint64_t)a.M * g.K * g.N >= 160000000ull)) {
+    // Short units (tile height 64) do not wait for that pipe: 6784 x 5168 takes 48.8 us at 16 rows without it, 51.8 with it.
+    if (!quads_ok || (a.x_scratch != nullptr && a.M >= 3 && p.step >= 64 && p.total >= 6 * P && (uint64_t)a.M * g.K * g.N >= 160000000ull)) {
         cfg.gridDim = dim3((g.K / 4 + 256) / 256, a.M);
         cfg.blockDim = dim3(256);
         CI_CUDA(cudaLaunchKernelEx(&cfg, k_interleave_x, a.x, a.ldx, a.M, g.K, (uint32_t)quads_ok,
