@@ -235,7 +235,9 @@ static int decode_tiled(const ci_tiled_weight *w, void *d_out, uint32_t ld, cuda
     if (rc) return rc;
     CI_REQUIRE(d_out != nullptr, "null output");
     DecArgs a = make_args(w);
-    rc = launch_decode4(a, w->max_tile_len, BF16, d_out, ld ? ld : w->N, s);   // 32-wide tiles
+    rc = launch_decode2(a, w->max_tile_len, BF16, d_out, ld ? ld : w->N, s);   // 32-wide tiles
+    if (rc <= 0) return rc;
+    rc = launch_decode4(a, w->max_tile_len, BF16, d_out, ld ? ld : w->N, s);
     if (rc <= 0) return rc;
     if (ld != 0 && ld != w->N) {
         set_error("this weight does not qualify for the staged decoder, the only one that writes padded rows");

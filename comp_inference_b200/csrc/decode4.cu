@@ -386,6 +386,49 @@ int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     return decode4(a, max_tile_len, bf16, out, ld, 0, nullptr, nullptr, s);
 }
 
+constexpr uint32_t kDec4Fixed = 2 * kLutBytes + kDec4BarBytes;  // up to one table size is lost to the table's alignment
+
+// As in the fused linear: the warp count with the cheapest rounds; a second window where it costs no warp that pays.
+static double plan_rounds(Dec4Args &p, uint32_t man_bytes, int max_smem, uint32_t &warps) {
+    const uint32_t P = (uint32_t)sm_count(), room = (uint32_t)max_smem - kDec4Fixed;
+    double best = 0.0;
+    warps = 0;
+    for (uint32_t stages = 2; stages >= 1; --stages) {
+        uint32_t w_max = room / (stages * p.stage_bytes + man_bytes);
+        if (w_max > kDec4Warps) w_max = kDec4Warps;
+        for (uint32_t w = 1; w <= w_max; ++w) {
+            const double cost = run_cost((p.total + P - 1) / P, w, 0.9) * (stages == 1 ? 1.02 : 1.0);
+            if (warps == 0 || cost < best) { best = cost; warps = w; p.stages = stages; }
+        }
+    }
+    return best;
+}
+
+static bool has_entries(const DecArgs &a, bool bf16) {
+    const Geom &g = a.g;
+    return bf16 && a.entry_step != 0 && a.entry_cap != 0 && g.half > a.entry_step && g.half % a.entry_step == 0 &&
+           a.entry_step % kChunkRows == 0 &&
+           ((reinterpret_cast<uintptr_t>(a.entry_states) | reinterpret_cast<uintptr_t>(a.entry_rows)) & 15u) == 0;
+}
+
+// Bytes of one window and the initial states (with entry points also the rows of the next bytes).
+static uint32_t stage_bytes4(uint32_t cap_rows, bool entry) { return (cap_rows * 128u + (entry ? 768u : 512u) + 127u) & ~127u; }
+
+double decode4_cost(const DecArgs &a, uint32_t max_tile_len, bool bf16) {
+    const Geom &g = a.g;
+    int dev = 0, max_smem = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return 0.0;
+    const bool entry = has_entries(a, bf16);
+    Dec4Args p;
+    p.stage_bytes = stage_bytes4(entry ? a.entry_cap : max_tile_len, entry);
+    p.total = g.tiles_k * ((g.tiles_n + 1) / 2) * (entry ? g.half / a.entry_step : 1u);
+    uint32_t warps;
+    const double cost = plan_rounds(p, bf16 ? kManBytes : 0u, max_smem, warps);
+    return entry ? cost * a.entry_step / g.half : cost;         // per 64 symbols of the whole stream
+}
+
 static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, uint32_t step,
                    uint32_t *entry_states, uint16_t *entry_rows, cudaStream_t s) {
     const Geom &g = a.g;
@@ -397,11 +440,9 @@ static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     CI_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     Dec4Args p;
     p.a = a;
-    const bool entry = bf16 && a.entry_step != 0 && a.entry_cap != 0 && g.half > a.entry_step && g.half % a.entry_step == 0 &&
-                       a.entry_step % kChunkRows == 0 &&
-                       ((reinterpret_cast<uintptr_t>(a.entry_states) | reinterpret_cast<uintptr_t>(a.entry_rows)) & 15u) == 0;
+    const bool entry = has_entries(a, bf16);
     p.cap_rows = entry ? a.entry_cap : max_tile_len;
-    p.stage_bytes = (p.cap_rows * 128u + (entry ? 768u : 512u) + 127u) & ~127u;
+    p.stage_bytes = stage_bytes4(p.cap_rows, entry);
     p.pairs_n = (g.tiles_n + 1) / 2;
     p.step = entry ? a.entry_step : step;
     p.subs = p.step ? g.half / p.step : 0;
@@ -409,24 +450,13 @@ static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     p.entry_states = entry ? const_cast<uint32_t *>(a.entry_states) : entry_states;
     p.entry_rows = entry ? const_cast<uint16_t *>(a.entry_rows) : entry_rows;
     p.entry_spans = a.entry_spans;
-    const uint32_t fixed = 2 * kLutBytes + kDec4BarBytes;           // up to one table size is lost to the table's alignment
-    const uint32_t room = (uint32_t)max_smem - fixed, man_bytes = bf16 ? kManBytes : 0u;
-    // As in the fused linear: the warp count with the cheapest rounds; a second window where it costs no warp that pays.
-    const uint32_t P = (uint32_t)sm_count();
+    const uint32_t P = (uint32_t)sm_count(), man_bytes = bf16 ? kManBytes : 0u;
     uint32_t warps = 0;
-    double best = 0.0;
-    for (uint32_t stages = 2; stages >= 1; --stages) {
-        uint32_t w_max = room / (stages * p.stage_bytes + man_bytes);
-        if (w_max > kDec4Warps) w_max = kDec4Warps;
-        for (uint32_t w = 1; w <= w_max; ++w) {
-            const double cost = run_cost((p.total + P - 1) / P, w, 0.9) * (stages == 1 ? 1.02 : 1.0);
-            if (warps == 0 || cost < best) { best = cost; warps = w; p.stages = stages; }
-        }
-    }
+    plan_rounds(p, man_bytes, max_smem, warps);
     if (warps == 0) return 1;
     uint32_t blocks = (p.total + warps - 1) / warps;
     if (blocks > P) blocks = P;
-    const size_t smem = fixed + (size_t)warps * (p.stages * p.stage_bytes + man_bytes);
+    const size_t smem = kDec4Fixed + (size_t)warps * (p.stages * p.stage_bytes + man_bytes);
     p.ld = ld;
     p.vec = ld % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & (bf16 ? 7u : 3u)) == 0;
     const bool edge = g.K % g.th != 0 || g.N % 4 != 0 || !p.vec;

@@ -100,6 +100,14 @@ def test_decoder_edges(K, N, th):
     assert torch.equal(plane, ci.extract_exp_and_mantissa(W)[0])
 
 
+# two streams a lane (few tiles: short and missing bottom halves, odd widths and rows, several rounds of tall tiles) and its
+# neighbour, four streams at sizes with many tiles
+@pytest.mark.parametrize("K,N,th", [(700, 33, 1024), (520, 130, 1024), (512, 64, 1024), (513, 4099, 1024), (8200, 1186, 2048),
+                                    (16, 31, 16), (4097, 2014, 128), (2111, 8222, 64), (4096, 4100, 128)])
+def test_decoder_few_and_many_tiles(K, N, th):
+    test_decoder_edges(K, N, th)
+
+
 # row gather: every row of small tables (each position inside a half tile), ids outside, one id, more ids than warps,
 # tall tiles (one window per warp), odd widths
 @pytest.mark.parametrize("V,H,th,n", [(96, 128, 16, 300), (300, 4096, 16, 1), (257, 100, 128, 257), (3000, 64, 1024, 500),
