@@ -8,8 +8,8 @@
 // chain of a stream, usually one a warp: nothing is fetched for the next one ahead.
 //
 // Measured on a B200 (graph replays over more than L2), four streams per lane -> two: 4096 x 11008 at tile height 1024 75.9 ->
-// 54.4 us (1376 tiles: nine or ten warps a multiprocessor, the fullest scheduler's three at 62 % of its issue slots),
-// 11008 x 4096 at 1024 95 -> 56, 1024 x 2048 at 128 9.3 -> 5.9, 777 x 1001 at 128 16.9 -> 8.
+// 54.4 us (1376 tiles: nine or ten warps a multiprocessor, 55 % of the issue slots; the waits that are left are the chain's own,
+// arithmetic and table look-ups), 11008 x 4096 at 1024 95 -> 56, 1024 x 2048 at 128 9.3 -> 5.9, 777 x 1001 at 128 16.9 -> 8.5.
 #include "decode.cuh"
 #include "ptx.cuh"
 
@@ -260,7 +260,8 @@ int launch_decode2(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     uint32_t w_max = ((uint32_t)max_smem - fixed) / warp_bytes;
     if (w_max > kDec2Warps) w_max = kDec2Warps;
     // us at 64 symbols per stream, as run_cost: a round of one warp per scheduler is the chain (4.2), with n it is n warps'
-    // instructions (measured 8 warps 4.9, 12 6.9, 16 9.1, 20 11.1).
+    // instructions.  Whole launches of one round took 6.2 us with 5 warps, 6.9 with 8, 8.9 with 12, 11.4 with 16 and 13.6 with
+    // 20; the 2 us or so that every launch has are left out, as they are in run_cost.
     auto round2 = [](uint32_t w) { return w <= 4 ? 4.2 : 1.0 + 2.0 * ((w + 3) / 4); };
     uint32_t warps = 0;
     double best = 0.0;

@@ -14,8 +14,9 @@
 // around them.  A warp therefore takes a run of consecutive tasks: eight at a time their ids are read and their tiles'
 // offsets and depths fetched, one tile per lane, while the eight before them are worked off; a task then costs two
 // shuffles for its lane's own tile, and no division.  Byte windows, initial states and the row's sign+mantissa bytes are
-// fetched one task ahead.  Tall tiles are entered at the entry point before the row where the caller has them.  Measured, 4096 ids of 32000 x 4096 at tile height 16: 148 us with one task at a time,
-// divisions in 64 bits and eight shuffles per task -> see the table in the design notes.
+// fetched one task ahead.  Tall tiles are entered at the entry point before the row where the caller has them.  Measured on
+// a B200, 4096 ids of 32000 x 4096 at tile height 16: 148 us with one task at a time, divisions in 64 bits and eight
+// shuffles per task -> 88.
 #include "embedding.cuh"
 #include "ptx.cuh"
 
@@ -36,7 +37,10 @@ struct Emb4Args {
 };
 
 // ENTRY: streams are entered at the entry point before the row (tall tiles), not at their start.
-template <bool ENTRY>
+// RAGGED: the last block of 128 columns lacks tiles.  A lane without one decodes the block's first tile along: real symbols,
+// where random ones would take the branch for a second byte at every step.  (An instantiation of its own: in all of them it cost
+// 2 %, 87.4 us to 89.3 at 4096 ids of 32000 x 4096.)
+template <bool ENTRY, bool RAGGED>
 __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_constant__ Emb4Args p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const EmbArgs &a = p.a;
@@ -103,23 +107,22 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
 
     // What the lane knows about one task.
     struct Task {
-        uint32_t ti, cb, inner, ml, tsel;
+        uint32_t ti, cb, inner, ml;
         bool live;             // the id is inside the table
         uint4 states;
         uint32_t man;
         uint2 rows;            // ENTRY: next byte's row of every stream
     };
+    // The tile of the column block whose streams this lane decodes.
+    auto tile_of = [&](uint32_t cb) { return !RAGGED || cb * 4 + tsel < g.tiles_n ? tsel : 0u; };
     // Task k of the batch: its copies into `stage`, its states and sign+mantissa bytes.
     auto open = [&](const Batch &b, uint32_t k, uint32_t stage, Task &t) {
         t.ti = __shfl_sync(kFull, b.ti, 4 * k);
         t.cb = __shfl_sync(kFull, b.cb, 4 * k);
-        // a lane without a tile of its own decodes the block's first one along: real symbols, whose steps do not take the
-        // branch for a second byte
-        t.tsel = t.cb * 4 + tsel < g.tiles_n ? tsel : 0u;
-        const uint32_t src_lane = 4 * k + t.tsel;
+        const uint32_t tsel_d = tile_of(t.cb), src_lane = 4 * k + tsel_d;
         const uint32_t row = __shfl_sync(kFull, b.row, 4 * k), off = __shfl_sync(kFull, b.off, src_lane);
         t.ml = __shfl_sync(kFull, b.ml, src_lane);
-        const uint32_t tn = t.cb * 4 + t.tsel;
+        const uint32_t tn = t.cb * 4 + tsel_d;
         t.live = row != 0xFFFFFFFFu;
         const uint32_t tk = row / g.th, rel = row - tk * g.th, h = rel >= g.half ? 1u : 0u;
         t.inner = t.live ? rel - h * g.half : 0u;
@@ -143,7 +146,8 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
             const uint32_t skip = t.ml - rows;
             const uint8_t *src = a.stream + off + h * 32 + (size_t)(skip + (quad >> 1)) * 64 + (quad & 1) * 16;
             const uint32_t dst = wbase_s + stage * p.stage_bytes + (skip + (quad >> 1)) * 128 + tsel * 32 + (quad & 1) * 16;
-            for (uint32_t i = t.tsel == tsel ? quad >> 1 : rows; i < rows; i += 4) cp_async16(dst + (i - (quad >> 1)) * 128, src + (size_t)(i - (quad >> 1)) * 64);
+            for (uint32_t i = tsel_d == tsel ? quad >> 1 : rows; i < rows; i += 4)
+                cp_async16(dst + (i - (quad >> 1)) * 128, src + (size_t)(i - (quad >> 1)) * 64);
         }
         cp_async_arrive(bar_base + stage * 8);
     };
@@ -175,7 +179,7 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
             z.s[1] = t.states.y;
             z.s[2] = t.states.z;
             z.s[3] = t.states.w;
-            const uint32_t start = win_s + t.tsel * 32 + quad * 4 + (!ENTRY && t.ml ? (t.ml - 1) * 128 : 0u);
+            const uint32_t start = win_s + tile_of(t.cb) * 32 + quad * 4 + (!ENTRY && t.ml ? (t.ml - 1) * 128 : 0u);
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j) z.p[j] = start + j;
             if constexpr (ENTRY) {
@@ -255,9 +259,11 @@ int launch_embedding4(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t s) {
     p.stages = room / (2 * p.stage_bytes) >= 12 ? 2 : 1;        // a deep window is worth doubling while 12 warps still fit
     uint32_t w_max = room / (p.stages * p.stage_bytes);
     if (w_max > kEmb4Warps) w_max = kEmb4Warps;
-    static SmemLimit lim[2] = {};
-    void (*const kernel)(Emb4Args) = entry ? k_embedding4<true> : k_embedding4<false>;
-    if (int rc = ensure_smem_limit(lim[entry], (const void *)kernel, (size_t)max_smem)) return rc;
+    const bool ragged = g.tiles_n % 4 != 0;
+    static SmemLimit lim[4] = {};
+    void (*const kernel)(Emb4Args) = entry ? (ragged ? k_embedding4<true, true> : k_embedding4<true, false>)
+                                           : (ragged ? k_embedding4<false, true> : k_embedding4<false, false>);
+    if (int rc = ensure_smem_limit(lim[entry + 2 * ragged], (const void *)kernel, (size_t)max_smem)) return rc;
     const uint32_t P = (uint32_t)sm_count();
     const uint64_t ids_per_launch = 0x40000000ull / p.blocks_n;     // task numbers fit 32 bits
     for (uint64_t i0 = 0; i0 < a.n_ids; i0 += ids_per_launch) {

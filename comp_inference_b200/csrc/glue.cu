@@ -313,8 +313,8 @@ static int launch_pdl(void (*kernel)(Args...), dim3 grid, dim3 block, size_t sme
 
 // One block per sequence: the token with the largest logit (a NaN is the largest, ties go to the lowest token, as
 // torch.argmax has it) becomes the input of the next step and joins the output; the block that finishes last advances
-// position and step count.  One launch for what took argmax, two additions, a copy and an indexed copy: 24 us of a step
-// of eight sequences over 32000 tokens.
+// position and step count.  One launch for what took argmax, two additions, a copy and an indexed copy: in a
+// captured step on a B200, eight sequences over 32000 tokens, 14.9 us -> 7.3.
 __global__ void __launch_bounds__(1024) k_greedy_step(const uint16_t *__restrict__ logits, int64_t ld, uint32_t V, uint32_t vec,
                                                       int64_t *tok, int64_t *pos, int64_t *steps, int64_t *out, int64_t T,
                                                       uint32_t *ticket) {

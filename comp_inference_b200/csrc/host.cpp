@@ -3,8 +3,8 @@
 // ctypes conversions.  Same checks and messages as the Python layer; anything rare (a workspace that has to grow, a table
 // that has to be prepared) is done by calling back into comp_inference_b200._lib, which stays the owner of those buffers.
 //
-// Measured, RansLinear.forward of a 512 x 4096 shard, one row, back to back: 25.5 us in Python, see the table in the
-// design notes for now; the kernel itself takes 5.6 us.
+// Measured, RansLinear.forward of a 512 x 4096 shard, one row, back to back: 25.5 us in Python, 7.0 to 7.4 here;
+// the kernel itself takes 5.6.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
