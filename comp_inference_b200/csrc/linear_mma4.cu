@@ -35,6 +35,8 @@
 // Measured (graph replays over more than L2 of weights), before -> after the chunks, the in-place renormalisation, the
 // wider choice of warp counts and the reordered activations: 4096 x 22016 at tile height 128, 1 row 90.4 -> 82.3 us,
 // 16 rows 126.7 -> 89.6; 4096 x 4096 at 1024 (was the generic kernel) 551 -> 68.
+#include <type_traits>
+
 #include "linear.cuh"
 #include "ptx.cuh"
 
@@ -504,67 +506,78 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
         }
         auto start_streams = [&]() {
             z.start(st_s, first);
-            if constexpr (!ENTRY) return;
-            // every stream has its own row of the window
-            const uint32_t rows_s = win_s + st_off + 512 + tsel_d * 128 + (hsel_d * 32 + gq * 4) * 2;
-            const uint32_t r01 = lds_u32(rows_s), r23 = lds_u32(rows_s + 4);
-            const uint32_t top = p.cap_rows - 1;
-            z.p[0] += min(r01 & 0xFFFFu, top) * 128;
-            z.p[1] += min(r01 >> 16, top) * 128;
-            z.p[2] += min(r23 & 0xFFFFu, top) * 128;
-            z.p[3] += min(r23 >> 16, top) * 128;
+            if constexpr (ENTRY) {                              // every stream has its own row of the window
+                const uint32_t rows_s = win_s + st_off + 512 + tsel_d * 128 + (hsel_d * 32 + gq * 4) * 2;
+                const uint32_t r01 = lds_u32(rows_s), r23 = lds_u32(rows_s + 4);
+                const uint32_t top = p.cap_rows - 1;
+                z.p[0] += min(r01 & 0xFFFFu, top) * 128;
+                z.p[1] += min(r01 >> 16, top) * 128;
+                z.p[2] += min(r23 & 0xFFFFu, top) * 128;
+                z.p[3] += min(r23 >> 16, top) * 128;
+            }
         };
         start_streams();
 
         uint32_t wb[4][2] = {};
         uint32_t xf[4] = {};                                     // the group before: its weights, its activations
         uint32_t blk = 0, left = len;                           // left: blocks until this lane's stream is used up
+        // Compiled for whole units and, in RAGGED, once more for the one of a column group that is not: with the tests in
+        // one loop for both, all units paid for them.
+        auto decode_unit = [&](auto rag_tag) {
+            constexpr bool RAG = decltype(rag_tag)::value;
 #pragma unroll 1
-        for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
-            const uint32_t buf = chunk & 1;
-            __syncwarp();                                       // every lane is done with the other chunk buffer
-            if (c + 1 < n_chunks) issue_man(man, two, c + 1, buf ^ 1);
-            else if (t + 1 < hi) issue_man(man_of(n_grp, n_pk, n_sub), 2 * n_pk + 1 < g.tiles_k, 0, buf ^ 1);
-            if (c == 0 && p.stages == 2) next_unit();   // behind it: a chunk's arrival waits for older copies
-            if (!mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1)) atomicExch(p.status, 1u);
-            z.clamp(win_s);
-            uint32_t ms = man_s + (buf * 4 + q) * kSegPitch + gq * 4;
-            const uint32_t end = RAGGED && empty ? 0u : min(blk + kChunkRows / 4, n_blocks);
+            for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
+                const uint32_t buf = chunk & 1;
+                __syncwarp();                                       // every lane is done with the other chunk buffer
+                if (c + 1 < n_chunks) issue_man(man, two, c + 1, buf ^ 1);
+                else if (t + 1 < hi) issue_man(man_of(n_grp, n_pk, n_sub), 2 * n_pk + 1 < g.tiles_k, 0, buf ^ 1);
+                if (c == 0 && p.stages == 2) next_unit();   // behind it: a chunk's arrival waits for older copies
+                if (!mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1)) atomicExch(p.status, 1u);
+                z.clamp(win_s);
+                uint32_t ms = man_s + (buf * 4 + q) * kSegPitch + gq * 4;
+                const uint32_t end = RAG && empty ? 0u : min(blk + kChunkRows / 4, n_blocks);
 #pragma unroll 1
-            for (; blk < end; ++blk) {
-                const uint2 v0 = __ldg(reinterpret_cast<const uint2 *>(xp0));   // used by the mma at the end
-                uint2 v1 = make_uint2(0u, 0u);
-                if constexpr (HI) v1 = __ldg(reinterpret_cast<const uint2 *>(xp1));
-                const uint32_t m[4] = {lds_u32(ms), lds_u32(ms + 32), lds_u32(ms + 64), lds_u32(ms + 96)};
-                // The tensor instruction of the group before comes first: behind it the compiler knows that the warp is
-                // converged, and the register copies that its checks of that need go.
-                mma4<HI>(acc, wb, xf);
-                group4(wb, z, lut_s, m);
-                if (rag) {
-                    const uint32_t n = blk + 1 < n_my ? 4u : blk >= n_my ? 0u : cut ? cut : 4u;   // rows of the block that exist
-                    if (n < 4) {
+                for (; blk < end; ++blk) {
+                    const uint2 v0 = __ldg(reinterpret_cast<const uint2 *>(xp0));   // used by the mma at the end
+                    uint2 v1 = make_uint2(0u, 0u);
+                    if constexpr (HI) v1 = __ldg(reinterpret_cast<const uint2 *>(xp1));
+                    const uint32_t m[4] = {lds_u32(ms), lds_u32(ms + 32), lds_u32(ms + 64), lds_u32(ms + 96)};
+                    // The tensor instruction of the group before comes first: behind it the compiler knows that the warp is
+                    // converged, and the register copies that its checks of that need go.
+                    mma4<HI>(acc, wb, xf);
+                    group4(wb, z, lut_s, m);
+                    if constexpr (RAG) {
+                        const uint32_t n = blk + 1 < n_my ? 4u : blk >= n_my ? 0u : cut ? cut : 4u;   // rows of the block that exist
+                        if (n < 4) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            wb[i][0] &= n == 0 ? 0u : n == 1 ? 0xFFFFu : 0xFFFFFFFFu;
-                            wb[i][1] &= n == 3 ? 0xFFFFu : 0u;
+                            for (int i = 0; i < 4; ++i) {
+                                wb[i][0] &= n == 0 ? 0u : n == 1 ? 0xFFFFu : 0xFFFFFFFFu;
+                                wb[i][1] &= n == 3 ? 0xFFFFu : 0u;
+                            }
+                        }
+                    }
+                    xf[0] = v0.x; xf[1] = v0.y; xf[2] = v1.x; xf[3] = v1.y;
+                    ms += 128;
+                    xp0 += xs;
+                    if constexpr (HI) xp1 += xs;
+                    if constexpr (RAG) {
+                        if (blk + 1 == n_my) {                      // rows beyond K from the next block on
+                            xp0 = xp1 = g_zero_activations;
+                            xs = 0;
+                        }
+                        if (--left == 0) {
+                            left = len;
+                            start_streams();
                         }
                     }
                 }
-                xf[0] = v0.x; xf[1] = v0.y; xf[2] = v1.x; xf[3] = v1.y;
-                ms += 128;
-                xp0 += xs;
-                if constexpr (HI) xp1 += xs;
-                if (rag) {
-                    if (blk + 1 == n_my) {                      // rows beyond K from the next block on
-                        xp0 = xp1 = g_zero_activations;
-                        xs = 0;
-                    }
-                    if (--left == 0) {
-                        left = len;
-                        start_streams();
-                    }
-                }
             }
+        };
+        if constexpr (RAGGED) {
+            if (rag) decode_unit(std::true_type{});
+            else decode_unit(std::false_type{});
+        } else {
+            decode_unit(std::false_type{});
         }
         mma4<HI>(acc, wb, xf);
         if (p.stages == 1) {
