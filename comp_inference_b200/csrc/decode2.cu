@@ -159,7 +159,14 @@ __global__ void __launch_bounds__(kDec2Warps * 32, 1) k_decode2(const __grid_con
         (void)mbar_wait(bar, parity);
         parity ^= 1;
         Pair z;
-        z.start(st_s, first);
+        auto start_streams = [&]() {
+            z.start(st_s, first);
+            if (EDGE && tn * 32 + c_d + 1 >= g.N) {             // as Quad::keep
+                z.s[1] = z.s[0];
+                z.p[1] = z.p[0];
+            }
+        };
+        start_streams();
 
         uint8_t *o = reinterpret_cast<uint8_t *>(out) + ((size_t)row * p.ld + col) * (BF16 ? 2 : 1);
         const size_t pitch = (size_t)p.ld * (BF16 ? 2 : 1);
@@ -218,7 +225,7 @@ __global__ void __launch_bounds__(kDec2Warps * 32, 1) k_decode2(const __grid_con
             }
             if (EDGE && --left == 0) {
                 left = len;
-                z.start(st_s, first);
+                start_streams();
             }
         }
     }

@@ -218,21 +218,26 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         };
 
         const uint32_t win_s = wbase_s + stage * p.stage_bytes;
-        const uint32_t st_s = win_s + st_off + tsel_d * 256 + (hsel_d * 32 + (quad & 7) * 4) * 4;
-        uint32_t first = win_s + tsel_d * 64 + hsel_d * 32 + (quad & 7) * 4;
+        // Columns beyond N: see Quad::keep; a lane without any takes the first ones of its tile.  (An index keeps the rows
+        // that its own streams have left, so there every stream is its own.)
+        const uint32_t quad_d = INDEX || cols != 0 ? quad & 7 : 0u;
+        const uint32_t cols_d = INDEX ? 4u : min(4u, g.N - (64 * tp + 32 * tsel_d + 4 * quad_d));
+        const uint32_t st_s = win_s + st_off + tsel_d * 256 + (hsel_d * 32 + quad_d * 4) * 4;
+        uint32_t first = win_s + tsel_d * 64 + hsel_d * 32 + quad_d * 4;
         if (!ENTRY && ml <= p.cap_rows) first += (ml - 1) * 128;  // last byte row; an empty tile starts one row below
         (void)mbar_wait(bar_base + stage * 8, stage ? parity1 : parity0);
         if (stage) parity1 ^= 1; else parity0 ^= 1;
         auto start_streams = [&]() {
             z.start(st_s, first);
-            if constexpr (!ENTRY) return;
-            // every stream has its own row of the window
-            const uint32_t rows_s = win_s + st_off + 512 + tsel_d * 128 + (hsel_d * 32 + (quad & 7) * 4) * 2;
-            const uint32_t r01 = lds_u32(rows_s), r23 = lds_u32(rows_s + 4), top = p.cap_rows - 1;
-            z.p[0] += min(r01 & 0xFFFFu, top) * 128;
-            z.p[1] += min(r01 >> 16, top) * 128;
-            z.p[2] += min(r23 & 0xFFFFu, top) * 128;
-            z.p[3] += min(r23 >> 16, top) * 128;
+            if constexpr (ENTRY) {                              // every stream has its own row of the window
+                const uint32_t rows_s = win_s + st_off + 512 + tsel_d * 128 + (hsel_d * 32 + quad_d * 4) * 2;
+                const uint32_t r01 = lds_u32(rows_s), r23 = lds_u32(rows_s + 4), top = p.cap_rows - 1;
+                z.p[0] += min(r01 & 0xFFFFu, top) * 128;
+                z.p[1] += min(r01 >> 16, top) * 128;
+                z.p[2] += min(r23 & 0xFFFFu, top) * 128;
+                z.p[3] += min(r23 >> 16, top) * 128;
+            }
+            if (EDGE && cols_d < 4) z.keep(cols_d);             // without EDGE N is a multiple of four
         };
         start_streams();
 

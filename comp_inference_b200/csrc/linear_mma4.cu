@@ -476,6 +476,9 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
             xp0 = xp1 = g_zero_activations;
             xs = 0;
         }
+        // Columns beyond N: see Quad::keep; a lane without any takes the first ones of its group.
+        const uint32_t left_n = g.N - grp * 32, gq_d = 4 * gq < left_n ? gq : 0u;
+        const uint32_t cols = min(4u, left_n - 4 * gq_d);
         const uint32_t ml = tsel_d ? nx_ml1 : nx_ml0;
         auto next_unit = [&]() {                                // every lane is done with the window it goes to
             if (t + 1 >= hi) return;
@@ -494,8 +497,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
 
         // ---- this lane's four streams --------------------------------------
         const uint32_t win_s = wbase_s + stage * p.stage_bytes;
-        const uint32_t st_s = win_s + st_off + tsel_d * 256 + (hsel_d * 32 + gq * 4) * 4;
-        uint32_t first = win_s + tsel_d * 64 + hsel_d * 32 + gq * 4;
+        const uint32_t st_s = win_s + st_off + tsel_d * 256 + (hsel_d * 32 + gq_d * 4) * 4;
+        uint32_t first = win_s + tsel_d * 64 + hsel_d * 32 + gq_d * 4;
         if (!ENTRY && ml <= p.cap_rows) first += (ml - 1) * 128;   // last byte row; an empty tile starts one row below
 
         // ---- wait for the bytes (bounded) -------------------------------------
@@ -507,7 +510,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
         auto start_streams = [&]() {
             z.start(st_s, first);
             if constexpr (ENTRY) {                              // every stream has its own row of the window
-                const uint32_t rows_s = win_s + st_off + 512 + tsel_d * 128 + (hsel_d * 32 + gq * 4) * 2;
+                const uint32_t rows_s = win_s + st_off + 512 + tsel_d * 128 + (hsel_d * 32 + gq_d * 4) * 2;
                 const uint32_t r01 = lds_u32(rows_s), r23 = lds_u32(rows_s + 4);
                 const uint32_t top = p.cap_rows - 1;
                 z.p[0] += min(r01 & 0xFFFFu, top) * 128;
@@ -515,6 +518,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
                 z.p[2] += min(r23 & 0xFFFFu, top) * 128;
                 z.p[3] += min(r23 >> 16, top) * 128;
             }
+            if (cols < 4) z.keep(cols);
         };
         start_streams();
 

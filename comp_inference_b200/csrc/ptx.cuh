@@ -214,6 +214,16 @@ struct Quad {
             : "+r"(s[0]), "+r"(s[1]), "+r"(s[2]), "+r"(s[3]), "+r"(p[0]), "+r"(p[1]), "+r"(p[2]), "+r"(p[3])
             : "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]));
     }
+    // Streams of columns that do not exist (`cols` of the four do) run along with the first one.  Their own would start at
+    // 2^16 over zero bytes: a symbol of frequency 1 at every step, and with it the branch for a second byte.
+    __device__ __forceinline__ void keep(uint32_t cols) {
+#pragma unroll
+        for (uint32_t j = 1; j < 4; ++j)
+            if (j >= cols) {
+                s[j] = s[0];
+                p[j] = p[0];
+            }
+    }
     // Keeps a malformed stream's cursors within reach of the window at `low`: call it at least every 32 symbols.
     __device__ __forceinline__ void clamp(uint32_t low) {
 #pragma unroll

@@ -162,3 +162,17 @@ def test_greedy_step(B, V):
         assert torch.equal(tok[:B], want) and torch.equal(out[:B, i], want)
         assert int(pos) == 7 + i and int(steps) == i and int(ticket) == 0
     assert int(tok[B]) == 0 and int(out[B].sum()) == 0
+
+
+# columns beyond N run along with others: one to three left in a lane's quad, lanes and tiles without any; whole and
+# ragged K, with and without entry points
+@pytest.mark.parametrize("K,N,th,M", [(8192, 4097, 128, 1), (8200, 4098, 64, 9), (8192, 4115, 128, 16), (2048, 35, 1024, 2),
+                                      (2049, 61, 1024, 5), (4100, 2020, 1024, 1)])
+def test_column_edges(K, N, th, M):
+    import comp_inference_b200 as ci
+    W = _weight(K, N)
+    c = ci.compress_weight_cuda(W, th, 32)
+    m = ci.RansLinear(K, N, c["tile_height"], c["tile_width"]).load_compressed(c).prepare()
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(K)).to(torch.bfloat16).cuda()
+    assert _close(m(x), x.float() @ W.float())
+    test_decoder_edges(K, N, th)
