@@ -11,12 +11,12 @@
 // weights leave as one 8-byte store.  Only the rows a stream can reach are copied: two bytes a symbol at most.
 //
 // At the tile heights that suit gathers only a few symbols are decoded per task, so what bounds the kernel is the work
-// around them.  A warp therefore takes a run of consecutive tasks: eight at a time their ids are read and their tiles'
+// around them.  A warp therefore takes many tasks: eight at a time their ids are read and their tiles'
 // offsets and depths fetched, one tile per lane, while the eight before them are worked off; a task then costs two
 // shuffles for its lane's own tile, and no division.  Byte windows, initial states and the row's sign+mantissa bytes are
 // fetched one task ahead.  Tall tiles are entered at the entry point before the row where the caller has them.  Measured on
 // a B200, 4096 ids of 32000 x 4096 at tile height 16: 148 us with one task at a time, divisions in 64 bits and eight
-// shuffles per task -> 88.
+// shuffles per task -> 72.
 #include "embedding.cuh"
 #include "ptx.cuh"
 
@@ -55,8 +55,11 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
     start_lut(lut_s, lut_bar, a.lut);
     const uint32_t wbase_s = lut_s + kLutBytes + kEmb4BarBytes + warp * p.stages * p.stage_bytes;
     const uint32_t bar_base = lut_s + kLutBytes + warp * 16;
-    const uint32_t gw = blockIdx.x * W + warp, n_warps = gridDim.x * W;
-    const uint32_t lo = (uint32_t)((uint64_t)gw * p.total / n_warps), hi = (uint32_t)((uint64_t)(gw + 1) * p.total / n_warps);
+    // Task n of this warp is gw + n * n_warps, the CTA running fastest in gw: the symbols to drop are a matter of the id, and a
+    // run of consecutive tasks has one or two ids.  4096 ids of 32000 x 4096, runs -> this: tile height 16 86 us -> 72, 128
+    // 460 -> 336, 1024 (2048 ids) 292 -> 209.
+    const uint32_t n_warps = gridDim.x * W;
+    const uint32_t gw = warp * gridDim.x + blockIdx.x, lo = 0, hi = gw < p.total ? (p.total - gw + n_warps - 1) / n_warps : 0u;
     const uint32_t tsel = lane >> 3, quad = lane & 7;           // tile of the block, column quad inside it
 
     if (lane == 0) {
@@ -80,7 +83,7 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
         uint32_t off, ml;      // the lane's tile: byte offset, depth (0 for a tile that is not read)
     };
     auto load_ids = [&](uint32_t first, Batch &b) {
-        const uint32_t t = min(first + (lane >> 2), hi - 1);
+        const uint32_t t = gw + min(first + (lane >> 2), hi - 1) * n_warps;
         b.ti = t / p.blocks_n;
         b.cb = t - b.ti * p.blocks_n;
         const int64_t id = __ldg(a.ids + b.ti);
