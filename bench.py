@@ -276,7 +276,7 @@ def secondary_metrics(mods, dense, device, peak_hbm, peak_tf, src):
     out["decode_bf16"] = {"effective_uncompressed_GBs": dense_bytes / (ms * 1e-3) / 1e9, "ms_per_block": ms,
                           "frac_of_hbm_peak": dense_bytes / (ms * 1e-3) / 1e9 / peak_hbm, "peak_source": f"of {src}"}
 
-    # ---- GPU encoder: whole pipeline (split, histogram, table, two encoder passes) and the encoder calls alone
+    # ---- GPU encoder: whole pipeline (split, histogram, table, encoder) and the encoder call alone
     W = dense["gate_up_proj"]
     ms = timed(lambda: ci.compress_weight_cuda(W, TILE_H, TILE_W), 3, warm=1)
     e, _ = ci.extract_exp_and_mantissa(W)
@@ -285,7 +285,7 @@ def secondary_metrics(mods, dense, device, peak_hbm, peak_tf, src):
     ms_enc = timed(lambda: mgr.compress_tiled(e, f, cdf, TILE_H, TILE_W, _keep_on_device=True), 3, warm=1)
     out["encode"] = {"shape_KN": list(W.shape), "pipeline_ms": ms, "pipeline_bf16_in_GBs": W.numel() * 2 / (ms * 1e-3) / 1e9,
                      "encoder_ms": ms_enc, "encoder_symbols_per_s": W.numel() / (ms_enc * 1e-3),
-                     "note": "encoder_ms = both passes (sizes, write) + the host wait between them"}
+                     "note": "encoder_ms = tables, encoder, packing and the host wait for the stream's length"}
     del e
 
     # ---- small batches through the block, ours and the dense library GEMV on the same rotation (> L2)

@@ -16,15 +16,15 @@ struct DecArgs {
     const uint16_t *entry_rows;
 };
 
-// Staged decoder (decode_staged.cu): CI_OK when launched, 1 when the tensor does not qualify
-// (the caller then uses the generic kernel), < 0 on error.
-// Four-streams-per-lane decoder for 32-wide tiles (decode4.cu); same return convention.
+// Every launcher: CI_OK when launched, 1 when the tensor does not qualify (the caller then tries the next one), < 0 on error.
+// Four-streams-per-lane decoder for 32-wide tiles (decode4.cu).
 int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, cudaStream_t s);
-// Two streams per lane (decode2.cu), where few streams leave that one too few warps; same return convention.
+// Two streams per lane (decode2.cu), where few streams leave that one too few warps.
 double decode4_cost(const DecArgs &a, uint32_t max_tile_len, bool bf16);   // run_cost of launch_decode4, 0: it does not qualify
 int launch_decode2(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, cudaStream_t s);
 int build_entry_points(const DecArgs &a, uint32_t max_tile_len, uint32_t step, uint32_t *d_states, uint16_t *d_rows,
                        uint32_t *d_spans, uint32_t *d_cap, cudaStream_t s);
+// Other tile widths (decode_staged.cu).
 int launch_decode_staged(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, cudaStream_t s);
 
 }  // namespace ci
