@@ -11,6 +11,7 @@
 #include <torch/extension.h>
 
 #include <mutex>
+#include <optional>
 #include <unordered_map>
 
 #include "../../include/comp_inference_b200.h"
@@ -127,8 +128,9 @@ void fill(Weight &h, int64_t K, int64_t N, int64_t th, int64_t tw, uint32_t max_
     h.w.max_tile_len = max_len;
 }
 
-// What is derived from a weight's tables and depths (the prepared decode table, the deepest tile) is kept per tensor
-// objects, as in the Python layer: weak references, data pointers and versions tell whether an entry still holds.
+// What is derived from a weight's arrays is kept per tensor objects, as in the Python layer, and holds only for what it was made
+// of: weak references, data pointers and versions tell.  A write that torch's version counter does not see (through .data, by
+// another library, by a replayed graph) is not seen here either.
 struct Ref {
     c10::weak_intrusive_ptr<c10::TensorImpl> impl;
     const void *data;
@@ -139,11 +141,20 @@ struct Ref {
                version == (t.is_inference() ? 0 : t._version());
     }
 };
+// The entry points of a weight: of its streams, not of its tables and depths alone.
+struct Index {
+    Ref stream, states, offsets;
+    int64_t K, N, th;
+    Entries entries;
+    bool is(const Tensor &s, const Tensor &st, const Tensor &o, int64_t k, int64_t n, int64_t h) const {
+        return stream.is(s) && states.is(st) && offsets.is(o) && K == k && N == n && th == h;
+    }
+};
 struct Derived {
     Ref tables, slot_map, lens;
-    Tensor lut;
-    uint32_t max_len;
-    Entries entries;
+    Tensor lut;                                                 // of tables and slot_map
+    uint32_t max_len;                                           // of lens
+    std::optional<Index> index;                                 // of all of them and what it names itself
 };
 std::mutex g_derived_mutex;
 std::unordered_map<const void *, Derived> &g_derived = *new std::unordered_map<const void *, Derived>;   // by tile_max_lens' impl
@@ -169,6 +180,7 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
                               std::to_string(tiles * th * tw) + " expected");
     uint32_t max_len = 0;
     bool keep = false;
+    std::optional<Index> index;
     // a contiguous copy made above is a new object on every call: nothing to remember
     if (h.tables.is_same(tables) && h.slot_map.is_same(slot_map) && h.lens.is_same(lens)) {
         const void *key = lens.unsafeGetTensorImpl();
@@ -178,7 +190,7 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
             if (it != g_derived.end() && it->second.lens.is(lens) && it->second.tables.is(tables) && it->second.slot_map.is(slot_map)) {
                 h.lut = it->second.lut;
                 max_len = it->second.max_len;
-                h.entries = it->second.entries;
+                index = it->second.index;
             }
         }
         if (!h.lut.defined()) {
@@ -188,8 +200,13 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
         }
     }
     fill(h, K, N, th, tw, max_len);
+    // Entry points are worth their making only where they can be kept: not for copies, nor for inference tensors, whose
+    // versions nobody counts.
+    auto kept = [](const Tensor &mine, const Tensor &given) { return mine.is_same(given) && !given.is_inference(); };
     const bool tall = entries && h.lut.defined() && tw == 32 && th > 2 * kEntryStep && th % (2 * kEntryStep) == 0 && th <= 65536 &&
+                      kept(h.stream, stream_t) && kept(h.states, states) && kept(h.offsets, offsets) && kept(h.lens, lens) &&
                       (reinterpret_cast<uintptr_t>(h.w.stream) & 15u) == 0 && (reinterpret_cast<uintptr_t>(h.w.states) & 15u) == 0;
+    if (tall && index && index->is(h.stream, h.states, h.offsets, K, N, th)) h.entries = index->entries;
     if (tall && !h.entries.states.defined() && max_len != 0) {
         Entries e;
         const int64_t n = tiles * (th / 2 / kEntryStep);
@@ -201,6 +218,7 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
                                     (uint32_t *)e.spans.data_ptr(), (uint32_t *)cap.data_ptr(), stream()));
         e.cap = std::max<uint32_t>(1, (uint32_t)cap.item<int32_t>());
         h.entries = e;
+        index.emplace(Index{Ref(h.stream), Ref(h.states), Ref(h.offsets), K, N, th, e});
         keep = true;
     }
     if (tall && h.entries.states.defined()) {
@@ -218,7 +236,7 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
         if (g_derived.size() > 4096) g_derived.clear();
         const void *key = lens.unsafeGetTensorImpl();
         g_derived.erase(key);
-        g_derived.emplace(key, Derived{Ref(tables), Ref(slot_map), Ref(lens), h.lut, max_len, h.entries});
+        g_derived.emplace(key, Derived{Ref(tables), Ref(slot_map), Ref(lens), h.lut, max_len, std::move(index)});
     }
     return h;
 }

@@ -1,0 +1,63 @@
+"""What is derived from a weight's arrays and kept between calls (decode table, deepest tile, entry points into tall tiles)
+follows the arrays."""
+import pytest
+import torch
+
+from conftest import make_weight
+
+pytestmark = pytest.mark.gpu
+
+ARRAYS = ("rans_exp_stream", "rans_exp_states", "rans_exp_tables", "rans_exp_slot_map", "rans_exp_tile_offsets",
+          "rans_exp_tile_max_lens", "rans_man_raw")
+K, N, TH, M = 2048, 96, 1024, 2
+
+
+def _two_weights():
+    """Two weights whose packages differ in stream, states and sign+mantissa bytes only: the columns of the second are the
+    first's, swapped in pairs, so every tile has the same streams in another order."""
+    import comp_inference_b200 as ci
+    a = make_weight(K, N, 5)
+    b = a.view(K, N // 2, 2).flip(-1).reshape(K, N)
+    ca, cb = (ci.compress_weight_cuda(w.cuda(), TH, 32) for w in (a, b))
+    for name in ARRAYS[2:6]:
+        assert torch.equal(ca[name].view(torch.uint8), cb[name].view(torch.uint8)), name
+    assert ca["rans_exp_stream"].numel() == cb["rans_exp_stream"].numel()
+    assert not torch.equal(ca["rans_exp_states"].view(torch.int32), cb["rans_exp_states"].view(torch.int32))
+    return a.cuda(), ca, b.cuda(), cb
+
+
+def _call(kind, c, x, ids):
+    import comp_inference_b200 as ci
+    args = [c[n] for n in ARRAYS[:4]] + [(K, N), c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"], TH, 32, c["rans_man_raw"]]
+    if kind == "linear":
+        return ci.fused_rans_linear_triton(x, *args)
+    if kind == "transposed":
+        return ci.fused_rans_linear_transposed_triton(x[:, :N], *args)
+    return ci.fused_rans_embedding_triton(ids, *args)
+
+
+def _right(kind, y, w, x, ids):
+    if kind == "embedding":
+        return torch.equal(y, w[ids])
+    ref = x.float() @ w.float() if kind == "linear" else x[:, :N].float() @ w.float().t()
+    return float((y.float() - ref).abs().max() / ref.abs().max()) <= 1e-2
+
+
+def _inputs():
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(7)).to(torch.bfloat16).cuda()
+    return x, torch.randint(0, K, (50,), generator=torch.Generator().manual_seed(8)).cuda()
+
+
+@pytest.mark.parametrize("kind", ["linear", "transposed", "embedding"])
+@pytest.mark.parametrize("how", ["other tensors", "overwritten"])
+def test_functional_calls_follow_the_streams(kind, how):
+    wa, ca, wb, cb = _two_weights()
+    x, ids = _inputs()
+    assert _right(kind, _call(kind, ca, x, ids), wa, x, ids)
+    if how == "other tensors":                          # a second weight that shares the arrays it can share
+        cb = dict(cb, **{n: ca[n] for n in ARRAYS[2:6]})
+        assert _right(kind, _call(kind, cb, x, ids), wb, x, ids)
+    else:
+        for n in ("rans_exp_stream", "rans_exp_states", "rans_man_raw"):
+            ca[n].copy_(cb[n])
+        assert _right(kind, _call(kind, ca, x, ids), wb, x, ids)
