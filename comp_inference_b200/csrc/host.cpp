@@ -86,15 +86,45 @@ struct Entries {
     uint32_t cap = 0;
 };
 
+// Inference tensors have no version.
+uint32_t version_of(const Tensor &t) {
+    return t.is_inference() ? 0 : t.unsafeGetTensorImpl()->version_counter().current_version();
+}
+
 // The arrays of one compressed weight and its descriptor.
 struct Weight {
     Tensor stream, states, tables, slot_map, offsets, lens, mantissa, lut;
     Entries entries;
     ci_tiled_weight w;
+    // What it was made from: the tensors as they were given, where their data lay and which version it was.
+    static constexpr int kArrays = 7;
+    Tensor given[kArrays];
+    const void *data[kArrays];
+    uint32_t version[kArrays];
 
-    bool matches(const Tensor &s, const Tensor &st, const Tensor &m, const Tensor &o, int64_t th, int64_t tw) const {
-        return s.data_ptr() == w.stream && st.data_ptr() == (const void *)w.states && m.data_ptr() == (const void *)w.mantissa &&
-               o.data_ptr() == (const void *)w.tile_offsets && (uint32_t)th == w.tile_h && (uint32_t)tw == w.tile_w;
+    void remember(std::initializer_list<Tensor> arrays) {
+        int i = 0;
+        for (const Tensor &t : arrays) {
+            given[i] = t;
+            data[i] = t.defined() ? t.data_ptr() : nullptr;
+            version[i++] = t.defined() ? version_of(t) : 0;
+        }
+    }
+    // Whether it still describes a module's buffers: none replaced, none moved, none written to.
+    bool matches(const py::dict &buffers, int64_t th, int64_t tw) const {
+        static PyObject *const names[kArrays] = {
+            PyUnicode_InternFromString("rans_exp_stream"), PyUnicode_InternFromString("rans_exp_states"),
+            PyUnicode_InternFromString("rans_exp_tables"), PyUnicode_InternFromString("rans_exp_slot_map"),
+            PyUnicode_InternFromString("rans_exp_tile_offsets"), PyUnicode_InternFromString("rans_exp_tile_max_lens"),
+            PyUnicode_InternFromString("rans_man_raw")};
+        if ((uint32_t)th != w.tile_h || (uint32_t)tw != w.tile_w) return false;
+        for (int i = 0; i < kArrays; ++i) {
+            PyObject *o = PyDict_GetItem(buffers.ptr(), names[i]);
+            if (o == nullptr || !THPVariable_Check(o)) return false;
+            const Tensor &t = THPVariable_Unpack(o);
+            if (!t.is_same(given[i]) || t.data_ptr() != data[i] || version_of(t) != version[i]) return false;
+        }
+        return true;
     }
 };
 
@@ -135,10 +165,10 @@ struct Ref {
     c10::weak_intrusive_ptr<c10::TensorImpl> impl;
     const void *data;
     uint32_t version;
-    explicit Ref(const Tensor &t) : impl(t.getIntrusivePtr()), data(t.data_ptr()), version(t.is_inference() ? 0 : t._version()) {}
+    explicit Ref(const Tensor &t) : impl(t.getIntrusivePtr()), data(t.data_ptr()), version(version_of(t)) {}
     bool is(const Tensor &t) const {
         return !impl.expired() && impl._unsafe_get_target() == t.unsafeGetTensorImpl() && data == t.data_ptr() &&
-               version == (t.is_inference() ? 0 : t._version());
+               version == version_of(t);
     }
 };
 // The entry points of a weight: of its streams, not of its tables and depths alone.
@@ -169,6 +199,7 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
     h.offsets = as_u32(offsets, "tile_offsets");
     h.lens = as_u32(lens, "tile_max_lens");
     if (mantissa.has_value()) h.mantissa = as_u8(*mantissa, "mantissas");
+    h.remember({stream_t, states, tables, slot_map, offsets, lens, mantissa.has_value() ? *mantissa : Tensor()});
     if (th <= 0 || tw <= 0) throw py::value_error("tile sizes must be positive");
     const int64_t tiles = ((K + th - 1) / th) * ((N + tw - 1) / tw);
     if (h.states.numel() != tiles * 2 * tw)

@@ -53,37 +53,35 @@ class _RansBase(nn.Module):
         return self
 
     def prepare(self):
-        """Everything a forward would otherwise do lazily on its first call (descriptor, prepared decode
-        table, the deepest tile -- one device-to-host read): call it once the buffers are on the GPU and
-        before a CUDA graph is captured.  Subclasses add their own one-time work."""
+        """Everything a forward would otherwise do lazily on its first call (descriptor, prepared decode table, the
+        deepest tile and, for tall tiles, the entry points into their streams -- one or two device-to-host reads): call it
+        once the buffers are on the GPU and before a CUDA graph is captured.  Subclasses add their own one-time work."""
         if self.rans_exp_stream.is_cuda and self.rans_exp_states.numel():
-            self._weight(*self._stored_shape())
             self._native()
         return self
 
     _handle = None
 
     def _weight(self, K, N):
-        """The ci_tiled_weight descriptor of this module's buffers, built once (with the prepared decode
-        table and the deepest tile) and rebuilt only if a buffer was replaced."""
-        key = (self.rans_exp_stream.data_ptr(), self.rans_exp_states.data_ptr(), self.rans_man_raw.data_ptr(),
-               self.rans_exp_tile_offsets.data_ptr(), self.tile_k, self.tile_n)
-        if self._handle is None or self._handle[0] != key:
+        """The ci_tiled_weight descriptor of this module's buffers (with the prepared decode table and the deepest tile,
+        without entry points) for calls through ctypes."""
+        native = self._native()
+        if self._handle is None or self._handle[0] is not native:
             w, keep = _lib.tiled_weight(self.rans_exp_stream, self.rans_exp_states, self.rans_exp_tables,
                                         self.rans_exp_slot_map, self.rans_exp_tile_offsets,
                                         self.rans_exp_tile_max_lens, self.rans_man_raw, K, N, int(self.tile_k),
                                         int(self.tile_n), want_max=True)
-            self._handle = (key, w, keep)
+            self._handle = (native, w, keep)
         return self._handle[1]
 
     _native_handle = None
     _entries = False                # whether the module's kernel uses entry points into the streams of tall tiles
 
     def _native(self):
-        """The same descriptor for the native host path (_lib.host()); rebuilt only if a buffer was replaced."""
+        """The descriptor for the native host path (_lib.host()), built once and rebuilt if a buffer was replaced, moved or
+        written to (as torch's version counters tell: not through ``.data``, nor by a replayed graph)."""
         b, h = self._buffers, self._native_handle
-        if h is None or not h.matches(b["rans_exp_stream"], b["rans_exp_states"], b["rans_man_raw"],
-                                      b["rans_exp_tile_offsets"], self.tile_k, self.tile_n):
+        if h is None or not h.matches(b, self.tile_k, self.tile_n):
             h = _lib.host().Weight(b["rans_exp_stream"], b["rans_exp_states"], b["rans_exp_tables"], b["rans_exp_slot_map"],
                                    b["rans_exp_tile_offsets"], b["rans_exp_tile_max_lens"], b["rans_man_raw"],
                                    *self._stored_shape(), int(self.tile_k), int(self.tile_n), self._entries)
@@ -207,7 +205,10 @@ class RansLMHead(_RansBase):
         self._register()
 
     _twin = None
-    _entries = True
+
+    @property
+    def _entries(self):
+        return not self.fast_twin                               # the twin is made from a plain decode
 
     def _stored_shape(self):
         return self.out_features, self.in_features
@@ -222,31 +223,21 @@ class RansLMHead(_RansBase):
 
     def _twin_weight(self):
         """Descriptor of the [H, V] re-encoding, built on first use and rebuilt if the buffers change."""
-        V, H = self.out_features, self.in_features
-        key = (self.rans_exp_stream.data_ptr(), self.rans_exp_states.data_ptr(), self.rans_man_raw.data_ptr())
-        if self._twin is None or self._twin[0] != key:
+        stored = self._native()
+        if self._twin is None or self._twin[0] is not stored or self._twin[2] != self.twin_tile:
             from . import comp_inference as ci_mod
-            w_vh = ops.rans_decompress_bf16(self.rans_exp_stream, self.rans_exp_states, self.rans_exp_tables,
-                                            self.rans_exp_slot_map, (V, H), self.rans_exp_tile_offsets,
-                                            self.rans_exp_tile_max_lens, int(self.tile_k), int(self.tile_n),
-                                            self.rans_man_raw)
-            c = ci_mod.compress_weight_cuda(w_vh.t().contiguous(), *self.twin_tile)
-            del w_vh
-            w, keep = _lib.tiled_weight(c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"],
-                                        c["rans_exp_slot_map"], c["rans_exp_tile_offsets"],
-                                        c["rans_exp_tile_max_lens"], c["rans_man_raw"], H, V, int(c["tile_height"]),
-                                        int(c["tile_width"]), want_max=True)
-            native = _lib.host().Weight(c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"],
-                                        c["rans_exp_slot_map"], c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"],
-                                        c["rans_man_raw"], H, V, int(c["tile_height"]), int(c["tile_width"]))
-            self._twin = (key, w, keep, c, native)
+            c = ci_mod.compress_weight_cuda(stored.decode(True).t().contiguous(), *self.twin_tile)
+            twin = _lib.host().Weight(c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"],
+                                      c["rans_exp_slot_map"], c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"],
+                                      c["rans_man_raw"], self.in_features, self.out_features, int(c["tile_height"]),
+                                      int(c["tile_width"]))
+            self._twin = (stored, twin, self.twin_tile, c)
         return self._twin[1]
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         rows = 0 if self.prefill_policy == "fused" else max(self.prefill_rows, 17)   # from here on: logits of a whole prompt
         if self.fast_twin:
-            self._twin_weight()
-            return self._twin[4].linear(x, None, None, 0, False, rows)
+            return self._twin_weight().linear(x, None, None, 0, False, rows)
         return self._native().linear(x, None, None, 0, True, rows)
 
 

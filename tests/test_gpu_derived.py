@@ -61,3 +61,40 @@ def test_functional_calls_follow_the_streams(kind, how):
         for n in ("rans_exp_stream", "rans_exp_states", "rans_man_raw"):
             ca[n].copy_(cb[n])
         assert _right(kind, _call(kind, ca, x, ids), wb, x, ids)
+
+
+def _module(kind, c):
+    import comp_inference_b200 as ci
+    m = {"linear": lambda: ci.RansLinear(K, N, TH, 32), "embedding": lambda: ci.RansEmbedding(K, N, TH, 32),
+         "transposed": lambda: ci.RansLMHead(N, K, TH, 32, fast_twin=False), "twin": lambda: ci.RansLMHead(N, K, TH, 32)}[kind]()
+    return m.load_compressed({n: c[n].clone() for n in ARRAYS}).prepare()
+
+
+@pytest.mark.parametrize("kind", ["linear", "embedding", "transposed", "twin"])
+@pytest.mark.parametrize("how", ["overwritten", "replaced"])
+@pytest.mark.parametrize("what", ["streams", "tables"])
+def test_modules_follow_their_buffers(kind, how, what):
+    wa, ca, wb, cb = _two_weights()
+    changed = ("rans_exp_stream", "rans_exp_states", "rans_man_raw")
+    if what == "tables":                                # the same bytes read as exponents one higher: twice the weight
+        wb, changed = wa * 2, ARRAYS[2:4]
+        cb = dict(ca, rans_exp_tables=ca["rans_exp_tables"].view(torch.int32).roll(1).view(torch.uint32),
+                  rans_exp_slot_map=ca["rans_exp_slot_map"] + 1)
+    x, ids = _inputs()
+    m = _module(kind, ca)
+
+    def right(w):
+        if kind == "embedding":
+            return _right(kind, m(ids), w, x, ids)
+        if kind == "linear":                            # and as a prompt: decoded first
+            xl = x.repeat(10, 1)
+            return _right(kind, m(x), w, x, ids) and _right(kind, m(xl), w, xl, ids)
+        return _right("transposed", m(x[:, :N].contiguous()), w, x, ids)
+
+    assert right(wa)
+    if how == "replaced":
+        m.load_compressed({n: cb[n].clone() for n in changed})
+    else:
+        for n in changed:
+            getattr(m, n).copy_(cb[n])
+    assert right(wb)
