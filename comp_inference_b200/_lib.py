@@ -191,18 +191,28 @@ def as_u8(t, name):
 _lut_cache = {}
 
 
+def _make_room(cache):
+    """Drops the entries of tensors that are gone (a captured graph may refer to those of the others)."""
+    if len(cache) > 4096:
+        for key in [k for k, hit in cache.items() if hit[0]() is None]:
+            del cache[key]
+
+
 def prepared_lut(tables, slot_map):
-    """Device uint32[4096] merged decode table for this tables/slot_map pair (cached per tensor object)."""
+    """Device uint32[4096] merged decode table for this tables/slot_map pair (cached per tensor object).  None while the
+    current stream captures and there is none yet: the kernels then build it, and a table made inside a graph would hold
+    nothing until that graph has run."""
     key = (tables.data_ptr(), slot_map.data_ptr())
     hit = _lut_cache.get(key)
     if hit is not None:
         ref_t, ref_s, ver, lut = hit
         if ref_t() is tables and ref_s() is slot_map and ver == (tables._version, slot_map._version):
             return lut
+    if torch.cuda.is_current_stream_capturing():
+        return None
     lut = torch.empty(4096, dtype=torch.int32, device=tables.device)
     check(load().ci_prepare_lut(ptr(tables), ptr(slot_map), ptr(lut), stream()))
-    if len(_lut_cache) > 4096:
-        _lut_cache.clear()
+    _make_room(_lut_cache)
     _lut_cache[key] = (weakref.ref(tables), weakref.ref(slot_map), (tables._version, slot_map._version), lut)
     return lut
 
@@ -218,8 +228,7 @@ def max_tile_len(tile_max_lens):
     if hit is not None and hit[0]() is tile_max_lens and hit[1] == tile_max_lens._version:
         return hit[2]
     v = int(tile_max_lens.view(torch.int32).max().item()) if tile_max_lens.numel() else 0
-    if len(_maxlen_cache) > 4096:
-        _maxlen_cache.clear()
+    _make_room(_maxlen_cache)
     _maxlen_cache[key] = (weakref.ref(tile_max_lens), tile_max_lens._version, v)
     return v
 

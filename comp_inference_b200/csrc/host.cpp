@@ -7,11 +7,11 @@
 // the kernel itself takes 5.6.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
 #include <mutex>
-#include <optional>
 #include <unordered_map>
 
 #include "../../include/comp_inference_b200.h"
@@ -95,6 +95,7 @@ uint32_t version_of(const Tensor &t) {
 struct Weight {
     Tensor stream, states, tables, slot_map, offsets, lens, mantissa, lut;
     Entries entries;
+    bool lasting = true;       // false: made under stream capture without what has to be derived first; not to be kept
     ci_tiled_weight w;
     // What it was made from: the tensors as they were given, where their data lay and which version it was.
     static constexpr int kArrays = 7;
@@ -160,7 +161,8 @@ void fill(Weight &h, int64_t K, int64_t N, int64_t th, int64_t tw, uint32_t max_
 
 // What is derived from a weight's arrays is kept per tensor objects, as in the Python layer, and holds only for what it was made
 // of: weak references, data pointers and versions tell.  A write that torch's version counter does not see (through .data, by
-// another library, by a replayed graph) is not seen here either.
+// another library, by a replayed graph) is not seen here either.  An entry stays until its tensors are gone or have changed: a
+// captured graph may refer to it.
 struct Ref {
     c10::weak_intrusive_ptr<c10::TensorImpl> impl;
     const void *data;
@@ -171,23 +173,55 @@ struct Ref {
                version == version_of(t);
     }
 };
-// The entry points of a weight: of its streams, not of its tables and depths alone.
+// The decode table of tables and slot_map, the depth of the deepest tile.
+struct Tables {
+    Ref lens, tables, slot_map;
+    Tensor lut;
+    uint32_t max_len;
+    bool is(const Weight &h) const { return lens.is(h.lens) && tables.is(h.tables) && slot_map.is(h.slot_map); }
+    bool expired() const { return lens.impl.expired() || tables.impl.expired() || slot_map.impl.expired(); }
+};
+// The entry points of all of a weight's streams.
 struct Index {
-    Ref stream, states, offsets;
+    Ref stream, states, tables, slot_map, offsets, lens;
     int64_t K, N, th;
     Entries entries;
-    bool is(const Tensor &s, const Tensor &st, const Tensor &o, int64_t k, int64_t n, int64_t h) const {
-        return stream.is(s) && states.is(st) && offsets.is(o) && K == k && N == n && th == h;
+    bool is(const Weight &h) const {
+        return stream.is(h.stream) && states.is(h.states) && tables.is(h.tables) && slot_map.is(h.slot_map) &&
+               offsets.is(h.offsets) && lens.is(h.lens) && K == h.w.K && N == h.w.N && th == h.w.tile_h;
+    }
+    bool expired() const {
+        return stream.impl.expired() || states.impl.expired() || tables.impl.expired() || slot_map.impl.expired() ||
+               offsets.impl.expired() || lens.impl.expired();
     }
 };
+// By the tensor that an entry begins with.
+template <class T>
 struct Derived {
-    Ref tables, slot_map, lens;
-    Tensor lut;                                                 // of tables and slot_map
-    uint32_t max_len;                                           // of lens
-    std::optional<Index> index;                                 // of all of them and what it names itself
+    std::mutex mutex;
+    std::unordered_map<const void *, T> map;
+
+    // Calls use(entry) if there is one that holds for h.
+    template <class Use>
+    bool find(const Tensor &first, const Weight &h, Use use) {
+        std::lock_guard<std::mutex> lock(mutex);
+        auto it = map.find(first.unsafeGetTensorImpl());
+        if (it == map.end() || !it->second.is(h)) return false;
+        use(it->second);
+        return true;
+    }
+    void keep(const Tensor &first, T entry) {
+        std::lock_guard<std::mutex> lock(mutex);
+        // what belongs to weights that are gone goes with the next new one
+        for (auto it = map.begin(); it != map.end();) it = it->second.expired() ? map.erase(it) : std::next(it);
+        map.insert_or_assign(first.unsafeGetTensorImpl(), std::move(entry));
+    }
 };
-std::mutex g_derived_mutex;
-std::unordered_map<const void *, Derived> &g_derived = *new std::unordered_map<const void *, Derived>;   // by tile_max_lens' impl
+Derived<Tables> &g_tables = *new Derived<Tables>;               // by tile_max_lens
+Derived<Index> &g_indexes = *new Derived<Index>;                // by the stream
+
+// While a stream captures, nothing can be read back, and what a kernel writes exists only once the graph has run.
+bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
 
 Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables, const Tensor &slot_map, const Tensor &offsets,
              const Tensor &lens, const OptTensor &mantissa, int64_t K, int64_t N, int64_t th, int64_t tw, bool entries) {
@@ -210,64 +244,54 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
         throw py::value_error("mantissa plane has " + std::to_string(h.mantissa.numel()) + " bytes, " +
                               std::to_string(tiles * th * tw) + " expected");
     uint32_t max_len = 0;
-    bool keep = false;
-    std::optional<Index> index;
     // a contiguous copy made above is a new object on every call: nothing to remember
     if (h.tables.is_same(tables) && h.slot_map.is_same(slot_map) && h.lens.is_same(lens)) {
-        const void *key = lens.unsafeGetTensorImpl();
-        {
-            std::lock_guard<std::mutex> lock(g_derived_mutex);
-            auto it = g_derived.find(key);
-            if (it != g_derived.end() && it->second.lens.is(lens) && it->second.tables.is(tables) && it->second.slot_map.is(slot_map)) {
-                h.lut = it->second.lut;
-                max_len = it->second.max_len;
-                index = it->second.index;
-            }
-        }
-        if (!h.lut.defined()) {
+        const bool known = g_tables.find(lens, h, [&](const Tables &t) {
+            h.lut = t.lut;
+            max_len = t.max_len;
+        });
+        if (known) {
+        } else if (capturing()) {
+            h.lasting = false;                                  // the kernels that build the table themselves and need no depth
+        } else {
             h.lut = lib_attr("prepared_lut")(tables, slot_map).cast<Tensor>();
             max_len = lib_attr("max_tile_len")(lens).cast<uint32_t>();
-            keep = true;
+            g_tables.keep(lens, Tables{Ref(lens), Ref(tables), Ref(slot_map), h.lut, max_len});
         }
     }
     fill(h, K, N, th, tw, max_len);
     // Entry points are worth their making only where they can be kept: not for copies, nor for inference tensors, whose
     // versions nobody counts.
     auto kept = [](const Tensor &mine, const Tensor &given) { return mine.is_same(given) && !given.is_inference(); };
-    const bool tall = entries && h.lut.defined() && tw == 32 && th > 2 * kEntryStep && th % (2 * kEntryStep) == 0 && th <= 65536 &&
-                      kept(h.stream, stream_t) && kept(h.states, states) && kept(h.offsets, offsets) && kept(h.lens, lens) &&
-                      (reinterpret_cast<uintptr_t>(h.w.stream) & 15u) == 0 && (reinterpret_cast<uintptr_t>(h.w.states) & 15u) == 0;
-    if (tall && index && index->is(h.stream, h.states, h.offsets, K, N, th)) h.entries = index->entries;
-    if (tall && !h.entries.states.defined() && max_len != 0) {
-        Entries e;
-        const int64_t n = tiles * (th / 2 / kEntryStep);
-        e.states = at::empty({n * 64}, h.states.options());
-        e.rows = at::empty({n * 64}, h.states.options().dtype(at::kShort));
-        e.spans = at::empty({n}, h.states.options());
-        Tensor cap = at::empty({1}, h.states.options().dtype(at::kInt));
-        check(ci_build_entry_points(&h.w, kEntryStep, (uint32_t *)e.states.data_ptr(), (uint16_t *)e.rows.data_ptr(),
-                                    (uint32_t *)e.spans.data_ptr(), (uint32_t *)cap.data_ptr(), stream()));
-        e.cap = std::max<uint32_t>(1, (uint32_t)cap.item<int32_t>());
-        h.entries = e;
-        index.emplace(Index{Ref(h.stream), Ref(h.states), Ref(h.offsets), K, N, th, e});
-        keep = true;
+    const bool tall = entries && h.lut.defined() && max_len != 0 && tw == 32 && th > 2 * kEntryStep && th % (2 * kEntryStep) == 0 &&
+                      th <= 65536 && kept(h.stream, stream_t) && kept(h.states, states) && kept(h.offsets, offsets) &&
+                      kept(h.lens, lens) && (reinterpret_cast<uintptr_t>(h.w.stream) & 15u) == 0 &&
+                      (reinterpret_cast<uintptr_t>(h.w.states) & 15u) == 0;
+    if (tall) {
+        if (g_indexes.find(h.stream, h, [&](const Index &i) { h.entries = i.entries; })) {
+        } else if (capturing()) {
+            h.lasting = false;
+        } else {
+            Entries e;
+            const int64_t n = tiles * (th / 2 / kEntryStep);
+            e.states = at::empty({n * 64}, h.states.options());
+            e.rows = at::empty({n * 64}, h.states.options().dtype(at::kShort));
+            e.spans = at::empty({n}, h.states.options());
+            Tensor cap = at::empty({1}, h.states.options().dtype(at::kInt));
+            check(ci_build_entry_points(&h.w, kEntryStep, (uint32_t *)e.states.data_ptr(), (uint16_t *)e.rows.data_ptr(),
+                                        (uint32_t *)e.spans.data_ptr(), (uint32_t *)cap.data_ptr(), stream()));
+            e.cap = std::max<uint32_t>(1, (uint32_t)cap.item<int32_t>());
+            h.entries = e;
+            g_indexes.keep(h.stream, Index{Ref(h.stream), Ref(h.states), Ref(h.tables), Ref(h.slot_map), Ref(h.offsets),
+                                           Ref(h.lens), K, N, th, e});
+        }
     }
-    if (tall && h.entries.states.defined()) {
+    if (h.entries.states.defined()) {
         h.w.entry_step = kEntryStep;
         h.w.entry_states = (const uint32_t *)h.entries.states.data_ptr();
         h.w.entry_rows = (const uint16_t *)h.entries.rows.data_ptr();
         h.w.entry_spans = (const uint32_t *)h.entries.spans.data_ptr();
         h.w.entry_cap = h.entries.cap;
-    }
-    if (keep) {
-        std::lock_guard<std::mutex> lock(g_derived_mutex);
-        // what belongs to weights that are gone goes with the next new one
-        for (auto it = g_derived.begin(); it != g_derived.end();)
-            it = it->second.lens.impl.expired() || it->second.tables.impl.expired() ? g_derived.erase(it) : std::next(it);
-        if (g_derived.size() > 4096) g_derived.clear();
-        const void *key = lens.unsafeGetTensorImpl();
-        g_derived.erase(key);
-        g_derived.emplace(key, Derived{Ref(tables), Ref(slot_map), Ref(lens), h.lut, max_len, std::move(index)});
     }
     return h;
 }
@@ -430,6 +454,7 @@ PYBIND11_MODULE(_ci_host, m) {
         .def(py::init(&tiled), py::arg("stream"), py::arg("states"), py::arg("tables"), py::arg("slot_map"), py::arg("tile_offsets"),
              py::arg("tile_max_lens"), py::arg("mantissas"), py::arg("K"), py::arg("N"), py::arg("tile_h"), py::arg("tile_w"), py::arg("entries") = false)
         .def("matches", &Weight::matches)
+        .def_readonly("lasting", &Weight::lasting)
         .def("linear", &linear_call, py::arg("x"), py::arg("bias") = py::none(), py::arg("out") = py::none(), py::arg("split_k") = 0,
              py::arg("transposed") = false, py::arg("prefill_rows") = 0)
         .def("embedding", &embedding_call, py::arg("x"), py::arg("out") = py::none())

@@ -13,7 +13,16 @@ public API of the reference; nothing here is Triton.)
 
 All tensor arguments must already be CUDA tensors; inputs are borrowed for the
 call, outputs are fresh tensors or the caller's ``out``.  Everything is queued on
-the current torch CUDA stream and nothing synchronises.
+the current torch CUDA stream.
+
+What the tiled kernels need beyond the arrays (the prepared decode table, the depth
+of the deepest tile, entry points into the streams of tall tiles) is derived at the
+first call that brings them and kept as long as the same tensor objects come again
+unchanged: that call waits for the stream once, or twice where a linear or a gather
+meets tiles taller than 128 rows; the others do not wait.  While the stream captures, nothing
+is derived: a weight that was not used before runs on the kernels that need nothing
+but the arrays.  A captured graph holds what was derived for the weight as it was;
+capture it again after overwriting one in place.
 """
 import torch
 

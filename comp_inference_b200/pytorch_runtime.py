@@ -85,7 +85,8 @@ class _RansBase(nn.Module):
             h = _lib.host().Weight(b["rans_exp_stream"], b["rans_exp_states"], b["rans_exp_tables"], b["rans_exp_slot_map"],
                                    b["rans_exp_tile_offsets"], b["rans_exp_tile_max_lens"], b["rans_man_raw"],
                                    *self._stored_shape(), int(self.tile_k), int(self.tile_n), self._entries)
-            self.__dict__["_native_handle"] = h
+            if h.lasting:
+                self.__dict__["_native_handle"] = h
         return h
 
 

@@ -98,3 +98,48 @@ def test_modules_follow_their_buffers(kind, how, what):
         for n in changed:
             getattr(m, n).copy_(cb[n])
     assert right(wb)
+
+
+def _captured(fn):
+    """fn captured on a stream of its own, replayed once: (graph, result)."""
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        y = fn()
+    y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    return graph, y
+
+
+@pytest.mark.parametrize("kind", ["linear", "transposed", "embedding", "prompt"])
+@pytest.mark.parametrize("before", ["nothing", "decoded", "called", "overwritten"])
+def test_first_call_under_capture(kind, before):
+    """Nothing is read back while a stream captures, and what a capture makes is not kept for calls outside it."""
+    import comp_inference_b200 as ci
+    from comp_inference_b200 import _lib
+    wa, ca, wb, cb = _two_weights()
+    x, ids = _inputs()
+    if kind == "prompt":
+        x = x.repeat(10, 1)
+        m = ci.RansLinear(K, N, TH, 32).load_compressed(ca)
+        call, kind = lambda: m(x), "linear"
+    else:
+        call = lambda: _call(kind, ca, x, ids)
+    w = wa
+    if before in ("decoded", "overwritten"):
+        args = [ca[n] for n in ARRAYS[:4]] + [(K, N), ca["rans_exp_tile_offsets"], ca["rans_exp_tile_max_lens"], TH, 32, ca["rans_man_raw"]]
+        assert torch.equal(ci.rans_decompress_bf16(*args), w)
+    if before in ("called", "overwritten"):
+        assert _right(kind, call(), w, x, ids)
+    if before == "overwritten":
+        w = wb
+        for n in ("rans_exp_stream", "rans_exp_states", "rans_man_raw"):
+            ca[n].copy_(cb[n])
+    graph, y = _captured(call)
+    assert _right(kind, y, w, x, ids)
+    assert _right(kind, call(), w, x, ids)
+    del graph, y
+    assert _right(kind, call(), w, x, ids)
+    assert _lib.kernel_status(x.device) == 0
