@@ -212,6 +212,7 @@ def prepared_lut(tables, slot_map):
         return None
     lut = torch.empty(4096, dtype=torch.int32, device=tables.device)
     check(load().ci_prepare_lut(ptr(tables), ptr(slot_map), ptr(lut), stream()))
+    torch.cuda.current_stream().synchronize()          # once per table: the next call may come on another stream
     _make_room(_lut_cache)
     _lut_cache[key] = (weakref.ref(tables), weakref.ref(slot_map), (tables._version, slot_map._version), lut)
     return lut

@@ -254,8 +254,12 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
         } else if (capturing()) {
             h.lasting = false;                                  // the kernels that build the table themselves and need no depth
         } else {
-            h.lut = lib_attr("prepared_lut")(tables, slot_map).cast<Tensor>();
+            (void)tables._version(), (void)slot_map._version();  // inference tensors are refused: nobody counts their versions
+            h.lut = at::empty({4096}, tables.options().dtype(at::kInt));
+            check(ci_prepare_lut((const uint32_t *)tables.data_ptr(), (const uint8_t *)slot_map.data_ptr(),
+                                 (uint32_t *)h.lut.data_ptr(), stream()));
             max_len = lib_attr("max_tile_len")(lens).cast<uint32_t>();
+            c10::cuda::stream_synchronize(c10::cuda::getCurrentCUDAStream().stream());   // the next call may come on another one
             g_tables.keep(lens, Tables{Ref(lens), Ref(tables), Ref(slot_map), h.lut, max_len});
         }
     }

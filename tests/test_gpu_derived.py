@@ -143,3 +143,35 @@ def test_first_call_under_capture(kind, before):
     del graph, y
     assert _right(kind, call(), w, x, ids)
     assert _lib.kernel_status(x.device) == 0
+
+
+@pytest.mark.parametrize("layout", ["tiled", "dense"])
+def test_table_prepared_on_another_stream(layout):
+    """A decode table made by a call on one stream is whole for a call on another one, which has waited for the arrays only."""
+    import comp_inference_b200 as ci
+    w = make_weight(256, 64, 5)
+    c = ci.compress_weight_cuda(w.cuda(), 64, 32, uncoalesced_interleaving=layout == "dense")
+    fn = ci.fused_rans_embedding_triton if layout == "tiled" else ci.fused_rans_embedding_triton_uncoalesced
+    places = ("rans_exp_tile_offsets", "rans_exp_tile_max_lens") if layout == "tiled" else ("rans_exp_stream_offsets", "output_sizes")
+    args = [c[n] for n in ARRAYS[:4]] + [(256, 64), *(c[n] for n in places), 64, 32, c["rans_man_raw"]]
+    tables, slot_map = args[2], args[3]
+    ids = torch.arange(256, device="cuda")
+    fn(ids, *args[:2], tables.clone(), slot_map.clone(), *args[4:])      # kernels are loaded: loading one waits for the device
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        if layout == "tiled":                           # everything known, then the tables change: exponents one higher
+            assert torch.equal(fn(ids, *args), w.cuda())
+            tables.copy_(tables.view(torch.int32).roll(1).view(torch.uint32))
+            slot_map.add_(1)
+            w = w * 2
+        stale = torch.full((4096,), -1, dtype=torch.int32, device="cuda")    # what the table's memory may hold before it is made
+        del stale
+        ready = a.record_event()
+        torch.cuda._sleep(100_000_000)
+        fn(ids, *args)
+    b.wait_event(ready)
+    with torch.cuda.stream(b):
+        y = fn(ids, *args)
+    torch.cuda.synchronize()
+    assert torch.equal(y, w.cuda())
