@@ -96,9 +96,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         auto range = [&](uint32_t t, uint32_t &off, uint32_t &ml) {
             off = __ldg(a.tile_offsets + t);
             if constexpr (ENTRY) {
-                const uint32_t span = __ldg(p.entry_spans + (size_t)t * subs + sub);   // first row | rows << 16
-                off += (span & 0xFFFFu) * 64;
-                ml = span >> 16;
+                ml = enter_span(__ldg(p.entry_spans + (size_t)t * subs + sub), __ldg(a.tile_max_lens + t), off);
             } else {
                 ml = __ldg(a.tile_max_lens + t);
             }

@@ -98,9 +98,7 @@ __global__ void __launch_bounds__(kEmb4Warps * 32, 1) k_embedding4(const __grid_
             b.off = __ldg(a.tile_offsets + tile);
             if constexpr (ENTRY) {
                 const uint32_t rel = b.row - tk * g.th, inner = rel >= g.half ? rel - g.half : rel;
-                const uint32_t span = __ldg(a.entry_spans + tile * p.subs + inner / a.entry_step);   // first row | rows << 16
-                b.off += (span & 0xFFFFu) * 64;
-                b.ml = span >> 16;
+                b.ml = enter_span(__ldg(a.entry_spans + tile * p.subs + inner / a.entry_step), __ldg(a.tile_max_lens + tile), b.off);
             } else {
                 b.ml = __ldg(a.tile_max_lens + tile);
             }

@@ -88,9 +88,7 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
         const size_t tile = (size_t)tk * g.tiles_n + ct;
         off = __ldg(a.tile_offsets + tile);
         if constexpr (ENTRY) {
-            const uint32_t span = __ldg(a.entry_spans + tile * subs + grp % subs);   // first row | rows << 16
-            off += (span & 0xFFFFu) * 64;
-            ml = span >> 16;
+            ml = enter_span(__ldg(a.entry_spans + tile * subs + grp % subs), __ldg(a.tile_max_lens + tile), off);
         } else {
             ml = __ldg(a.tile_max_lens + tile);
         }

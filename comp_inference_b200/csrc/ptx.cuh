@@ -245,6 +245,15 @@ __device__ __forceinline__ void start_lut(uint32_t lut_s, uint32_t bar, const ui
 }
 __device__ __forceinline__ bool wait_lut(uint32_t bar, const uint32_t *lut) { return lut == nullptr || mbar_wait(bar, 0); }
 
+// A span of an entry point (first row | rows << 16): moves `off` from the tile's byte block to the span and returns its rows, or
+// more than any window holds where it reaches beyond the tile's `depth` rows -- entry points made of other arrays than these --
+// so that the copy is refused like that of any wrong depth.
+__device__ __forceinline__ uint32_t enter_span(uint32_t span, uint32_t depth, uint32_t &off) {
+    const uint32_t first = span & 0xFFFFu, rows = span >> 16;
+    off += first * 64;
+    return first + rows <= depth ? rows : 0xFFFFFFFFu;
+}
+
 // Sign+mantissa bytes on their way through a warp that decodes four segments (two tiles, both halves) at once: chunks of
 // kChunkRows rows of 32 bytes per segment, double buffered.  The segments of a chunk start 8 banks apart, so a row of
 // the warp's 128 columns is one conflict-free wavefront.

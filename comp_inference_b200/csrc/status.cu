@@ -26,7 +26,7 @@ int ci_status(uint32_t *d_status_word, uint32_t *code, int clear, ci_stream_t st
     if (v == 0) return CI_OK;
     if (clear) CI_CUDA(cudaMemsetAsync(d_status_word, 0, sizeof v, s));
     const char *what = v == 1   ? "a bounded wait for a copy into shared memory ran out"
-                       : v == 2 ? "tile_max_lens holds an entry above the descriptor's max_tile_len"
+                       : v == 2 ? "tile_max_lens contradicts the descriptor's max_tile_len or its entry points"
                        : v == 9 ? "a bounded wait for a peer rank ran out"
                                 : "a kernel reported a pipeline error";
     set_error("device status %u: %s; the outputs of the affected calls are not valid", v, what);

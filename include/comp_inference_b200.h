@@ -94,8 +94,8 @@ const char *ci_last_error(void);
 /* ---- errors found on the device, malformed metadata ---------------------- */
 
 /* The staged kernels never trap and never wait without a bound.  When a wait runs out, or a tile's
- * entry in tile_max_lens contradicts the descriptor's max_tile_len, they write a code into a status
- * word and finish with invalid output: 1 = a copy into shared memory did not arrive, 2 = metadata
+ * entry in tile_max_lens contradicts the descriptor's max_tile_len or its entry points, they write a code into a
+ * status word and finish with invalid output: 1 = a copy into shared memory did not arrive, 2 = metadata
  * mismatch, 9 = a peer rank did not answer (the tensor-parallel exchanges), other values = a pipeline
  * stage of the prefill GEMM gave up.  For ci_linear / ci_linear_transposed / ci_linear_dense the word
  * lives inside the workspace, at the address ci_workspace_status_word() returns (host arithmetic, no

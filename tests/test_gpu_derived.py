@@ -175,3 +175,19 @@ def test_table_prepared_on_another_stream(layout):
         y = fn(ids, *args)
     torch.cuda.synchronize()
     assert torch.equal(y, w.cuda())
+
+
+@pytest.mark.parametrize("kind", ["linear", "transposed"])
+def test_entry_points_that_contradict_the_depths_are_reported(kind):
+    """A write that no version counter sees leaves entry points behind which reach beyond a tile's byte block (here: by one
+    row, inside the stream): nothing is read there, and the status word says so."""
+    import comp_inference_b200 as ci
+    wa, ca, _, _ = _two_weights()
+    x, ids = _inputs()
+    assert _right(kind, _call(kind, ca, x, ids), wa, x, ids)
+    ci.check_status()
+    ca["rans_exp_tile_max_lens"].view(torch.int32).data.sub_(1)
+    _call(kind, ca, x, ids)
+    with pytest.raises(RuntimeError, match="status 2"):
+        ci.check_status()
+    ci.check_status()
