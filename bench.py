@@ -229,10 +229,7 @@ def block_step(mods, x):
 
 
 def block_routes(mods, M):
-    from comp_inference_b200 import _lib
-    lib = _lib.load()
-    return sorted({ROUTES.get(lib.ci_linear_route(m._weight(m.in_features, m.out_features), M), "?")
-                   for m in mods.values()})
+    return sorted({ROUTES.get(m._native().route(M), "?") for m in mods.values()})
 
 
 def parity_table(mods, dense, device):
@@ -700,7 +697,7 @@ def shards_once(args):
         torch.cuda.synchronize()
         ref = x.float() @ dense[name].float()
         row = {"shape_in_out": [m.in_features, m.out_features],
-               "kernel": ROUTES[_lib.load().ci_linear_route(m._weight(m.in_features, m.out_features), 1)],
+               "kernel": ROUTES[m._native().route(1)],
                "rel_err": float((y.float() - ref).abs().max() / ref.abs().max())}
         if args.shards_time:
             def many():

@@ -25,7 +25,9 @@ class TiledWeight(C.Structure):
     _fields_ = [("stream", C.c_void_p), ("states", C.c_void_p), ("tables", C.c_void_p), ("slot_map", C.c_void_p),
                 ("tile_offsets", C.c_void_p), ("tile_max_lens", C.c_void_p), ("mantissa", C.c_void_p),
                 ("lut", C.c_void_p), ("stream_len", C.c_uint64), ("K", C.c_uint32), ("N", C.c_uint32),
-                ("tile_h", C.c_uint32), ("tile_w", C.c_uint32), ("max_tile_len", C.c_uint32), ("reserved", C.c_uint32)]
+                ("tile_h", C.c_uint32), ("tile_w", C.c_uint32), ("max_tile_len", C.c_uint32), ("entry_step", C.c_uint32),
+                ("entry_states", C.c_void_p), ("entry_rows", C.c_void_p), ("entry_spans", C.c_void_p),
+                ("entry_cap", C.c_uint32), ("reserved", C.c_uint32)]
 
 
 class DenseWeight(C.Structure):
@@ -341,7 +343,7 @@ def tiled_weight(stream_t, states, tables, slot_map, tile_offsets, tile_max_lens
         lut = prepared_lut(tb, sm) if (tb is tables and sm is slot_map) else None
     deepest = max_tile_len(tile_max_lens) if (want_max and ml is tile_max_lens) else 0
     w = TiledWeight(ptr(st), ptr(sts), ptr(tb), ptr(sm), ptr(off), ptr(ml), ptr(man), ptr(lut), st.numel(),
-                    K, N, th, tw, deepest, 0)
+                    K, N, th, tw, deepest)
     return w, (st, sts, tb, sm, off, ml, man, lut, keep)
 
 

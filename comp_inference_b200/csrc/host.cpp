@@ -459,6 +459,11 @@ PYBIND11_MODULE(_ci_host, m) {
              py::arg("tile_max_lens"), py::arg("mantissas"), py::arg("K"), py::arg("N"), py::arg("tile_h"), py::arg("tile_w"), py::arg("entries") = false)
         .def("matches", &Weight::matches)
         .def_readonly("lasting", &Weight::lasting)
+        .def("route", [](const Weight &h, int64_t rows) {           // the kernel that linear runs (ci_linear_route), entry points included
+            const int route = ci_linear_route(&h.w, (uint32_t)rows);
+            if (route < 0) check(route);
+            return route;
+        })
         .def("linear", &linear_call, py::arg("x"), py::arg("bias") = py::none(), py::arg("out") = py::none(), py::arg("split_k") = 0,
              py::arg("transposed") = false, py::arg("prefill_rows") = 0)
         .def("embedding", &embedding_call, py::arg("x"), py::arg("out") = py::none())

@@ -191,3 +191,11 @@ def test_entry_points_that_contradict_the_depths_are_reported(kind):
     with pytest.raises(RuntimeError, match="status 2"):
         ci.check_status()
     ci.check_status()
+
+
+@pytest.mark.parametrize("k,n,th,rows,route", [(1024, 256, 256, 1, 2), (1024, 256, 256, 16, 2), (1024, 256, 128, 1, 1), (4096, 2048, 128, 1, 2),
+                                               (1024, 256, 256, 17, 3)])
+def test_route_of_a_module_counts_its_entry_points(k, n, th, rows, route):
+    import comp_inference_b200 as ci
+    m = ci.RansLinear(k, n, th, 32).load_compressed(ci.compress_weight_cuda(make_weight(k, n, 5).cuda(), th, 32)).prepare()
+    assert m._native().route(rows) == route             # 1: two streams a lane, 2: four, 3: decode-GEMM (ci_linear_route)
