@@ -258,7 +258,6 @@ def secondary_metrics(mods, dense, device, peak_hbm, peak_tf, src):
     """The other parts of the headline metric on the same block, N = 1 only, short runs outside the timed
     region."""
     import comp_inference_b200 as ci
-    from comp_inference_b200 import ops
     out = {}
 
     # ---- stand-alone rANS decode to bf16
@@ -329,9 +328,7 @@ def secondary_metrics(mods, dense, device, peak_hbm, peak_tf, src):
 
     def block_split(x, split_k):
         def lin(m, xx):
-            x2 = ops._check_x(xx, m.in_features)
-            return ops._linear_call(m._weight(m.in_features, m.out_features), x2, x2.shape[0], m.out_features, None,
-                                    None, split_k, False)
+            return m._native().linear(xx, None, None, split_k)
         qkv = lin(mods["qkv_proj"], x)
         h = lin(mods["o_proj"], qkv[..., :HIDDEN])
         gu = lin(mods["gate_up_proj"], h)

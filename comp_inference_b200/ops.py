@@ -84,26 +84,6 @@ def rans_decompress_bf16(compressed_streams, initial_states, tables, slot_map, w
                               int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n)).decode(True)
 
 
-def _linear_call(w, x2, M, n_out, bias, out, split_k, transposed):
-    dev = x2.device
-    lib = _lib.load()
-    y = out.view(M, n_out) if out is not None else torch.empty((M, n_out), device=dev, dtype=torch.bfloat16)
-    if y.dtype != torch.bfloat16 or y.stride(1) != 1:
-        raise RuntimeError("out must be a bfloat16 tensor with unit inner stride")
-    nbytes = lib.ci_linear_workspace_bytes(M, n_out, 0 if transposed else w.K, w.tile_h)
-    if M > 16 and not transposed and split_k > 1:               # an explicit split-K of the prefill GEMM: room for its partials
-        nbytes = max(nbytes, (1 << 14) + min(int(split_k), 8) * M * n_out * 4)
-    ws = _lib.workspace(dev, nbytes)
-    b = _bias(bias, n_out)
-    if transposed:
-        _lib.check(lib.ci_linear_transposed(w, _lib.ptr(x2), x2.stride(0), M, _lib.ptr(b), _lib.ptr(y), y.stride(0),
-                                            _lib.ptr(ws), ws.numel(), _lib.stream()))
-    else:
-        _lib.check(lib.ci_linear(w, _lib.ptr(x2), x2.stride(0), M, _lib.ptr(b), _lib.ptr(y), y.stride(0),
-                                 _lib.ptr(ws), ws.numel(), int(split_k), _lib.stream()))
-    return y
-
-
 def fused_rans_linear_triton(x, compressed_data, initial_states, tables, slot_map, weight_shape, tile_offsets,
                              tile_max_lens, tile_k, tile_n, mantissas, accum_block_size=32, bias=None, out=None,
                              SPLIT_K=8, workspace=None):
