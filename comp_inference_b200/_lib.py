@@ -51,6 +51,7 @@ SIGNATURES = {
                                              C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32]),
     "ci_build_tables": (C.c_int, [_V, _V, _V, _V]),
     "ci_prepare_lut": (C.c_int, [_V, _V, _V, _S]),
+    "ci_weight_written": (C.c_int, [_S]),
     "ci_split_bf16": (C.c_int, [_V, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, _V, _V, _V, _V, _S]),
     "ci_histogram_u8": (C.c_int, [_V, C.c_uint64, _V, _S]),
     "ci_normalize_freqs": (C.c_int, [_V, _V, _V]),

@@ -12,6 +12,7 @@
 #include <torch/extension.h>
 
 #include <mutex>
+#include <optional>
 #include <unordered_map>
 
 #include "../../include/comp_inference_b200.h"
@@ -170,14 +171,26 @@ struct Ref {
     explicit Ref(const Tensor &t) : impl(t.getIntrusivePtr()), data(t.data_ptr()), version(version_of(t)) {}
     bool is(const Tensor &t) const {
         return !impl.expired() && impl._unsafe_get_target() == t.unsafeGetTensorImpl() && data == t.data_ptr() &&
-               version == version_of(t);
+               !t.is_inference() && version == version_of(t);
     }
 };
-// The decode table of tables and slot_map, the depth of the deepest tile.
+// The decode table of tables and slot_map, the depth of the deepest tile, and the other arrays that came with them last.
 struct Tables {
     Ref lens, tables, slot_map;
     Tensor lut;
     uint32_t max_len;
+    std::optional<Ref> last[4] = {};
+    // Whether all of h's arrays have come before as they are now.
+    bool seen(const Weight &h) {
+        const Tensor *arrays[4] = {&h.stream, &h.states, &h.offsets, &h.mantissa};
+        bool all = true;
+        for (int i = 0; i < 4; ++i) {
+            if (!arrays[i]->defined() || (last[i] && last[i]->is(*arrays[i]))) continue;
+            last[i].emplace(*arrays[i]);
+            all = false;
+        }
+        return all;
+    }
     bool is(const Weight &h) const { return lens.is(h.lens) && tables.is(h.tables) && slot_map.is(h.slot_map); }
     bool expired() const { return lens.impl.expired() || tables.impl.expired() || slot_map.impl.expired(); }
 };
@@ -246,11 +259,14 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
     uint32_t max_len = 0;
     // a contiguous copy made above is a new object on every call: nothing to remember
     if (h.tables.is_same(tables) && h.slot_map.is_same(slot_map) && h.lens.is_same(lens)) {
-        const bool known = g_tables.find(lens, h, [&](const Tables &t) {
+        bool seen = false;
+        const bool known = g_tables.find(lens, h, [&](Tables &t) {
             h.lut = t.lut;
             max_len = t.max_len;
+            seen = t.seen(h);
         });
         if (known) {
+            if (!seen) check(ci_weight_written(stream()));      // they may be the previous kernel's product
         } else if (capturing()) {
             h.lasting = false;                                  // the kernels that build the table themselves and need no depth
         } else {
@@ -260,7 +276,9 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
                                  (uint32_t *)h.lut.data_ptr(), stream()));
             max_len = lib_attr("max_tile_len")(lens).cast<uint32_t>();
             c10::cuda::stream_synchronize(c10::cuda::getCurrentCUDAStream().stream());   // the next call may come on another one
-            g_tables.keep(lens, Tables{Ref(lens), Ref(tables), Ref(slot_map), h.lut, max_len});
+            Tables t{Ref(lens), Ref(tables), Ref(slot_map), h.lut, max_len};
+            t.seen(h);
+            g_tables.keep(lens, std::move(t));
         }
     }
     fill(h, K, N, th, tw, max_len);

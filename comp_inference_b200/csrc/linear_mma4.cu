@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     }
     if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
-    // Everything above touches only the weight, which no kernel writes.  When this launch was allowed to
+    // Everything above touches only the weight, which the previous kernel has not written (ci_weight_written).  When this launch was allowed to
     // start before its predecessor in the stream has finished (programmatic dependent launch), wait here
     // for it -- activations, workspace and output may be its products -- and let the next launch start
     // its own preamble while this grid works.  Both are no-ops in an ordinary launch.

@@ -74,6 +74,8 @@ __global__ void k_prepare_lut(const uint32_t *__restrict__ tables, const uint8_t
     }
 }
 
+__global__ void k_weight_written() {}
+
 // One thread per element of the row-major [K,N] matrix.
 __global__ void k_split_bf16(const uint16_t *__restrict__ w, uint32_t K, uint32_t N, uint32_t th, uint32_t tw,
                              uint32_t tiles_n, uint8_t *__restrict__ exp_plane, uint8_t *__restrict__ man_tiled,
@@ -197,6 +199,12 @@ int ci_prepare_lut(const uint32_t *d_tables, const uint8_t *d_slot_map, uint32_t
     CI_REQUIRE(d_tables && d_slot_map && d_lut, "null pointer");
     k_prepare_lut<<<kProbScale / 256, 256, 0, (cudaStream_t)stream>>>(d_tables, d_slot_map, d_lut);
     CI_LAUNCH_CHECK(k_prepare_lut);
+    return CI_OK;
+}
+
+int ci_weight_written(ci_stream_t stream) {
+    k_weight_written<<<1, 1, 0, (cudaStream_t)stream>>>();
+    CI_LAUNCH_CHECK(k_weight_written);
     return CI_OK;
 }
 

@@ -136,6 +136,13 @@ int ci_build_tables(const uint16_t *freqs, const uint16_t *cdf, uint32_t *tables
  * lookups per symbol instead: comp_inference/rans_triton.py:95-105.) */
 int ci_prepare_lut(const uint32_t *d_tables, const uint8_t *d_slot_map, uint32_t *d_lut, ci_stream_t stream);
 
+/* Device.  An empty kernel behind the one that has written a weight's arrays.  The decoders, linears and gathers are launched
+ * with programmatic dependent launch: while the previous kernel of the stream drains they already read the weight (never
+ * activations, ids or outputs), and a kernel's stores are sure to be seen only by what waits for its completion, as every
+ * ordinary launch, copy and host wait does.  Call it where neither of those lies between a kernel that writes a weight
+ * and the first call that reads it. */
+int ci_weight_written(ci_stream_t stream);
+
 /* ---- bf16 split / merge, histogram ------------------------------------- */
 
 /* Device.  bf16 bits [K,N] -> exponent plane u8 [K,N], sign+mantissa bytes

@@ -199,3 +199,27 @@ def test_route_of_a_module_counts_its_entry_points(k, n, th, rows, route):
     import comp_inference_b200 as ci
     m = ci.RansLinear(k, n, th, 32).load_compressed(ci.compress_weight_cuda(make_weight(k, n, 5).cuda(), th, 32)).prepare()
     assert m._native().route(rows) == route             # 1: two streams a lane, 2: four, 3: decode-GEMM (ci_linear_route)
+
+
+@pytest.mark.parametrize("kind", ["linear", "transposed", "embedding", "module"])
+@pytest.mark.parametrize("th", [1024, 128])
+def test_a_weight_written_by_the_kernel_before(kind, th):
+    """The arrays may be products of the kernel that comes right before a call, which starts to read the weight early."""
+    import comp_inference_b200 as ci
+    a = make_weight(K, N, 5)
+    ws = [a.cuda(), a.view(K, N // 2, 2).flip(-1).reshape(K, N).cuda()]
+    cs = [ci.compress_weight_cuda(w, th, 32) for w in ws]
+    x, ids = _inputs()
+    c = {n: cs[0][n].clone() for n in ARRAYS}
+    m = ci.RansLinear(K, N, th, 32).load_compressed(c)
+    args = [c[n] for n in ARRAYS[:4]] + [(K, N), c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"], th, 32, c["rans_man_raw"]]
+    call = {"linear": lambda: ci.fused_rans_linear_triton(x, *args), "module": lambda: m(x),
+            "transposed": lambda: ci.fused_rans_linear_transposed_triton(x[:, :N], *args),
+            "embedding": lambda: ci.fused_rans_embedding_triton(ids, *args)}[kind]
+    out = []
+    for i in range(20):
+        for n, dt in (("rans_exp_stream", torch.uint8), ("rans_man_raw", torch.uint8), ("rans_exp_states", torch.int32)):
+            torch.add(cs[i % 2][n].view(dt), 0, out=c[n].view(dt))      # a kernel, where copy_ would be a copy
+        out.append(call())
+    for i, y in enumerate(out):
+        assert _right("linear" if kind == "module" else kind, y, ws[i % 2], x, ids)
