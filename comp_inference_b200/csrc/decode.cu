@@ -57,7 +57,7 @@ __device__ __forceinline__ bool stage_bytes(const DecArgs &a, const LaneTask &L,
 template <bool BF16>
 __device__ __forceinline__ void emit(const DecArgs &a, const LaneTask &L, void *out, uint32_t row, uint32_t lr,
                                      uint32_t entry) {
-    size_t o = (size_t)row * a.g.N + L.n;
+    size_t o = (size_t)row * a.ld + L.n;
     uint32_t sym = lut_sym(entry);
     if (BF16) {
         uint32_t m = __ldg(a.mantissa + (size_t)L.t * a.g.th * a.g.tw + (size_t)lr * a.g.tw + L.lc);
@@ -219,6 +219,7 @@ static DecArgs make_args(const ci_tiled_weight *w) {
     a.tile_max_lens = w->tile_max_lens; a.lut = w->lut; a.slot_map = w->slot_map; a.mantissa = w->mantissa;
     a.g = make_geom(w->K, w->N, w->tile_h, w->tile_w);
     a.stream_aligned = (reinterpret_cast<uintptr_t>(w->stream) & 15u) == 0;
+    a.ld = w->N;
     a.entry_step = w->entry_step;
     if (a.entry_step != 0) {
         a.entry_cap = w->entry_cap;
@@ -235,14 +236,11 @@ static int decode_tiled(const ci_tiled_weight *w, void *d_out, uint32_t ld, cuda
     if (rc) return rc;
     CI_REQUIRE(d_out != nullptr, "null output");
     DecArgs a = make_args(w);
-    rc = launch_decode2(a, w->max_tile_len, BF16, d_out, ld ? ld : w->N, s);   // 32-wide tiles
+    if (ld) a.ld = ld;
+    rc = launch_decode2(a, w->max_tile_len, BF16, d_out, s);         // 32-wide tiles
     if (rc <= 0) return rc;
-    rc = launch_decode4(a, w->max_tile_len, BF16, d_out, ld ? ld : w->N, s);
+    rc = launch_decode4(a, w->max_tile_len, BF16, d_out, s);
     if (rc <= 0) return rc;
-    if (ld != 0 && ld != w->N) {
-        set_error("this weight does not qualify for the staged decoder, the only one that writes padded rows");
-        return CI_E_INVALID;
-    }
     rc = launch_decode_staged(a, w->max_tile_len, BF16, d_out, s);   // other staged shapes
     if (rc <= 0) return rc;
     uint32_t n_tasks = a.g.tiles_k * a.g.groups;

@@ -25,7 +25,6 @@ struct Dec2Args {
     uint32_t cap_rows;     // rows of the byte window (>= every tile_max_len)
     uint32_t win_bytes;    // window + 64 initial states
     uint32_t total;        // tiles
-    uint32_t ld;           // elements from one output row to the next
     uint32_t vec;          // output rows can be written as aligned pairs
 };
 
@@ -168,8 +167,8 @@ __global__ void __launch_bounds__(kDec2Warps * 32, 1) k_decode2(const __grid_con
         };
         start_streams();
 
-        uint8_t *o = reinterpret_cast<uint8_t *>(out) + ((size_t)row * p.ld + col) * (BF16 ? 2 : 1);
-        const size_t pitch = (size_t)p.ld * (BF16 ? 2 : 1);
+        uint8_t *o = reinterpret_cast<uint8_t *>(out) + ((size_t)row * a.ld + col) * (BF16 ? 2 : 1);
+        const size_t pitch = (size_t)a.ld * (BF16 ? 2 : 1);
         const uint8_t *man = a.mantissa + (size_t)t * g.th * 32 + lane * 16;
 #pragma unroll 1
         for (uint32_t c = 0; c < n_chunks; ++c) {
@@ -249,7 +248,7 @@ static int launch_dec2(const Dec2Args &p, uint32_t blocks, uint32_t warps, size_
     return CI_OK;
 }
 
-int launch_decode2(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, cudaStream_t s) {
+int launch_decode2(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, cudaStream_t s) {
     const Geom &g = a.g;
     if (g.tw != 32 || g.th % 16 != 0 || max_tile_len == 0) return 1;
     if (!a.stream_aligned || (reinterpret_cast<uintptr_t>(a.states) & 15u)) return 1;
@@ -280,8 +279,7 @@ int launch_decode2(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     const double four = decode4_cost(a, max_tile_len, bf16);   // 0: not a weight for it
     if (four > 0.0 && four <= 1.05 * best) return 1;
     const uint32_t blocks = p.total < P ? p.total : P;
-    p.ld = ld;
-    p.vec = ld % 2 == 0 && g.N % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & (bf16 ? 3u : 1u)) == 0;
+    p.vec = a.ld % 2 == 0 && g.N % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & (bf16 ? 3u : 1u)) == 0;
     const bool edge = g.K % g.th != 0 || !p.vec;
     const size_t smem = fixed + (size_t)warps * warp_bytes;
     if (bf16) return edge ? launch_dec2<true, true>(p, blocks, warps, smem, max_smem, out, s)

@@ -31,7 +31,6 @@ struct Dec4Args {
     uint32_t stages;       // windows per warp
     uint32_t pairs_n;      // tile pairs per tile row = ceil(tiles_n / 2)
     uint32_t total;        // units
-    uint32_t ld;           // elements from one output row to the next
     uint32_t vec;          // output rows can be written as aligned quads
     uint32_t step, subs;   // INDEX, ENTRY: rows between entry points, entry points per half tile
     uint32_t *entry_states;
@@ -239,8 +238,8 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         };
         start_streams();
 
-        uint8_t *o8 = reinterpret_cast<uint8_t *>(out) + ((size_t)row * p.ld + col0) * (BF16 ? 2 : 1);
-        const size_t o_pitch = (size_t)p.ld * (BF16 ? 2 : 1);
+        uint8_t *o8 = reinterpret_cast<uint8_t *>(out) + ((size_t)row * a.ld + col0) * (BF16 ? 2 : 1);
+        const size_t o_pitch = (size_t)a.ld * (BF16 ? 2 : 1);
 #pragma unroll 1
         for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
             const uint32_t buf = chunk & 1;
@@ -370,12 +369,12 @@ static int launch_dec4(const Dec4Args &p, uint32_t blocks, uint32_t warps, size_
     return CI_OK;
 }
 
-static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, uint32_t step,
+static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t step,
                    uint32_t *entry_states, uint16_t *entry_rows, cudaStream_t s);
 
 int build_entry_points(const DecArgs &a, uint32_t max_tile_len, uint32_t step, uint32_t *d_states, uint16_t *d_rows,
                        uint32_t *d_spans, uint32_t *d_cap, cudaStream_t s) {
-    const int rc = decode4(a, max_tile_len, false, nullptr, a.g.N, step, d_states, d_rows, s);
+    const int rc = decode4(a, max_tile_len, false, nullptr, step, d_states, d_rows, s);
     if (rc) return rc;
     CI_CUDA(cudaMemsetAsync(d_cap, 0, sizeof(uint32_t), s));
     const uint32_t tiles = a.g.tiles_k * a.g.tiles_n;
@@ -385,8 +384,8 @@ int build_entry_points(const DecArgs &a, uint32_t max_tile_len, uint32_t step, u
 }
 
 // Returns CI_OK when it launched, 1 when the tensor does not qualify, < 0 on error.
-int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, cudaStream_t s) {
-    return decode4(a, max_tile_len, bf16, out, ld, 0, nullptr, nullptr, s);
+int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, cudaStream_t s) {
+    return decode4(a, max_tile_len, bf16, out, 0, nullptr, nullptr, s);
 }
 
 constexpr uint32_t kDec4Fixed = 2 * kLutBytes + kDec4BarBytes;  // up to one table size is lost to the table's alignment
@@ -432,7 +431,7 @@ double decode4_cost(const DecArgs &a, uint32_t max_tile_len, bool bf16) {
     return entry ? cost * a.entry_step / g.half : cost;         // per 64 symbols of the whole stream
 }
 
-static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t ld, uint32_t step,
+static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t step,
                    uint32_t *entry_states, uint16_t *entry_rows, cudaStream_t s) {
     const Geom &g = a.g;
     if (g.tw != 32 || g.th % 16 != 0 || max_tile_len == 0) return 1;
@@ -460,8 +459,7 @@ static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     uint32_t blocks = (p.total + warps - 1) / warps;
     if (blocks > P) blocks = P;
     const size_t smem = kDec4Fixed + (size_t)warps * (p.stages * p.stage_bytes + man_bytes);
-    p.ld = ld;
-    p.vec = ld % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & (bf16 ? 7u : 3u)) == 0;
+    p.vec = a.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & (bf16 ? 7u : 3u)) == 0;
     const bool edge = g.K % g.th != 0 || g.N % 4 != 0 || !p.vec;
     if (step) return launch_dec4<false, false, true, false>(p, blocks, warps, smem, max_smem, nullptr, s);
     if (entry) return edge ? launch_dec4<true, true, false, true>(p, blocks, warps, smem, max_smem, out, s)

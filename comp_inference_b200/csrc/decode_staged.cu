@@ -3,7 +3,11 @@
 // decode + uninterleave + reconstruct chain of rans_decompress_module_weight_bf16
 // (comp_inference/comp_inference.py:633-711).
 //
-// Same unit and staging as the fused linear: one warp per (tile row, 32-column group), the unit's
+// Takes tiles 8 and 16 wide, and 32-wide ones whose initial states lie on no 16-byte boundary (a slice of a larger buffer),
+// which decode2.cu and decode4.cu copy in bulk and refuse: 4096 x 4096 at tile height 128 25 us, where the kernel for the
+// rest takes 66 (decode4: 16).
+//
+// Unit and staging as in linear_mma.cu: one warp per (tile row, 32-column group), the unit's
 // compressed byte block (and, for bf16 output, its sign+mantissa block) arrive by bulk async copy
 // into a per-warp double buffer while the previous unit is decoded.  Units are dealt to the warps of
 // the persistent grid round-robin with the column group running fastest, so warps that run at the
@@ -93,7 +97,7 @@ __global__ void __launch_bounds__(512, 1) k_decode_staged(const __grid_constant_
         if (ok) {
             uint8_t *o8 = reinterpret_cast<uint8_t *>(out);
             uint16_t *o16 = reinterpret_cast<uint16_t *>(out);
-            size_t oA = (size_t)row0 * g.N + n, oB = oA + (size_t)g.half * g.N;
+            size_t oA = (size_t)row0 * a.ld + n, oB = oA + (size_t)g.half * a.ld;
             uint32_t i = 0;
             for (; i + 8 <= nB; i += 8) {                        // eight rows of both halves, no bounds tests
                 const uint32_t mA = man_s + i * TW, mB = mA + g.half * TW;
@@ -115,8 +119,8 @@ __global__ void __launch_bounds__(512, 1) k_decode_staged(const __grid_constant_
                             o8[oB] = (uint8_t)lut_sym(f);
                         }
                     }
-                    oA += g.N;
-                    oB += g.N;
+                    oA += a.ld;
+                    oB += a.ld;
                 }
             }
             for (; i < nA; ++i) {                                // ragged end of the last tile row
@@ -138,8 +142,8 @@ __global__ void __launch_bounds__(512, 1) k_decode_staged(const __grid_constant_
                         else o8[oB] = (uint8_t)lut_sym(f);
                     }
                 }
-                oA += g.N;
-                oB += g.N;
+                oA += a.ld;
+                oB += a.ld;
             }
         }
         __syncwarp();

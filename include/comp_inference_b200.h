@@ -231,7 +231,7 @@ int ci_decode_plane(const ci_tiled_weight *w, uint8_t *d_out, ci_stream_t stream
  * tiled decode, uninterleave_mantissas, reconstruct_from_exp_and_mantissa). */
 int ci_decode_bf16(const ci_tiled_weight *w, uint16_t *d_out, ci_stream_t stream);
 
-/* The same with rows `ld` elements apart (32-wide tiles and a known max_tile_len only); what lies between is not written. */
+/* The same with rows `ld` elements apart; what lies between is not written. */
 int ci_decode_bf16_ld(const ci_tiled_weight *w, uint16_t *d_out, int64_t ld, ci_stream_t stream);
 
 /* Dense-layout counterparts. */

@@ -176,3 +176,19 @@ def test_column_edges(K, N, th, M):
     x = torch.randn(M, K, generator=torch.Generator().manual_seed(K)).to(torch.bfloat16).cuda()
     assert _close(m(x), x.float() @ W.float())
     test_decoder_edges(K, N, th)
+
+
+# prompts whose buffers the staged decoders do not take (slices of a larger buffer): odd sizes are decoded into padded rows all the same
+@pytest.mark.parametrize("K,N,th", [(1000, 776, 128), (1000, 777, 128), (515, 131, 1024)])
+@pytest.mark.parametrize("name", ["rans_exp_stream", "rans_exp_states", "rans_man_raw"])
+def test_prompt_from_unaligned_buffers(K, N, th, name):
+    import comp_inference_b200 as ci
+    W = _weight(K, N)
+    c = ci.compress_weight_cuda(W, th, 32)
+    t = c[name]
+    c[name] = torch.empty(t.numel() + 1, dtype=torch.uint8 if t.dtype == torch.uint8 else torch.int32, device="cuda").view(t.dtype)[1:]
+    c[name].copy_(t)
+    m = ci.RansLinear(K, N, c["tile_height"], c["tile_width"]).load_compressed(c).prepare()
+    x = torch.randn(20, K, generator=torch.Generator().manual_seed(N)).to(torch.bfloat16).cuda()
+    for rows in (20, 3):
+        assert _close(m(x[:rows]), x[:rows].float() @ W.float())
