@@ -300,9 +300,14 @@ Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables,
             e.rows = at::empty({n * 64}, h.states.options().dtype(at::kShort));
             e.spans = at::empty({n}, h.states.options());
             Tensor cap = at::empty({1}, h.states.options().dtype(at::kInt));
-            check(ci_build_entry_points(&h.w, kEntryStep, (uint32_t *)e.states.data_ptr(), (uint16_t *)e.rows.data_ptr(),
-                                        (uint32_t *)e.spans.data_ptr(), (uint32_t *)cap.data_ptr(), stream()));
-            e.cap = std::max<uint32_t>(1, (uint32_t)cap.item<int32_t>());
+            const int rc = ci_build_entry_points(&h.w, kEntryStep, (uint32_t *)e.states.data_ptr(), (uint16_t *)e.rows.data_ptr(),
+                                                 (uint32_t *)e.spans.data_ptr(), (uint32_t *)cap.data_ptr(), stream());
+            if (rc == CI_E_INVALID) {
+                e = Entries();                                  // tiles too deep for the staged decoder's window: none
+            } else {
+                check(rc);
+                e.cap = std::max<uint32_t>(1, (uint32_t)cap.item<int32_t>());
+            }
             h.entries = e;
             g_indexes.keep(h.stream, Index{Ref(h.stream), Ref(h.states), Ref(h.tables), Ref(h.slot_map), Ref(h.offsets),
                                            Ref(h.lens), K, N, th, e});

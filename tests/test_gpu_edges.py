@@ -192,3 +192,20 @@ def test_prompt_from_unaligned_buffers(K, N, th, name):
     x = torch.randn(20, K, generator=torch.Generator().manual_seed(N)).to(torch.bfloat16).cuda()
     for rows in (20, 3):
         assert _close(m(x[:rows]), x[:rows].float() @ W.float())
+
+
+# tall tiles of incompressible exponents: a window of the staged decoder does not fit, so there are no entry points
+@pytest.mark.parametrize("K,N,th", [(4096, 64, 4096), (4100, 40, 4096)])
+def test_tiles_too_deep_for_entry_points(K, N, th):
+    import comp_inference_b200 as ci
+    g = torch.Generator().manual_seed(K)
+    W = (torch.randn(K, N, generator=g) * 2.0 ** torch.randint(-100, 1, (K, N), generator=g)).to(torch.bfloat16).cuda()
+    c = ci.compress_weight_cuda(W, th, 32)
+    assert c["tile_height"] == th and int(c["rans_exp_tile_max_lens"].view(torch.int32).max()) > 1550
+    m = ci.RansLinear(K, N, th, 32).load_compressed(c).prepare()
+    x = torch.randn(20, K, generator=g).to(torch.bfloat16).cuda()
+    for rows in (1, 20):
+        assert _close(m(x[:rows]), x[:rows].float() @ W.float())
+    e = ci.RansEmbedding(K, N, th, 32).load_compressed(c).prepare()
+    ids = torch.tensor([0, K // 2 - 1, K // 2, K - 1], device="cuda")
+    assert torch.equal(e(ids), W[ids])
