@@ -393,7 +393,8 @@ static size_t workspace_bytes(uint32_t M, uint32_t n_out) {
 }
 
 // Behind those, where the caller's workspace has room: up to 16 rows of activations reordered (linear_mma4.cu).
-static size_t x_scratch_bytes(uint32_t K) { return K ? (size_t)K * 16 * sizeof(uint16_t) + 256 : 0; }
+// A group of four rows is stored whole, the first one at the next 256-byte boundary.
+static size_t x_scratch_bytes(uint32_t K) { return K ? ((size_t)K + 3) / 4 * 4 * 16 * sizeof(uint16_t) + 256 : 0; }
 
 template <int MT>
 static int launch_linear(LinArgs a, cudaStream_t s) {

@@ -209,3 +209,23 @@ def test_tiles_too_deep_for_entry_points(K, N, th):
     e = ci.RansEmbedding(K, N, th, 32).load_compressed(c).prepare()
     ids = torch.tensor([0, K // 2 - 1, K // 2, K - 1], device="cuda")
     assert torch.equal(e(ids), W[ids])
+
+
+# the workspace of the size that the library names is all that a call touches: activations reordered behind the partial sums,
+# fewer rows than a group of four, workspaces that end off a 256-byte boundary
+@pytest.mark.parametrize("K,N,M", [(1, 28419, 15), (5, 28419, 15), (9, 28419, 15), (1, 28419, 13), (1001, 28419, 15), (18, 28419, 16)])
+def test_linear_stays_inside_its_workspace(K, N, M):
+    from comp_inference_b200 import _lib
+    lib = _lib.load()
+    W = _weight(K, N)
+    stream, states, _, tables, slot_map, offsets, lens, man, *_ = _lib.host().compress(W, 16, 32, False)
+    w, keep = _lib.tiled_weight(stream, states, tables, slot_map, offsets, lens, man, K, N, 16, 32, want_max=True)
+    assert lib.ci_linear_route(w, M) == 2
+    n = lib.ci_linear_workspace_bytes(M, N, K, 16)
+    ws = torch.zeros(n + 4096, dtype=torch.uint8, device="cuda")
+    ws[n:] = 0xA5
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).cuda()
+    y = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    _lib.check(lib.ci_linear(w, _lib.ptr(x), K, M, None, _lib.ptr(y), N, _lib.ptr(ws), n, 0, _lib.stream()))
+    assert _close(y, x.float() @ W.float())
+    assert bool((ws[n:] == 0xA5).all())
