@@ -795,7 +795,7 @@ int ci_linear_static(const ci_tiled_weight *w, const uint16_t *d_x, int64_t ldx,
         ci::set_error("ci_linear_static takes at most %u activation rows per call, got %u", ci::kStaticMaxRows, M);
         return CI_E_WORKSPACE;
     }
-    const size_t need = ci_linear_workspace_bytes(M, w->N, w->K, w->tile_h);
+    const size_t need = ci::workspace_bytes(M, w->N);   // activations are reordered only where there is room left
     if (need > ci::kStaticScratchBytes) {
         ci::set_error("ci_linear_static: %u x %u outputs need %zu bytes of scratch, the built-in array holds %zu; "
                       "use ci_linear with a caller-provided workspace", M, w->N, need, ci::kStaticScratchBytes);

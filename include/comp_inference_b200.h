@@ -282,8 +282,8 @@ int ci_linear_route(const ci_tiled_weight *w, uint32_t M);
  * (ci_linear_static_max_bytes()); every GPU that loads the library holds that array until exit.
  * The call itself allocates nothing and frees nothing.
  *
- * Limits: M <= 16 activation rows, and ci_linear_workspace_bytes(M, N, K, tile_h) must fit in the
- * array (true for N up to about 16000 at M = 16); otherwise CI_E_WORKSPACE with the sizes in
+ * Limits: M <= 16 activation rows, and the tickets and partial sums must fit in the array (true for N
+ * up to 16368 at M = 16); otherwise CI_E_WORKSPACE with the sizes in
  * ci_last_error().  The first call on a device looks up the array's device address (with that
  * device current); make that first call outside any stream capture.  All calls on a device share
  * the array: two calls that overlap on the GPU (different streams, no ordering) race on it. */

@@ -84,3 +84,21 @@ def test_static_scratch_rejects_what_does_not_fit():
     big.N = 40000                                         # 16 rows x 40000 outputs would need ~41 MB of partials
     rc = lib.ci_linear_static(big, _lib.ptr(x), K, 16, None, _lib.ptr(y), 40000, _lib.stream())
     assert rc == -4 and b"built-in array" in lib.ci_last_error()
+
+
+def test_static_scratch_holds_the_widest_outputs():
+    """What the array is sized for is what ci_linear cannot do without: 16360 outputs at 16 rows fit."""
+    import comp_inference_b200 as ci
+    from comp_inference_b200 import _lib
+    lib = _lib.load()
+    K, N, M = 512, 16360, 16
+    W = make_weight(K, N, seed=2).cuda()
+    c = ci.compress_weight_cuda(W, 64, 32)
+    w, keep = _lib.tiled_weight(c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"], c["rans_exp_slot_map"],
+                                c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"], c["rans_man_raw"], K, N, 64, 32,
+                                want_max=True)
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).cuda()
+    y = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    _call(lib, lib.ci_linear_static, w, x, y)
+    ref = x.float() @ W.float()
+    assert float((y.float() - ref).abs().max() / ref.abs().max()) <= 1e-2
