@@ -422,7 +422,8 @@ template <bool PLANE>
 static int encode32(Enc32Args a, uint32_t *d_offsets, EncResult *d_res, uint64_t *stream_len, cudaStream_t s) {
     // Two columns a lane halve the loads, stores and address arithmetic per symbol, but also the warps: only where a
     // multiprocessor keeps 16 of them.
-    const bool aligned = a.N % 2 == 0 && (reinterpret_cast<uintptr_t>(a.src) & (PLANE ? 1u : 3u)) == 0;
+    const bool aligned = a.N % 2 == 0 && (reinterpret_cast<uintptr_t>(a.src) & (PLANE ? 1u : 3u)) == 0 &&
+                         (reinterpret_cast<uintptr_t>(a.mantissa) & 1u) == 0;
     const uint64_t warps2 = (uint64_t)(a.tiles_n + 1) / 2 * 2 * a.tiles_k;
     CI_CUDA(cudaMemsetAsync(a.max_lens, 0, (size_t)a.tiles_k * a.tiles_n * 4, s));
     int rc = aligned && warps2 >= 16ull * sm_count() ? launch_encode32<2, PLANE>(a, s) : launch_encode32<1, PLANE>(a, s);

@@ -229,3 +229,25 @@ def test_linear_stays_inside_its_workspace(K, N, M):
     _lib.check(lib.ci_linear(w, _lib.ptr(x), K, M, None, _lib.ptr(y), N, _lib.ptr(ws), n, 0, _lib.stream()))
     assert _close(y, x.float() @ W.float())
     assert bool((ws[n:] == 0xA5).all())
+
+
+# the encoder's sign+mantissa bytes to an odd address, at sizes where a lane takes two columns and one
+@pytest.mark.parametrize("K,N", [(2048, 4800), (1000, 78)])
+def test_encoder_to_an_odd_address(K, N):
+    import ctypes as C
+    import comp_inference_b200 as ci
+    from comp_inference_b200 import _lib
+    lib = _lib.load()
+    W = _weight(K, N)
+    c = ci.compress_weight_cuda(W, 64, 32)
+    tiles, want = -(-K // 64) * -(-N // 32), c["rans_man_raw"]
+    man = torch.zeros(want.numel() + 1, dtype=torch.uint8, device="cuda")[1:]
+    u32 = lambda n: torch.empty(n, dtype=torch.int32, device="cuda")
+    states, sizes, offsets, lens, tables = u32(tiles * 64), u32(tiles * 64), u32(tiles), u32(tiles), u32(256)
+    slot_map, freqs, cdf = torch.empty(4096, dtype=torch.uint8, device="cuda"), torch.empty(256, dtype=torch.uint16), torch.empty(256, dtype=torch.uint16)
+    n_scratch, n = lib.ci_compress_scratch_bytes(K, N, 64, 32), C.c_uint64(0)
+    scratch = torch.empty(n_scratch, dtype=torch.uint8, device="cuda")
+    _lib.check(lib.ci_compress_bf16(_lib.ptr(W), K, N, 64, 32, *map(_lib.ptr, (man, states, sizes, offsets, lens, tables, slot_map, scratch)),
+                                    n_scratch, _lib.ptr(freqs), _lib.ptr(cdf), None, C.byref(n), _lib.stream()))
+    assert torch.equal(man, want) and n.value == c["rans_exp_stream"].numel()
+    assert torch.equal(states, c["rans_exp_states"].view(torch.int32))
