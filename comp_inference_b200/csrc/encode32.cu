@@ -402,10 +402,16 @@ __global__ void __launch_bounds__(256) k_pack32(const uint32_t *__restrict__ wor
 // ------------------------------------------------------------------------ host
 
 // Page-locked landing place of the results, one per host thread: a pageable copy would be staged by the driver.
+struct PinnedResult {
+    EncResult *p = nullptr;
+    ~PinnedResult() {
+        if (p != nullptr) (void)cudaFreeHost(p);                // idle: every call that used it has waited
+    }
+};
 static EncResult *pinned_result() {
-    static thread_local EncResult *p = nullptr;
-    if (p == nullptr && cudaHostAlloc((void **)&p, sizeof *p, cudaHostAllocPortable) != cudaSuccess) p = nullptr;
-    return p;
+    static thread_local PinnedResult r;
+    if (r.p == nullptr && cudaHostAlloc((void **)&r.p, sizeof *r.p, cudaHostAllocPortable) != cudaSuccess) r.p = nullptr;
+    return r.p;
 }
 
 static bool encode32_takes(const Geom &g) { return g.tw == 32 && g.th >= 16 && g.th % 16 == 0; }

@@ -251,3 +251,16 @@ def test_encoder_to_an_odd_address(K, N):
                                     n_scratch, _lib.ptr(freqs), _lib.ptr(cdf), None, C.byref(n), _lib.stream()))
     assert torch.equal(man, want) and n.value == c["rans_exp_stream"].numel()
     assert torch.equal(states, c["rans_exp_states"].view(torch.int32))
+
+
+# threads that compress one after the other: each has a landing place of its own, given back when it ends
+def test_encoder_from_threads_that_end():
+    import threading
+    import comp_inference_b200 as ci
+    W = _weight(256, 64)
+    want, got = ci.compress_weight_cuda(W, 64, 32), []
+    for _ in range(8):
+        t = threading.Thread(target=lambda: got.append(ci.compress_weight_cuda(W, 64, 32)))
+        t.start()
+        t.join()
+    assert len(got) == 8 and all(torch.equal(c["rans_exp_stream"], want["rans_exp_stream"]) for c in got)
