@@ -242,10 +242,12 @@ def max_tile_len(tile_max_lens):
 # ticket counters zeroed, so they can share; two streams may overlap on the GPU and must not (the
 # reference keeps one global buffer for every layer and stream, comp_inference/pytorch_runtime.py:386-394).
 # A buffer that was handed out is never freed: a CUDA graph captured earlier keeps replaying into the
-# address it saw, so when a larger one is needed the old tensor is retired, not dropped.
+# address it saw, so when a larger one is needed the old tensor is retired, not dropped.  A call that is captured on a
+# stream without one of that size takes memory of the graph instead.
 _workspaces = {}
 _retired = []
 _MIN_WORKSPACE = 8 << 20
+_TICKET_BYTES = 4096 * 4            # the counters at the head of a workspace; partial sums are written before they are read
 
 
 def workspace(device, nbytes):
@@ -255,6 +257,11 @@ def workspace(device, nbytes):
     key = (device, torch.cuda.current_stream(device).cuda_stream)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
+        if torch.cuda.is_current_stream_capturing():
+            # memory of this graph, its ticket counters zeroed in it: another graph or an eager call cannot count on that
+            ws = torch.empty(max(int(nbytes), _TICKET_BYTES), dtype=torch.uint8, device=device)
+            ws[:_TICKET_BYTES].zero_()
+            return ws
         if ws is not None:
             _retired.append((key[0], ws))
         ws = torch.zeros(max(int(nbytes), _MIN_WORKSPACE), dtype=torch.uint8, device=device)
@@ -290,7 +297,8 @@ def kernel_status(device):
 def check_status(device=None, clear=True):
     """Raises RuntimeError (CI_E_DEVICE) if any kernel that used one of this device's workspaces reported an
     error through its status word; call it wherever the host waits for results anyway.  Goes through the C ABI
-    (ci_status), which waits for the current stream."""
+    (ci_status), which waits for the current stream.  A graph captured on a stream that no call had run on keeps its words
+    to itself: run the step once on the capture stream first, as a warm-up does."""
     lib = load()
     device = torch.device(device if device is not None else f"cuda:{torch.cuda.current_device()}")
     for ws in _status_words(device):

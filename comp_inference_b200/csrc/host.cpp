@@ -36,6 +36,9 @@ py::object lib_attr(const char *name) { return py::module_::import("comp_inferen
 // Launches go to the current stream of the current device, as everywhere in this package.
 ci_stream_t stream() { return reinterpret_cast<ci_stream_t>(c10::cuda::getCurrentCUDAStream().stream()); }
 
+// While a stream captures, nothing can be read back, and what a kernel writes exists only once the graph has run.
+bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
+
 struct StreamKey {
     int device;
     void *stream;
@@ -60,6 +63,7 @@ struct BufferCache {
             if (it != map.end() && (size_t)it->second.nbytes() >= bytes) return it->second;
         }
         Tensor t = ask();
+        if (capturing()) return t;                              // a graph's own memory
         std::lock_guard<std::mutex> lock(mutex);
         map[key] = t;
         return t;
@@ -232,9 +236,6 @@ struct Derived {
 };
 Derived<Tables> &g_tables = *new Derived<Tables>;               // by tile_max_lens
 Derived<Index> &g_indexes = *new Derived<Index>;                // by the stream
-
-// While a stream captures, nothing can be read back, and what a kernel writes exists only once the graph has run.
-bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
 
 Weight tiled(const Tensor &stream_t, const Tensor &states, const Tensor &tables, const Tensor &slot_map, const Tensor &offsets,
              const Tensor &lens, const OptTensor &mantissa, int64_t K, int64_t N, int64_t th, int64_t tw, bool entries) {

@@ -250,6 +250,8 @@ def _attention_workspace(device, nbytes):
     key = (device, torch.cuda.current_stream(device).cuda_stream)
     ws = _attn_ws.get(key)
     if ws is None or ws.numel() < nbytes:
+        if torch.cuda.is_current_stream_capturing():           # of this graph alone, as in _lib.workspace
+            return torch.zeros(int(nbytes), dtype=torch.uint8, device=device)
         if ws is not None:
             _attn_retired.append(ws)
         ws = torch.zeros(max(int(nbytes), 1 << 20), dtype=torch.uint8, device=device)

@@ -101,6 +101,8 @@ def _decode_scratch(device, K, N):
     key = (device, torch.cuda.current_stream(device).cuda_stream)
     buf = _scratch.get(key)
     if buf is None or buf.numel() < K * N:
+        if torch.cuda.is_current_stream_capturing():           # of this graph alone, as in _lib.workspace
+            return torch.empty((K, N), dtype=torch.bfloat16, device=device)
         if buf is not None:
             _scratch_retired.append(buf)
         buf = torch.empty(K * N, dtype=torch.bfloat16, device=device)

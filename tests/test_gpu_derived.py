@@ -223,3 +223,49 @@ def test_a_weight_written_by_the_kernel_before(kind, th):
         out.append(call())
     for i, y in enumerate(out):
         assert _right("linear" if kind == "module" else kind, y, ws[i % 2], x, ids)
+
+
+@pytest.mark.parametrize("kind", ["linear", "transposed", "prompt", "dense"])
+def test_graphs_replayed_in_another_order_than_captured(kind):
+    """Two graphs captured on one stream that no call ran on before, in a pool they share with others: neither counts on
+    what the other would have zeroed."""
+    import comp_inference_b200 as ci
+    from comp_inference_b200 import _lib
+    wa, ca, _, _ = _two_weights()
+    x, _ = _inputs()
+    if kind == "dense":
+        c = ci.compress_weight_cuda(wa, 64, 32, uncoalesced_interleaving=True)
+        call = lambda: ci.fused_rans_linear_triton_uncoalesced(
+            x, c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"], c["rans_exp_slot_map"], (K, N),
+            c["rans_exp_stream_offsets"], c["output_sizes"], c["tile_height"], 32, c["rans_man_raw"])
+    elif kind == "prompt":
+        x = x.repeat(10, 1)
+        m = ci.RansLinear(K, N, TH, 32).load_compressed(ca).prepare()
+        call = lambda: m(x)
+    else:
+        call = lambda: _call(kind, ca, x, None)
+    kind = "linear" if kind in ("dense", "prompt") else kind
+    assert _right(kind, call(), wa, x, None)
+    used = {key[1] for key in _lib._workspaces}
+    side = next(s for s in (torch.cuda.Stream() for _ in range(64)) if s.cuda_stream not in used)
+    pool, graphs = torch.cuda.graph_pool_handle(), []
+
+    def capture(fn):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side, pool=pool):
+            y = fn()
+        return g, y
+
+    before, _ = capture(lambda: torch.full((64 << 20,), 255, dtype=torch.uint8, device="cuda").sum())
+    before.replay()                                     # what the pool's memory holds
+    torch.cuda.synchronize()
+    graphs = [capture(call), capture(call)]
+    for g, y in reversed(graphs):
+        g.replay()
+        torch.cuda.synchronize()
+        assert _right(kind, y, wa, x, None)
+    with torch.cuda.stream(side):
+        y = call()
+    torch.cuda.synchronize()
+    assert _right(kind, y, wa, x, None)
+    assert _lib.kernel_status(x.device) == 0
