@@ -21,7 +21,7 @@
 
 namespace ci {
 
-constexpr uint32_t kDec4Warps = 21;          // x 32 threads x 96 registers
+constexpr uint32_t kDec4Warps = 21;          // six on one scheduler: 80 registers a thread, which it needs (none spilled)
 constexpr uint32_t kDec4BarBytes = 768;      // up to 21 warps x (2 window stages + 2 mantissa chunks) x 8 B, the table's
 
 struct Dec4Args {

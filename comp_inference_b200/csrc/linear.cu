@@ -526,7 +526,7 @@ static int linear_impl(const ci_tiled_weight *w, const uint16_t *d_x, int64_t ld
         // depth, aligned buffers, a workspace): it splits K by itself, so split_k -- a hint about how to run,
         // not about the result -- only shapes the generic kernel that takes the rest
         if (have_ws) {
-            rc = launch_linear_mma4(a, w->max_tile_len, s);     // 32-wide tiles, whole tile rows
+            rc = launch_linear_mma4(a, w->max_tile_len, s);     // 32-wide tiles
             if (rc == CI_OK) continue;
             if (rc < 0) return rc;
             rc = launch_linear_mma(a, w->max_tile_len, s);

@@ -13,11 +13,11 @@
 // instantiation for 9..16 activation rows issues a second pair of mma for row g + 8.  No shared-memory
 // transpose, no ldmatrix.
 //
-// Measured on a B200 this kernel is bound neither by HBM (10 %) nor by one on-chip unit alone: issue
-// slots are 41 % busy with about 20 integer-heavy instructions per decoded symbol on half-rate pipes,
-// the shared-memory / L1 pipeline 48 %, and every mma.sync costs as much as several ordinary
-// instructions.  So the data movement around the decode step is arranged to cost as few instructions,
-// wavefronts and tensor instructions as possible:
+// Measured on a B200 this kernel is bound neither by HBM (12 %) nor by one on-chip unit alone: over a launch at
+// 4096 x 4096, one row, issue slots are 54 % busy (61 % at 4096 x 8192, where the fixed part of a launch weighs less)
+// with 21 integer-heavy instructions per 32 symbols, the ALU pipe 40 % and L1 / shared memory 53 %; what a warp waits
+// for is its own dependent chain.  So the data movement around the decode step is arranged to cost as few
+// instructions, wavefronts and tensor instructions as possible:
 //  * compressed bytes: the two tiles' byte blocks ([row][64 B] each) are copied by cp.async into one
 //    window of 128-byte rows (upper tile in bytes 0..63, lower tile in 64..127).  The four streams of a
 //    lane are the four bytes of one word column, so every lane reads its own bank whatever row each of
@@ -34,7 +34,7 @@
 //
 // Measured (graph replays over more than L2 of weights), before -> after the chunks, the in-place renormalisation, the
 // wider choice of warp counts and the reordered activations: 4096 x 22016 at tile height 128, 1 row 90.4 -> 82.3 us,
-// 16 rows 126.7 -> 89.6; 4096 x 4096 at 1024 (was the generic kernel) 551 -> 68.
+// 16 rows 126.7 -> 89.6; 4096 x 4096 at 1024, one row, 551 (the generic kernel) -> 63, and with entry points (ENTRY) 18.9.
 #include <type_traits>
 
 #include "linear.cuh"
@@ -44,7 +44,9 @@ namespace ci {
 
 constexpr uint32_t kBar4Bytes = 768;         // up to 21 warps x (2 window stages + 2 mantissa chunks) x 8 B, the table's
 constexpr uint32_t kMma4Warps = 16;          // x 32 threads x 128 registers = the register file
-constexpr uint32_t kMma4ManyWarps = 21;      // with 96 registers (some spilled): where it saves a round of units
+// Where it saves a round of units.  21 warps are six on one scheduler, so all of its launches have 80 registers a thread: up to
+// eight rows 4 bytes are spilled, 40 with ragged K, 56 and 108 above eight rows, up to 140 with entry points.
+constexpr uint32_t kMma4ManyWarps = 21;
 
 struct Mma4Args {
     LinArgs a;
@@ -113,7 +115,7 @@ __device__ __forceinline__ void group4(uint32_t (&b)[4][2], Quad &z, uint32_t lu
 //
 // ENTRY: a unit is not a pair of whole tiles but the rows between two entry points of it (tall tiles: 512 symbols are one
 // serial chain).  The states and cursors of its streams come from the index, its window holds just the rows of the byte
-// blocks that those symbols touch.  4096 x 4096 at tile height 1024, one row: 63 us -> 18.4.
+// blocks that those symbols touch.  4096 x 4096 at tile height 1024, one row: 63 us -> 18.9.
 __device__ __align__(16) uint16_t g_zero_activations[256];
 template <bool HI, bool RAGGED, bool ENTRY, uint32_t MAX_WARPS>
 __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_constant__ Mma4Args p) {
@@ -242,8 +244,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     }
     if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
-    // Everything above touches only the weight, which the previous kernel has not written (ci_weight_written).  When this launch was allowed to
-    // start before its predecessor in the stream has finished (programmatic dependent launch), wait here
+    // Everything above touches only the weight, which the previous kernel has not written (ci_weight_written).  When
+    // this launch was allowed to start before its predecessor in the stream has finished (programmatic dependent launch), wait here
     // for it -- activations, workspace and output may be its products -- and let the next launch start
     // its own preamble while this grid works.  Both are no-ops in an ordinary launch.
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -658,9 +660,11 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     // (measured cross-over: 4096 x 2048 at tile height 128).  The two-streams kernel takes tiles of up to 256 rows.
     if (g.th <= 256 && !entry && p.total < P * CI_MMA4_MIN_UNITS) return 1;
     // One CTA per multiprocessor, the units dealt out in equal runs (they differ by one at most).  The warp count decides
-    // how well the last round is filled: 11008 x 4096 takes two rounds of 19 warps (41.5 us) or three of 13 (46.7),
-    // 4096 x 22016 five of 15 or 16 (77) instead of six of 14 (86).  A second window per warp, which hides the copies of
-    // the next unit, is worth 2 %: less than a warp that would not fit beside it.
+    // how well the last round is filled.  One row, us: 11008 x 4096 takes two rounds of 19 warps 41.0, three of 13 46.0;
+    // 4096 x 22016 takes 3.75 rounds of 20 warps 75.8, five of 16 or 15 76.1 and 76.5, six of 14 84.5.  Sixteen rows, where the
+    // many-warp kernel's second accumulators are spilled: 16 warps 84.7, 20 89.3, 14 92.3.  The two constants for more than 16
+    // warps stand for those registers.  A second window per warp, which hides the copies of the next unit, is worth 2 %:
+    // less than a warp that would not fit beside it.
     uint32_t warps = 0;
     bool many = false;
     double best = 0.0;

@@ -91,7 +91,9 @@ def fused_rans_linear_triton(x, compressed_data, initial_states, tables, slot_ma
 
     ``accum_block_size`` and ``workspace`` are accepted for source compatibility: blocking is internal,
     and split-K partials live in this package's own fp32 workspace (the reference's is a bf16 buffer
-    of another size).  ``SPLIT_K`` is honoured up to 16; 0 lets the library choose.
+    of another size).  ``SPLIT_K`` is a hint: the kernels of up to 16 rows split K by themselves, only the generic one
+    and the decode-GEMM (more than 16 rows) go by it; 0 lets the library choose.  Many rows are faster through RansLinear,
+    whose default decodes the weight once and multiplies with a library GEMM.
     """
     return _lib.host().Weight(compressed_data, initial_states, tables, slot_map, tile_offsets, tile_max_lens, mantissas,
                               int(weight_shape[0]), int(weight_shape[1]), int(tile_k), int(tile_n), True).linear(
