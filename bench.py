@@ -624,34 +624,46 @@ def reference_triton_subprocess():
 
 
 def kernels_once(args):
-    """One small invocation of each hot kernel on one 4096x4096 weight (24 MB compressed, nothing else resident):
-    the case the ncu captures summarised under profiles/ are taken on.  Prints parity figures, no timing."""
+    """Three small invocations of each hot kernel, in rounds: the case the ncu captures summarised under profiles/ are
+    taken on.  A 4096x4096 weight (24 MB compressed) at two tile heights and a 32000x4096 table at two; nothing else is
+    resident.  Prints parity figures, no timing."""
     import comp_inference_b200 as ci
     torch.cuda.set_device(0)
     K = N = HIDDEN
-    W = make_weight_kn(K, N, 1001).cuda()
-    c = ci.compress_weight_cuda(W, TILE_H, TILE_W)
-    m = ci.RansLinear(K, N, c["tile_height"], c["tile_width"], prefill_policy="fused").load_compressed(c).cuda()
+    W, T = make_weight_kn(K, N, 1001).cuda(), make_weight_kn(HIDDEN, VOCAB, 1004).t().contiguous().cuda()
     g = torch.Generator().manual_seed(7)
-    x1 = torch.randn(1, K, generator=g).to(torch.bfloat16).cuda()
-    x512 = torch.randn(512, K, generator=g).to(torch.bfloat16).cuda()
-    ids = torch.randint(0, K, (4096,), generator=g).cuda()
+    x = {M: torch.randn(M, K, generator=g).to(torch.bfloat16).cuda() for M in (1, 16, 512)}
+    ids = torch.randint(0, VOCAB, (4096,), generator=g).cuda()
+
+    def arrays(c, shape):
+        return dict(initial_states=c["rans_exp_states"], tables=c["rans_exp_tables"], slot_map=c["rans_exp_slot_map"],
+                    weight_shape=shape, tile_offsets=c["rans_exp_tile_offsets"],
+                    tile_max_lens=c["rans_exp_tile_max_lens"], tile_k=c["tile_height"], tile_n=c["tile_width"],
+                    mantissas=c["rans_man_raw"])
+
+    tall = ci.compress_weight_cuda(W, 1024, TILE_W)
+    tables = {h: ci.compress_weight_cuda(T, h, TILE_W) for h in (16, TILE_H)}
+    head = tables[TILE_H]
+    emb = {h: ci.RansEmbedding(VOCAB, HIDDEN, h, TILE_W).load_compressed(c).prepare() for h, c in tables.items()}
+    lin = {h: ci.RansLinear(K, N, h, TILE_W, prefill_policy="fused") for h in (TILE_H, 1024)}
     for _ in range(3):
-        y1 = m(x1)                                                    # k_linear_mma4
-        y512 = m(x512)                                                # k_linear_gemm + k_splitk_reduce
-        w = ci.rans_decompress_bf16(m.rans_exp_stream, m.rans_exp_states, m.rans_exp_tables, m.rans_exp_slot_map,
-                                    (K, N), m.rans_exp_tile_offsets, m.rans_exp_tile_max_lens, m.tile_k, m.tile_n,
-                                    m.rans_man_raw)                   # k_decode4
-        rows = ci.fused_rans_embedding_triton(ids, m.rans_exp_stream, m.rans_exp_states, m.rans_exp_tables,
-                                              m.rans_exp_slot_map, (K, N), m.rans_exp_tile_offsets,
-                                              m.rans_exp_tile_max_lens, m.tile_k, m.tile_n, m.rans_man_raw)  # k_embedding4
+        c = ci.compress_weight_cuda(W, TILE_H, TILE_W)                    # k_exp_histogram, k_encode32, k_pack32
+        lin[TILE_H].load_compressed(c).prepare()
+        lin[1024].load_compressed(tall).prepare()
+        y = {M: lin[TILE_H](x[M]) for M in x}                             # k_linear_mma4<0,..>, <1,..>, k_linear_gemm + k_splitk_reduce
+        y_tall = lin[1024](x[1])                                          # k_linear_mma4<..,1,..>: entry points
+        logits = ci.fused_rans_linear_transposed_triton(x[1], head["rans_exp_stream"], **arrays(head, (VOCAB, HIDDEN)))   # k_linear_t4
+        w = {h: ci.rans_decompress_bf16(p["rans_exp_stream"], **arrays(p, (K, N))) for h, p in ((TILE_H, c), (1024, tall))}   # k_decode4, k_decode2
+        rows = {h: m(ids) for h, m in emb.items()}                        # k_embedding4
     torch.cuda.synchronize()
     ci.check_status()
-    ref1, ref512 = x1.float() @ W.float(), x512.float() @ W.float()
-    print(json.dumps({"kernels_once": True, "decode_bit_exact": bool(torch.equal(w.view(torch.int16), W.view(torch.int16))),
-                      "embedding_bit_exact": bool(torch.equal(rows.view(torch.int16), W[ids].view(torch.int16))),
-                      "gemv_rel_err": float((y1.float() - ref1).abs().max() / ref1.abs().max()),
-                      "gemm_rel_err": float((y512.float() - ref512).abs().max() / ref512.abs().max())}))
+    rel = lambda got, ref: float((got.float() - ref).abs().max() / ref.abs().max())
+    print(json.dumps({"kernels_once": True,
+                      "decode_bit_exact": all(torch.equal(v.view(torch.int16), W.view(torch.int16)) for v in w.values()),
+                      "embedding_bit_exact": all(torch.equal(v.view(torch.int16), T[ids].view(torch.int16)) for v in rows.values()),
+                      "linear_rel_err": {M: rel(y[M], x[M].float() @ W.float()) for M in x},
+                      "linear_tile_1024_rel_err": rel(y_tall, x[1].float() @ W.float()),
+                      "head_rel_err": rel(logits, x[1].float() @ T.float().t())}))
 
 
 def shards_once(args):
@@ -1074,7 +1086,7 @@ def main():
                          "dense product (the case the shard kernels are profiled on)")
     ap.add_argument("--shards-time", action="store_true", help="with --shards-once: per-launch and per-step times")
     ap.add_argument("--kernels-once", action="store_true",
-                    help="run each hot kernel three times on one 4096x4096 weight and exit (the ncu capture case)")
+                    help="run each hot kernel three times on small cases and exit (the ncu capture case)")
     args = ap.parse_args()
     # Tile height is a per-tensor parameter of the stored format.  One GPU: 128 rows (fewest bytes, longest
     # streams).  Tensor-parallel shards are small enough for a launch to be bounded by the length of one stream,
