@@ -62,7 +62,7 @@ REPEATS = 7
 # compressed size, so a step's average launch is scaled by its compressed bytes.
 NCU_TRAFFIC_4096 = 24.17e6
 NCU_BYTES_4096 = 24.06e6
-NCU_CAPTURE = "ncu --set full of k_linear_mma4 on the 4096x4096 layer (bench.py --kernels-once), scaled by compressed bytes"
+NCU_CAPTURE = "ncu dram__bytes_read.sum + write of k_linear_mma4 on the 4096x4096 layer (bench.py --kernels-once), scaled by compressed bytes"
 ROUTES = {0: "k_linear (generic split-K)", 1: "k_linear_mma", 2: "k_linear_mma4", 3: "k_linear_gemm"}
 
 
