@@ -255,9 +255,10 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
                     const size_t at = (((size_t)t0 + tsel) * p.subs + c * kChunkRows / p.step) * 64 + hsel * 32 + (quad & 7) * 4;
                     const uint32_t below = win_s + tsel * 64 + hsel * 32 + (quad & 7) * 4 - 128;
                     *reinterpret_cast<uint4 *>(p.entry_states + at) = make_uint4(z.s[0], z.s[1], z.s[2], z.s[3]);
-                    uint32_t left[4];                           // a used-up stream's cursor was clamped to the window: none or one
+                    // A used-up stream's cursor was clamped to the window: none or one, but none in a tile without bytes.
+                    uint32_t left[4];
 #pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j) left[j] = z.p[j] > below + j ? (z.p[j] - below - j) >> 7 : 0u;
+                    for (uint32_t j = 0; j < 4; ++j) left[j] = z.p[j] > below + j ? min((z.p[j] - below - j) >> 7, ml) : 0u;
                     *reinterpret_cast<uint2 *>(p.entry_rows + at) = make_uint2(left[0] | left[1] << 16, left[2] | left[3] << 16);
                 }
             }

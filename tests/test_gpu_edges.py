@@ -264,3 +264,24 @@ def test_encoder_from_threads_that_end():
         t.start()
         t.join()
     assert len(got) == 8 and all(torch.equal(c["rans_exp_stream"], want["rans_exp_stream"]) for c in got)
+
+
+# one symbol only: a last tile row too short to emit a byte, below tiles that have some, entered at entry points
+@pytest.mark.parametrize("K,N,th", [(342, 64, 256), (342, 2647, 256), (1100, 33, 1024), (3072 + 40, 96, 1024)])
+def test_entry_points_of_tiles_without_bytes(K, N, th):
+    import comp_inference_b200 as ci
+    from comp_inference_b200 import _lib
+    W = torch.full((K, N), 1.5, dtype=torch.bfloat16, device="cuda")
+    c = ci.compress_weight_cuda(W, th, 32)
+    depths = c["rans_exp_tile_max_lens"].view(torch.int32)
+    assert int(depths.min()) == 0 and int(depths.max()) > 0
+    m = ci.RansLinear(K, N, th, 32).load_compressed(c).prepare()
+    h = ci.RansLMHead(N, K, th, 32, fast_twin=False).load_compressed(c).prepare()
+    for M in (1, 9, 20):
+        x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).cuda()
+        assert _close(m(x), x.float() @ W.float())
+        xh = x.repeat(1, -(-N // K))[:, :N]
+        assert _close(h(xh), xh.float() @ W.float().t())
+    ids = torch.tensor([0, th // 2, th, K - 1], device="cuda")
+    assert torch.equal(ci.RansEmbedding(K, N, th, 32).load_compressed(c).prepare()(ids), W[ids])
+    assert _lib.kernel_status(W.device) == 0
