@@ -394,7 +394,9 @@ static size_t workspace_bytes(uint32_t M, uint32_t n_out) {
 
 // Behind those, where the caller's workspace has room: up to 16 rows of activations reordered (linear_mma4.cu).
 // A group of four rows is stored whole, the first one at the next 256-byte boundary.
-static size_t x_scratch_bytes(uint32_t K) { return K ? ((size_t)K + 3) / 4 * 4 * 16 * sizeof(uint16_t) + 256 : 0; }
+static size_t x_scratch_bytes(uint32_t K, uint32_t th) {
+    return K && th ? ((size_t)K + 2 * th - 1) / (2 * th) * (2 * th) * 16 * sizeof(uint16_t) + 256 : 0;
+}
 
 template <int MT>
 static int launch_linear(LinArgs a, cudaStream_t s) {
@@ -466,7 +468,7 @@ size_t ci_linear_workspace_bytes(uint32_t M, uint32_t n_out, uint32_t K, uint32_
         const size_t fast = (size_t)kTicketBytes * 4 + linear_t4_workspace_bytes(M, n_out, tile_h);
         return generic > fast ? generic : fast;
     }
-    size_t small = workspace_bytes(M, n_out) + x_scratch_bytes(K);
+    size_t small = workspace_bytes(M, n_out) + x_scratch_bytes(K, tile_h);
     size_t big = (size_t)kTicketBytes * 4 + gemm_workspace_bytes(M, n_out, K, tile_h);    // prefill path, split-K partials
     return small > big ? small : big;
 }
@@ -491,7 +493,7 @@ static int linear_impl(const ci_tiled_weight *w, const uint16_t *d_x, int64_t ld
     a.tickets = reinterpret_cast<uint32_t *>(d_ws);
     a.partial = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(d_ws) + kTicketBytes * 4);
     a.bias = d_bias; a.ldx = ldx; a.ldy = ldy;
-    if (have_ws && ws_bytes >= workspace_bytes(M, w->N) + x_scratch_bytes(w->K))
+    if (have_ws && ws_bytes >= workspace_bytes(M, w->N) + x_scratch_bytes(w->K, w->tile_h))
         a.x_scratch = reinterpret_cast<uint16_t *>(reinterpret_cast<uint8_t *>(d_ws) +
                                                    ((workspace_bytes(M, w->N) + 255) & ~(size_t)255));
     cudaStream_t s = (cudaStream_t)stream;

@@ -13,11 +13,10 @@
 // instantiation for 9..16 activation rows issues a second pair of mma for row g + 8.  No shared-memory
 // transpose, no ldmatrix.
 //
-// Measured on a B200 this kernel is bound neither by HBM (12 %) nor by one on-chip unit alone: over a launch at
-// 4096 x 4096, one row, issue slots are 54 % busy (61 % at 4096 x 8192, where the fixed part of a launch weighs less)
-// with 21 integer-heavy instructions per 32 symbols, the ALU pipe 40 % and L1 / shared memory 53 %; what a warp waits
-// for is its own dependent chain.  So the data movement around the decode step is arranged to cost as few
-// instructions, wavefronts and tensor instructions as possible:
+// Bound by the on-chip units, not by HBM (15 to 20 %): in full rounds of 16 warps, 19.4 instructions and 5.4 load / shared-memory
+// wavefronts per 32 symbols, which take 6.7 cycles: issue slots 72 % busy, that pipe 80 %; the decode step alone, without its
+// surroundings, 16.5, 5.1 and 5.6.  So the data movement around the step is arranged to cost as few instructions and
+// wavefronts as possible:
 //  * compressed bytes: the two tiles' byte blocks ([row][64 B] each) are copied by cp.async into one
 //    window of 128-byte rows (upper tile in bytes 0..63, lower tile in 64..127).  The four streams of a
 //    lane are the four bytes of one word column, so every lane reads its own bank whatever row each of
@@ -25,16 +24,22 @@
 //  * sign+mantissa bytes: chunks of 16 rows of the four segments, double buffered per warp by cp.async, the segments
 //    8 banks apart so that a row of the warp's 128 columns is one conflict-free wavefront (read straight from
 //    global memory a row took four, one per 32-byte sector: a quarter of the pipe's load);
-//  * initial states arrive by bulk copy with the rest of the unit (no global load at a unit's start).
-// The byte windows are double buffered per warp where they fit (tall tiles: one window); byte ranges of the next units
-// are loaded one unit ahead by all lanes in parallel.
+//  * all copies of a warp are its own, so it waits for them by cp.async.wait_all and a __syncwarp; an mbarrier per
+//    buffer cost 0.5 instructions per 32 symbols more, bulk copies issued by one lane more than that;
+//  * activations: the load of four rows of a unit touches four segments, a wavefront for each of them, activation row and half
+//    warp.  Lanes without an activation row take no part (half of the wavefronts at up to four rows), and from a certain size on
+//    the activations are put in the order of the loads first (k_interleave_x).  A copy in shared memory for one or two rows
+//    saved another 1.5 % of a long launch and cost 1 us at the start of every one.
+// The byte windows are double buffered per warp where they fit; byte ranges of the next units are loaded one unit ahead by
+// all lanes in parallel.
 //
 // Scheduling: warp-level stream-K as in linear_mma.cu (units ordered by column group then tile-row
 // pair, equal contiguous runs per warp, fp32 partials + ticket, fixed summation order).
 //
-// Measured (graph replays over more than L2 of weights), before -> after the chunks, the in-place renormalisation, the
-// wider choice of warp counts and the reordered activations: 4096 x 22016 at tile height 128, 1 row 90.4 -> 82.3 us,
-// 16 rows 126.7 -> 89.6; 4096 x 4096 at 1024, one row, 551 (the generic kernel) -> 63, and with entry points (ENTRY) 18.9.
+// Measured (graph replays over more than L2 of weights) before -> with Quad::step_together, the waits and
+// activations as above and 96 registers for 17 to 20 warps: 4096 x 22016 at tile height 128, 1 row 76.3 -> 67.1 us, 16 rows
+// 84.7 -> 74.7; 11008 x 4096, 1 row 40.3 -> 36.9; 4096 x 12288 46.3 -> 42.6; 4096 x 4096 18.0 -> 17.1, at tile height 1024 with
+// entry points (ENTRY) 18.7 -> 17.8.
 #include <type_traits>
 
 #include "linear.cuh"
@@ -42,11 +47,11 @@
 
 namespace ci {
 
-constexpr uint32_t kBar4Bytes = 768;         // up to 21 warps x (2 window stages + 2 mantissa chunks) x 8 B, the table's
+constexpr uint32_t kBar4Bytes = 128;         // the table's barrier
 constexpr uint32_t kMma4Warps = 16;          // x 32 threads x 128 registers = the register file
-// Where it saves a round of units.  21 warps are six on one scheduler, so all of its launches have 80 registers a thread: up to
-// eight rows 4 bytes are spilled, 40 with ragged K, 56 and 108 above eight rows, up to 140 with entry points.
-constexpr uint32_t kMma4ManyWarps = 21;
+// Where it saves a round of units: 96 registers a thread, without spills (one instantiation spills 16 bytes).  Bounded for 21
+// warps it would be 80, with up to 160 bytes spilled: 4096 x 22016 on 20 warps, one row 67.2 us -> 72.6, 16 rows 74.7 -> 77.3.
+constexpr uint32_t kMma4ManyWarps = 20;
 
 struct Mma4Args {
     LinArgs a;
@@ -60,7 +65,7 @@ struct Mma4Args {
     uint32_t per_group;    // units of a column group = pairs_k * subs
     uint32_t stages;       // byte windows per warp: 2, or 1 where tall tiles leave no room for two
     uint32_t y_vec;        // outputs can be written as 16-byte rows of eight
-    uint32_t x_step;       // elements from one row's activations k .. k+3 to k+4 .. k+7
+    uint32_t x_order;      // activations are in the order of k_interleave_x
     uint32_t *status;      // set non-zero if a wait ran out
 };
 
@@ -93,17 +98,23 @@ __device__ __forceinline__ void mma4(float (&acc)[4][4], const uint32_t (&b)[4][
         mma_bf16(acc[3], w23, xf[2], xf[3]);
     }
 }
-__device__ __forceinline__ void group4(uint32_t (&b)[4][2], Quad &z, uint32_t lut_s, const uint32_t (&m)[4]) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {                               // two rows -> one packed pair per column
-        uint32_t e[4], f[4];
-        z.step(lut_s, e);
-        z.step(lut_s, f);
-        b[0][h] = weight_pair4<0>(e[0], f[0], m[2 * h], m[2 * h + 1]);
-        b[1][h] = weight_pair4<1>(e[1], f[1], m[2 * h], m[2 * h + 1]);
-        b[2][h] = weight_pair4<2>(e[2], f[2], m[2 * h], m[2 * h + 1]);
-        b[3][h] = weight_pair4<3>(e[3], f[3], m[2 * h], m[2 * h + 1]);
-    }
+// Four activations into the registers that the mma before has just read, where the lane has a row.
+__device__ __forceinline__ void load_x(uint32_t &lo, uint32_t &hi, const uint16_t *src, bool has) {
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.u32 p, %3, 0;\n\t"
+                 "@p ld.global.nc.v2.u32 {%0, %1}, [%2];\n\t}"
+                 : "+r"(lo), "+r"(hi)
+                 : "l"(src), "r"((uint32_t)has));
+}
+// Two symbols of each stream -> one packed pair per column.
+__device__ __forceinline__ void rows2(uint32_t (&b)[4][2], int h, Quad &z, uint32_t lut_s, uint32_t m0, uint32_t m1) {
+    uint32_t e[4], f[4];
+    z.step_together(lut_s, e);
+    z.step_together(lut_s, f);
+    b[0][h] = weight_pair4<0>(e[0], f[0], m0, m1);
+    b[1][h] = weight_pair4<1>(e[1], f[1], m0, m1);
+    b[2][h] = weight_pair4<2>(e[2], f[2], m0, m1);
+    b[3][h] = weight_pair4<3>(e[3], f[3], m0, m1);
 }
 
 // RAGGED: K is not a whole number of tile pairs, so the last units of a column group lack their lower tile or end
@@ -117,6 +128,22 @@ __device__ __forceinline__ void group4(uint32_t (&b)[4][2], Quad &z, uint32_t lu
 // serial chain).  The states and cursors of its streams come from the index, its window holds just the rows of the byte
 // blocks that those symbols touch.  4096 x 4096 at tile height 1024, one row: 63 us -> 18.9.
 __device__ __align__(16) uint16_t g_zero_activations[256];
+
+// Place of the four activations k4 of row m in that order, in 8-byte pieces, and back: what the 32 lanes read for four rows
+// of a unit are neighbours.
+struct XOrder {
+    uint32_t half4;        // k4 per row segment (half a tile)
+    uint32_t M;
+    __device__ __forceinline__ uint32_t place(uint32_t pk, uint32_t r4, uint32_t m, uint32_t q) const {
+        return ((pk * half4 + r4) * M + m) * 4 + q;
+    }
+    __device__ __forceinline__ uint32_t k4(uint32_t place, uint32_t &m) const {
+        const uint32_t row = place / (4 * M), in = place - row * 4 * M, pk = row / half4;
+        m = in >> 2;
+        return (4 * pk + (in & 3)) * half4 + row - pk * half4;
+    }
+};
+
 template <bool HI, bool RAGGED, bool ENTRY, uint32_t MAX_WARPS>
 __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_constant__ Mma4Args p) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -132,7 +159,6 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     start_lut(lut_s, lut_bar, a.lut);
     const uint32_t wbase_s = lut_s + kLutBytes + kBar4Bytes + W * kManBytes + warp * p.stages * p.stage_bytes;
     const uint32_t man_s = lut_s + kLutBytes + kBar4Bytes + warp * kManBytes;
-    const uint32_t bar_base = lut_s + kLutBytes + warp * 32, man_bar = bar_base + 16;
     const uint32_t seg_bytes = g.th * 16;                       // half a tile of sign+mantissa bytes
     const uint32_t st_off = p.cap_rows * 128;
 
@@ -172,64 +198,46 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     auto issue = [&](uint32_t grp, uint32_t pk, uint32_t sub, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
         const uint32_t t0 = (2 * pk) * g.tiles_n + grp;
         const bool two = 2 * pk + 1 < g.tiles_k;
-        const uint32_t bar = bar_base + stage * 8;
         const uint32_t dst = wbase_s + stage * p.stage_bytes;
         if (ml0 > p.cap_rows || ml1 > p.cap_rows) {             // metadata disagrees with the declared maximum
             if (lane == 0) atomicExch(p.status, 2u);
             ml0 = ml1 = 0;
         }
-        if (lane == 0) {
-            fence_async_proxy();
-            if constexpr (ENTRY) {
-                const size_t e0 = ((size_t)t0 * subs + sub) * 64, e1 = e0 + (size_t)g.tiles_n * subs * 64;
-                mbar_expect_tx(bar, two ? 768u : 384u);
-                bulk_load(dst + st_off, a.entry_states + e0, 256, bar);
-                bulk_load(dst + st_off + 512, a.entry_rows + e0, 128, bar);
-                if (two) {
-                    bulk_load(dst + st_off + 256, a.entry_states + e1, 256, bar);
-                    bulk_load(dst + st_off + 640, a.entry_rows + e1, 128, bar);
-                }
-            } else {
-                mbar_expect_tx(bar, two ? 512u : 256u);
-                bulk_load(dst + st_off, a.states + (size_t)t0 * 64, 256, bar);
-                if (two) bulk_load(dst + st_off + 256, a.states + ((size_t)t0 + g.tiles_n) * 64, 256, bar);
-            }
+        // states, 16 lanes a tile, and for entry points the rows of their next bytes, 8 lanes a tile
+        const bool lower = lane >= 16;
+        if constexpr (ENTRY) {
+            const size_t e = ((size_t)t0 * subs + sub) * 64, d = (size_t)g.tiles_n * subs * 64;
+            if (!lower || two) cp_async16(dst + st_off + lane * 16, a.entry_states + e + (lower ? d : 0) + (lane & 15) * 4);
+            if (lane < 8 || (two && lane < 16))
+                cp_async16(dst + st_off + 512 + lane * 16, a.entry_rows + e + (lane < 8 ? 0 : d) + (lane & 7) * 8);
+        } else {
+            if (!lower || two) cp_async16(dst + st_off + lane * 16, a.states + (size_t)(t0 + (lower ? g.tiles_n : 0u)) * 64 + (lane & 15) * 4);
         }
         // byte blocks: 16-byte pieces, piece i of a tile = (row i / 4, quarter i % 4)
         const uint8_t *s0 = a.stream + off0, *s1 = a.stream + off1;
         for (uint32_t i = lane; i < ml0 * 4; i += 32) cp_async16(dst + (i >> 2) * 128 + (i & 3) * 16, s0 + i * 16);
         for (uint32_t i = lane; i < ml1 * 4; i += 32) cp_async16(dst + (i >> 2) * 128 + 64 + (i & 3) * 16, s1 + i * 16);
-        cp_async_arrive(bar);
     };
 
     // Sign+mantissa bytes of a unit's upper tile, this lane's 16-byte piece of every chunk row pair.
     auto man_of = [&](uint32_t grp, uint32_t pk, uint32_t sub) {
         return a.mantissa + ((size_t)2 * pk * g.tiles_n + grp) * (2 * seg_bytes) + (ENTRY ? sub * step * 32 : 0u) + lane * 16;
     };
-    // Rows [kChunkRows * c, + kChunkRows) of the four segments of a unit into chunk buffer `buf`; src: man_of the unit.
-    auto issue_man = [&](const uint8_t *src, bool two, uint32_t c, uint32_t buf) {
+    // Rows [row, + kChunkRows) of the four segments of a unit into chunk buffer `buf`; src: this lane's piece of them.
+    const size_t tile_step = (size_t)g.tiles_n * (2 * seg_bytes);
+    auto issue_man = [&](const uint8_t *src, bool two, uint32_t row, uint32_t buf) {
         const uint32_t dst = man_s + buf * (4 * kSegPitch) + lane * 16;
-        if (c * kChunkRows + (lane >> 1) < step) {
-            src += c * (kChunkRows * 32);
+        if (row + (lane >> 1) < step) {
             cp_async16(dst, src);
             cp_async16(dst + kSegPitch, src + seg_bytes);
             if (two) {
-                src += (size_t)g.tiles_n * (2 * seg_bytes);
+                src += tile_step;
                 cp_async16(dst + 2 * kSegPitch, src);
                 cp_async16(dst + 3 * kSegPitch, src + seg_bytes);
             }
         }
-        cp_async_arrive(man_bar + buf * 8);
     };
 
-    if (lane == 0) {
-        mbar_init(bar_base, 33);                                // 32 cp.async arrivals + the bulk copies' expect_tx
-        mbar_init(bar_base + 8, 33);
-        mbar_init(man_bar, 32);
-        mbar_init(man_bar + 8, 32);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
     load_desc();
     uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
     uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
@@ -428,13 +436,13 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
         if (lane == 0) a.tickets[grp] = 0;                      // ready for the next call
     };
 
-    // Activations of rows gq and gq + 8, eight consecutive k at a time (two groups of four rows).
-    // Rows beyond the batch read the last real row instead: their products land in output rows that are
-    // never stored, so no guard (and no branch) is needed in the loop.
-    const uint32_t m_last = a.M - 1;
-    const uint16_t *x0 = a.x + (size_t)min(gq, m_last) * a.ldx;
-    const uint16_t *x1 = a.x + (size_t)min(gq + 8, m_last) * a.ldx;
-    uint32_t parity0 = 0, parity1 = 0, stage = 0;
+    // Activations of rows gq and gq + 8, four consecutive k of the lane's segment at a time.  Lanes without a row load nothing
+    // (from rows that lie apart a load is a wavefront per segment and half warp).
+    const bool has0 = gq < a.M, has1 = gq + 8 < a.M;
+    const uint16_t *x0 = a.x + (p.x_order ? lane * 4 : (size_t)(has0 ? gq : 0) * a.ldx);
+    const uint16_t *x1 = a.x + (p.x_order ? 128 + lane * 4 : (size_t)(has1 ? gq + 8 : 0) * a.ldx);
+    const uint32_t x_step = p.x_order ? 16 * a.M : 4;
+    uint32_t stage = 0;
     uint32_t cur_grp = grp;
     zero_acc();
     const uint32_t n_blocks = step / 4;                         // blocks of four symbols per stream
@@ -443,11 +451,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     uint32_t chunk = 0;                                         // sign+mantissa chunks consumed: buffer and phase parity
 
     Quad z;
+    const uint8_t *man = man_of(grp, pk, sub);                  // the sign+mantissa chunk that was asked for last
+    bool two = 2 * pk + 1 < g.tiles_k;
     for (uint32_t t = lo; t < hi; ++t) {
         const bool last_sub = !ENTRY || sub + 1 == subs, wrap = last_sub && pk + 1 == p.pairs_k;
         const uint32_t n_grp = grp + wrap, n_pk = wrap ? 0u : pk + last_sub, n_sub = last_sub ? 0u : sub + 1;   // of unit t + 1
-        const uint8_t *man = man_of(grp, pk, sub);
-        const bool two = 2 * pk + 1 < g.tiles_k;
         if (grp != cur_grp) {
             flush(cur_grp);
             zero_acc();
@@ -470,9 +478,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
                 len = (top_rows + 3) >> 2;
             }
         }
-        uint32_t xs = p.x_step;
-        const uint16_t *xp0 = x0 + (size_t)(krow >> 2) * xs, *xp1 = x1 + (size_t)(krow >> 2) * xs;
-        if (RAGGED && n_my == 0) {
+        const uint32_t r4 = pk * (g.half / 4) + (ENTRY ? sub * step / 4 : 0u);
+        uint32_t xs = x_step;
+        const size_t x_at = p.x_order ? (size_t)r4 * x_step : krow;
+        const uint16_t *xp0 = x0 + x_at, *xp1 = x1 + x_at;
+        if (RAGGED && n_my == 0 && !p.x_order) {
             xp0 = xp1 = g_zero_activations;
             xs = 0;
         }
@@ -493,20 +503,14 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
             nx_ml1 = __shfl_sync(kFull, d_ml1, j);
             issue(n_grp, n_pk, n_sub, p.stages == 1 ? 0u : stage ^ 1, nx_off0, nx_ml0, nx_off1, nx_ml1);
         };
-        __syncwarp();
-
         // ---- this lane's four streams --------------------------------------
         const uint32_t win_s = wbase_s + stage * p.stage_bytes;
         const uint32_t st_s = win_s + st_off + tsel_d * 256 + (hsel_d * 32 + gq_d * 4) * 4;
         uint32_t first = win_s + tsel_d * 64 + hsel_d * 32 + gq_d * 4;
         if (!ENTRY && ml <= p.cap_rows) first += (ml - 1) * 128;   // last byte row; an empty tile starts one row below
 
-        // ---- wait for the bytes (bounded) -------------------------------------
-        {
-            const uint32_t bar = bar_base + stage * 8, par = stage ? parity1 : parity0;
-            if (!mbar_wait(bar, par)) atomicExch(p.status, 1u);  // the result is invalid; the loop still ends
-            if (stage) parity1 ^= 1; else parity0 ^= 1;
-        }
+        cp_async_wait();                                        // this unit's bytes and states, the first sign+mantissa chunk
+        __syncwarp();
         auto start_streams = [&]() {
             z.start(st_s, first);
             if constexpr (ENTRY) {                              // every stream has its own row of the window
@@ -532,24 +536,32 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
 #pragma unroll 1
             for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
                 const uint32_t buf = chunk & 1;
-                __syncwarp();                                       // every lane is done with the other chunk buffer
-                if (c + 1 < n_chunks) issue_man(man, two, c + 1, buf ^ 1);
-                else if (t + 1 < hi) issue_man(man_of(n_grp, n_pk, n_sub), 2 * n_pk + 1 < g.tiles_k, 0, buf ^ 1);
-                if (c == 0 && p.stages == 2) next_unit();   // behind it: a chunk's arrival waits for older copies
-                if (!mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1)) atomicExch(p.status, 1u);
+                if (c != 0) {
+                    cp_async_wait();                                // this chunk is here
+                    __syncwarp();                                   // for every lane, and all are done with the other buffer
+                }
+                const bool last = c + 1 == n_chunks;
+                if (last) {                                         // the next unit's first chunk
+                    man = man_of(n_grp, n_pk, n_sub);
+                    two = 2 * n_pk + 1 < g.tiles_k;
+                } else {
+                    man += kChunkRows * 32;
+                }
+                if (!last || t + 1 < hi) issue_man(man, two, last ? 0u : (c + 1) * kChunkRows, buf ^ 1);
+                if (c == 0 && p.stages == 2) next_unit();
                 z.clamp(win_s);
                 uint32_t ms = man_s + (buf * 4 + q) * kSegPitch + gq * 4;
                 const uint32_t end = RAG && empty ? 0u : min(blk + kChunkRows / 4, n_blocks);
 #pragma unroll 1
                 for (; blk < end; ++blk) {
-                    const uint2 v0 = __ldg(reinterpret_cast<const uint2 *>(xp0));   // used by the mma at the end
-                    uint2 v1 = make_uint2(0u, 0u);
-                    if constexpr (HI) v1 = __ldg(reinterpret_cast<const uint2 *>(xp1));
                     const uint32_t m[4] = {lds_u32(ms), lds_u32(ms + 32), lds_u32(ms + 64), lds_u32(ms + 96)};
                     // The tensor instruction of the group before comes first: behind it the compiler knows that the warp is
                     // converged, and the register copies that its checks of that need go.
                     mma4<HI>(acc, wb, xf);
-                    group4(wb, z, lut_s, m);
+                    load_x(xf[0], xf[1], xp0, has0);                // used by the mma at the end
+                    if constexpr (HI) load_x(xf[2], xf[3], xp1, has1);
+                    rows2(wb, 0, z, lut_s, m[0], m[1]);
+                    rows2(wb, 1, z, lut_s, m[2], m[3]);
                     if constexpr (RAG) {
                         const uint32_t n = blk + 1 < n_my ? 4u : blk >= n_my ? 0u : cut ? cut : 4u;   // rows of the block that exist
                         if (n < 4) {
@@ -560,12 +572,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
                             }
                         }
                     }
-                    xf[0] = v0.x; xf[1] = v0.y; xf[2] = v1.x; xf[3] = v1.y;
                     ms += 128;
                     xp0 += xs;
                     if constexpr (HI) xp1 += xs;
                     if constexpr (RAG) {
-                        if (blk + 1 == n_my) {                      // rows beyond K from the next block on
+                        if (blk + 1 == n_my && !p.x_order) { // rows beyond K from the next block on
                             xp0 = xp1 = g_zero_activations;
                             xs = 0;
                         }
@@ -597,27 +608,29 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     flush(cur_grp);
 }
 
-// x[M][K] -> scratch[ceil(K / 4)][M][4], zeros beyond K.  A warp's activation load reads four consecutive k of every row: from rows K elements
-// apart that is a cache line, and a wavefront of the load pipe, per row and segment (32 a load for 8 rows, 60 % of the
-// kernel's pipe time at 16 rows); in this order a segment's rows are neighbours.
-__global__ void __launch_bounds__(256) k_interleave_x(const uint16_t *__restrict__ x, int64_t ldx, uint32_t M, uint32_t K,
-                                                      uint32_t aligned, uint2 *__restrict__ out) {
+// The activations in the order in which the kernel's warps read them, [tile pair][four rows][M][segment][4], zeros beyond K: a
+// warp's load of four rows is then one run of 32 M bytes (of 256 where M is larger than eight).  From rows K elements apart it is
+// a cache line, and a wavefront of the load pipe, per row and segment.
+__global__ void __launch_bounds__(256) k_interleave_x(const uint16_t *__restrict__ x, int64_t ldx, uint32_t K, XOrder order,
+                                                      uint32_t pieces, uint32_t aligned, uint2 *__restrict__ out) {
     asm volatile("griddepcontrol.wait;" ::: "memory");          // the activations may be the previous kernel's product
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint32_t k4 = blockIdx.x * 256 + threadIdx.x;
-    if (4 * k4 >= K) return;
-    for (uint32_t m = blockIdx.y; m < M; m += gridDim.y) {
-        const uint16_t *src = x + (size_t)m * ldx + 4 * k4;
-        uint2 v = make_uint2(0u, 0u);
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= pieces) return;
+    uint32_t m;
+    const uint32_t k = 4 * order.k4(i, m);
+    uint2 v = make_uint2(0u, 0u);
+    if (k < K) {
+        const uint16_t *src = x + (size_t)m * ldx + k;
         if (aligned) {
             v = __ldg(reinterpret_cast<const uint2 *>(src));
         } else {
-            const uint32_t n = K - 4 * k4;
+            const uint32_t n = K - k;
             v.x = __ldg(src) | (n > 1 ? (uint32_t)__ldg(src + 1) << 16 : 0u);
             v.y = (n > 2 ? (uint32_t)__ldg(src + 2) : 0u) | (n > 3 ? (uint32_t)__ldg(src + 3) << 16 : 0u);
         }
-        out[(size_t)k4 * M + m] = v;
     }
+    out[i] = v;
 }
 
 // ------------------------------------------------------------------------ host
@@ -660,11 +673,11 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     // (measured cross-over: 4096 x 2048 at tile height 128).  The two-streams kernel takes tiles of up to 256 rows.
     if (g.th <= 256 && !entry && p.total < P * CI_MMA4_MIN_UNITS) return 1;
     // One CTA per multiprocessor, the units dealt out in equal runs (they differ by one at most).  The warp count decides
-    // how well the last round is filled.  One row, us: 11008 x 4096 takes two rounds of 19 warps 41.0, three of 13 46.0;
-    // 4096 x 22016 takes 3.75 rounds of 20 warps 75.8, five of 16 or 15 76.1 and 76.5, six of 14 84.5.  Sixteen rows, where the
-    // many-warp kernel's second accumulators are spilled: 16 warps 84.7, 20 89.3, 14 92.3.  The two constants for more than 16
-    // warps stand for those registers.  A second window per warp, which hides the copies of the next unit, is worth 2 %:
-    // less than a warp that would not fit beside it.
+    // how well the last round is filled.  One row, us: 11008 x 4096 takes two rounds of 19 warps 36.9, 2.7 of 14 41.1;
+    // 4096 x 22016 takes 3.7 rounds of 20 warps 67.2, 4.7 of 16 70.1, 5.4 of 14 78.1; 4096 x 12288 2.6 of 16 42.6, 2.1 of
+    // 20 45.7.  A second window per warp, which hides the copies of the next unit, is worth 2 %: less than a warp that would
+    // not fit beside it.
+    const uint32_t x_rows = p.pairs_k * 2 * g.th;               // K, rounded up to whole tile pairs
     uint32_t warps = 0;
     bool many = false;
     double best = 0.0;
@@ -673,9 +686,8 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
         uint32_t w_max = room / (stages * p.stage_bytes + kManBytes);
         if (w_max > kMma4ManyWarps) w_max = kMma4ManyWarps;
         for (uint32_t w = 1; w <= w_max; ++w) {
-            const bool m = w > kMma4Warps;                      // more spilled registers with a second set of accumulators
-            const double cost = run_cost(units, w, 0.9) * (stages == 1 ? 1.02 : 1.0) * (m && a.M > 8 ? 1.12 : 1.0);
-            if (warps == 0 || cost < best) { best = cost; warps = w; many = m; p.stages = stages; }
+            const double cost = run_cost(units, w, 0.3) * (stages == 1 ? 1.02 : 1.0);
+            if (warps == 0 || cost < best) { best = cost; warps = w; many = w > kMma4Warps; p.stages = stages; }
         }
     }
     if (warps == 0 || (g.th <= 256 && !entry && warps < 4)) return 1;
@@ -685,7 +697,7 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     p.slots = blocks * warps < p.total ? blocks * warps : p.total;
     if ((uint64_t)p.slots * (p.total + 1) >> 32) return 1;      // 1.8 million units
     p.y_vec = ((reinterpret_cast<uintptr_t>(a.y) & 15u) == 0 && (a.ldy & 7) == 0) ? 1u : 0u;
-    p.x_step = 4;
+    p.x_order = 0;
     p.status = a.tickets + (kTicketBytes - 1);
     if (a.dry_run) return CI_OK;                                // qualification only
 
@@ -709,17 +721,20 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    // The extra launch takes 2.7 us and saves about 1.7e-8 us per activation row and weight, where the multiprocessors are
-    // busy at all: it pays from 1.6e8 of them (4096 x 22016: 119 -> 90 us at 16 rows, 94 -> 85 at 8, 87 -> 85 at 4).
-    // Short units (tile height 64) do not wait for that pipe: 6784 x 5168 takes 48.8 us at 16 rows without it, 51.8 with it.
-    if (!quads_ok || (a.x_scratch != nullptr && a.M >= 3 && p.step >= 64 && p.total >= 6 * P && (uint64_t)a.M * g.K * g.N >= 160000000ull)) {
-        cfg.gridDim = dim3((g.K / 4 + 256) / 256, a.M);
+    // The launch in front costs about 2 us and takes a wavefront per row beyond the first, segment and four rows of a unit out of
+    // the load pipe.  us without -> with: 4096 x 4096 at 6 rows 20.1 -> 20.9, 8 21.3 -> 20.9, 16 27.7 -> 22.2; 5504 x 4100 at
+    // 2 rows 22.3 -> 24.1, 5 26.7 -> 25.9; 4096 x 22016 at 2 rows 70.9 -> 71.5, 3 74.0 -> 72.0, 16 121.2 -> 75.8; at tile
+    // height 64, where the steps of a short unit wait for less, 6784 x 5168 at 4 rows 32.9 -> 33.7, 8 34.9 -> 34.1.
+    const uint64_t x_lines = (uint64_t)(a.M - 1) * g.K * g.N;
+    const bool reorder = a.x_scratch != nullptr && a.M >= 3 && x_lines >= (p.step >= 64 ? 90000000ull : 200000000ull);
+    if (!quads_ok || reorder) {
+        const uint32_t pieces = x_rows / 4 * a.M;
+        cfg.gridDim = dim3((pieces + 255) / 256);
         cfg.blockDim = dim3(256);
-        CI_CUDA(cudaLaunchKernelEx(&cfg, k_interleave_x, a.x, a.ldx, a.M, g.K, (uint32_t)quads_ok,
+        CI_CUDA(cudaLaunchKernelEx(&cfg, k_interleave_x, a.x, a.ldx, g.K, XOrder{g.half / 4, a.M}, pieces, (uint32_t)quads_ok,
                                    reinterpret_cast<uint2 *>(a.x_scratch)));
         p.a.x = a.x_scratch;
-        p.a.ldx = 4;
-        p.x_step = 4 * a.M;
+        p.x_order = 1;
     }
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(warps * 32);

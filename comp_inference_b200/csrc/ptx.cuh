@@ -36,6 +36,8 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+// All cp.async issued so far by this thread have landed (for the other lanes of the warp behind a __syncwarp).
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // The mbarrier gets one arrival when all cp.async issued so far by this thread have landed.
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
@@ -146,8 +148,13 @@ __device__ __forceinline__ void renorm_fast(uint32_t &state, uint32_t &pos) {
 // every step), which takes one shared-memory latency off the decode chain; about one symbol in three merges it, under
 // a predicate.  A second byte is needed only after a symbol of frequency below 16: one test for the four streams, one
 // branch.  The whole renormalisation is one asm block so that the rare branch updates the registers in place; with the
-// branch in C++ the compiler copies all eight of them on the common path (2 of 22 instructions per symbol).  A warp vote in
-// front of the branch made the stand-alone decoder 3 % slower and the fused linear no faster.
+// branch in C++ the compiler copies all eight of them on the common path (2 of 22 instructions per symbol).
+//
+// step_together(): the whole warp takes that branch or does not, by a vote on a test that does not wait for the first bytes
+// (the state before them is below 2^8).  Where tensor instructions follow, lanes that part in every step have to be brought
+// together again: in a loop of steps, packing and mma alone one warp a scheduler took 211 cycles a step and takes 166,
+// 16 warps 378 and 359.  The decoders and the gather, without such instructions, are 0.2 to 0.4 % slower with it.  Second bytes
+// under predicates instead of a branch: 403 at 16 warps.
 struct Quad {
     uint32_t s[4], p[4];                                        // states, shared addresses of the next bytes
 
@@ -202,6 +209,34 @@ struct Quad {
             "DONE:\n\t}"
             : "+r"(s[0]), "+r"(s[1]), "+r"(s[2]), "+r"(s[3]), "+r"(p[0]), "+r"(p[1]), "+r"(p[2]), "+r"(p[3])
             : "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]));
+    }
+    __device__ __forceinline__ void step_together(uint32_t lut_s, uint32_t (&e)[4]) {
+        uint32_t y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = lds_u8(p[j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e[j] = decode_aligned(s[j], lut_s);
+        const uint32_t low = min(min(s[0], s[1]), min(s[2], s[3]));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            asm("{\n\t.reg .pred p;\n\t"
+                "setp.lt.u32 p, %0, 65536;\n\t"
+                "@p mad.lo.u32 %0, %0, 256, %2;\n\t"
+                "@p sub.u32 %1, %1, 128;\n\t}"
+                : "+r"(s[j]), "+r"(p[j])
+                : "r"(y[j]));
+        if (__any_sync(kFull, low < 256u)) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[j] = lds_u8(p[j]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                asm volatile("{\n\t.reg .pred p;\n\t"
+                             "setp.lt.u32 p, %0, 65536;\n\t"
+                             "@p mad.lo.u32 %0, %0, 256, %2;\n\t"
+                             "@p sub.u32 %1, %1, 128;\n\t}"
+                             : "+r"(s[j]), "+r"(p[j])
+                             : "r"(y[j]));
+        }
     }
     // Streams of columns that do not exist (`cols` of the four do) run along with the first one.  Their own would start at
     // 2^16 over zero bytes: a symbol of frequency 1 at every step, and with it the branch for a second byte.
@@ -261,12 +296,13 @@ constexpr uint32_t kChunkRows = 16;
 constexpr uint32_t kSegPitch = kChunkRows * 32 + 32;
 constexpr uint32_t kManBytes = 2 * 4 * kSegPitch;
 // Cost model of the persistent kernels' launches, in us at 64 symbols per stream.  A round of units -- every one of w warps
-// takes one -- lasts 3.6 + 0.75 x warps, where a scheduler with a warp more than the others counts half (measured in full
-// rounds of the fused linear: 12 warps 12.7, 14 14.8, 16 15.6; up to four warps have a scheduler each and take 7.2).
+// takes one -- lasts 2.6 + 0.7 x warps, where a scheduler with a warp more than the others counts half (measured in full
+// rounds of the fused linear: 12 warps 11.2, 14 13.1, 16 13.7, 19 16.4; two warps a scheduler 9, one 7.4).
 // `extra` is what a round of more than 16 warps costs on top, where they have fewer registers or a pipe is full already.
 inline double round_cost(uint32_t w, double extra) {
-    if (w <= 4) return 7.2;
-    return 3.6 + 0.375 * (w + (w + 3) / 4 * 4) + (w > 16 ? extra : 0.0);
+    if (w <= 4) return 7.4;
+    if (w <= 8) return 9.0;
+    return 2.6 + 0.35 * (w + (w + 3) / 4 * 4) + (w > 16 ? extra : 0.0);
 }
 // `units` units on a multiprocessor with w warps: full rounds, then what is left on fewer warps.
 inline double run_cost(uint32_t units, uint32_t w, double extra) {
