@@ -9,41 +9,67 @@
 // activations of the sixteen columns -- stays in registers for the whole unit.  (The kernel for forced cases in linear.cu
 // reduces every row over the lanes with 31 shuffles per 32 rows instead.)
 //
-// A unit yields a sum for every row, so the sums live in shared memory, private to the warp: read as the mma's C operand
+// A unit yields a sum for every row.  For one or two activation rows and up to 64 rows a segment they stay in registers from
+// one column block to the next (REG); otherwise they live in shared memory, private to the warp: read as the mma's C operand
 // and written back, two 8-byte loads and stores per two rows.  The warps of a CTA take column blocks of the same four
 // tiles ("group"); at the end of its run in a group the CTA adds its warps' sums, writes an fp32 partial and draws a
-// ticket; the CTA that draws the last one adds the partials in a fixed order and writes bf16.
+// ticket; the CTA that draws the last one adds the partials in a fixed order and writes bf16.  Where there is room for two
+// sets of sums a CTA deals the units of two groups out as one sequence before it does so.
 //
 // Bytes are staged as in linear_mma4.cu: one window of 128-byte rows per unit (a shared-memory bank per lane), sign and
-// mantissa in 16-row chunks.  Bound by the decode step like that kernel.  Measured on a B200, 32000 x 4096, one row, tile
-// height 128: 1000 us (the shuffle kernel) -> 139; 32000 x 5120 at tile height 1024: 516 us without entry points -> 274 with
-// them, eight rows 3590 -> 444.
+// mantissa in 16-row chunks, initial states with the window, all waited for with cp.async.wait_all.  Bound by the instructions
+// of the decode step like that kernel: 21 per 32 symbols, 75 % of the issue slots in long runs (32000 x 4096, one row).
+//
+// Measured on a B200, us, before -> with sums in registers, two sets, states among the copies and the chunks of three warps
+// in front of the table: 32000 x 4096 at tile height 128, one row 139 -> 118, two 145 -> 131, eight 215 -> 195; at 64 155 -> 128; at
+// 1024 with entry points 273 -> 194, eight rows 366 -> 328; 8000 x 1024 at 128 31.5 -> 22.3.  The shuffle kernel takes 1000 and 3590
+// for the first and for eight rows at 1024.
 #include "linear.cuh"
 #include "ptx.cuh"
 
 namespace ci {
 
 constexpr uint32_t kT4Warps = 16;
-constexpr uint32_t kT4BarBytes = 640;        // up to 16 warps x (2 window stages + 2 chunks) x 8 B
+constexpr uint32_t kT4BarBytes = 128;        // the table's barrier, the flag of the last arrival
 constexpr uint32_t kT4SegPitch = kChunkRows * 16 + 16;       // eight segments of a chunk, 4 banks apart
 constexpr uint32_t kT4ManBytes = 2 * 8 * kT4SegPitch;
+constexpr uint32_t kT4RegChunks = 4;         // chunks of a segment whose sums a lane holds in registers
 
 struct T4Args {
     LinArgs a;
     uint32_t cap_rows;     // rows of a byte window (>= every tile_max_len)
-    uint32_t stage_bytes;
+    uint32_t stage_bytes;  // window + initial states (with entry points also the rows of the next bytes)
     uint32_t stages;       // windows per warp
-    uint32_t acc_bytes;    // sums of a warp
+    uint32_t front;        // warps whose sign+mantissa chunks lie in front of the table
+    uint32_t acc_bytes;    // sums of a warp in one group
+    uint32_t sets;         // groups that a CTA works on between two barriers
     uint32_t cblocks;      // 16-column blocks per group
     uint32_t subs, step;   // ENTRY: groups per four tiles, the rows of a segment in each; else 1, half a tile
     uint32_t total;        // units
+    uint32_t x_wide;       // four activations are one aligned 8-byte load
+    uint32_t wide;         // states (and rows) can be copied 16 bytes at a time
     uint32_t *status;
 };
 
-// MT: sums per row in shared memory (1, 2 or 8 activation rows).
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+// d = w . x with nothing added: the sums of two rows of each segment over the unit's columns.
+__device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const uint32_t (&w)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+// MT: activation rows that a pass takes (1, 2 or 8).
+// REG: the sums of up to 64 rows a segment stay in registers (one or two activation rows).  Every column of D is made a row of
+// activations -- column n is row n % MT -- so that all four lanes of a segment hold the sums of its two rows, and lane q adds
+// those of rows 4q .. 4q + 3 of a 16-row chunk to its own: 16 MT registers, turned by one chunk at a time because a loop cannot
+// index them.  (One activation column per row pair in one D instead would let an infinite weight reach its neighbours' sums.)
 // ENTRY: a group is the rows of four tiles between two entry points (see linear_mma4.cu), so its sums are those of a short
 // tile; without, a tall tile's sums and window leave room for three warps.
-template <int MT, bool ENTRY>
+template <int MT, bool ENTRY, bool REG>
 __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_constant__ T4Args p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const LinArgs &a = p.a;
@@ -53,107 +79,148 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     const uint32_t lut_s = (smem_s + kLutBytes - 1) & ~(kLutBytes - 1);    // see linear_mma4.cu
     uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + (lut_s - smem_s));
     const uint32_t lut_bar = lut_s + kLutBytes + kT4BarBytes - 16;
+    if (lut_s - smem_s < p.front * kT4ManBytes) {               // the table does not lie where the launcher takes it to
+        if (threadIdx.x == 0) atomicExch(p.status, 1u);
+        return;
+    }
     start_lut(lut_s, lut_bar, a.lut);
-    const uint32_t bar_base = lut_s + kLutBytes + warp * 32, man_bar = bar_base + 16;
-    const uint32_t man_s = lut_s + kLutBytes + kT4BarBytes + warp * kT4ManBytes;
-    const uint32_t acc0_s = lut_s + kLutBytes + kT4BarBytes + W * kT4ManBytes, acc_s = acc0_s + warp * p.acc_bytes;
-    const uint32_t wbase_s = acc0_s + W * p.acc_bytes + warp * p.stages * p.stage_bytes;
+    const uint32_t behind_s = lut_s + kLutBytes + kT4BarBytes;
+    const uint32_t man_s = warp < p.front ? smem_s + warp * kT4ManBytes : behind_s + (warp - p.front) * kT4ManBytes;
+    const uint32_t acc0_s = behind_s + (W - p.front) * kT4ManBytes, set_bytes = W * p.acc_bytes;
+    const uint32_t acc_s = acc0_s + warp * p.acc_bytes;         // of the first set; the others set_bytes further each
+    const uint32_t wbase_s = acc0_s + p.sets * set_bytes + warp * p.stages * p.stage_bytes;
+    const uint32_t st_off = p.cap_rows * 128;
     const uint32_t subs = ENTRY ? p.subs : 1u, step = ENTRY ? p.step : g.half;
     const uint32_t seg_acc = step * (MT * 4) + (MT == 8 ? 32 : MT * 4);  // bytes between the sums of two segments
-    __shared__ uint32_t s_flag;
+    uint32_t *const s_flag = reinterpret_cast<uint32_t *>(smem + (lut_bar + 8 - smem_s));
 
     const uint32_t sg = lane >> 2, q = lane & 3;                // row segment and column quad of this lane
-    // Units of this CTA: [lo, hi), column block running fastest; those of a group are dealt to the warps in turn.
+    // Units of this CTA: [lo, hi), column block running fastest.  Those of `sets` groups, a span, are dealt to the warps in
+    // turn; a span ends with a barrier.
     const uint32_t lo = (uint32_t)((uint64_t)blockIdx.x * p.total / gridDim.x);
     const uint32_t hi = (uint32_t)((uint64_t)(blockIdx.x + 1) * p.total / gridDim.x);
 
-    auto group_end = [&](uint32_t u) { return min(hi, (u / p.cblocks + 1) * p.cblocks); };
-    // u: a unit of this warp in the run that began at base -> the next one, base updated; hi when there is none
-    auto advance = [&](uint32_t u, uint32_t &base) {
-        uint32_t n = u + W;
-        while (n >= group_end(base)) {
-            base = group_end(base);
-            if (base >= hi) return hi;
-            n = base + warp;
+    struct Unit {
+        uint32_t u, grp, cb;   // unit, its group and column block; u = hi: none
+        uint32_t span;         // first group of its span
+    };
+    auto span_end = [&](uint32_t grp0) { return (uint32_t)min((uint64_t)hi, (uint64_t)(grp0 + p.sets) * p.cblocks); };
+    auto settle = [&](Unit &x) {                                // after x.u and x.cb have moved
+        for (uint32_t end = span_end(x.span); x.u >= end; end = span_end(x.span)) {
+            if (end >= hi) {
+                x.u = hi;
+                return;
+            }
+            x.span += p.sets;
+            x.u = end + warp;
+            x.grp = x.span;
+            x.cb = warp;
         }
-        return n;
+        for (; x.cb >= p.cblocks; x.cb -= p.cblocks) ++x.grp;
+    };
+    auto advance = [&](Unit &x) {
+        if (x.u >= hi) return;
+        x.u += W;
+        x.cb += W;
+        settle(x);
     };
 
-    // Lanes 0..3: byte offset and depth of the group's four tiles in unit u's tile column.
-    auto load_desc = [&](uint32_t u, uint32_t &off, uint32_t &ml) {
+    // Lanes 0..3: byte offset and depth of the group's four tiles in a unit's tile column.
+    auto load_desc = [&](const Unit &x, uint32_t &off, uint32_t &ml) {
         off = ml = 0;
-        if (u >= hi || lane >= 4) return;
-        const uint32_t grp = u / p.cblocks, ct = (u - grp * p.cblocks) >> 1, tk = 4 * (grp / subs) + lane;
+        if (x.u >= hi || lane >= 4) return;
+        const uint32_t tk = 4 * (x.grp / subs) + lane;
         if (tk >= g.tiles_k) return;
-        const size_t tile = (size_t)tk * g.tiles_n + ct;
+        const size_t tile = (size_t)tk * g.tiles_n + (x.cb >> 1);
         off = __ldg(a.tile_offsets + tile);
         if constexpr (ENTRY) {
-            ml = enter_span(__ldg(a.entry_spans + tile * subs + grp % subs), __ldg(a.tile_max_lens + tile), off);
+            ml = enter_span(__ldg(a.entry_spans + tile * subs + x.grp % subs), __ldg(a.tile_max_lens + tile), off);
         } else {
             ml = __ldg(a.tile_max_lens + tile);
         }
     };
-    auto issue = [&](uint32_t u, uint32_t stage, uint32_t off, uint32_t ml) {
-        const uint32_t hb = u % p.cblocks & 1, dst = wbase_s + stage * p.stage_bytes;
+    auto issue = [&](const Unit &x, uint32_t stage, uint32_t off, uint32_t ml) {
+        const uint32_t hb = x.cb & 1, dst = wbase_s + stage * p.stage_bytes;
         if (ml > p.cap_rows) {                                  // metadata disagrees with the declared maximum
             atomicExch(p.status, 2u);
             ml = 0;
         }
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            const uint32_t n = __shfl_sync(kFull, ml, j) * 2;
-            const uint8_t *src = a.stream + __shfl_sync(kFull, off, j) + hb * 16;
-            for (uint32_t i = lane; i < n; i += 32)             // (row i / 2, half i % 2)
-                cp_async16(dst + (i >> 1) * 128 + j * 32 + (i & 1) * 16, src + (size_t)(i >> 1) * 64 + (i & 1) * 32);
+        // byte blocks: eight lanes a row of the window, two (one a half) for every tile
+        const uint32_t n = __shfl_sync(kFull, ml, lane >> 1 & 3), from = __shfl_sync(kFull, off, lane >> 1 & 3);
+        const uint8_t *bytes = a.stream + from + hb * 16 + (lane & 1) * 32 + (lane >> 3) * 64;
+        uint32_t to = dst + lane * 16;
+        for (uint32_t r = lane >> 3; r < n; r += 4, to += 512, bytes += 256) cp_async16(to, bytes);
+        // States of the unit's 16 columns, segment by segment: four columns a lane.
+        const uint32_t grp4 = x.grp / subs, tk = 4 * grp4 + (lane >> 3);
+        if (tk < g.tiles_k) {
+            const size_t at = (((size_t)tk * g.tiles_n + (x.cb >> 1)) * subs + (ENTRY ? x.grp - grp4 * subs : 0u)) * 64 +
+                              (lane >> 2 & 1) * 32 + hb * 16 + (lane & 3) * 4;
+            const uint32_t *src = (ENTRY ? a.entry_states : a.states) + at, d = dst + st_off + lane * 16;
+            if (p.wide) {
+                cp_async16(d, src);
+            } else {
+                for (uint32_t j = 0; j < 4; ++j) cp_async4(d + 4 * j, src + j);
+            }
+            if constexpr (ENTRY) {                              // two lanes' rows are 16 bytes
+                const uint16_t *rows = a.entry_rows + at;
+                if (p.wide) {
+                    if ((lane & 1) == 0) cp_async16(dst + st_off + 512 + lane * 8, rows);
+                } else {
+                    for (uint32_t j = 0; j < 2; ++j) cp_async4(dst + st_off + 512 + lane * 8 + 4 * j, rows + 2 * j);
+                }
+            }
         }
-        cp_async_arrive(bar_base + stage * 8);
     };
-    auto issue_man = [&](uint32_t u, uint32_t c, uint32_t buf) {
-        const uint32_t grp = u / p.cblocks, cb = u - grp * p.cblocks;
-        const uint32_t row = lane & 15, h = lane >> 4;          // a lane copies one row of one half of every tile
-        if (c * kChunkRows + row < step) {
-            const uint32_t tk0 = 4 * (grp / subs), sub_row = ENTRY ? grp % subs * step : 0u;
-            const uint8_t *src = a.mantissa + (((size_t)tk0 * g.tiles_n + (cb >> 1)) * g.th + h * g.half + sub_row + c * kChunkRows + row) * 32 +
-                                 (cb & 1) * 16;
-            const uint32_t dst = man_s + (buf * 8 + h) * kT4SegPitch + row * 16;
-#pragma unroll
-            for (uint32_t j = 0; j < 4; ++j)
-                if (tk0 + j < g.tiles_k) cp_async16(dst + 2 * j * kT4SegPitch, src + (size_t)j * g.tiles_n * g.th * 32);
-        }
-        cp_async_arrive(man_bar + buf * 8);
+    // Sign+mantissa bytes: a lane copies one row of one half of every tile, 16 columns.
+    const uint32_t man_row = lane & 15, man_half = lane >> 4;
+    auto man_of = [&](const Unit &x) {
+        const uint32_t grp4 = x.grp / subs, sub_row = ENTRY ? (x.grp - grp4 * subs) * step : 0u;
+        return a.mantissa + (((size_t)4 * grp4 * g.tiles_n + (x.cb >> 1)) * g.th + man_half * g.half + sub_row + man_row) * 32 +
+               (x.cb & 1) * 16;
     };
-    // The segment whose streams this lane decodes: its own, or, where the group has no such tile, the same half of the
-    // first one (real symbols; random ones would take the branch for a second byte at every step).
-    auto seg_of = [&](uint32_t grp) { return 4 * (grp / subs) + (sg >> 1) < g.tiles_k ? sg : sg & 1; };
-    // Initial states of this lane's streams in unit u; a column beyond the matrix repeats the block's first one (its
-    // weights are finite and meet zero activations).
-    auto load_states = [&](uint32_t u, uint32_t (&s)[4], uint32_t (&rows)[4]) {
-        const uint32_t grp = u / p.cblocks, cb = u - grp * p.cblocks, tk = 4 * (grp / subs) + (seg_of(grp) >> 1);
-        rows[0] = rows[1] = rows[2] = rows[3] = 0;
-        const size_t at = (((size_t)tk * g.tiles_n + (cb >> 1)) * subs + (ENTRY ? grp % subs : 0u)) * 64 + (sg & 1) * 32 + (cb & 1) * 16;
-        const uint32_t *src = (ENTRY ? a.entry_states : a.states) + at;
+    const size_t tile_step = (size_t)g.tiles_n * g.th * 32;
+    // Rows [row, + kChunkRows) into chunk buffer `buf`; src: this lane's piece of them, `tiles` of the group exist.
+    auto issue_man = [&](const uint8_t *src, uint32_t tiles, uint32_t row, uint32_t buf) {
+        if (row + man_row >= step) return;
+        const uint32_t dst = man_s + (buf * 8 + man_half) * kT4SegPitch + man_row * 16;
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            const uint32_t c = cb * 16 + 4 * q + j < g.N ? 4 * q + j : 0u;
-            s[j] = __ldg(src + c);
-            if constexpr (ENTRY) rows[j] = min((uint32_t)__ldg(a.entry_rows + at + c), p.cap_rows - 1);
+        for (uint32_t j = 0; j < 4; ++j)
+            if (j < tiles) cp_async16(dst + 2 * j * kT4SegPitch, src + j * tile_step);
+    };
+    auto tiles_of = [&](const Unit &x) { return g.tiles_k - 4 * (x.grp / subs); };
+    // Activations of the lane's column of D, columns col .. col + 3 of the weight.
+    const uint32_t x_row = REG ? sg % MT : sg;
+    auto load_x = [&](const Unit &x, uint32_t (&xb)[2]) {
+        xb[0] = xb[1] = 0;
+        if (x.u >= hi || x_row >= a.M) return;
+        const uint32_t col = x.cb * 16 + 4 * q;
+        const uint16_t *src = a.x + (size_t)x_row * a.ldx + col;
+        if (p.x_wide) {
+            if (col < g.N) {
+                const uint2 v = __ldg(reinterpret_cast<const uint2 *>(src));
+                xb[0] = v.x;
+                xb[1] = v.y;
+            }
+            return;
         }
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            if (col + j < g.N) xb[j >> 1] |= (uint32_t)__ldg(src + j) << (16 * (j & 1));
     };
 
-    if (lane == 0) {
-        for (uint32_t i = 0; i < 4; ++i) mbar_init(bar_base + 8 * i, 32);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
-    uint32_t base = lo;
-    uint32_t u = lo + warp < group_end(lo) ? lo + warp : advance(lo + warp - W, base);
-    uint32_t nbase = base, nu = u < hi ? advance(u, nbase) : hi;
+    Unit cur{lo + warp, lo / p.cblocks, 0, lo / p.cblocks};
+    cur.cb = lo - cur.grp * p.cblocks + warp;
+    settle(cur);
+    Unit nxt = cur;
+    advance(nxt);
     uint32_t off, ml, noff, nml;
-    load_desc(u, off, ml);
-    load_desc(nu, noff, nml);
-    if (u < hi) {
-        issue(u, 0, off, ml);
-        issue_man(u, 0, 0);
+    load_desc(cur, off, ml);
+    load_desc(nxt, noff, nml);
+    const uint8_t *man = man_of(cur);                           // the sign+mantissa chunk that was asked for last
+    uint32_t man_tiles = tiles_of(cur);
+    if (cur.u < hi) {
+        issue(cur, 0, off, ml);
+        issue_man(man, man_tiles, 0, 0);
     }
     if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
@@ -161,59 +228,114 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (!wait_lut(lut_bar, a.lut)) atomicExch(p.status, 1u);
-    const bool live_m = MT == 8 ? 2 * q < a.M : q == 0;         // lanes whose two D columns are activation rows
+    const bool live_m = MT == 8 ? 2 * q < a.M : q == 0;         // !REG: lanes whose two D columns are activation rows
     const uint32_t n_chunks = (step + kChunkRows - 1) / kChunkRows;
-    uint32_t parity0 = 0, parity1 = 0, stage = 0, chunk = 0;
+    uint32_t stage = 0, chunk = 0;
+    uint32_t xb[2], nxb[2];
+    load_x(cur, xb);
     Quad z;
-    for (uint32_t run = lo; run < hi; run = group_end(run)) {   // the CTA's runs: one per group it touches
-        const uint32_t end = group_end(run), grp = run / p.cblocks;
-        for (uint32_t i = lane * 4; i < p.acc_bytes; i += 128) asm volatile("st.shared.u32 [%0], %1;" ::"r"(acc_s + i), "r"(0u) : "memory");
-        __syncwarp();
-        for (; u < end; u = nu, base = nbase, nu = u < hi ? advance(u, nbase) : hi) {
-            const uint32_t cb = u - grp * p.cblocks, col = cb * 16 + 4 * q;
-            uint32_t next_row[4];
-            load_states(u, z.s, next_row);
-            uint32_t xb[2] = {0u, 0u};                          // activations of row sg, columns col .. col + 3
-            if (sg < a.M) {
-                const uint16_t *x = a.x + (size_t)sg * a.ldx + col;
+    float sum[kT4RegChunks][4 * MT];                            // REG: [chunk][row 4q + 0..3][activation row]
+    auto zero_sums = [&]() {
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j)
-                    if (col + j < g.N) xb[j >> 1] |= (uint32_t)__ldg(x + j) << (16 * (j & 1));
+        for (uint32_t f = 0; f < kT4RegChunks; ++f)
+#pragma unroll
+            for (int i = 0; i < 4 * MT; ++i) sum[f][i] = 0.f;
+    };
+    auto turn_sums = [&]() {
+#pragma unroll
+        for (int i = 0; i < 4 * MT; ++i) {
+            const float t = sum[0][i];
+#pragma unroll
+            for (uint32_t f = 0; f + 1 < kT4RegChunks; ++f) sum[f][i] = sum[f + 1][i];
+            sum[kT4RegChunks - 1][i] = t;
+        }
+    };
+    auto store_sums = [&](uint32_t set) {
+#pragma unroll
+        for (uint32_t f = 0; f < kT4RegChunks; ++f)
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const uint32_t r = f * kChunkRows + 4 * q + i;
+                if (r < step) {
+#pragma unroll
+                    for (uint32_t m = 0; m < MT; ++m)
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(acc_s + set * set_bytes + sg * seg_acc + (r * MT + m) * 4),
+                                     "f"(sum[f][i * MT + m]) : "memory");
+                }
             }
-            const uint32_t sd = seg_of(grp), my_ml = __shfl_sync(kFull, ml, sd >> 1);
+    };
+    for (uint32_t run = lo; run < hi;) {                        // the CTA's spans
+        const uint32_t grp0 = run / p.cblocks, end = span_end(grp0), n_sets = (end - 1) / p.cblocks - grp0 + 1;
+        uint32_t set = 0;                                       // REG: whose sums the registers hold
+        if constexpr (REG) {
+            zero_sums();
+        } else {
+            for (uint32_t k = 0; k < n_sets; ++k)
+                for (uint32_t i = lane * 4; i < p.acc_bytes; i += 128)
+                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(acc_s + k * set_bytes + i), "r"(0u) : "memory");
+            __syncwarp();
+        }
+        while (cur.u < end) {
+            if constexpr (REG) {
+                for (; set < cur.grp - grp0; ++set) {
+                    store_sums(set);
+                    zero_sums();
+                }
+            }
+            load_x(nxt, nxb);
+            // The segment whose streams this lane decodes: its own, or, where the group has no such tile, the same half of the
+            // first one (real symbols; random ones would take the branch for a second byte at every step).
+            const uint32_t sd = 4 * (cur.grp / subs) + (sg >> 1) < g.tiles_k ? sg : sg & 1;
+            const uint32_t my_ml = __shfl_sync(kFull, ml, sd >> 1), col = cur.cb * 16 + 4 * q;
             const uint32_t win_s = wbase_s + stage * p.stage_bytes;
             const uint32_t first = win_s + (!ENTRY && my_ml <= p.cap_rows ? my_ml - 1 : 0u) * 128 + sd * 16;
+            cp_async_wait();                                    // this unit's bytes and states, its first sign+mantissa chunk
+            __syncwarp();
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) z.p[j] = first + next_row[j] * 128 + (col + j < g.N ? 4 * q + j : 0u);
-            if (!mbar_wait(bar_base + stage * 8, stage ? parity1 : parity0)) atomicExch(p.status, 1u);
-            if (stage) parity1 ^= 1; else parity0 ^= 1;
+            for (uint32_t j = 0; j < 4; ++j) {
+                // a column beyond the matrix repeats the block's first one (its weights are finite and meet zero activations)
+                const uint32_t c = col + j < g.N ? 4 * q + j : 0u;
+                z.s[j] = lds_u32(win_s + st_off + sd * 64 + c * 4);
+                z.p[j] = first + c;
+                if constexpr (ENTRY) z.p[j] += min(lds_u16(win_s + st_off + 512 + sd * 32 + c * 2), p.cap_rows - 1) * 128;
+            }
             auto next_unit = [&]() {
                 off = noff;
                 ml = nml;
-                if (nu >= hi) return;
-                issue(nu, p.stages == 2 ? stage ^ 1 : 0u, off, ml);
-                uint32_t b2 = nbase;
-                load_desc(advance(nu, b2), noff, nml);
+                if (nxt.u >= hi) return;
+                issue(nxt, p.stages == 2 ? stage ^ 1 : 0u, off, ml);
+                Unit after = nxt;
+                advance(after);
+                load_desc(after, noff, nml);
             };
-            uint32_t ac = acc_s + sg * seg_acc + (MT == 8 ? q * 8 : 0u);
+            uint32_t ac = acc_s + (REG ? 0u : (cur.grp - grp0) * set_bytes) + sg * seg_acc + (MT == 8 ? q * 8 : 0u);
 #pragma unroll 1
             for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
                 const uint32_t buf = chunk & 1;
-                __syncwarp();                                   // every lane is done with the other buffers
-                if (c + 1 < n_chunks) issue_man(u, c + 1, buf ^ 1);
-                else if (nu < hi) issue_man(nu, 0, buf ^ 1);
-                if (c == 0 && p.stages == 2) next_unit();       // behind it: a chunk's arrival waits for older copies
-                if (!mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1)) atomicExch(p.status, 1u);
+                if (c != 0) {
+                    cp_async_wait();                            // this chunk is here
+                    __syncwarp();                               // for every lane, and all are done with the other buffer
+                }
+                const bool last = c + 1 == n_chunks;
+                if (last) {                                     // the next unit's first chunk
+                    man = man_of(nxt);
+                    man_tiles = tiles_of(nxt);
+                } else {
+                    man += kChunkRows * 32;
+                }
+                if (!last || nxt.u < hi) issue_man(man, man_tiles, last ? 0u : (c + 1) * kChunkRows, buf ^ 1);
+                if (c == 0 && p.stages == 2) next_unit();
                 z.clamp(win_s);
                 uint32_t ms = man_s + (buf * 8 + sg) * kT4SegPitch + q * 4;
                 const uint32_t n = min(kChunkRows, step - c * kChunkRows);
 #pragma unroll 1
                 for (uint32_t r = 0; r < n; r += 4) {
+                    const bool mine = q == r >> 2;              // REG
 #pragma unroll
                     for (uint32_t i = 0; i < 4; i += 2) {
                         float d[4] = {0.f, 0.f, 0.f, 0.f};
                         const uint32_t ad = ac + i * (MT * 4);
-                        if (live_m) {
+                        if (!REG && live_m) {
                             if constexpr (MT == 1) {
                                 d[0] = __uint_as_float(lds_u32(ad));
                                 d[2] = __uint_as_float(lds_u32(ad + 4));
@@ -226,26 +348,42 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
 #pragma unroll
                         for (uint32_t k = 0; k < 2; ++k) {      // rows i, i + 1: columns 0, 1 and 2, 3 of the lane
                             uint32_t e[4];
-                            z.step(lut_s, e);
+                            if constexpr (REG) z.step_together(lut_s, e);
+                            else z.step(lut_s, e);
                             const uint32_t m = lds_u32(ms + (i + k) * 16);
                             const uint32_t e01 = __byte_perm(e[0], e[1], 0x6521) << 3, e23 = __byte_perm(e[2], e[3], 0x6521) << 3;
                             w[k] = exp_or_man(e01, __byte_perm(m, 0u, 0x1100));
                             w[2 + k] = exp_or_man(e23, __byte_perm(m, 0u, 0x3322));
                         }
-                        mma_bf16(d, w, xb[0], xb[1]);
-                        if (live_m) {
-                            if constexpr (MT == 1) {
-                                asm volatile("st.shared.f32 [%0], %1;" ::"r"(ad), "f"(d[0]) : "memory");
-                                asm volatile("st.shared.f32 [%0], %1;" ::"r"(ad + 4), "f"(d[2]) : "memory");
-                            } else {
-                                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ad), "f"(d[0]), "f"(d[1]) : "memory");
-                                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ad + MT * 4), "f"(d[2]), "f"(d[3]) : "memory");
+                        if constexpr (REG) {
+                            mma_bf16_zero(d, w, xb[0], xb[1]);
+                            if (mine) {
+#pragma unroll
+                                for (int m = 0; m < MT; ++m) {
+                                    sum[0][i * MT + m] += d[m];
+                                    sum[0][(i + 1) * MT + m] += d[2 + m];
+                                }
+                            }
+                        } else {
+                            mma_bf16(d, w, xb[0], xb[1]);
+                            if (live_m) {
+                                if constexpr (MT == 1) {
+                                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(ad), "f"(d[0]) : "memory");
+                                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(ad + 4), "f"(d[2]) : "memory");
+                                } else {
+                                    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ad), "f"(d[0]), "f"(d[1]) : "memory");
+                                    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ad + MT * 4), "f"(d[2]), "f"(d[3]) : "memory");
+                                }
                             }
                         }
                     }
                     ac += 4 * (MT * 4);
                     ms += 64;
                 }
+                if constexpr (REG) turn_sums();
+            }
+            if constexpr (REG) {
+                for (uint32_t c = n_chunks; c < kT4RegChunks; ++c) turn_sums();
             }
             if (p.stages == 2) {
                 stage ^= 1;
@@ -253,53 +391,67 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
                 __syncwarp();                                   // every lane is done with the only window
                 next_unit();
             }
+            cur = nxt;
+            advance(nxt);
+            xb[0] = nxb[0];
+            xb[1] = nxb[1];
         }
-        // ---- the group's sums of this CTA ------------------------------------------------------------------
-        __syncthreads();
-        const uint32_t rows = 8 * step, first_cta = (uint32_t)(((uint64_t)(grp * p.cblocks + 1) * gridDim.x - 1) / p.total);
-        const uint32_t last_cta = (uint32_t)(((uint64_t)min((grp + 1) * p.cblocks, p.total) * gridDim.x - 1) / p.total);
-        const uint32_t count = last_cta - first_cta + 1;
-        // row r of the group = row r % step of its segment r / step
-        auto out_row = [&](uint32_t r) {
-            const uint32_t seg = r / step;
-            return (4 * (grp / subs) * 2 + seg) * g.half + (ENTRY ? grp % subs * step : 0u) + r - seg * step;
-        };
-        float *mine = a.partial + (size_t)(blockIdx.x + grp) * rows * a.M;
-        for (uint32_t i = threadIdx.x; i < rows * a.M; i += blockDim.x) {
-            const uint32_t m = i / rows, r = i - m * rows, seg = r / step, v = out_row(r);
-            const uint32_t at = acc0_s + seg * seg_acc + (r - seg * step) * (MT * 4) + m * 4;
-            float sum = 0.f;
-            for (uint32_t w = 0; w < W; ++w) sum += __uint_as_float(lds_u32(at + w * p.acc_bytes));
-            if (count > 1) {
-                mine[i] = sum;
-            } else if (v < g.K) {
-                if (a.bias) sum += load_bf16(a.bias + v);
-                a.y[(size_t)m * a.ldy + v] = float_to_bf16_bits(sum);
+        if constexpr (REG) {
+            for (; set < n_sets; ++set) {
+                store_sums(set);
+                zero_sums();
             }
         }
-        if (count > 1) {
-            if (last_arrival(a.tickets + grp, count, &s_flag)) {
-                for (uint32_t i = threadIdx.x; i < rows * a.M; i += blockDim.x) {
-                    const uint32_t m = i / rows, v = out_row(i - m * rows);
-                    if (v >= g.K) continue;
-                    float sum = 0.f;
-                    for (uint32_t c = first_cta; c <= last_cta; ++c) sum += __ldcg(a.partial + (size_t)(c + grp) * rows * a.M + i);
-                    if (a.bias) sum += load_bf16(a.bias + v);
-                    a.y[(size_t)m * a.ldy + v] = float_to_bf16_bits(sum);
+        // ---- the span's sums of this CTA, group by group -----------------------------------------------------
+        __syncthreads();
+        for (uint32_t k = 0; k < n_sets; ++k) {
+            const uint32_t grp = grp0 + k, rows = 8 * step;
+            const uint32_t first_cta = (uint32_t)(((uint64_t)(grp * p.cblocks + 1) * gridDim.x - 1) / p.total);
+            const uint32_t last_cta = (uint32_t)(((uint64_t)min((grp + 1) * p.cblocks, p.total) * gridDim.x - 1) / p.total);
+            const uint32_t count = last_cta - first_cta + 1;
+            // row r of the group = row r % step of its segment r / step
+            auto out_row = [&](uint32_t r) {
+                const uint32_t seg = r / step;
+                return (4 * (grp / subs) * 2 + seg) * g.half + (ENTRY ? grp % subs * step : 0u) + r - seg * step;
+            };
+            float *mine = a.partial + (size_t)(blockIdx.x + grp) * rows * a.M;
+            for (uint32_t i = threadIdx.x; i < rows * a.M; i += blockDim.x) {
+                const uint32_t m = i / rows, r = i - m * rows, seg = r / step, v = out_row(r);
+                const uint32_t at = acc0_s + k * set_bytes + seg * seg_acc + (r - seg * step) * (MT * 4) + m * 4;
+                float total = 0.f;
+                for (uint32_t w = 0; w < W; ++w) total += __uint_as_float(lds_u32(at + w * p.acc_bytes));
+                if (count > 1) {
+                    mine[i] = total;
+                } else if (v < g.K) {
+                    if (a.bias) total += load_bf16(a.bias + v);
+                    a.y[(size_t)m * a.ldy + v] = float_to_bf16_bits(total);
                 }
-                if (threadIdx.x == 0) a.tickets[grp] = 0;       // ready for the next call
+            }
+            if (count > 1) {
+                if (last_arrival(a.tickets + grp, count, s_flag)) {
+                    for (uint32_t i = threadIdx.x; i < rows * a.M; i += blockDim.x) {
+                        const uint32_t m = i / rows, v = out_row(i - m * rows);
+                        if (v >= g.K) continue;
+                        float total = 0.f;
+                        for (uint32_t c = first_cta; c <= last_cta; ++c) total += __ldcg(a.partial + (size_t)(c + grp) * rows * a.M + i);
+                        if (a.bias) total += load_bf16(a.bias + v);
+                        a.y[(size_t)m * a.ldy + v] = float_to_bf16_bits(total);
+                    }
+                    if (threadIdx.x == 0) a.tickets[grp] = 0;   // ready for the next call
+                }
             }
         }
         __syncthreads();                                        // the sums may be cleared
+        run = end;
     }
 }
 
 // ------------------------------------------------------------------------ host
 
-template <int MT, bool ENTRY>
+template <int MT, bool ENTRY, bool REG>
 static int launch_t4_pass(T4Args p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, cudaStream_t s) {
     static SmemLimit lim = {};
-    if (int rc = ensure_smem_limit(lim, (const void *)k_linear_t4<MT, ENTRY>, (size_t)max_smem - 1024)) return rc;
+    if (int rc = ensure_smem_limit(lim, (const void *)k_linear_t4<MT, ENTRY, REG>, (size_t)max_smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(warps * 32);
@@ -310,7 +462,7 @@ static int launch_t4_pass(T4Args p, uint32_t blocks, uint32_t warps, size_t smem
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CI_CUDA(cudaLaunchKernelEx(&cfg, k_linear_t4<MT, ENTRY>, p));
+    CI_CUDA(cudaLaunchKernelEx(&cfg, k_linear_t4<MT, ENTRY, REG>, p));
     return CI_OK;
 }
 
@@ -325,7 +477,7 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
     if ((reinterpret_cast<uintptr_t>(a.stream) & 15u) || (reinterpret_cast<uintptr_t>(a.mantissa) & 15u)) return 1;
     if (partial_capacity < linear_t4_workspace_bytes(a.M, g.K, g.th)) return 1;
     const bool entry = a.entry_step != 0 && a.entry_cap != 0 && g.half > a.entry_step && g.half % a.entry_step == 0 &&
-                       a.entry_step % kChunkRows == 0;
+                       a.entry_step % kChunkRows == 0 && (reinterpret_cast<uintptr_t>(a.entry_rows) & 3u) == 0;
     const uint32_t step = entry ? a.entry_step : g.half, subs = g.half / step, groups = (g.tiles_k + 3) / 4 * subs;
     if (groups >= kTicketBytes - 1) return 1;
     int dev = 0, max_smem = 0;
@@ -335,51 +487,62 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
     p.cap_rows = entry ? a.entry_cap : max_tile_len;
     p.step = step;
     p.subs = subs;
-    p.stage_bytes = p.cap_rows * 128u;
+    p.stage_bytes = p.cap_rows * 128u + (entry ? 768u : 512u);
     p.cblocks = (g.N + 15) / 16;
     p.total = groups * p.cblocks;
     p.status = a.tickets + (kTicketBytes - 1);
-    const uint32_t P = (uint32_t)sm_count(), fixed = 2 * kLutBytes + kT4BarBytes + 1024, room = (uint32_t)max_smem - fixed;
+    p.wide = ((entry ? reinterpret_cast<uintptr_t>(a.entry_states) | reinterpret_cast<uintptr_t>(a.entry_rows)
+                     : reinterpret_cast<uintptr_t>(a.states)) & 15u) == 0;
+    const uint32_t P = (uint32_t)sm_count(), fixed = 2 * kLutBytes + kT4BarBytes, room = (uint32_t)max_smem - fixed;
     const uint32_t blocks = p.total < P ? p.total : P;
     // Passes over the weight x rounds of units: sums for eight activation rows take eight times the shared memory of one,
-    // which a tall tile cannot afford at a useful number of warps.  The units of a CTA count as one sequence here, without the
-    // barrier that ends each of its groups: at 32000 x 4096 and tile height 128, 47 of 148 CTAs take 8 rounds for 6.8 rounds of work.
+    // which a tall tile cannot afford at a useful number of warps.  Two sets of sums where there is room: a CTA with the units
+    // of two groups then deals them out as one sequence, and without a second one rounds its units up in each.
+    const uint32_t units = (p.total + blocks - 1) / blocks;
+    uint32_t front = 0;
+    if (int rc = front_bytes(dev, front)) return rc;
+    front /= kT4ManBytes;
     uint32_t warps = 0, rows_per_pass = 0;
     double best = 0.0;
     for (uint32_t mt = 1; mt <= 8; mt = mt == 2 ? 8 : mt * 2)
-        for (uint32_t stages = 1; stages <= 2; ++stages) {
-            const uint32_t acc = (8 * (step * (mt * 4) + (mt == 8 ? 32 : mt * 4)) + 15) & ~15u;
-            const uint32_t warp_bytes = stages * p.stage_bytes + kT4ManBytes + acc;
-            uint32_t w_max = room / warp_bytes;
-            if (w_max > kT4Warps) w_max = kT4Warps;
-            for (uint32_t w = 1; w <= w_max; ++w) {
-                const double cost = (double)((a.M + mt - 1) / mt) * run_cost((p.total + blocks - 1) / blocks, w, 0.0) *
-                                    (stages == 1 ? 1.02 : 1.0);
-                if (warps == 0 || cost < best) {
-                    best = cost;
-                    warps = w;
-                    rows_per_pass = mt;
-                    p.stages = stages;
-                    p.acc_bytes = acc;
+        for (uint32_t stages = 1; stages <= 2; ++stages)
+            for (uint32_t sets = 1; sets <= (mt == 8 ? 1u : 2u); ++sets) {
+                const uint32_t acc = (8 * (step * (mt * 4) + (mt == 8 ? 32 : mt * 4)) + 15) & ~15u;
+                const uint32_t own = stages * p.stage_bytes + sets * acc;
+                uint32_t w_max = (room + front * kT4ManBytes) / (own + kT4ManBytes);
+                if (w_max < front) w_max = room / own;
+                if (w_max > kT4Warps) w_max = kT4Warps;
+                for (uint32_t w = 1; w <= w_max; ++w) {
+                    const bool split = groups > 1 && (sets == 1 || units > p.cblocks);   // some CTA's units end in two rounds
+                    const double cost = (double)((a.M + mt - 1) / mt) *
+                                        (run_cost(units, w, 0.0) + (split ? 0.5 * round_cost(w, 0.0) : 0.0)) * (stages == 1 ? 1.02 : 1.0);
+                    if (warps == 0 || cost < best) {
+                        best = cost;
+                        warps = w;
+                        rows_per_pass = mt;
+                        p.stages = stages;
+                        p.sets = sets;
+                        p.front = w < front ? w : front;
+                        p.acc_bytes = acc;
+                    }
                 }
             }
-        }
     if (warps == 0) return 1;
-    const size_t smem = fixed - 1024 + (size_t)warps * (p.stages * p.stage_bytes + kT4ManBytes + p.acc_bytes);
+    const size_t smem = fixed + (size_t)warps * (p.stages * p.stage_bytes + p.sets * p.acc_bytes) + (size_t)(warps - p.front) * kT4ManBytes;
     for (uint32_t m0 = 0; m0 < a.M; m0 += rows_per_pass) {
         p.a = a;
         p.a.x = a.x + (size_t)m0 * a.ldx;
         p.a.y = a.y + (size_t)m0 * a.ldy;
+        p.x_wide = ((reinterpret_cast<uintptr_t>(p.a.x) & 7u) == 0 && (a.ldx & 3) == 0 && g.N % 4 == 0) ? 1u : 0u;
         p.a.M = a.M - m0 < rows_per_pass ? a.M - m0 : rows_per_pass;
-        int rc;
-        if (entry)
-            rc = rows_per_pass == 1   ? launch_t4_pass<1, true>(p, blocks, warps, smem, max_smem, s)
-                 : rows_per_pass == 2 ? launch_t4_pass<2, true>(p, blocks, warps, smem, max_smem, s)
-                                      : launch_t4_pass<8, true>(p, blocks, warps, smem, max_smem, s);
-        else
-            rc = rows_per_pass == 1   ? launch_t4_pass<1, false>(p, blocks, warps, smem, max_smem, s)
-                 : rows_per_pass == 2 ? launch_t4_pass<2, false>(p, blocks, warps, smem, max_smem, s)
-                                      : launch_t4_pass<8, false>(p, blocks, warps, smem, max_smem, s);
+        using Pass = int (*)(T4Args, uint32_t, uint32_t, size_t, int, cudaStream_t);
+        static const Pass pass[2][5] = {
+            {launch_t4_pass<1, false, true>, launch_t4_pass<2, false, true>, launch_t4_pass<1, false, false>,
+             launch_t4_pass<2, false, false>, launch_t4_pass<8, false, false>},
+            {launch_t4_pass<1, true, true>, launch_t4_pass<2, true, true>, launch_t4_pass<1, true, false>,
+             launch_t4_pass<2, true, false>, launch_t4_pass<8, true, false>}};
+        const bool reg = step <= kT4RegChunks * kChunkRows;
+        const int rc = pass[entry][rows_per_pass == 8 ? 4 : rows_per_pass - 1 + (reg ? 0 : 2)](p, blocks, warps, smem, max_smem, s);
         if (rc) return rc;
     }
     return CI_OK;
