@@ -13,7 +13,7 @@
 //    were the kernel's largest stall (1.9 of 6 cycles per instruction) and four wavefronts a row;
 //  * a decoded row of the lane is four adjacent weights: one 8-byte store (4 bytes for the plane), and the
 //    sixteen lanes of a half write 128 contiguous bytes of an output row.
-// Initial states arrive by bulk copy with the unit, byte ranges of later units are loaded ahead by all
+// Initial states arrive with the unit's bytes, byte ranges of later units are loaded ahead by all
 // lanes in parallel, windows are double buffered per warp where they fit (tall tiles: one window), and the kernel is
 // launched with programmatic dependent launch (its preamble overlaps the previous kernel of the stream).
 #include "decode.cuh"
@@ -22,7 +22,7 @@
 namespace ci {
 
 constexpr uint32_t kDec4Warps = 21;          // six on one scheduler: 80 registers a thread, which it needs (none spilled)
-constexpr uint32_t kDec4BarBytes = 768;      // up to 21 warps x (2 window stages + 2 mantissa chunks) x 8 B, the table's
+constexpr uint32_t kDec4BarBytes = 128;      // the table's barrier
 
 struct Dec4Args {
     DecArgs a;
@@ -58,7 +58,6 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     start_lut(lut_s, lut_bar, a.lut);
     const uint32_t man_s = lut_s + kLutBytes + kDec4BarBytes + (BF16 ? warp * kManBytes : 0);
     const uint32_t wbase_s = lut_s + kLutBytes + kDec4BarBytes + (BF16 ? W * kManBytes : 0) + warp * p.stages * p.stage_bytes;
-    const uint32_t bar_base = lut_s + kLutBytes + warp * 32, man_bar = bar_base + 16;
     const uint32_t st_off = p.cap_rows * 128;
     const uint32_t seg_bytes = g.th * 16;                       // half a tile of sign+mantissa bytes
 
@@ -105,37 +104,33 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     };
 
     auto issue = [&](uint32_t t0, uint32_t sub, bool two, uint32_t stage, uint32_t off0, uint32_t ml0, uint32_t off1, uint32_t ml1) {
-        const uint32_t bar = bar_base + stage * 8;
         const uint32_t dst = wbase_s + stage * p.stage_bytes;
         if (ml0 > p.cap_rows || ml1 > p.cap_rows) ml0 = ml1 = 0;   // metadata disagrees with the declared maximum
-        if (lane == 0) {
-            fence_async_proxy();
-            if constexpr (ENTRY) {
-                const size_t e0 = ((size_t)t0 * subs + sub) * 64, e1 = e0 + (size_t)subs * 64;
-                mbar_expect_tx(bar, two ? 768u : 384u);
-                bulk_load(dst + st_off, p.entry_states + e0, 256, bar);
-                bulk_load(dst + st_off + 512, p.entry_rows + e0, 128, bar);
-                if (two) {
-                    bulk_load(dst + st_off + 256, p.entry_states + e1, 256, bar);
-                    bulk_load(dst + st_off + 640, p.entry_rows + e1, 128, bar);
-                }
-            } else {
-                mbar_expect_tx(bar, two ? 512u : 256u);
-                bulk_load(dst + st_off, a.states + (size_t)t0 * 64, two ? 512u : 256u, bar);   // the tiles are neighbours
-            }
+        // states, 16 lanes a tile, and for entry points the rows of the next bytes, 8 lanes a tile
+        if constexpr (ENTRY) {
+            const size_t e = ((size_t)t0 * subs + sub) * 64, d = (size_t)subs * 64;
+            if (lane < 16 || two) cp_async16(dst + st_off + lane * 16, p.entry_states + e + (lane < 16 ? 0 : d) + (lane & 15) * 4);
+            if (lane < 8 || (two && lane < 16))
+                cp_async16(dst + st_off + 512 + lane * 16, p.entry_rows + e + (lane < 8 ? 0 : d) + (lane & 7) * 8);
+        } else {
+            if (lane < 16 || two) cp_async16(dst + st_off + lane * 16, a.states + (size_t)t0 * 64 + lane * 4);   // the tiles are neighbours
         }
-        const uint8_t *s0 = a.stream + off0, *s1 = a.stream + off1;
-        for (uint32_t i = lane; i < ml0 * 4; i += 32) cp_async16(dst + (i >> 2) * 128 + (i & 3) * 16, s0 + i * 16);
-        for (uint32_t i = lane; i < ml1 * 4; i += 32) cp_async16(dst + (i >> 2) * 128 + 64 + (i & 3) * 16, s1 + i * 16);
-        cp_async_arrive(bar);
+        // byte blocks: eight lanes a row of the window, four for each tile
+        const bool right = lane & 4;
+        const uint8_t *src = a.stream + (right ? off1 : off0) + (lane & 3) * 16 + (lane >> 3) * 64;
+        const uint32_t rows = right ? ml1 : ml0;
+        uint32_t to = dst + lane * 16;
+        for (uint32_t r = lane >> 3; r < rows; r += 4, to += 512, src += 256) cp_async16(to, src);
     };
-    // Sign+mantissa rows [kChunkRows * c, + kChunkRows) of the segments (left A, left B, right A, right B) of the unit whose
-    // first tile is t0.
-    auto issue_man = [&](uint32_t t0, uint32_t sub, bool two, uint32_t c, uint32_t buf) {
-        const uint8_t *src = a.mantissa + (size_t)t0 * (2 * seg_bytes) + (ENTRY ? sub * step * 32 : 0u) +
-                             c * (kChunkRows * 32) + lane * 16;
+    // Sign+mantissa bytes of the segments (left A, left B, right A, right B) of the unit whose first tile is t0: this lane's
+    // piece of the first chunk.
+    auto man_of = [&](uint32_t t0, uint32_t sub) {
+        return a.mantissa + (size_t)t0 * (2 * seg_bytes) + (ENTRY ? sub * step * 32 : 0u) + lane * 16;
+    };
+    // Rows [row, + kChunkRows) of the four segments into chunk buffer `buf`; src: this lane's piece of them.
+    auto issue_man = [&](const uint8_t *src, bool two, uint32_t row, uint32_t buf) {
         const uint32_t dst = man_s + buf * (4 * kSegPitch) + lane * 16;
-        if (c * kChunkRows + (lane >> 1) < step) {
+        if (row + (lane >> 1) < step) {
             cp_async16(dst, src);
             cp_async16(dst + kSegPitch, src + seg_bytes);
             if (two) {
@@ -143,17 +138,8 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
                 cp_async16(dst + 3 * kSegPitch, src + 3 * seg_bytes);
             }
         }
-        cp_async_arrive(man_bar + buf * 8);
     };
 
-    if (lane == 0) {
-        mbar_init(bar_base, 33);                                // 32 cp.async arrivals + the bulk copy's expect_tx
-        mbar_init(bar_base + 8, 33);
-        mbar_init(man_bar, 32);
-        mbar_init(man_bar + 8, 32);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
     load_desc();
     uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
     uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
@@ -162,7 +148,7 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
     if (gw < p.total) {
         unit_tiles(gw, tk, sub, tp, t0, two);
         issue(t0, sub, two, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
-        if (BF16) issue_man(t0, sub, two, 0, 0);
+        if (BF16) issue_man(man_of(t0, sub), two, 0, 0);
     }
     if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
@@ -173,7 +159,8 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
 
     (void)wait_lut(lut_bar, a.lut);
     const uint32_t n_chunks = (step + kChunkRows - 1) / kChunkRows;
-    uint32_t parity0 = 0, parity1 = 0, stage = 0, li = 0, chunk = 0;
+    uint32_t stage = 0, li = 0, chunk = 0;
+    const uint8_t *man = BF16 ? man_of(t0, sub) : nullptr;      // the sign+mantissa chunk that was asked for last
     Quad z;
 
     for (uint32_t t = gw; t < p.total; t += n_warps, ++li) {
@@ -222,8 +209,8 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
         const uint32_t st_s = win_s + st_off + tsel_d * 256 + (hsel_d * 32 + quad_d * 4) * 4;
         uint32_t first = win_s + tsel_d * 64 + hsel_d * 32 + quad_d * 4;
         if (!ENTRY && ml <= p.cap_rows) first += (ml - 1) * 128;  // last byte row; an empty tile starts one row below
-        (void)mbar_wait(bar_base + stage * 8, stage ? parity1 : parity0);
-        if (stage) parity1 ^= 1; else parity0 ^= 1;
+        cp_async_wait();                                        // this unit's bytes and states, its first sign+mantissa chunk
+        __syncwarp();
         auto start_streams = [&]() {
             z.start(st_s, first);
             if constexpr (ENTRY) {                              // every stream has its own row of the window
@@ -243,13 +230,16 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
 #pragma unroll 1
         for (uint32_t c = 0; c < n_chunks; ++c, ++chunk) {
             const uint32_t buf = chunk & 1;
-            __syncwarp();                                       // every lane is done with the other buffers
-            if (BF16) {
-                if (c + 1 < n_chunks) issue_man(t0, sub, two, c + 1, buf ^ 1);
-                else if (more) issue_man(n_t0, n_sub, n_two, 0, buf ^ 1);
+            if (BF16 && c != 0) {
+                cp_async_wait();                                // this chunk is here
+                __syncwarp();                                   // for every lane, and all are done with the other buffer
             }
-            if (c == 0 && p.stages == 2) next_unit();           // behind it: a chunk's arrival waits for older copies
-            if (BF16) (void)mbar_wait(man_bar + buf * 8, (chunk >> 1) & 1);
+            if constexpr (BF16) {
+                const bool last = c + 1 == n_chunks;
+                man = last ? man_of(n_t0, n_sub) : man + kChunkRows * 32;
+                if (!last || more) issue_man(man, last ? n_two : two, last ? 0u : (c + 1) * kChunkRows, buf ^ 1);
+            }
+            if (c == 0 && p.stages == 2) next_unit();
             if constexpr (INDEX) {
                 if (c * kChunkRows % p.step == 0 && tile_live) {
                     const size_t at = (((size_t)t0 + tsel) * p.subs + c * kChunkRows / p.step) * 64 + hsel * 32 + (quad & 7) * 4;

@@ -213,10 +213,12 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
         } else {
             if (!lower || two) cp_async16(dst + st_off + lane * 16, a.states + (size_t)(t0 + (lower ? g.tiles_n : 0u)) * 64 + (lane & 15) * 4);
         }
-        // byte blocks: 16-byte pieces, piece i of a tile = (row i / 4, quarter i % 4)
-        const uint8_t *s0 = a.stream + off0, *s1 = a.stream + off1;
-        for (uint32_t i = lane; i < ml0 * 4; i += 32) cp_async16(dst + (i >> 2) * 128 + (i & 3) * 16, s0 + i * 16);
-        for (uint32_t i = lane; i < ml1 * 4; i += 32) cp_async16(dst + (i >> 2) * 128 + 64 + (i & 3) * 16, s1 + i * 16);
+        // byte blocks: eight lanes a row of the window, four for each tile
+        const bool low_tile = lane & 4;
+        const uint8_t *src = a.stream + (low_tile ? off1 : off0) + (lane & 3) * 16 + (lane >> 3) * 64;
+        const uint32_t rows = low_tile ? ml1 : ml0;
+        uint32_t to = dst + lane * 16;
+        for (uint32_t r = lane >> 3; r < rows; r += 4, to += 512, src += 256) cp_async16(to, src);
     };
 
     // Sign+mantissa bytes of a unit's upper tile, this lane's 16-byte piece of every chunk row pair.
