@@ -129,7 +129,8 @@ int ci_embedding(const ci_tiled_weight *w, const int64_t *d_ids, uint64_t n_ids,
         a.entry_rows = w->entry_rows;
         a.entry_spans = w->entry_spans;
     }
-    rc = launch_embedding4(a, w->max_tile_len, (cudaStream_t)stream);  // 32-wide tiles: four streams per lane
+    rc = launch_embedding_group(a, w->max_tile_len, (cudaStream_t)stream);     // 32-wide tiles: four streams per lane
+    if (rc == 1) rc = launch_embedding4(a, w->max_tile_len, (cudaStream_t)stream);
     if (rc <= 0) return rc;
     uint64_t tasks = n_ids * a.g.groups, blocks = (tasks + kEmbWarps - 1) / kEmbWarps, cap = (uint64_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;

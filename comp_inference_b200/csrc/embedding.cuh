@@ -22,5 +22,7 @@ struct EmbArgs {
 // Four-streams-per-lane gather for 32-wide tiles (embedding4.cu): CI_OK when launched, 1 when the
 // table does not qualify (the caller then uses the generic kernel), < 0 on error.
 int launch_embedding4(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t s);
+// The same for many ids at a time (embedding_group.cu); same return convention.
+int launch_embedding_group(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t s);
 
 }  // namespace ci

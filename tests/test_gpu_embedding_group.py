@@ -1,0 +1,34 @@
+"""The row gather where ids share streams (embedding_group.cu): exact, whatever the ids and however they are spread."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("V,H,th", [
+    (4000, 512, 64),       # 32 rows a bin
+    (4001, 1100, 128),     # columns beyond the matrix, the last tile not whole
+    (9000, 260, 1024),     # entry points
+    (16000, 2048, 16),     # eight rows a bin
+])
+@pytest.mark.parametrize("ids", ["spread", "sorted", "one", "few", "invalid", "most"])
+def test_grouped_gather(V, H, th, ids):
+    import comp_inference_b200 as ci
+    g = torch.Generator("cuda").manual_seed(V)
+    W = (torch.randn(V, H, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    c = ci.compress_weight_cuda(W, th, 32)
+    m = ci.RansEmbedding(V, H, c["tile_height"], 32).load_compressed(c).prepare()
+    n = 4096 if ids != "most" else 9001                 # three launches, the last one short
+    i = torch.randint(0, V, (n,), generator=g, device="cuda")
+    if ids == "sorted":
+        i = i.sort().values
+    elif ids == "one":
+        i[:] = V - 1                                    # one bin of all ids
+    elif ids == "few":
+        i = i % 200 * (V // 200)                        # bins of one row and 20 ids, and of several
+    elif ids == "invalid":
+        i[::3], i[1::7] = -1, V                         # a bin of ids outside the table
+    out = m(i)
+    ok = (i >= 0) & (i < V)
+    want = torch.where(ok[:, None], W[i.clamp(0, V - 1)], torch.zeros((), dtype=torch.bfloat16, device="cuda"))
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
