@@ -65,6 +65,28 @@ struct Pair {
             : "+r"(s[0]), "+r"(s[1]), "+r"(p[0]), "+r"(p[1])
             : "r"(y0), "r"(y1));
     }
+    // The same with the second bytes loaded ahead too, see Quad::step_ahead.
+    __device__ __forceinline__ void step_ahead(uint32_t lut_s, uint32_t (&e)[2]) {
+        uint32_t y[2], v[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            y[j] = lds_u8(p[j]);
+            v[j] = lds_u8(p[j] - 64);
+        }
+        e[0] = decode_aligned(s[0], lut_s);
+        e[1] = decode_aligned(s[1], lut_s);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            asm("{\n\t.reg .pred p, q;\n\t"
+                "setp.lt.u32 p, %0, 65536;\n\t"
+                "setp.lt.u32 q, %0, 256;\n\t"
+                "@p mad.lo.u32 %0, %0, 256, %2;\n\t"
+                "@p sub.u32 %1, %1, 64;\n\t"
+                "@q mad.lo.u32 %0, %0, 256, %3;\n\t"
+                "@q sub.u32 %1, %1, 64;\n\t}"
+                : "+r"(s[j]), "+r"(p[j])
+                : "r"(y[j]), "r"(v[j]));
+    }
     __device__ __forceinline__ void clamp(uint32_t low) {
         p[0] = max(p[0], low);
         p[1] = max(p[1], low);
@@ -72,7 +94,9 @@ struct Pair {
 };
 
 // EDGE: the last tile row is not whole, or output rows cannot be written as aligned pairs.
-template <bool BF16, bool EDGE>
+// AHEAD: at most a warp a scheduler, so the chain alone counts.  4096 x 2048 at tile height 1024 (1.7 warps a multiprocessor) 36.5 us ->
+// 30.7; with nine or ten warps it costs 6 %.
+template <bool BF16, bool EDGE, bool AHEAD>
 __global__ void __launch_bounds__(kDec2Warps * 32, 1) k_decode2(const __grid_constant__ Dec2Args p, void *out) {
     extern __shared__ __align__(128) uint8_t smem[];
     const DecArgs &a = p.a;
@@ -190,7 +214,8 @@ __global__ void __launch_bounds__(kDec2Warps * 32, 1) k_decode2(const __grid_con
                     for (uint32_t i = 0; i < 8; ++i) {
                         const uint32_t m = BF16 ? lds_u16(ms + i * 32) : 0u;
                         uint32_t e[2];
-                        z.step(lut_s, e);
+                        if constexpr (AHEAD) z.step_ahead(lut_s, e);
+                        else z.step(lut_s, e);
                         store(r + i, BF16 ? exp_or_man(__byte_perm(e[0], e[1], 0x6521) << 3, __byte_perm(m, 0u, 0x1100))
                                           : (e[0] >> 12 & 0xFFu) | (e[1] >> 4 & 0xFF00u));
                         o += pitch;
@@ -230,10 +255,10 @@ __global__ void __launch_bounds__(kDec2Warps * 32, 1) k_decode2(const __grid_con
     }
 }
 
-template <bool BF16, bool EDGE>
-static int launch_dec2(const Dec2Args &p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, void *out, cudaStream_t s) {
+template <bool BF16, bool EDGE, bool AHEAD>
+static int launch_dec2_as(const Dec2Args &p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, void *out, cudaStream_t s) {
     static SmemLimit lim = {};
-    if (int rc = ensure_smem_limit(lim, (const void *)k_decode2<BF16, EDGE>, (size_t)max_smem)) return rc;
+    if (int rc = ensure_smem_limit(lim, (const void *)k_decode2<BF16, EDGE, AHEAD>, (size_t)max_smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(warps * 32);
@@ -244,8 +269,14 @@ static int launch_dec2(const Dec2Args &p, uint32_t blocks, uint32_t warps, size_
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CI_CUDA(cudaLaunchKernelEx(&cfg, k_decode2<BF16, EDGE>, p, out));
+    CI_CUDA(cudaLaunchKernelEx(&cfg, k_decode2<BF16, EDGE, AHEAD>, p, out));
     return CI_OK;
+}
+
+template <bool BF16, bool EDGE>
+static int launch_dec2(const Dec2Args &p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, void *out, cudaStream_t s) {
+    return warps <= 4 ? launch_dec2_as<BF16, EDGE, true>(p, blocks, warps, smem, max_smem, out, s)
+                      : launch_dec2_as<BF16, EDGE, false>(p, blocks, warps, smem, max_smem, out, s);
 }
 
 int launch_decode2(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, cudaStream_t s) {
@@ -265,10 +296,10 @@ int launch_decode2(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     const uint32_t warp_bytes = p.win_bytes + (bf16 ? kDec2Man : 0u), units = (p.total + P - 1) / P;
     uint32_t w_max = ((uint32_t)max_smem - fixed) / warp_bytes;
     if (w_max > kDec2Warps) w_max = kDec2Warps;
-    // us at 64 symbols per stream, as run_cost: a round of one warp per scheduler is the chain (4.2), with n it is n warps'
-    // instructions.  Whole launches of one round took 6.2 us with 5 warps, 6.9 with 8, 8.9 with 12, 11.4 with 16 and 13.6 with
-    // 20; the 2 us or so that every launch has are left out, as they are in run_cost.
-    auto round2 = [](uint32_t w) { return w <= 4 ? 4.2 : 1.0 + 2.0 * ((w + 3) / 4); };
+    // us at 64 symbols per stream, as run_cost: a round of one warp per scheduler is the chain (3.5), with n it is n warps'
+    // instructions.  512 symbols a stream took 31 us with up to 4 warps, 46 with 8, 54 with 10, 60 with 12, 90 with 16; the 2 us or
+    // so that every launch has are left out, as they are in run_cost.
+    auto round2 = [](uint32_t w) { return w <= 4 ? 3.5 : 1.2 + 2.0 * ((w + 3) / 4) + (w > 12 ? 1.3 : 0.0); };
     uint32_t warps = 0;
     double best = 0.0;
     for (uint32_t w = 1; w <= w_max; ++w) {

@@ -22,6 +22,7 @@
 namespace ci {
 
 constexpr uint32_t kDec4Warps = 21;          // six on one scheduler: 80 registers a thread, which it needs (none spilled)
+constexpr uint32_t kDec4AheadWarps = 8;      // up to here the chain is what counts: Quad::step_ahead
 constexpr uint32_t kDec4BarBytes = 128;      // the table's barrier
 
 struct Dec4Args {
@@ -43,8 +44,8 @@ struct Dec4Args {
 // that are left then.
 // EDGE: the last tile row is not whole (rows beyond K are decoded to garbage and not stored), or output rows cannot be
 // written as aligned quads (N or the address is odd).
-template <bool BF16, bool EDGE, bool INDEX, bool ENTRY>
-__global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_constant__ Dec4Args p, void *out) {
+template <bool BF16, bool EDGE, bool INDEX, bool ENTRY, bool AHEAD>
+__global__ void __launch_bounds__((AHEAD ? kDec4AheadWarps : kDec4Warps) * 32, 1) k_decode4(const __grid_constant__ Dec4Args p, void *out) {
     extern __shared__ __align__(128) uint8_t smem[];
     const DecArgs &a = p.a;
     const Geom &g = a.g;
@@ -260,7 +261,8 @@ __global__ void __launch_bounds__(kDec4Warps * 32, 1) k_decode4(const __grid_con
 #pragma unroll
                 for (uint32_t i = 0; i < 4; ++i) {
                     uint32_t e[4];
-                    z.step(lut_s, e);
+                    if constexpr (AHEAD) z.step_ahead(lut_s, e);
+                    else z.step(lut_s, e);
                     // bits 8..23 of two entries side by side: the symbols sit at bits 4..11 / 20..27
                     const uint32_t a01 = __byte_perm(e[0], e[1], 0x6521), a23 = __byte_perm(e[2], e[3], 0x6521);
                     if constexpr (INDEX) continue;
@@ -341,11 +343,11 @@ __global__ void __launch_bounds__(256) k_entry_spans(uint16_t *rows, uint32_t *s
 
 // ------------------------------------------------------------------------ host
 
-template <bool BF16, bool EDGE, bool INDEX, bool ENTRY>
-static int launch_dec4(const Dec4Args &p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, void *out,
+template <bool BF16, bool EDGE, bool INDEX, bool ENTRY, bool AHEAD>
+static int launch_dec4_as(const Dec4Args &p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, void *out,
                        cudaStream_t s) {
     static SmemLimit lim = {};
-    if (int rc = ensure_smem_limit(lim, (const void *)k_decode4<BF16, EDGE, INDEX, ENTRY>, (size_t)max_smem)) return rc;
+    if (int rc = ensure_smem_limit(lim, (const void *)k_decode4<BF16, EDGE, INDEX, ENTRY, AHEAD>, (size_t)max_smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(warps * 32);
@@ -356,8 +358,15 @@ static int launch_dec4(const Dec4Args &p, uint32_t blocks, uint32_t warps, size_
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CI_CUDA(cudaLaunchKernelEx(&cfg, k_decode4<BF16, EDGE, INDEX, ENTRY>, p, out));
+    CI_CUDA(cudaLaunchKernelEx(&cfg, k_decode4<BF16, EDGE, INDEX, ENTRY, AHEAD>, p, out));
     return CI_OK;
+}
+
+template <bool BF16, bool EDGE, bool INDEX, bool ENTRY>
+static int launch_dec4(const Dec4Args &p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, void *out,
+                       cudaStream_t s) {
+    return warps <= kDec4AheadWarps ? launch_dec4_as<BF16, EDGE, INDEX, ENTRY, true>(p, blocks, warps, smem, max_smem, out, s)
+                                    : launch_dec4_as<BF16, EDGE, INDEX, ENTRY, false>(p, blocks, warps, smem, max_smem, out, s);
 }
 
 static int decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out, uint32_t step,
@@ -381,6 +390,10 @@ int launch_decode4(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
 
 constexpr uint32_t kDec4Fixed = 2 * kLutBytes + kDec4BarBytes;  // up to one table size is lost to the table's alignment
 
+// A round of w warps, as round_cost: up to a warp a scheduler it is the chain of Quad::step_ahead (512 symbols a stream took 39 us
+// with one to four warps, 60 with five, 62 with six; with step() 61, 72 and 74).
+static double round4(uint32_t w) { return w <= 4 ? 4.6 : w <= kDec4AheadWarps ? 8.2 : round_cost(w, 0.9); }
+
 // As in the fused linear: the warp count with the cheapest rounds; a second window where it costs no warp that pays.
 static double plan_rounds(Dec4Args &p, uint32_t man_bytes, int max_smem, uint32_t &warps) {
     const uint32_t P = (uint32_t)sm_count(), room = (uint32_t)max_smem - kDec4Fixed;
@@ -390,7 +403,8 @@ static double plan_rounds(Dec4Args &p, uint32_t man_bytes, int max_smem, uint32_
         uint32_t w_max = room / (stages * p.stage_bytes + man_bytes);
         if (w_max > kDec4Warps) w_max = kDec4Warps;
         for (uint32_t w = 1; w <= w_max; ++w) {
-            const double cost = run_cost((p.total + P - 1) / P, w, 0.9) * (stages == 1 ? 1.02 : 1.0);
+            const uint32_t units = (p.total + P - 1) / P;
+            const double cost = ((units / w) * round4(w) + (units % w ? round4(units % w) : 0.0)) * (stages == 1 ? 1.02 : 1.0);
             if (warps == 0 || cost < best) { best = cost; warps = w; p.stages = stages; }
         }
     }
@@ -418,7 +432,10 @@ double decode4_cost(const DecArgs &a, uint32_t max_tile_len, bool bf16) {
     p.stage_bytes = stage_bytes4(entry ? a.entry_cap : max_tile_len, entry);
     p.total = g.tiles_k * ((g.tiles_n + 1) / 2) * (entry ? g.half / a.entry_step : 1u);
     uint32_t warps;
-    const double cost = plan_rounds(p, bf16 ? kManBytes : 0u, max_smem, warps);
+    double cost = plan_rounds(p, bf16 ? kManBytes : 0u, max_smem, warps);
+    if (warps <= kDec4AheadWarps && (g.K % g.th != 0 || g.N % 4 != 0)) cost *= 1.3;     // the chain of EDGE is longer
+    // A launch takes 1 us longer to its first symbol than one of decode2.cu: 2048 x 2048 at tile height 128 6.6 us there, 8.2 here.
+    if (warps <= kDec4AheadWarps && !entry) cost += 64.0 / g.half;
     return entry ? cost * a.entry_step / g.half : cost;         // per 64 symbols of the whole stream
 }
 

@@ -155,6 +155,10 @@ __device__ __forceinline__ void renorm_fast(uint32_t &state, uint32_t &pos) {
 // together again: in a loop of steps, packing and mma alone one warp a scheduler took 211 cycles a step and takes 166,
 // 16 warps 378 and 359.  The decoders and the gather, without such instructions, are 0.2 to 0.4 % slower with it.  Second bytes
 // under predicates instead of a branch: 403 at 16 warps.
+//
+// step_ahead(): both bytes are loaded before they are known to be needed and merged under predicates: the shortest chain, for
+// launches of so few warps that nothing else happens meanwhile.  In that loop one warp a scheduler takes 131 cycles a step, but
+// 16 warps 403.
 struct Quad {
     uint32_t s[4], p[4];                                        // states, shared addresses of the next bytes
 
@@ -237,6 +241,27 @@ struct Quad {
                              : "+r"(s[j]), "+r"(p[j])
                              : "r"(y[j]));
         }
+    }
+    __device__ __forceinline__ void step_ahead(uint32_t lut_s, uint32_t (&e)[4]) {
+        uint32_t y[4], v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            y[j] = lds_u8(p[j]);
+            v[j] = lds_u8(p[j] - 128);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e[j] = decode_aligned(s[j], lut_s);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            asm("{\n\t.reg .pred p, q;\n\t"
+                "setp.lt.u32 p, %0, 65536;\n\t"
+                "setp.lt.u32 q, %0, 256;\n\t"
+                "@p mad.lo.u32 %0, %0, 256, %2;\n\t"
+                "@p sub.u32 %1, %1, 128;\n\t"
+                "@q mad.lo.u32 %0, %0, 256, %3;\n\t"
+                "@q sub.u32 %1, %1, 128;\n\t}"
+                : "+r"(s[j]), "+r"(p[j])
+                : "r"(y[j]), "r"(v[j]));
     }
     // Streams of columns that do not exist (`cols` of the four do) run along with the first one.  Their own would start at
     // 2^16 over zero bytes: a symbol of frequency 1 at every step, and with it the branch for a second byte.
