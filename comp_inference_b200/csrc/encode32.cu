@@ -17,7 +17,11 @@
 // m f - 2^(32+s) < f <= 2^(s+1) (Granlund and Montgomery, "Division by Invariant Integers using Multiplication").
 //
 // Measured, 4096 x 11008 at tile height 128 through compress_weight_cuda on a B200: 1650 us (and up to 6000 when the
-// stream-ordered allocator returned its memory) -> 168, of which the encoder itself 79, the histogram 18, packing 12.
+// stream-ordered allocator returned its memory) -> 162, of which the encoder itself 78, the histogram 20, packing 11; with pointers that
+// step from row to row instead of a 64-bit product for each, the encoder 64; with the kernels launched ahead of the end of the
+// one before and the depths cleared by one of them, 141 in all, and 2048 x 2048 84 -> 68.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace ci {
@@ -34,6 +38,27 @@ struct EncResult {                           // copied to the host in one piece
 // Words of one stream's slot: a symbol costs at most 12 bits plus log2(1 + 1/16) of rounding.
 __host__ __device__ inline uint32_t stream_words(uint32_t half) { return (half * 3 / 2 + half / 32 + 8 + 3) / 4; }
 
+// Every kernel behind the first is launched with programmatic dependent launch: it waits here until the one before has finished,
+// and lets the next one be scheduled.
+__device__ __forceinline__ void behind_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... Params, class... Args>
+static int launch_behind(void (*kernel)(Params...), uint32_t blocks, uint32_t threads, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CI_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+    return CI_OK;
+}
+
 // ---------------------------------------------------------------- 1. histogram
 
 // Counters [bin][lane]: a warp's increments never meet in a bank, however few different symbols there are.
@@ -41,6 +66,7 @@ template <bool MAN>
 __global__ void __launch_bounds__(512) k_exp_histogram(const uint16_t *__restrict__ w, uint64_t n, unsigned long long *hist,
                                                        unsigned long long *man_hist) {
     extern __shared__ uint32_t s_cnt[];                         // [256][32], with MAN twice
+    behind_previous();
     const uint32_t lane = threadIdx.x & 31;
     for (uint32_t i = threadIdx.x; i < 8192 * (MAN ? 2 : 1); i += blockDim.x) s_cnt[i] = 0;
     __syncthreads();
@@ -79,12 +105,16 @@ __device__ __forceinline__ uint4 encoder_entry(uint32_t f, uint32_t start) {
     return make_uint4(m, start, (4096u - f) << 5 | s, f << 12);
 }
 
-// One block.  hist != null: the frequency rule of ci_normalize_freqs; null: frequencies are in res already.
+// One block.  hist != null: the frequency rule of ci_normalize_freqs; null: frequencies are in res already.  Also clears the
+// tiles' depths, which the encoder takes the maximum into.
 __global__ void __launch_bounds__(256) k_make_tables(const unsigned long long *hist, const unsigned long long *man_hist,
-                                                     EncResult *res, uint4 *enc, uint32_t *tables, uint8_t *slot_map) {
+                                                     EncResult *res, uint4 *enc, uint32_t *tables, uint8_t *slot_map,
+                                                     uint32_t *max_lens, uint32_t tiles) {
     __shared__ uint32_t s_f[256], s_c[256];
     __shared__ unsigned long long s_tot[8];
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    behind_previous();
+    for (uint32_t i = t; i < tiles; i += 256) max_lens[i] = 0;
     if (hist != nullptr) {
         unsigned long long h = hist[t], sum = h;
         for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(kFull, sum, d);
@@ -231,9 +261,14 @@ struct Chain {
 // One warp takes one half (top or bottom streams) of COLS neighbouring tiles, a lane one or two columns.  Rows are taken
 // last first, four at a time, loaded one batch ahead of the chains.  (Both halves in one lane, twice the independent
 // chains and half the warps, was slower: 95 to 141 us against 80 for 4096 x 11008.)
+// Warps of a block: 4096 x 11008 65 us with eight, 64 with four; one column a lane, 2048 x 2048, 9.7 and 10.2.
+template <int COLS>
+constexpr uint32_t kEncWarps = COLS == 2 ? 4 : 8;
+
 template <int COLS, bool PLANE>
-__global__ void __launch_bounds__(256, 4) k_encode32(const __grid_constant__ Enc32Args a) {
+__global__ void __launch_bounds__(kEncWarps<COLS> * 32, 32 / kEncWarps<COLS>) k_encode32(const __grid_constant__ Enc32Args a) {
     __shared__ uint4 s_tab[256];
+    behind_previous();
     for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab[i] = a.table[i];
     __syncthreads();
     const uint32_t lane = lane_id(), per_row = (a.tiles_n + COLS - 1) / COLS * 2;
@@ -254,46 +289,52 @@ __global__ void __launch_bounds__(256, 4) k_encode32(const __grid_constant__ Enc
     }
     const uint32_t row0 = tk * a.th + h * a.half;
     if (live && row0 < a.K) {
-        const size_t first = (size_t)row0 * a.N + col;
-        auto fetch = [&](uint32_t i) -> uint32_t {              // row i of the half: the symbols of the lane's columns
-            const size_t at = first + (size_t)i * a.N;
-            if constexpr (PLANE) {
-                const uint8_t *s = static_cast<const uint8_t *>(a.src) + at;
-                return COLS == 2 ? *reinterpret_cast<const uint16_t *>(s) : *s;
+        constexpr int kBatch = 4;
+        using Src = std::conditional_t<PLANE, uint8_t, uint16_t>;
+        uint32_t i = min(a.half, a.K - row0);                   // rows left
+        const Src *src = static_cast<const Src *>(a.src) + (size_t)(row0 + i) * a.N + col;      // one row behind the next
+        uint8_t *man = a.mantissa + t * a.th * 32 + ((size_t)h * a.half + i) * 32 + c;
+        const size_t pitch = a.N;
+        auto fetch = [&]() -> uint32_t {                        // the symbols of the lane's columns, a row further up
+            src -= pitch;
+            if constexpr (COLS == 2) {
+                if constexpr (PLANE) return *reinterpret_cast<const uint16_t *>(src);
+                else return *reinterpret_cast<const uint32_t *>(src);
             } else {
-                const uint16_t *s = static_cast<const uint16_t *>(a.src) + at;
-                return COLS == 2 ? *reinterpret_cast<const uint32_t *>(s) : *s;
+                return *src;
             }
         };
-        uint8_t *man = a.mantissa + t * a.th * 32 + (size_t)h * a.half * 32 + c;
-        auto code = [&](uint32_t i, uint32_t w) {
+        auto code = [&](int up, uint32_t w) {                   // `up` rows above man
             if constexpr (PLANE) {
                 z[0].put(s_tab[w & 0xFFu]);
                 if constexpr (COLS == 2) z[1].put(s_tab[w >> 8]);
             } else {
                 const uint32_t m = ((w >> 8) & 0x00800080u) | (w & 0x007F007Fu);
-                uint8_t *dst = man + i * 32;
+                uint8_t *dst = man - up * 32;
                 if constexpr (COLS == 2) *reinterpret_cast<uint16_t *>(dst) = (uint16_t)__byte_perm(m, 0u, 0x4420);
                 else *dst = (uint8_t)m;
                 z[0].put(s_tab[(w >> 7) & 0xFFu]);
                 if constexpr (COLS == 2) z[1].put(s_tab[(w >> 23) & 0xFFu]);
             }
         };
-        uint32_t i = min(a.half, a.K - row0);
-        for (; i & 3u; --i) code(i - 1, fetch(i - 1));
+        for (; i % kBatch; --i) {
+            code(1, fetch());
+            man -= 32;
+        }
         if (i) {
-            uint32_t w[4], nx[4];
+            uint32_t w[kBatch], nx[kBatch];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) w[r] = fetch(i - 1 - r);
-            for (; i; i -= 4) {
-                if (i > 4) {
+            for (int r = 0; r < kBatch; ++r) w[r] = fetch();
+            for (; i; i -= kBatch) {
+                if (i > kBatch) {
 #pragma unroll
-                    for (int r = 0; r < 4; ++r) nx[r] = fetch(i - 5 - r);
+                    for (int r = 0; r < kBatch; ++r) nx[r] = fetch();
                 }
 #pragma unroll
-                for (int r = 0; r < 4; ++r) code(i - 1 - r, w[r]);
+                for (int r = 0; r < kBatch; ++r) code(r + 1, w[r]);
+                man -= 32 * kBatch;
 #pragma unroll
-                for (int r = 0; r < 4; ++r) w[r] = nx[r];
+                for (int r = 0; r < kBatch; ++r) w[r] = nx[r];
             }
         }
     }
@@ -319,6 +360,7 @@ __global__ void __launch_bounds__(256, 4) k_encode32(const __grid_constant__ Enc
 __global__ void __launch_bounds__(1024) k_scan_tiles(const uint32_t *__restrict__ max_lens, uint32_t tiles,
                                                      uint32_t *__restrict__ offsets, EncResult *res) {
     __shared__ unsigned long long s_warp[33];
+    behind_previous();
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     unsigned long long base = 0;
     for (uint32_t first = 0; first < tiles; first += 16384) {
@@ -419,9 +461,7 @@ static bool encode32_takes(const Geom &g) { return g.tw == 32 && g.th >= 16 && g
 template <int COLS, bool PLANE>
 static int launch_encode32(const Enc32Args &a, cudaStream_t s) {
     const uint32_t warps = (a.tiles_n + COLS - 1) / COLS * 2 * a.tiles_k;
-    k_encode32<COLS, PLANE><<<(warps + 7) / 8, 256, 0, s>>>(a);
-    CI_LAUNCH_CHECK(k_encode32);
-    return CI_OK;
+    return launch_behind(k_encode32<COLS, PLANE>, (warps + kEncWarps<COLS> - 1) / kEncWarps<COLS>, kEncWarps<COLS> * 32, s, a);
 }
 
 template <bool PLANE>
@@ -431,11 +471,9 @@ static int encode32(Enc32Args a, uint32_t *d_offsets, EncResult *d_res, uint64_t
     const bool aligned = a.N % 2 == 0 && (reinterpret_cast<uintptr_t>(a.src) & (PLANE ? 1u : 3u)) == 0 &&
                          (reinterpret_cast<uintptr_t>(a.mantissa) & 1u) == 0;
     const uint64_t warps2 = (uint64_t)(a.tiles_n + 1) / 2 * 2 * a.tiles_k;
-    CI_CUDA(cudaMemsetAsync(a.max_lens, 0, (size_t)a.tiles_k * a.tiles_n * 4, s));
     int rc = aligned && warps2 >= 16ull * sm_count() ? launch_encode32<2, PLANE>(a, s) : launch_encode32<1, PLANE>(a, s);
     if (rc) return rc;
-    k_scan_tiles<<<1, 1024, 0, s>>>(a.max_lens, a.tiles_k * a.tiles_n, d_offsets, d_res);
-    CI_LAUNCH_CHECK(k_scan_tiles);
+    if ((rc = launch_behind(k_scan_tiles, 1, 1024, s, a.max_lens, a.tiles_k * a.tiles_n, d_offsets, d_res))) return rc;
     EncResult *h = pinned_result();
     CI_REQUIRE(h != nullptr, "no page-locked memory for the encoder's results");
     CI_CUDA(cudaMemcpyAsync(h, d_res, sizeof *h, cudaMemcpyDeviceToHost, s));
@@ -511,9 +549,9 @@ int ci_compress_bf16(const uint16_t *d_w, uint32_t K, uint32_t N, uint32_t th, u
     if (man_hist) k_exp_histogram<true><<<(uint32_t)blocks, 512, smem, s>>>(d_w, n, hist, mh);
     else k_exp_histogram<false><<<(uint32_t)blocks, 512, smem, s>>>(d_w, n, hist, nullptr);
     CI_LAUNCH_CHECK(k_exp_histogram);
-    k_make_tables<<<1, 256, 0, s>>>(hist, man_hist ? mh : nullptr, res, reinterpret_cast<uint4 *>(base + kOffEncTab), d_tables,
-                                    d_slot_map);
-    CI_LAUNCH_CHECK(k_make_tables);
+    if ((rc = launch_behind(k_make_tables, 1, 256, s, hist, man_hist ? mh : nullptr, res, reinterpret_cast<uint4 *>(base + kOffEncTab),
+                            d_tables, d_slot_map, a.max_lens, a.tiles_k * a.tiles_n)))
+        return rc;
     rc = encode32<false>(a, d_tile_offsets, res, stream_len, s);
     const EncResult *h = pinned_result();
     if (rc == CI_OK) {
@@ -546,8 +584,9 @@ int ci_compress_plane(const uint8_t *d_plane, uint32_t K, uint32_t N, const uint
     memcpy(h->freqs, freqs, sizeof h->freqs);                   // idle: every call that used it has waited
     memcpy(h->cdf, cdf, sizeof h->cdf);
     CI_CUDA(cudaMemcpyAsync(res, h, sizeof *res, cudaMemcpyHostToDevice, s));
-    k_make_tables<<<1, 256, 0, s>>>(nullptr, nullptr, res, reinterpret_cast<uint4 *>(base + kOffEncTab), d_tables, d_slot_map);
-    CI_LAUNCH_CHECK(k_make_tables);
+    if ((rc = launch_behind(k_make_tables, 1, 256, s, nullptr, nullptr, res, reinterpret_cast<uint4 *>(base + kOffEncTab), d_tables,
+                            d_slot_map, a.max_lens, a.tiles_k * a.tiles_n)))
+        return rc;
     return encode32<true>(a, d_tile_offsets, res, stream_len, s);
 }
 
