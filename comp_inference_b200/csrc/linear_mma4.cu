@@ -726,9 +726,10 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     // The launch in front costs about 2 us and takes a wavefront per row beyond the first, segment and four rows of a unit out of
     // the load pipe.  us without -> with: 4096 x 4096 at 6 rows 20.1 -> 20.9, 8 21.3 -> 20.9, 16 27.7 -> 22.2; 5504 x 4100 at
     // 2 rows 22.3 -> 24.1, 5 26.7 -> 25.9; 4096 x 22016 at 2 rows 70.9 -> 71.5, 3 74.0 -> 72.0, 16 121.2 -> 75.8; at tile
-    // height 64, where the steps of a short unit wait for less, 6784 x 5168 at 4 rows 32.9 -> 33.7, 8 34.9 -> 34.1.
+    // height 64, where the steps of a short unit wait for less, 6784 x 5168 at 4 rows 32.9 -> 33.7, 8 34.9 -> 34.1; with so few units
+    // that the pipe is not busy, 4936 x 2120 at tile height 1024 and 13 rows 27.6 -> 28.9.
     const uint64_t x_lines = (uint64_t)(a.M - 1) * g.K * g.N;
-    const bool reorder = a.x_scratch != nullptr && a.M >= 3 && x_lines >= (p.step >= 64 ? 90000000ull : 200000000ull);
+    const bool reorder = a.x_scratch != nullptr && a.M >= 3 && x_lines >= (p.step < 64 ? 200000000ull : units >= 16 ? 90000000ull : 150000000ull);
     if (!quads_ok || reorder) {
         const uint32_t pieces = x_rows / 4 * a.M;
         cfg.gridDim = dim3((pieces + 255) / 256);

@@ -21,8 +21,8 @@
 // of the decode step like that kernel: 21 per 32 symbols, 75 % of the issue slots in long runs (32000 x 4096, one row).
 //
 // Measured on a B200, us, before -> with sums in registers, two sets, states among the copies and the chunks of three warps
-// in front of the table: 32000 x 4096 at tile height 128, one row 139 -> 118, two 145 -> 131, eight 215 -> 195; at 64 155 -> 128; at
-// 1024 with entry points 273 -> 194, eight rows 366 -> 328; 8000 x 1024 at 128 31.5 -> 22.3.  The shuffle kernel takes 1000 and 3590
+// in front of the table: 32000 x 4096 at tile height 128, one row 139 -> 118, two 145 -> 131, eight 215 -> 196; at 64 155 -> 128; at
+// 1024 with entry points 273 -> 194; 16000 x 4096 at 1024, four rows 208 -> 187; 8000 x 1024 at 128 31.5 -> 22.3.  The shuffle kernel takes 1000 and 3590
 // for the first and for eight rows at 1024.
 #include "linear.cuh"
 #include "ptx.cuh"
@@ -348,8 +348,7 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
 #pragma unroll
                         for (uint32_t k = 0; k < 2; ++k) {      // rows i, i + 1: columns 0, 1 and 2, 3 of the lane
                             uint32_t e[4];
-                            if constexpr (REG) z.step_together(lut_s, e);
-                            else z.step(lut_s, e);
+                            z.step_together(lut_s, e);
                             const uint32_t m = lds_u32(ms + (i + k) * 16);
                             const uint32_t e01 = __byte_perm(e[0], e[1], 0x6521) << 3, e23 = __byte_perm(e[2], e[3], 0x6521) << 3;
                             w[k] = exp_or_man(e01, __byte_perm(m, 0u, 0x1100));
