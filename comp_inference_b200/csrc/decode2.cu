@@ -297,9 +297,9 @@ int launch_decode2(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     uint32_t w_max = ((uint32_t)max_smem - fixed) / warp_bytes;
     if (w_max > kDec2Warps) w_max = kDec2Warps;
     // us at 64 symbols per stream, as run_cost: a round of one warp per scheduler is the chain (3.5), with n it is n warps'
-    // instructions.  512 symbols a stream took 31 us with up to 4 warps, 46 with 8, 54 with 10, 60 with 12, 90 with 16; the 2 us or
-    // so that every launch has are left out, as they are in run_cost.
-    auto round2 = [](uint32_t w) { return w <= 4 ? 3.5 : 1.2 + 2.0 * ((w + 3) / 4) + (w > 12 ? 1.3 : 0.0); };
+    // instructions.  512 symbols a stream took 31 us with up to 4 warps, 46 with 8, 54 with 10, 60 with 12, 256 symbols 42.5 with 17;
+    // the 2 us or so that every launch has are left out, as they are in run_cost.
+    auto round2 = [](uint32_t w) { return w <= 4 ? 3.5 : w <= 8 ? 5.3 : w <= 12 ? 7.2 : w <= 16 ? 8.8 : 10.0; };
     uint32_t warps = 0;
     double best = 0.0;
     for (uint32_t w = 1; w <= w_max; ++w) {
@@ -308,7 +308,7 @@ int launch_decode2(const DecArgs &a, uint32_t max_tile_len, bool bf16, void *out
     }
     if (warps == 0) return 1;
     const double four = decode4_cost(a, max_tile_len, bf16);   // 0: not a weight for it
-    if (four > 0.0 && four <= 1.05 * best) return 1;
+    if (four > 0.0 && four <= best) return 1;
     const uint32_t blocks = p.total < P ? p.total : P;
     p.vec = a.ld % 2 == 0 && g.N % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & (bf16 ? 3u : 1u)) == 0;
     const bool edge = g.K % g.th != 0 || !p.vec;
