@@ -475,9 +475,34 @@ py::tuple compress(const Tensor &w, int64_t th, int64_t tw, bool want_man_hist) 
                           want_man_hist ? py::cast(man_hist) : py::none());
 }
 
+// linear_of(weight, buffers, tile_h, tile_w, x, bias, split_k, prefill_rows): a module's call in one step, None where `buffers`
+// are no longer what the descriptor was made from.  A plain C function: the binding layer's own argument handling costs a call as
+// much as the allocation of its result.
+PyObject *linear_of(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 8) throw py::type_error("linear_of takes 8 arguments");
+    const Weight &h = *py::cast<const Weight *>(py::handle(args[0]));
+    TORCH_CHECK_TYPE(PyDict_Check(args[1]) && THPVariable_Check(args[4]), "linear_of needs a module's buffers and a tensor");
+    long long v[4];
+    for (int i = 0; i < 4; ++i) {
+        v[i] = PyLong_AsLongLong(args[i < 2 ? 2 + i : 4 + i]);
+        if (v[i] == -1 && PyErr_Occurred()) throw py::error_already_set();
+    }
+    if (!h.matches(py::reinterpret_borrow<py::dict>(args[1]), v[0], v[1])) Py_RETURN_NONE;
+    OptTensor bias;
+    if (args[5] != Py_None) {
+        TORCH_CHECK_TYPE(THPVariable_Check(args[5]), "bias must be a tensor");
+        bias = THPVariable_Unpack(args[5]);
+    }
+    return THPVariable_Wrap(linear_call(h, THPVariable_Unpack(args[4]), bias, std::nullopt, v[2], false, v[3]));
+    END_HANDLE_TH_ERRORS
+}
+PyMethodDef fast_calls[] = {{"linear_of", (PyCFunction)(void (*)(void))linear_of, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
+
 }  // namespace
 
 PYBIND11_MODULE(_ci_host, m) {
+    if (PyModule_AddFunctions(m.ptr(), fast_calls) != 0) throw py::error_already_set();
     py::class_<Weight>(m, "Weight", "Descriptor of a compressed weight and the tensors it points into")
         .def(py::init(&tiled), py::arg("stream"), py::arg("states"), py::arg("tables"), py::arg("slot_map"), py::arg("tile_offsets"),
              py::arg("tile_max_lens"), py::arg("mantissas"), py::arg("K"), py::arg("N"), py::arg("tile_h"), py::arg("tile_w"), py::arg("entries") = false)
