@@ -142,15 +142,15 @@ __global__ void __launch_bounds__((AHEAD ? kDec4AheadWarps : kDec4Warps) * 32, 1
     };
 
     load_desc();
-    uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
-    uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
     uint32_t tk = 0, sub = 0, tp = 0, t0 = 0;                   // of unit t
     bool two = false;
     if (gw < p.total) {
         unit_tiles(gw, tk, sub, tp, t0, two);
-        issue(t0, sub, two, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
-        if (BF16) issue_man(man_of(t0, sub), two, 0, 0);
+        if (BF16) issue_man(man_of(t0, sub), two, 0, 0);        // does not wait for the byte ranges
     }
+    uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
+    uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
+    if (gw < p.total) issue(t0, sub, two, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
     if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
     // Only the weight was touched so far.  With programmatic dependent launch the output buffer may still

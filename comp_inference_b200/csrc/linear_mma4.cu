@@ -241,17 +241,16 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) k_linear_mma4(const __grid_
     };
 
     load_desc();
-    uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
-    uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
     uint32_t grp = lo / p.per_group, pk = lo - grp * p.per_group, sub = 0;   // of unit t
     if constexpr (ENTRY) {
         sub = pk % subs;
         pk /= subs;
     }
-    if (lo < hi) {
-        issue(grp, pk, sub, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
-        issue_man(man_of(grp, pk, sub), 2 * pk + 1 < g.tiles_k, 0, 0);
-    }
+    // The sign+mantissa bytes do not wait for the byte ranges: they are asked for while those are on their way.
+    if (lo < hi) issue_man(man_of(grp, pk, sub), 2 * pk + 1 < g.tiles_k, 0, 0);
+    uint32_t nx_off0 = __shfl_sync(kFull, d_off0, 0), nx_ml0 = __shfl_sync(kFull, d_ml0, 0);
+    uint32_t nx_off1 = __shfl_sync(kFull, d_off1, 0), nx_ml1 = __shfl_sync(kFull, d_ml1, 0);
+    if (lo < hi) issue(grp, pk, sub, 0, nx_off0, nx_ml0, nx_off1, nx_ml1);
     if (a.lut == nullptr) load_lut(s_lut, nullptr, a.tables, a.slot_map);
     __syncthreads();
     // Everything above touches only the weight, which the previous kernel has not written (ci_weight_written).  When
