@@ -123,9 +123,14 @@ __global__ void __launch_bounds__(kDec2Warps * 32, 1) k_decode2(const __grid_con
         cp_async_arrive(man_bar + buf * 8);
     };
     // Starts the copies of tile t (whole warp).
+    // The sign+mantissa bytes do not wait for the byte range.  Where many warps start at once asking for them first spreads their copies
+    // (1500 x 4000 at tile height 128 8.8 us -> 8.5, 3000 x 1500 at 64 6.7 -> 6.4); where few do, it is 0.5 % slower.
+    const bool man_first = W > 8;
     auto issue = [&](uint32_t t, uint32_t &ml) {
         ml = __ldg(a.tile_max_lens + t);
         const uint32_t off = __ldg(a.tile_offsets + t);
+        const uint8_t *man = a.mantissa + (size_t)t * g.th * 32 + lane * 16;
+        if (BF16 && man_first) issue_man(man, 0, 0);
         if (ml > p.cap_rows) ml = 0;                            // metadata disagrees with the declared maximum
         if (lane == 0) {
             fence_async_proxy();
@@ -133,7 +138,7 @@ __global__ void __launch_bounds__(kDec2Warps * 32, 1) k_decode2(const __grid_con
             if (ml) bulk_load(win_s, a.stream + off, ml * 64, bar);
             bulk_load(win_s + p.cap_rows * 64, a.states + (size_t)t * 64, 256, bar);
         }
-        if constexpr (BF16) issue_man(a.mantissa + (size_t)t * g.th * 32 + lane * 16, 0, 0);
+        if (BF16 && !man_first) issue_man(man, 0, 0);
     };
 
     if (lane == 0) {
