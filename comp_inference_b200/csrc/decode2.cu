@@ -7,9 +7,9 @@
 // and initial states arrive by bulk copy, sign+mantissa bytes in double-buffered chunks of 16 rows.  A unit is the whole
 // chain of a stream, usually one a warp: nothing is fetched for the next one ahead.
 //
-// Measured on a B200 (graph replays over more than L2), four streams per lane -> two: 4096 x 11008 at tile height 1024 75.9 ->
-// 54.4 us (1376 tiles: nine or ten warps a multiprocessor, 55 % of the issue slots; the waits that are left are the chain's own,
-// arithmetic and table look-ups), 11008 x 4096 at 1024 95 -> 56, 1024 x 2048 at 128 9.3 -> 5.9, 777 x 1001 at 128 16.9 -> 8.5.
+// Measured on a B200 (graph replays over more than L2), four streams per lane -> two: 4096 x 11008 at tile height 1024 59.8 ->
+// 51.9 us (1376 tiles: nine or ten warps a multiprocessor, so three on some scheduler and 2.3 on average; the waits that are left are
+// the chain's own, arithmetic and table look-ups), 1000 x 1000 at 512 34 -> 17, 777 x 1001 at 128 13.3 -> 7.3.
 #include "decode.cuh"
 #include "ptx.cuh"
 
