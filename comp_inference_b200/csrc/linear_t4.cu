@@ -69,7 +69,11 @@ __device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const uint32_t (&w)
 // index them.  (One activation column per row pair in one D instead would let an infinite weight reach its neighbours' sums.)
 // ENTRY: a group is the rows of four tiles between two entry points (see linear_mma4.cu), so its sums are those of a short
 // tile; without, a tall tile's sums and window leave room for three warps.
-template <int MT, bool ENTRY, bool REG>
+// RAGGED: the matrix ends inside a column block.  Zero activations alone would not do for the columns that are missing: the
+// symbols they repeat may be those of an infinite weight, and zero times that is not a number.  Their exponents are masked to
+// zero.  An instantiation of its own (32000 x 4090, one row 121.7 us -> 125.7): in all of them the masks cost 32000 x 4096 2.6 %,
+// a second loop for the last block 2.8 %.
+template <int MT, bool ENTRY, bool REG, bool RAGGED>
 __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_constant__ T4Args p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const LinArgs &a = p.a;
@@ -293,12 +297,15 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
             __syncwarp();
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j) {
-                // a column beyond the matrix repeats the block's first one (its weights are finite and meet zero activations)
+                // a column beyond the matrix repeats the symbols of the block's first one
                 const uint32_t c = col + j < g.N ? 4 * q + j : 0u;
                 z.s[j] = lds_u32(win_s + st_off + sd * 64 + c * 4);
                 z.p[j] = first + c;
                 if constexpr (ENTRY) z.p[j] += min(lds_u16(win_s + st_off + 512 + sd * 32 + c * 2), p.cap_rows - 1) * 128;
             }
+            // RAGGED: exponent bits of the columns that exist
+            const uint32_t exp01 = (col < g.N ? 0x7F80u : 0u) | (col + 1 < g.N ? 0x7F800000u : 0u);
+            const uint32_t exp23 = (col + 2 < g.N ? 0x7F80u : 0u) | (col + 3 < g.N ? 0x7F800000u : 0u);
             auto next_unit = [&]() {
                 off = noff;
                 ml = nml;
@@ -351,8 +358,9 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
                             z.step_together(lut_s, e);
                             const uint32_t m = lds_u32(ms + (i + k) * 16);
                             const uint32_t e01 = __byte_perm(e[0], e[1], 0x6521) << 3, e23 = __byte_perm(e[2], e[3], 0x6521) << 3;
-                            w[k] = exp_or_man(e01, __byte_perm(m, 0u, 0x1100));
-                            w[2 + k] = exp_or_man(e23, __byte_perm(m, 0u, 0x3322));
+                            const uint32_t m01 = __byte_perm(m, 0u, 0x1100), m23 = __byte_perm(m, 0u, 0x3322);
+                            w[k] = RAGGED ? (e01 & exp01) | (m01 & 0x807F807Fu) : exp_or_man(e01, m01);
+                            w[2 + k] = RAGGED ? (e23 & exp23) | (m23 & 0x807F807Fu) : exp_or_man(e23, m23);
                         }
                         if constexpr (REG) {
                             mma_bf16_zero(d, w, xb[0], xb[1]);
@@ -447,10 +455,10 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
 
 // ------------------------------------------------------------------------ host
 
-template <int MT, bool ENTRY, bool REG>
+template <int MT, bool ENTRY, bool REG, bool RAGGED>
 static int launch_t4_pass(T4Args p, uint32_t blocks, uint32_t warps, size_t smem, int max_smem, cudaStream_t s) {
     static SmemLimit lim = {};
-    if (int rc = ensure_smem_limit(lim, (const void *)k_linear_t4<MT, ENTRY, REG>, (size_t)max_smem)) return rc;
+    if (int rc = ensure_smem_limit(lim, (const void *)k_linear_t4<MT, ENTRY, REG, RAGGED>, (size_t)max_smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(warps * 32);
@@ -461,7 +469,7 @@ static int launch_t4_pass(T4Args p, uint32_t blocks, uint32_t warps, size_t smem
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CI_CUDA(cudaLaunchKernelEx(&cfg, k_linear_t4<MT, ENTRY, REG>, p));
+    CI_CUDA(cudaLaunchKernelEx(&cfg, k_linear_t4<MT, ENTRY, REG, RAGGED>, p));
     return CI_OK;
 }
 
@@ -535,13 +543,14 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
         p.x_wide = ((reinterpret_cast<uintptr_t>(p.a.x) & 7u) == 0 && (a.ldx & 3) == 0 && g.N % 4 == 0) ? 1u : 0u;
         p.a.M = a.M - m0 < rows_per_pass ? a.M - m0 : rows_per_pass;
         using Pass = int (*)(T4Args, uint32_t, uint32_t, size_t, int, cudaStream_t);
-        static const Pass pass[2][5] = {
-            {launch_t4_pass<1, false, true>, launch_t4_pass<2, false, true>, launch_t4_pass<1, false, false>,
-             launch_t4_pass<2, false, false>, launch_t4_pass<8, false, false>},
-            {launch_t4_pass<1, true, true>, launch_t4_pass<2, true, true>, launch_t4_pass<1, true, false>,
-             launch_t4_pass<2, true, false>, launch_t4_pass<8, true, false>}};
+#define CI_T4_SET(E, R)                                                                                      \
+    {launch_t4_pass<1, E, true, R>, launch_t4_pass<2, E, true, R>, launch_t4_pass<1, E, false, R>,           \
+     launch_t4_pass<2, E, false, R>, launch_t4_pass<8, E, false, R>}
+        static const Pass pass[4][5] = {CI_T4_SET(false, false), CI_T4_SET(true, false), CI_T4_SET(false, true), CI_T4_SET(true, true)};
+#undef CI_T4_SET
         const bool reg = step <= kT4RegChunks * kChunkRows;
-        const int rc = pass[entry][rows_per_pass == 8 ? 4 : rows_per_pass - 1 + (reg ? 0 : 2)](p, blocks, warps, smem, max_smem, s);
+        const int rc = pass[entry + 2 * (g.N % 16 != 0)][rows_per_pass == 8 ? 4 : rows_per_pass - 1 + (reg ? 0 : 2)](p, blocks, warps, smem,
+                                                                                                                  max_smem, s);
         if (rc) return rc;
     }
     return CI_OK;

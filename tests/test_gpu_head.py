@@ -49,3 +49,26 @@ def test_infinite_weight_stays_in_its_row(M):
     y = _call(c, (V, H), x)
     bad = (~torch.isfinite(y)).any(0).nonzero().flatten().tolist()
     assert bad == [77, 300]
+
+
+@pytest.mark.parametrize("V,H,th,M", [
+    (600, 250, 128, 1),    # sums in registers, the last column block has ten columns
+    (600, 90, 64, 2),
+    (600, 333, 16, 8),     # sums in shared memory
+    (1500, 1003, 1024, 1), # entry points
+    (1500, 1003, 1024, 5),
+])
+def test_infinite_weight_beside_missing_columns(V, H, th, M):
+    import comp_inference_b200 as ci
+    g = torch.Generator("cuda").manual_seed(V + H)
+    W = (torch.randn(V, H, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    W[7, H // 16 * 16], W[V - 1, H // 16 * 16], W[40, H - 1] = float("inf"), float("-inf"), float("inf")
+    c = ci.compress_weight_cuda(W, th, 32)
+    x = torch.randn(M, H, generator=g, device="cuda").to(torch.bfloat16)
+    y = _call(c, (V, H), x).double()
+    ref = x.double() @ W.double().t()
+    inf = ref.isinf()
+    assert inf.sum() == 3 * M and torch.equal(y[inf], ref[inf])
+    Wf = torch.where(W.isinf(), torch.zeros_like(W), W).double()
+    bound = ref.abs() * 2.0 ** -8 + (x.double().abs() @ Wf.abs().t()) * (H * 2.0 ** -23)   # as above
+    assert bool(((y - ref).abs() <= bound)[~inf].all())
