@@ -9,9 +9,12 @@
 //
 // The groups are made by every CTA for itself, in shared memory: a counting sort of the ids by bin.  It costs 3 us and 148
 // reads of the ids from L2, and no launch, no workspace and no second pass over memory; groups come in the order of their bins, so
-// that all CTAs mean the same ones.
+// that all CTAs mean the same ones.  Bins of more than 128 ids -- padding, tokens that repeat -- are ordered by the ids' ranks: with a
+// sort of such a bin by the whole CTA, a barrier a step, 4096 ids of which half are one token took 16000 x 2048 at tile height
+// 16 49.3 us and now 33.3, all of them one 57.4 -> 22.8, in Zipf's distribution 44.0 -> 35.4; 32000 x 4096 there 74.1 -> 58.1,
+// 63.5 -> 29.2, 66.1 -> 58.5.
 //
-// Bound by instructions (73 % of the issue slots at tile height 16, where a group is 1.6 ids and 5 rows), about 700 a task there, of
+// Bound by instructions (75 % of the issue slots at tile height 16, where a group is 1.6 ids and 5 rows), 680 a task there, of
 // which the decode step 300.
 #include <math.h>
 
@@ -25,7 +28,7 @@ constexpr uint32_t kEmbGBarBytes = 256;      // the table's barrier, the number 
 constexpr uint32_t kEmbGIds = 4096;          // ids of one launch
 constexpr uint32_t kEmbGroup = 8;            // ids of a group
 constexpr uint32_t kEmbGRanked = 128;        // ids of a bin that a warp sorts
-constexpr uint32_t kEmbGFull = 512;          // at least kEmbGIds / (kEmbGroup + 1)
+constexpr uint32_t kEmbGSorts = 512;         // at least kEmbGIds / (kEmbGroup + 1)
 constexpr uint32_t kEmbGBins = 16384;        // counters of the sort
 
 struct EmbGArgs {
@@ -55,12 +58,13 @@ __global__ void __launch_bounds__(kEmbGWarps * 32, 1) k_embedding_group(const __
     const uint32_t lut_s = (smem_s + kLutBytes - 1) & ~(kLutBytes - 1);
     const uint32_t lut_bar = lut_s + kLutBytes;
     start_lut(lut_s, lut_bar, a.lut);
-    uint32_t *const head = reinterpret_cast<uint32_t *>(smem + (lut_bar - smem_s));   // [4]: groups, [5], [6]: full bins, [8..]: the scan's sums
+    uint32_t *const head = reinterpret_cast<uint32_t *>(smem + (lut_bar - smem_s));   // [4]: groups, [5]: sorts, [6]: bins of very many ids, [8..]: the scan's sums
     uint32_t *const tokens = head + kEmbGBarBytes / 4;          // [n]: row in the bin << 16 | id
     uint32_t *const groups = tokens + p.n;                      // [<= n]: bin << 16 | first token << 3 | ids - 1
-    uint32_t *const full = groups + p.n;                        // bins of more than one group; from the end, those of very many ids
-    uint32_t *const count = full + kEmbGFull;                   // [bins + 1]: ids of a bin, later where the next bin's begin
-    const uint32_t wbase_s = ((smem_u32(count) + (p.bins + 1) * 4 + 127) & ~127u) + warp * p.stages * p.stage_bytes;
+    uint32_t *const sorts = groups + p.n;                       // tokens to sort: first one << 16 | in order of ids << 15 | their number
+    uint32_t *const count = sorts + kEmbGSorts;                 // [bins + 1]: ids of a bin, later where the next bin's begin (low half)
+    const uint32_t windows_s = (smem_u32(count) + (p.bins + 1) * 4 + 127) & ~127u;
+    const uint32_t wbase_s = windows_s + warp * p.stages * p.stage_bytes;
     const uint32_t man_off = p.cap_rows * 128;
 
     for (uint32_t i = threadIdx.x; i <= p.bins; i += blockDim.x) count[i] = 0;
@@ -99,22 +103,69 @@ __global__ void __launch_bounds__(kEmbGWarps * 32, 1) k_embedding_group(const __
             count[b] = at;
             for (uint32_t j = 0; j < k; j += kEmbGroup) groups[grp++] = b << 16 | (at + j) << 3 | (min(k - j, kEmbGroup) - 1);
             at += k;
-            if (k > kEmbGRanked) full[kEmbGFull - 1 - atomicAdd(head + 6, 1u)] = b;
-            else if (k > kEmbGroup) full[atomicAdd(head + 5, 1u)] = b;
+            if (k > kEmbGRanked) {                              // its number, and behind it where it ends
+                count[b] = (atomicAdd(head + 6, 1u) + 1) << 16 | at;
+                for (uint32_t j = 0; j < k; j += kEmbGRanked)
+                    sorts[atomicAdd(head + 5, 1u)] = (at - k + j) << 16 | 0x8000u | min(k - j, kEmbGRanked);
+            } else if (k > kEmbGroup) {
+                sorts[atomicAdd(head + 5, 1u)] = (at - k) << 16 | k;
+            }
         }
         if (threadIdx.x == blockDim.x - 1) head[4] = grp;
     }
     __syncthreads();
+    auto token_of = [&](uint32_t i, uint32_t row, uint32_t bin) { return (row != 0xFFFFFFFFu ? row - bin * p.seg : 0u) << 16 | i; };
+    const uint32_t heavy = head[6];                             // bins of more ids than a warp sorts
+    if (heavy == 0) {
 #pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < p.n; i += blockDim.x) {
-        const uint32_t row = row_of(i), bin = bin_of(row);
-        tokens[atomicAdd(count + bin, 1u)] = (row != 0xFFFFFFFFu ? row - bin * p.seg : 0u) << 16 | i;
+        for (uint32_t i = threadIdx.x; i < p.n; i += blockDim.x) {
+            const uint32_t row = row_of(i), bin = bin_of(row);
+            tokens[atomicAdd(count + bin, 1u)] = token_of(i, row, bin);
+        }
+    } else {
+        // Tokens that repeat, padding, ids outside the table.  In such a bin an id's place is its rank among the bin's ids: from a
+        // bit for every id of the launch, in the windows' memory, which nobody uses yet, and the number of bits before each word.
+        const uint32_t words = (p.n + 31) / 32;
+        uint32_t *const bits = reinterpret_cast<uint32_t *>(smem + (windows_s - smem_s));      // [heavy][words]
+        uint16_t *const before = reinterpret_cast<uint16_t *>(bits + heavy * words);
+        for (uint32_t i = threadIdx.x; i < heavy * words; i += blockDim.x) bits[i] = 0;
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t i0 = warp * 32; i0 < p.n; i0 += blockDim.x) {
+            const uint32_t i = i0 + lane, row = i < p.n ? row_of(i) : 0xFFFFFFFFu, bin = bin_of(row);
+            const uint32_t l = i < p.n ? count[bin] >> 16 : 0u;
+            if (l == 0 && i < p.n) tokens[atomicAdd(count + bin, 1u)] = token_of(i, row, bin);
+            const uint32_t same = __match_any_sync(kFull, l);
+            if (l != 0 && lane == __ffs(same) - 1) bits[(l - 1) * words + i0 / 32] = same;     // a word is one warp's
+        }
+        __syncthreads();
+        for (uint32_t l = warp; l < heavy; l += W) {
+            uint32_t sum = 0;
+            for (uint32_t w0 = 0; w0 < words; w0 += 32) {
+                const uint32_t mine = w0 + lane < words ? __popc(bits[l * words + w0 + lane]) : 0u;
+                uint32_t run = mine;
+                for (uint32_t d = 1; d < 32; d <<= 1) {
+                    const uint32_t o = __shfl_up_sync(kFull, run, d);
+                    if (lane >= d) run += o;
+                }
+                if (w0 + lane < words) before[l * words + w0 + lane] = (uint16_t)(sum + run - mine);
+                sum += __shfl_sync(kFull, run, 31);
+            }
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < p.n; i += blockDim.x) {
+            const uint32_t row = row_of(i), bin = bin_of(row), l = count[bin] >> 16;
+            if (l == 0) continue;
+            const uint32_t first = bin ? count[bin - 1] & 0xFFFFu : 0u, at = (l - 1) * words + i / 32;
+            tokens[first + before[at] + __popc(bits[at] & ((1u << (i & 31)) - 1))] = token_of(i, row, bin);
+        }
     }
     __syncthreads();
     // A bin of more than one group in order of rows (and ids), so that every CTA splits it alike and a group's rows are near one
-    // another: by rank, a warp a bin; by Batcher's odd-even merge sort, the whole CTA, where very many ids share a bin.
+    // another: by rank, a warp a bin; one whose tokens are in order of ids by runs of 128.
     for (uint32_t l = warp; l < head[5]; l += W) {
-        const uint32_t b = full[l], first = b ? count[b - 1] : 0u, k = count[b] - first;
+        const uint32_t first = sorts[l] >> 16, k = sorts[l] & 0x7FFFu;
         if (k <= 32) {
             const uint32_t mine = lane < k ? tokens[first + lane] : 0xFFFFFFFFu;
             uint32_t rank = 0;
@@ -128,6 +179,13 @@ __global__ void __launch_bounds__(kEmbGWarps * 32, 1) k_embedding_group(const __
             mine[j] = lane + 32 * j < k ? tokens[first + lane + 32 * j] : 0xFFFFFFFFu;
             rank[j] = 0;
         }
+        if (sorts[l] & 0x8000u) {                               // all of one row: they are in order
+            const uint32_t row = tokens[first] >> 16;
+            bool same = true;
+#pragma unroll
+            for (uint32_t j = 0; j < kEmbGRanked / 32; ++j) same &= lane + 32 * j >= k || mine[j] >> 16 == row;
+            if (__all_sync(kFull, same)) continue;
+        }
         for (uint32_t i = 0; i < k; ++i) {
             const uint32_t v = tokens[first + i];
 #pragma unroll
@@ -137,22 +195,6 @@ __global__ void __launch_bounds__(kEmbGWarps * 32, 1) k_embedding_group(const __
 #pragma unroll
         for (uint32_t j = 0; j < kEmbGRanked / 32; ++j)
             if (lane + 32 * j < k) tokens[first + rank[j]] = mine[j];
-    }
-    for (uint32_t l = 0; l < head[6]; ++l) {
-        const uint32_t b = full[kEmbGFull - 1 - l], first = b ? count[b - 1] : 0u, k = count[b] - first;
-        for (uint32_t w = 1; w < k; w *= 2)
-            for (uint32_t d = w; d; d /= 2) {
-                __syncthreads();
-                for (uint32_t i = threadIdx.x; i + d < k; i += blockDim.x) {
-                    // comparators of the merge of runs of w: distance d, behind the first step only between neighbouring pairs
-                    const bool pair = d == w ? (i & (2 * w - 1)) < w : i % (2 * w) >= d && (i - d) % (2 * d) < d && (i & (2 * w - 1)) + d < 2 * w;
-                    const uint32_t lo = tokens[first + i], hi = tokens[first + i + d];
-                    if (pair && lo > hi) {
-                        tokens[first + i] = hi;
-                        tokens[first + i + d] = lo;
-                    }
-                }
-            }
     }
     __syncthreads();
     const uint32_t total = head[4] * p.blocks_n, n_warps = gridDim.x * W, gw = warp * gridDim.x + blockIdx.x;
@@ -341,7 +383,11 @@ __global__ void __launch_bounds__(kEmbGWarps * 32, 1) k_embedding_group(const __
 // 3.5 us for the sort.  us, embedding4.cu -> groups: 32000 x 4096 at tile height 16, 2048 ids 39 -> 44, 4096 71 -> 70; at 64,
 // 256 ids 18 -> 19, 1024 50 -> 41, 4096 180 -> 84; at 128, 128 ids 20 -> 20, 512 47 -> 39, 4096 327 -> 132; at 1024 with entry
 // points, 4096 376 -> 148; 16000 x 2048 at 16, 2048 ids 20.6 -> 20.8, 4096 37.6 -> 29.9; 8000 x 1000 at 128, 256 ids 13.1 -> 13.3,
-// 1024 34.5 -> 17.8.  (A table of a few bins would spend its time on sorting them.)
+// 1024 34.5 -> 17.8.  (A table of a few bins would spend its time on sorting them.)  How the ids are spread is not known here.
+// 4096 ids in Zipf's distribution gain too (32000 x 4096 at 16 71 -> 59, at 128 338 -> 128; 16000 x 2048 at 16 38 -> 35, 37 -> 37 where
+// frequent tokens are neighbours).  Where groups pay little, a batch padded with token 0, the first of its streams, which
+// embedding4.cu has at once, loses up to 3 us: half of them padding, 16000 x 2048 at 16, 4096 ids 31.0 -> 33.3, 32000 x 1024 at 64,
+// 2048 ids 19.5 -> 21.9, 8000 x 1000 at 128, 512 ids 12.9 -> 16.1; 32000 x 4096 at 64, 4096 ids 113 -> 77.
 static bool groups_pay(uint32_t bins, uint32_t seg, double ids, uint32_t blocks_n) {
     const double each = ids / bins, hit = 1.0 - exp(-each);
     if (each > 64.0) return false;
@@ -376,8 +422,8 @@ int launch_embedding_group(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t
     p.blocks_n = (g.tiles_n + 3) / 4;
     p.out_vec = ((reinterpret_cast<uintptr_t>(a.out) & 7u) == 0 && (a.ldo & 3) == 0) ? 1u : 0u;
     // up to one table size is lost to the table's alignment
-    const uint32_t fixed = 2 * kLutBytes + kEmbGBarBytes + (uint32_t)(ids * 8) + kEmbGFull * 4 + (p.bins + 1) * 4 + 128;
-    if (fixed + p.stage_bytes > (uint32_t)max_smem) return 1;
+    const uint32_t fixed = 2 * kLutBytes + kEmbGBarBytes + (uint32_t)(ids * 8) + kEmbGSorts * 4 + (p.bins + 1) * 4 + 128;
+    if (fixed + p.stage_bytes > (uint32_t)max_smem) return 1;   // the ranks of 4096 ids, 24 KB, fit in any case
     const uint32_t room = (uint32_t)max_smem - fixed;
     p.stages = room / (2 * p.stage_bytes) >= 12 ? 2 : 1;        // as in embedding4.cu
     uint32_t w_max = room / (p.stages * p.stage_bytes);
@@ -399,7 +445,8 @@ int launch_embedding_group(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(blocks);
         cfg.blockDim = dim3(warps * 32);
-        cfg.dynamicSmemBytes = fixed + (size_t)warps * p.stages * p.stage_bytes;
+        const size_t ranks = (size_t)p.n / (kEmbGRanked + 1) * ((p.n + 31) / 32) * 6, windows = (size_t)warps * p.stages * p.stage_bytes;
+        cfg.dynamicSmemBytes = fixed + (ranks > windows ? ranks : windows);
         cfg.stream = s;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

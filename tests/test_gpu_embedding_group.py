@@ -1,4 +1,6 @@
 """The row gather where ids share streams (embedding_group.cu): exact, whatever the ids and however they are spread."""
+import math
+
 import pytest
 import torch
 
@@ -7,11 +9,13 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("V,H,th", [
     (4000, 512, 64),       # 32 rows a bin
-    (4001, 1100, 128),     # columns beyond the matrix, the last tile not whole
-    (9000, 260, 1024),     # entry points
+    (4001, 1100, 128),     # 63 bins of 65 ids: too few, ungrouped
+    (5001, 1100, 128),     # columns beyond the matrix, the last tile not whole
+    (9000, 260, 1024),     # entry points, columns beyond the matrix
+    (9000, 256, 1024),     # entry points, whole blocks of columns
     (16000, 2048, 16),     # eight rows a bin
 ])
-@pytest.mark.parametrize("ids", ["spread", "sorted", "one", "few", "invalid", "most"])
+@pytest.mark.parametrize("ids", ["spread", "sorted", "one", "few", "invalid", "most", "skewed", "padded"])
 def test_grouped_gather(V, H, th, ids):
     import comp_inference_b200 as ci
     g = torch.Generator("cuda").manual_seed(V)
@@ -26,6 +30,10 @@ def test_grouped_gather(V, H, th, ids):
         i[:] = V - 1                                    # one bin of all ids
     elif ids == "few":
         i = i % 200 * (V // 200)                        # bins of one row and 20 ids, and of several
+    elif ids == "skewed":                               # several bins of more than 128 ids, of one row and of many
+        i = (torch.rand(n, generator=g, device="cuda") * math.log(V)).exp().long() - 1
+    elif ids == "padded":                               # two bins of more, in runs and in between
+        i[:1300], i[2000::2] = 0, V - 1
     elif ids == "invalid":
         i[::3], i[1::7] = -1, V                         # a bin of ids outside the table
     out = m(i)
