@@ -436,6 +436,7 @@ double decode4_cost(const DecArgs &a, uint32_t max_tile_len, bool bf16) {
     p.total = g.tiles_k * ((g.tiles_n + 1) / 2) * (entry ? g.half / a.entry_step : 1u);
     uint32_t warps;
     double cost = plan_rounds(p, bf16 ? kManBytes : 0u, max_smem, warps);
+    if (warps == 0) return 0.0;                                 // too deep for a window of four streams a lane
     if (warps <= kDec4AheadWarps && (g.K % g.th != 0 || g.N % 4 != 0)) cost *= 1.3;     // the chain of EDGE is longer
     // A launch takes 1 us longer to its first symbol than one of decode2.cu: 2048 x 2048 at tile height 128 6.6 us there, 8.2 here.
     if (warps <= kDec4AheadWarps && !entry) cost += 64.0 / g.half;
