@@ -35,12 +35,18 @@ constexpr uint32_t kT4SegPitch = kChunkRows * 16 + 16;       // eight segments o
 constexpr uint32_t kT4ManBytes = 2 * 8 * kT4SegPitch;
 constexpr uint32_t kT4RegChunks = 4;         // chunks of a segment whose sums a lane holds in registers
 
+// The table's alignment leaves up to a table's size unused in front of the table, where the chunks of three warps have room; the
+// rest of it is left at the end of the window.  With this much in the two together, a chunk that does not fit in front, where the
+// window begins elsewhere, moves everything behind the table up by one and still fits.
+constexpr uint32_t kT4Front = 3, kT4SpareBytes = (kT4Front + 1) * kT4ManBytes;
+static_assert(kT4SpareBytes >= kLutBytes, "the table's alignment may cost a table's size");
+
 struct T4Args {
     LinArgs a;
     uint32_t cap_rows;     // rows of a byte window (>= every tile_max_len)
     uint32_t stage_bytes;  // window + initial states (with entry points also the rows of the next bytes)
     uint32_t stages;       // windows per warp
-    uint32_t front;        // warps whose sign+mantissa chunks lie in front of the table
+    uint32_t front;        // warps whose sign+mantissa chunks lie in front of the table, as far as there is room
     uint32_t acc_bytes;    // sums of a warp in one group
     uint32_t sets;         // groups that a CTA works on between two barriers
     uint32_t cblocks;      // 16-column blocks per group
@@ -83,14 +89,11 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     const uint32_t lut_s = (smem_s + kLutBytes - 1) & ~(kLutBytes - 1);    // see linear_mma4.cu
     uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + (lut_s - smem_s));
     const uint32_t lut_bar = lut_s + kLutBytes + kT4BarBytes - 16;
-    if (lut_s - smem_s < p.front * kT4ManBytes) {               // the table does not lie where the launcher takes it to
-        if (threadIdx.x == 0) atomicExch(p.status, 1u);
-        return;
-    }
     start_lut(lut_s, lut_bar, a.lut);
     const uint32_t behind_s = lut_s + kLutBytes + kT4BarBytes;
-    const uint32_t man_s = warp < p.front ? smem_s + warp * kT4ManBytes : behind_s + (warp - p.front) * kT4ManBytes;
-    const uint32_t acc0_s = behind_s + (W - p.front) * kT4ManBytes, set_bytes = W * p.acc_bytes;
+    const uint32_t front = min(p.front, (lut_s - smem_s) / kT4ManBytes);
+    const uint32_t man_s = warp < front ? smem_s + warp * kT4ManBytes : behind_s + (warp - front) * kT4ManBytes;
+    const uint32_t acc0_s = behind_s + (W - front) * kT4ManBytes, set_bytes = W * p.acc_bytes;
     const uint32_t acc_s = acc0_s + warp * p.acc_bytes;         // of the first set; the others set_bytes further each
     const uint32_t wbase_s = acc0_s + p.sets * set_bytes + warp * p.stages * p.stage_bytes;
     const uint32_t st_off = p.cap_rows * 128;
@@ -500,15 +503,12 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
     p.status = a.tickets + (kTicketBytes - 1);
     p.wide = ((entry ? reinterpret_cast<uintptr_t>(a.entry_states) | reinterpret_cast<uintptr_t>(a.entry_rows)
                      : reinterpret_cast<uintptr_t>(a.states)) & 15u) == 0;
-    const uint32_t P = (uint32_t)sm_count(), fixed = 2 * kLutBytes + kT4BarBytes, room = (uint32_t)max_smem - fixed;
+    const uint32_t P = (uint32_t)sm_count(), fixed = kLutBytes + kT4SpareBytes + kT4BarBytes, room = (uint32_t)max_smem - fixed;
     const uint32_t blocks = p.total < P ? p.total : P;
     // Passes over the weight x rounds of units: sums for eight activation rows take eight times the shared memory of one,
     // which a tall tile cannot afford at a useful number of warps.  Two sets of sums where there is room: a CTA with the units
     // of two groups then deals them out as one sequence, and without a second one rounds its units up in each.
     const uint32_t units = (p.total + blocks - 1) / blocks;
-    uint32_t front = 0;
-    if (int rc = front_bytes(dev, front)) return rc;
-    front /= kT4ManBytes;
     uint32_t warps = 0, rows_per_pass = 0;
     double best = 0.0;
     for (uint32_t mt = 1; mt <= 8; mt = mt == 2 ? 8 : mt * 2)
@@ -516,8 +516,8 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
             for (uint32_t sets = 1; sets <= (mt == 8 ? 1u : 2u); ++sets) {
                 const uint32_t acc = (8 * (step * (mt * 4) + (mt == 8 ? 32 : mt * 4)) + 15) & ~15u;
                 const uint32_t own = stages * p.stage_bytes + sets * acc;
-                uint32_t w_max = (room + front * kT4ManBytes) / (own + kT4ManBytes);
-                if (w_max < front) w_max = room / own;
+                uint32_t w_max = (room + kT4Front * kT4ManBytes) / (own + kT4ManBytes);
+                if (w_max < kT4Front) w_max = room / own;
                 if (w_max > kT4Warps) w_max = kT4Warps;
                 for (uint32_t w = 1; w <= w_max; ++w) {
                     const bool split = groups > 1 && (sets == 1 || units > p.cblocks);   // some CTA's units end in two rounds
@@ -529,7 +529,7 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
                         rows_per_pass = mt;
                         p.stages = stages;
                         p.sets = sets;
-                        p.front = w < front ? w : front;
+                        p.front = w < kT4Front ? w : kT4Front;
                         p.acc_bytes = acc;
                     }
                 }

@@ -314,15 +314,6 @@ __device__ __forceinline__ uint32_t enter_span(uint32_t span, uint32_t depth, ui
     return first + rows <= depth ? rows : 0xFFFFFFFFu;
 }
 
-// The table's boundary leaves most of a table's size unused in front of it: the launchers put the sign+mantissa chunks of the
-// first warps there.  How much there is follows from what the system reserves at the start of the window; kernels check it.
-inline int front_bytes(int dev, uint32_t &bytes) {
-    int reserved = 0;
-    CI_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
-    bytes = (kLutBytes - (uint32_t)reserved % kLutBytes) % kLutBytes;
-    return CI_OK;
-}
-
 // Sign+mantissa bytes on their way through a warp that decodes four segments (two tiles, both halves) at once: chunks of
 // kChunkRows rows of 32 bytes per segment, double buffered.  The segments of a chunk start 8 banks apart, so a row of
 // the warp's 128 columns is one conflict-free wavefront.
