@@ -45,6 +45,19 @@ def bits(t):
     return t.contiguous().view(torch.uint16).cpu().numpy()
 
 
+def captured_kernels(call):
+    """The kernels that `call` launches, as the driver writes out the graph that it is captured into.  It has to have run once."""
+    import ctypes
+    import tempfile
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    with tempfile.NamedTemporaryFile(suffix=".dot") as f:
+        rc = ctypes.CDLL("libcuda.so.1").cuGraphDebugDotPrint(ctypes.c_void_p(graph.raw_cuda_graph()), f.name.encode(), ctypes.c_uint(0))
+        assert rc == 0
+        return open(f.name).read()
+
+
 def golden_case(golden, i):
     p = f"t{i}_"
     K, N, th, tw, seed = (int(v) for v in golden[p + "geom"])

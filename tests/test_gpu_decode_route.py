@@ -5,6 +5,8 @@ at 1500 rows or so and one of 64-byte rows (decode2.cu) at 3000."""
 import pytest
 import torch
 
+from conftest import captured_kernels
+
 pytestmark = pytest.mark.gpu
 
 
@@ -18,20 +20,20 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("N", [64, 2000])
 def test_deep_tiles(th, exps, staged, N):
     import comp_inference_b200 as ci
-    from torch.profiler import ProfilerActivity, profile
+    from comp_inference_b200 import _lib
     g = torch.Generator("cuda").manual_seed(th + exps + N)
     bits = torch.randint(0, exps, (th, N), generator=g, device="cuda") << 7 | torch.randint(0, 128, (th, N), generator=g, device="cuda")
-    W = bits.to(torch.int16).view(torch.bfloat16)
-    c = ci.compress_weight_cuda(W, th, 32)
+    W = bits.to(torch.int16)
+    c = ci.compress_weight_cuda(W.view(torch.bfloat16), th, 32)
     assert c["tile_height"] == th
-    args = dict(initial_states=c["rans_exp_states"], tables=c["rans_exp_tables"], slot_map=c["rans_exp_slot_map"], weight_shape=(th, N),
-                tile_offsets=c["rans_exp_tile_offsets"], tile_max_lens=c["rans_exp_tile_max_lens"], tile_k=th, tile_n=32,
-                mantissas=c["rans_man_raw"])
-    call = lambda: ci.rans_decompress_bf16(c["rans_exp_stream"], **args)
-    assert torch.equal(call().view(torch.int16), W.view(torch.int16))
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        call()
-        torch.cuda.synchronize()
-    kernels = [e.key for e in p.key_averages() if "k_decode" in e.key]
-    assert len(kernels) == 1
-    assert staged == any(k in kernels[0] for k in ("k_decode2", "k_decode4")), kernels
+    w, keep = _lib.tiled_weight(c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"], c["rans_exp_slot_map"],
+                                c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"], c["rans_man_raw"], th, N, th, 32,
+                                want_max=True)
+    out = torch.zeros_like(W)
+
+    def call():
+        _lib.check(_lib.load().ci_decode_bf16(w, out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    call()
+    assert torch.equal(out, W)
+    launched = captured_kernels(call)
+    assert staged == ("k_decode2" in launched or "k_decode4" in launched) and ("k_decode_tiled" in launched) == (not staged)
