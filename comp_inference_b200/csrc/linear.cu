@@ -393,7 +393,7 @@ static size_t workspace_bytes(uint32_t M, uint32_t n_out) {
 }
 
 // Behind those, where the caller's workspace has room: up to 16 rows of activations reordered (linear_mma4.cu).
-// A group of four rows is stored whole, the first one at the next 256-byte boundary.
+// They are stored in whole tile pairs, zeros beyond K, the first one at the next 256-byte boundary.
 static size_t x_scratch_bytes(uint32_t K, uint32_t th) {
     return K && th ? ((size_t)K + 2 * th - 1) / (2 * th) * (2 * th) * 16 * sizeof(uint16_t) + 256 : 0;
 }

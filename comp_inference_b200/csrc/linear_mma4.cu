@@ -126,17 +126,15 @@ __device__ __forceinline__ void rows2(uint32_t (&b)[4][2], int h, Quad &z, uint3
 //
 // ENTRY: a unit is not a pair of whole tiles but the rows between two entry points of it (tall tiles: 512 symbols are one
 // serial chain).  The states and cursors of its streams come from the index, its window holds just the rows of the byte
-// blocks that those symbols touch.  4096 x 4096 at tile height 1024, one row: 63 us -> 18.9.
+// blocks that those symbols touch.  4096 x 4096 at tile height 1024, one row: 63 us -> 17.8.
 __device__ __align__(16) uint16_t g_zero_activations[256];
 
-// Place of the four activations k4 of row m in that order, in 8-byte pieces, and back: what the 32 lanes read for four rows
-// of a unit are neighbours.
+// The order of k_interleave_x in 8-byte pieces of four activations: piece q of row m of the four rows r4 of a unit's segments is at
+// ((pair * half4 + r4) * M + m) * 4 + q, so that what the 32 lanes read for four rows of a unit are neighbours.
 struct XOrder {
     uint32_t half4;        // k4 per row segment (half a tile)
     uint32_t M;
-    __device__ __forceinline__ uint32_t place(uint32_t pk, uint32_t r4, uint32_t m, uint32_t q) const {
-        return ((pk * half4 + r4) * M + m) * 4 + q;
-    }
+    // Which four activations stand there, and of which row.
     __device__ __forceinline__ uint32_t k4(uint32_t place, uint32_t &m) const {
         const uint32_t row = place / (4 * M), in = place - row * 4 * M, pk = row / half4;
         m = in >> 2;

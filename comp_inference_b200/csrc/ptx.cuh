@@ -153,8 +153,9 @@ __device__ __forceinline__ void renorm_fast(uint32_t &state, uint32_t &pos) {
 // step_together(): the whole warp takes that branch or does not, by a vote on a test that does not wait for the first bytes
 // (the state before them is below 2^8).  Where tensor instructions follow, lanes that part in every step have to be brought
 // together again: in a loop of steps, packing and mma alone one warp a scheduler took 211 cycles a step and takes 166,
-// 16 warps 378 and 359.  The decoders and the gather, without such instructions, are 0.2 to 0.4 % slower with it.  Second bytes
-// under predicates instead of a branch: 403 at 16 warps.
+// 16 warps 378 and 359.  Without such instructions there is little in it: the decoders take 0.5 to 1.6 % longer with it, the
+// gather between 2 % less (few ids, or entry points) and 1 % more (tile height 16).  Second bytes under predicates instead of a
+// branch: 403 at 16 warps.
 //
 // step_ahead(): both bytes are loaded before they are known to be needed and merged under predicates: the shortest chain, for
 // launches of so few warps that nothing else happens meanwhile.  In that loop one warp a scheduler takes 131 cycles a step, but
