@@ -253,6 +253,33 @@ def test_encoder_to_an_odd_address(K, N):
     assert torch.equal(states, c["rans_exp_states"].view(torch.int32))
 
 
+# depths left over in the output array, in as many tiles as one block clears, one more, and several blocks' worth
+@pytest.mark.parametrize("K,N", [(8176, 1024), (8192, 1024), (16 * 1171, 32 * 43)])
+def test_encoder_clears_the_depths(K, N):
+    import ctypes as C
+    import comp_inference_b200 as ci
+    from comp_inference_b200 import _lib
+    lib = _lib.load()
+    W = _weight(K, N)
+    c = ci.compress_weight_cuda(W, 16, 32)
+    tiles, want = -(-K // 16) * -(-N // 32), c["rans_exp_tile_max_lens"].view(torch.int32)
+    assert 0 < int(want.max()) <= 16
+    u32 = lambda n: torch.full((n,), 0x7FFFFFFF, dtype=torch.int32, device="cuda")
+    man = torch.empty_like(c["rans_man_raw"])
+    states, sizes, offsets, lens, tables = u32(tiles * 64), u32(tiles * 64), u32(tiles), u32(tiles), u32(256)
+    slot_map, freqs, cdf = torch.empty(4096, dtype=torch.uint8, device="cuda"), torch.empty(256, dtype=torch.uint16), torch.empty(256, dtype=torch.uint16)
+    n_scratch, n = lib.ci_compress_scratch_bytes(K, N, 16, 32), C.c_uint64(0)
+    scratch = torch.empty(n_scratch, dtype=torch.uint8, device="cuda")
+    _lib.check(lib.ci_compress_bf16(_lib.ptr(W), K, N, 16, 32, *map(_lib.ptr, (man, states, sizes, offsets, lens, tables, slot_map, scratch)),
+                                    n_scratch, _lib.ptr(freqs), _lib.ptr(cdf), None, C.byref(n), _lib.stream()))
+    assert torch.equal(lens, want) and n.value == c["rans_exp_stream"].numel()
+    plane, _ = ci.extract_exp_and_mantissa(W)
+    lens.fill_(0x7FFFFFFF)
+    _lib.check(lib.ci_compress_plane(_lib.ptr(plane), K, N, _lib.ptr(freqs), _lib.ptr(cdf), 16, 32, *map(
+        _lib.ptr, (states, sizes, offsets, lens, tables, slot_map, scratch)), n_scratch, C.byref(n), _lib.stream()))
+    assert torch.equal(lens, want) and n.value == c["rans_exp_stream"].numel()
+
+
 # threads that compress one after the other: each has a landing place of its own, given back when it ends
 def test_encoder_from_threads_that_end():
     import threading
