@@ -19,7 +19,7 @@
 // Measured, 4096 x 11008 at tile height 128 through compress_weight_cuda on a B200: 1650 us (and up to 6000 when the
 // stream-ordered allocator returned its memory) -> 162, of which the encoder itself 78, the histogram 20, packing 11; with pointers that
 // step from row to row instead of a 64-bit product for each, the encoder 64; with the kernels launched ahead of the end of the
-// one before and the depths cleared by one of them, 141 in all, and 2048 x 2048 84 -> 68.
+// one before and the depths cleared beside the tables, 141 in all, and 2048 x 2048 84 -> 68.
 #include <type_traits>
 
 #include "common.cuh"

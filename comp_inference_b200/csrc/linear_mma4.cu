@@ -724,7 +724,9 @@ int launch_linear_mma4(const LinArgs &a, uint32_t max_tile_len, cudaStream_t s) 
     // the load pipe.  us without -> with: 4096 x 4096 at 6 rows 20.1 -> 20.9, 8 21.3 -> 20.9, 16 27.7 -> 22.2; 5504 x 4100 at
     // 2 rows 22.3 -> 24.1, 5 26.7 -> 25.9; 4096 x 22016 at 2 rows 70.9 -> 71.5, 3 74.0 -> 72.0, 16 121.2 -> 75.8; at tile
     // height 64, where the steps of a short unit wait for less, 6784 x 5168 at 4 rows 32.9 -> 33.7, 8 34.9 -> 34.1; with so few units
-    // that the pipe is not busy, 4936 x 2120 at tile height 1024 and 13 rows 27.6 -> 28.9.
+    // that the pipe is not busy, 4936 x 2120 at tile height 1024 and 13 rows 27.6 -> 28.9.  The lines lie so that none of these
+    // loses; the number of products alone does not tell gain from loss to the last 2 %, so that 4096 x 4096 at 8 and 9 rows, for
+    // one, goes without.
     const uint64_t x_lines = (uint64_t)(a.M - 1) * g.K * g.N;
     const bool reorder = a.x_scratch != nullptr && a.M >= 3 && x_lines >= (p.step < 64 ? 200000000ull : units >= 16 ? 90000000ull : 150000000ull);
     if (!quads_ok || reorder) {

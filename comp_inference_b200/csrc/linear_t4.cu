@@ -22,7 +22,7 @@
 //
 // Measured on a B200, us, before -> with sums in registers, two sets, states among the copies and the chunks of three warps
 // in front of the table: 32000 x 4096 at tile height 128, one row 139 -> 118, two 145 -> 131, eight 215 -> 196; at 64 155 -> 128; at
-// 1024 with entry points 273 -> 194; 16000 x 4096 at 1024, four rows 208 -> 187; 8000 x 1024 at 128 31.5 -> 22.3.  The shuffle kernel takes 1000 and 3590
+// 1024 with entry points 273 -> 194; 16000 x 4096 at 1024, four rows 208 -> 187; 8000 x 1024 at 128 31.5 -> 21.5.  The shuffle kernel takes 1000 and 3590
 // for the first and for eight rows at 1024.
 #include "linear.cuh"
 #include "ptx.cuh"
