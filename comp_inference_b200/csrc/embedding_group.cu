@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kEmbGWarps * 32, 1) k_embedding_group(const __
 
 // ------------------------------------------------------------------------ host
 
-// Whether groups are worth their making, for ids spread evenly over the table.  Rows to decode, 128 columns each, for one id
+// What groups gain in us, for ids spread evenly over the table.  Rows to decode, 128 columns each, for one id
 // at a time and for groups (a bin is decoded to the last of its rows); 7.2e-5 us a row, about as much on top for a group,
 // 3.5 us for the sort.  us, embedding4.cu -> groups: 32000 x 4096 at tile height 16, 2048 ids 39 -> 44, 4096 71 -> 70; at 64,
 // 256 ids 18 -> 19, 1024 50 -> 41, 4096 180 -> 84; at 128, 128 ids 20 -> 20, 512 47 -> 39, 4096 327 -> 132; at 1024 with entry
@@ -388,14 +388,30 @@ __global__ void __launch_bounds__(kEmbGWarps * 32, 1) k_embedding_group(const __
 // frequent tokens are neighbours).  Where groups pay little, a batch padded with token 0, the first of its streams, which
 // embedding4.cu has at once, loses up to 3 us: half of them padding, 16000 x 2048 at 16, 4096 ids 31.0 -> 33.3, 32000 x 1024 at 64,
 // 2048 ids 19.5 -> 21.9, 8000 x 1000 at 128, 512 ids 12.9 -> 16.1; 32000 x 4096 at 64, 4096 ids 113 -> 77.
-static bool groups_pay(uint32_t bins, uint32_t seg, double ids, uint32_t blocks_n) {
+static double one_by_one(uint32_t seg, double ids, uint32_t blocks_n) { return ids * (seg + 1) / 2 * blocks_n * 7.2e-5; }
+static double groups_gain(uint32_t bins, uint32_t seg, double ids, uint32_t blocks_n) {
     const double each = ids / bins, hit = 1.0 - exp(-each);
-    if (each > 64.0) return false;
+    if (each > 64.0) return -1e9;
     const double full = ids / kEmbGroup, bins_hit = bins * hit;
     const double groups = bins_hit > full ? bins_hit : full;
     const double deep = bins * seg * (1.0 - hit / each), split = full * seg * 0.55;
     const double rows = deep > split ? deep : split;
-    return (ids * (seg + 1) / 2 - rows - groups) * blocks_n * 7.2e-5 > 3.5;
+    return one_by_one(seg, ids, blocks_n) - (rows + groups) * blocks_n * 7.2e-5 - 3.5;
+}
+// More ids than one launch takes, in which embedding4.cu does not have to stop: a launch behind the first costs 6 us, and where
+// groups gain less than a fifth the ids behind the first 4096 lose it again, since embedding4.cu takes those in less time than the
+// first ones.  What is left behind the whole launches goes to embedding4.cu unless it is enough for groups of its own.  us, embedding4.cu
+// -> groups throughout -> this rule: 32000 x 4096 at tile height 16, 4097 ids 71.0 -> 85.6 -> 71.0, 6144 104 -> 113 -> 104, 8200 137 ->
+// 155 -> 137, 12288 200 -> 207 -> 200; at 64, 4100 ids 179 -> 88.3 -> 86.2; 16000 x 2048 at 16, 4097 ids 38.5 -> 40.2 -> 38.4,
+// 8192 71.3 -> 64.8 -> 64.6; 8000 x 1000 at 128, 4100 ids 108 -> 52.6 -> 50.9.  Returns how many ids groups take.
+static uint64_t grouped_ids(uint32_t bins, uint32_t seg, uint64_t ids, uint32_t blocks_n) {
+    if (ids <= kEmbGIds) return groups_gain(bins, seg, (double)ids, blocks_n) > 0.0 ? ids : 0;
+    const uint64_t rest = ids % kEmbGIds, whole = ids - rest;
+    const double gain = groups_gain(bins, seg, (double)kEmbGIds, blocks_n);
+    const double rest_gain = rest ? groups_gain(bins, seg, (double)rest, blocks_n) : 0.0;
+    if (gain < 0.2 * one_by_one(seg, (double)kEmbGIds, blocks_n)) return 0;
+    if (whole / kEmbGIds * gain + (rest_gain > 0.0 ? rest_gain : 0.0) <= (ids - 1) / kEmbGIds * 6.0) return 0;
+    return rest_gain > 0.0 ? ids : whole;
 }
 
 int launch_embedding_group(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t s) {
@@ -412,14 +428,15 @@ int launch_embedding_group(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t
     p.bins = (g.K + p.seg - 1) / p.seg;
     if (p.seg > 0xFFFFu || p.bins > kEmbGBins) return 1;        // rows in a bin and bins are 16-bit numbers below 0xFFFF
     const uint64_t ids = a.n_ids < kEmbGIds ? a.n_ids : kEmbGIds;
-    if (!groups_pay(p.bins, p.seg, (double)ids, (g.tiles_n + 3) / 4)) return 1;
+    p.blocks_n = (g.tiles_n + 3) / 4;
+    const uint64_t grouped = grouped_ids(p.bins, p.seg, a.n_ids, p.blocks_n);
+    if (grouped == 0) return 1;
     int dev = 0, max_smem = 0;
     CI_CUDA(cudaGetDevice(&dev));
     CI_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     p.cap_rows = entry ? a.entry_cap : max_tile_len;
     p.subs = entry ? g.half / a.entry_step : 1u;
     p.stage_bytes = p.cap_rows * 128u + kEmbGroup * 128u;
-    p.blocks_n = (g.tiles_n + 3) / 4;
     p.out_vec = ((reinterpret_cast<uintptr_t>(a.out) & 7u) == 0 && (a.ldo & 3) == 0) ? 1u : 0u;
     // up to one table size is lost to the table's alignment
     const uint32_t fixed = 2 * kLutBytes + kEmbGBarBytes + (uint32_t)(ids * 8) + kEmbGSorts * 4 + (p.bins + 1) * 4 + 128;
@@ -434,8 +451,8 @@ int launch_embedding_group(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t
                                            : (ragged ? k_embedding_group<false, true> : k_embedding_group<false, false>);
     if (int rc = ensure_smem_limit(lim[entry + 2 * ragged], (const void *)kernel, (size_t)max_smem)) return rc;
     const uint32_t P = (uint32_t)sm_count();
-    for (uint64_t i0 = 0; i0 < a.n_ids; i0 += kEmbGIds) {
-        p.n = (uint32_t)(a.n_ids - i0 < kEmbGIds ? a.n_ids - i0 : kEmbGIds);
+    for (uint64_t i0 = 0; i0 < grouped; i0 += kEmbGIds) {
+        p.n = (uint32_t)(grouped - i0 < kEmbGIds ? grouped - i0 : kEmbGIds);
         p.a.ids = a.ids + i0;
         p.a.out = a.out + i0 * a.ldo;
         const uint64_t most = (uint64_t)p.n * p.blocks_n;       // units, if no two ids shared a bin
@@ -455,7 +472,12 @@ int launch_embedding_group(const EmbArgs &a, uint32_t max_tile_len, cudaStream_t
         cfg.numAttrs = 1;
         CI_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
     }
-    return CI_OK;
+    if (grouped == a.n_ids) return CI_OK;
+    EmbArgs rest = a;
+    rest.ids += grouped;
+    rest.out += grouped * a.ldo;
+    rest.n_ids -= grouped;
+    return launch_embedding4(rest, max_tile_len, s);
 }
 
 }  // namespace ci
