@@ -14,7 +14,7 @@
 // 16 49.3 us and now 33.3, all of them one 57.4 -> 22.8, in Zipf's distribution 44.0 -> 35.4; 32000 x 4096 there 74.1 -> 58.1,
 // 63.5 -> 29.2, 66.1 -> 58.5.
 //
-// Bound by instructions (75 % of the issue slots at tile height 16, where a group is 1.6 ids and 5 rows), 680 a task there, of
+// Bound by instructions (76 % of the issue slots at tile height 16, where a group is 1.6 ids and 5 rows), 680 a task there, of
 // which the decode step 300.
 #include <math.h>
 
