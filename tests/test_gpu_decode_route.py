@@ -37,3 +37,26 @@ def test_deep_tiles(th, exps, staged, N):
     assert torch.equal(out, W)
     launched = captured_kernels(call)
     assert staged == ("k_decode2" in launched or "k_decode4" in launched) and ("k_decode_tiled" in launched) == (not staged)
+
+
+@pytest.mark.parametrize("K,N,th,kernel", [
+    (4096, 4096, 128, "k_decode4"),
+    (4096, 22016, 128, "k_decode4"),
+    (2048, 2048, 128, "k_decode2"),     # one warp a scheduler: two streams a lane start sooner
+    (777, 1001, 128, "k_decode2"),
+    (4096, 11008, 1024, "k_decode2"),   # long streams, few tiles
+])
+def test_choice_of_decoder(K, N, th, kernel):
+    import comp_inference_b200 as ci
+    from comp_inference_b200 import _lib
+    W = (torch.randn(K, N, generator=torch.Generator("cuda").manual_seed(K), device="cuda") * 0.02).to(torch.bfloat16)
+    c = ci.compress_weight_cuda(W, th, 32)
+    w, keep = _lib.tiled_weight(c["rans_exp_stream"], c["rans_exp_states"], c["rans_exp_tables"], c["rans_exp_slot_map"],
+                                c["rans_exp_tile_offsets"], c["rans_exp_tile_max_lens"], c["rans_man_raw"], K, N, th, 32, want_max=True)
+    out = torch.empty_like(W)
+
+    def call():
+        _lib.check(_lib.load().ci_decode_bf16(w, out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    call()
+    assert torch.equal(out.view(torch.int16), W.view(torch.int16))
+    assert kernel in captured_kernels(call)
