@@ -36,8 +36,8 @@ constexpr uint32_t kT4ManBytes = 2 * 8 * kT4SegPitch;
 constexpr uint32_t kT4RegChunks = 4;         // chunks of a segment whose sums a lane holds in registers
 
 // The table's alignment leaves up to a table's size unused in front of the table, where the chunks of three warps have room; the
-// rest of it is left at the end of the window.  With this much in the two together, a chunk that does not fit in front, where the
-// window begins elsewhere, moves everything behind the table up by one and still fits.
+// rest of it is left at the end of the window.  With this much in the two together, chunks that do not fit in front, where the
+// window begins elsewhere, fit there.
 constexpr uint32_t kT4Front = 3, kT4SpareBytes = (kT4Front + 1) * kT4ManBytes;
 static_assert(kT4SpareBytes >= kLutBytes, "the table's alignment may cost a table's size");
 
@@ -91,9 +91,13 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     const uint32_t lut_bar = lut_s + kLutBytes + kT4BarBytes - 16;
     start_lut(lut_s, lut_bar, a.lut);
     const uint32_t behind_s = lut_s + kLutBytes + kT4BarBytes;
-    const uint32_t front = min(p.front, (lut_s - smem_s) / kT4ManBytes);
-    const uint32_t man_s = warp < front ? smem_s + warp * kT4ManBytes : behind_s + (warp - front) * kT4ManBytes;
-    const uint32_t acc0_s = behind_s + (W - front) * kT4ManBytes, set_bytes = W * p.acc_bytes;
+    uint32_t man_s = warp < p.front ? smem_s + warp * kT4ManBytes : behind_s + (warp - p.front) * kT4ManBytes;
+    const uint32_t acc0_s = behind_s + (W - p.front) * kT4ManBytes, set_bytes = W * p.acc_bytes;
+    if (lut_s - smem_s < p.front * kT4ManBytes && warp < p.front) {
+        const uint32_t front = (lut_s - smem_s) / kT4ManBytes;
+        if (warp >= front) man_s = acc0_s + p.sets * set_bytes + W * p.stages * p.stage_bytes + (warp - front) * kT4ManBytes;
+    }
+    asm volatile("" : "+r"(man_s));                             // not worked out again in the loops
     const uint32_t acc_s = acc0_s + warp * p.acc_bytes;         // of the first set; the others set_bytes further each
     const uint32_t wbase_s = acc0_s + p.sets * set_bytes + warp * p.stages * p.stage_bytes;
     const uint32_t st_off = p.cap_rows * 128;
