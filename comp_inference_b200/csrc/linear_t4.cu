@@ -21,8 +21,8 @@
 // of the decode step like that kernel: 21 per 32 symbols, 75 % of the issue slots in long runs (32000 x 4096, one row).
 //
 // Measured on a B200, us, before -> with sums in registers, two sets, states among the copies and the chunks of three warps
-// in front of the table: 32000 x 4096 at tile height 128, one row 139 -> 118, two 145 -> 131, eight 215 -> 196; at 64 155 -> 128; at
-// 1024 with entry points 273 -> 194; 16000 x 4096 at 1024, four rows 208 -> 187; 8000 x 1024 at 128 31.5 -> 21.5.  The shuffle kernel takes 1000 and 3590
+// in front of the table: 32000 x 4096 at tile height 128, one row 139 -> 118, two 145 -> 129, eight 215 -> 194; at 64 155 -> 129; at
+// 1024 with entry points 273 -> 194; 16000 x 4096 at 1024, four rows 208 -> 187; 8000 x 1024 at 128 31.5 -> 21.2.  The shuffle kernel takes 1000 and 3590
 // for the first and for eight rows at 1024.
 #include "linear.cuh"
 #include "ptx.cuh"
@@ -32,14 +32,20 @@ namespace ci {
 constexpr uint32_t kT4Warps = 16;
 constexpr uint32_t kT4BarBytes = 128;        // the table's barrier, the flag of the last arrival
 constexpr uint32_t kT4SegPitch = kChunkRows * 16 + 16;       // eight segments of a chunk, 4 banks apart
-constexpr uint32_t kT4ManBytes = 2 * 8 * kT4SegPitch;
+constexpr uint32_t kT4ManBuf = 8 * kT4SegPitch;              // one of the two chunk buffers of a warp
+constexpr uint32_t kT4ManBytes = 2 * kT4ManBuf;
 constexpr uint32_t kT4RegChunks = 4;         // chunks of a segment whose sums a lane holds in registers
 
 // The table's alignment leaves up to a table's size unused in front of the table, where the chunks of three warps have room; the
-// rest of it is left at the end of the window.  With this much in the two together, chunks that do not fit in front, where the
-// window begins elsewhere, fit there.
-constexpr uint32_t kT4Front = 3, kT4SpareBytes = (kT4Front + 1) * kT4ManBytes;
-static_assert(kT4SpareBytes >= kLutBytes, "the table's alignment may cost a table's size");
+// rest of it is left at the end of the window.  Wherever the window begins, their buffers have room in the two together, one by one.
+// (Whole chunks would need 1 KB more: 30000 x 3000 at tile height 1024, eight rows, then has room for a warp less, 237 us -> 255.)
+constexpr uint32_t kT4Front = 3;
+constexpr bool front_fits() {
+    for (uint32_t gap = 0; gap < kLutBytes; gap += 16)
+        if (gap / kT4ManBuf + (kLutBytes - gap) / kT4ManBuf < 2 * kT4Front) return false;
+    return true;
+}
+static_assert(front_fits(), "no room for the chunk buffers beside the table");
 
 struct T4Args {
     LinArgs a;
@@ -77,7 +83,7 @@ __device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const uint32_t (&w)
 // tile; without, a tall tile's sums and window leave room for three warps.
 // RAGGED: the matrix ends inside a column block.  Zero activations alone would not do for the columns that are missing: the
 // symbols they repeat may be those of an infinite weight, and zero times that is not a number.  Their exponents are masked to
-// zero.  An instantiation of its own (32000 x 4090, one row 121.7 us -> 125.7): in all of them the masks cost 32000 x 4096 2.6 %,
+// zero.  An instantiation of its own (32000 x 4090, one row 116.8 us -> 118.5): in all of them the masks cost 32000 x 4096 2.6 %,
 // a second loop for the last block 2.8 %.
 template <int MT, bool ENTRY, bool REG, bool RAGGED>
 __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_constant__ T4Args p) {
@@ -93,11 +99,13 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     const uint32_t behind_s = lut_s + kLutBytes + kT4BarBytes;
     uint32_t man_s = warp < p.front ? smem_s + warp * kT4ManBytes : behind_s + (warp - p.front) * kT4ManBytes;
     const uint32_t acc0_s = behind_s + (W - p.front) * kT4ManBytes, set_bytes = W * p.acc_bytes;
+    uint32_t man_step = kT4ManBuf;                              // from the warp's first chunk buffer to its second
     if (lut_s - smem_s < p.front * kT4ManBytes && warp < p.front) {
-        const uint32_t front = (lut_s - smem_s) / kT4ManBytes;
-        if (warp >= front) man_s = acc0_s + p.sets * set_bytes + W * p.stages * p.stage_bytes + (warp - front) * kT4ManBytes;
+        const uint32_t front = (lut_s - smem_s) / kT4ManBuf, end_s = acc0_s + p.sets * set_bytes + W * p.stages * p.stage_bytes;
+        auto buffer = [&](uint32_t i) { return i < front ? smem_s + i * kT4ManBuf : end_s + (i - front) * kT4ManBuf; };
+        man_s = buffer(2 * warp);
+        man_step = buffer(2 * warp + 1) - man_s;
     }
-    asm volatile("" : "+r"(man_s));                             // not worked out again in the loops
     const uint32_t acc_s = acc0_s + warp * p.acc_bytes;         // of the first set; the others set_bytes further each
     const uint32_t wbase_s = acc0_s + p.sets * set_bytes + warp * p.stages * p.stage_bytes;
     const uint32_t st_off = p.cap_rows * 128;
@@ -193,7 +201,7 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
     // Rows [row, + kChunkRows) into chunk buffer `buf`; src: this lane's piece of them, `tiles` of the group exist.
     auto issue_man = [&](const uint8_t *src, uint32_t tiles, uint32_t row, uint32_t buf) {
         if (row + man_row >= step) return;
-        const uint32_t dst = man_s + (buf * 8 + man_half) * kT4SegPitch + man_row * 16;
+        const uint32_t dst = man_s + buf * man_step + man_half * kT4SegPitch + man_row * 16;
 #pragma unroll
         for (uint32_t j = 0; j < 4; ++j)
             if (j < tiles) cp_async16(dst + 2 * j * kT4SegPitch, src + j * tile_step);
@@ -340,7 +348,7 @@ __global__ void __launch_bounds__(kT4Warps * 32, 1) k_linear_t4(const __grid_con
                 if (!last || nxt.u < hi) issue_man(man, man_tiles, last ? 0u : (c + 1) * kChunkRows, buf ^ 1);
                 if (c == 0 && p.stages == 2) next_unit();
                 z.clamp(win_s);
-                uint32_t ms = man_s + (buf * 8 + sg) * kT4SegPitch + q * 4;
+                uint32_t ms = man_s + buf * man_step + sg * kT4SegPitch + q * 4;
                 const uint32_t n = min(kChunkRows, step - c * kChunkRows);
 #pragma unroll 1
                 for (uint32_t r = 0; r < n; r += 4) {
@@ -507,7 +515,7 @@ int launch_linear_t4(const LinArgs &a, uint32_t max_tile_len, size_t partial_cap
     p.status = a.tickets + (kTicketBytes - 1);
     p.wide = ((entry ? reinterpret_cast<uintptr_t>(a.entry_states) | reinterpret_cast<uintptr_t>(a.entry_rows)
                      : reinterpret_cast<uintptr_t>(a.states)) & 15u) == 0;
-    const uint32_t P = (uint32_t)sm_count(), fixed = kLutBytes + kT4SpareBytes + kT4BarBytes, room = (uint32_t)max_smem - fixed;
+    const uint32_t P = (uint32_t)sm_count(), fixed = 2 * kLutBytes + kT4BarBytes, room = (uint32_t)max_smem - fixed;
     const uint32_t blocks = p.total < P ? p.total : P;
     // Passes over the weight x rounds of units: sums for eight activation rows take eight times the shared memory of one,
     // which a tall tile cannot afford at a useful number of warps.  Two sets of sums where there is room: a CTA with the units
